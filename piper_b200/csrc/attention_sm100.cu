@@ -29,10 +29,6 @@
 // recorded and the CTA unwinds and frees its TMEM.
 #include "attention_sm100.h"
 
-#include <cstdlib>
-#include <map>
-#include <mutex>
-
 #include "ptx.cuh"
 
 namespace piper {
@@ -59,7 +55,7 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
@@ -78,73 +74,86 @@ __device__ __forceinline__ void store_row_chunk_sw128(uint8_t* tile, int row, in
 }
 
 // ================================================================= forward
-// warps 0-3 and 6-9: two softmax groups of 128 threads (each takes half the key columns of every score
-// tile and half the head dimension of the output); warp 4: TMA; warp 5: MMA
+// Bound by the tensor cores and the exponential unit alike: a 128x128 score tile of head dimension 128 costs 1,024
+// cycles of MMA and 1,024 cycles of ex2 (16 per cycle and SM).  A CTA therefore works on two query tiles (A, B) that
+// share one K/V stream: while four softmax warps turn the scores of one tile into probabilities, the MMAs of the
+// other tile run.  The probabilities go back to the tensor memory columns of their scores and feed P V from there, so
+// no thread writes shared memory in the loop; the output accumulates in tensor memory and is rescaled only when a
+// row maximum has grown by more than 2^kRescaleLog2 (the row sums use the same, possibly stale, maximum).
+// Tiles of one kv head are numbered query block major, so a pair is two heads of the group on the same rows where
+// the group is even, and neighbouring query blocks otherwise.
+// One CTA per 128 query rows, probabilities through shared memory: 254 us at S = 4096, 32 q / 8 kv heads.
+//
+// Warps 0-3: softmax of tile A, 4-7: of tile B (one query row per thread, row == TMEM lane); 8: TMA; 9: MMA.
 constexpr int FWD_THREADS = 320;
+constexpr float kRescaleLog2 = 8.f;      // probabilities stay below 2^8 of the stale maximum: no range is lost
 
 template <int HD>
 struct FwdSmem {
   static constexpr int HALVES = HD / 64;
   static constexpr int TILE = 128 * HD * 2;     // Q, K or V tile
-  static constexpr int P_BYTES = 128 * 128 * 2;
-  static constexpr int Q_OFF = 0;
-  static constexpr int K_OFF = TILE;            // 2 stages
-  static constexpr int V_OFF = 3 * TILE;        // 2 stages
-  static constexpr int P_OFF = 5 * TILE;
-  static constexpr int X_OFF = P_OFF + P_BYTES;   // row-max exchange [2 tiles][2 groups][128] + row-sum [2][128]
-  static constexpr int BAR_OFF = X_OFF + 6 * 128 * 4;
+  static constexpr int STAGES = 5;              // K0, V0, K1, V1, ... through one ring
+  static constexpr int Q_OFF = 0;               // 2 tiles; each takes its output tile at the end
+  static constexpr int KV_OFF = 2 * TILE;
+  static constexpr int BAR_OFF = KV_OFF + STAGES * TILE;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
 struct FwdBars {
   uint64_t q_full;
-  uint64_t k_full[2], k_empty[2];     // K is free again once S = Q K^T of its block has been computed ...
-  uint64_t v_full[2], v_empty[2];     // ... V only after P V, so the two rings run at different distances
-  uint64_t s_full[2], s_empty[2];
-  uint64_t p_full, p_empty;
-  uint64_t o_full[2], o_empty[2];
-  uint64_t mx_full[2], l_full;        // the two softmax groups exchange row maxima / row sums
+  uint64_t kv_full[5], kv_empty[5];
+  uint64_t s_full[2];          // scores of tile t are in tensor memory
+  uint64_t p_full[2][2];       // first / second 64 key columns of its probabilities are
+  uint64_t o_done[2];          // P V of the tile's last block has been accumulated
   uint32_t tmem_base;
 };
 
 template <int HD>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, __nv_bfloat16* __restrict__ out,
-                float* __restrict__ lse, int S, int Hq, int Hkv, float scale_log2, int* status) {
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_out,
+                float* __restrict__ lse, int S, int Hq, int Hkv, int B, int tiles_per_cta, float scale_log2,
+                int* status) {
   using L = FwdSmem<HD>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   FwdBars* bars = reinterpret_cast<FwdBars*>(smem + L::BAR_OFF);
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
-  const int qblk = gridDim.x - 1 - blockIdx.x;   // longest rows first
-  const int head = blockIdx.y;
-  const int b = blockIdx.z;
-  const int g = head / (Hq / Hkv);
-  const int n_blocks = qblk + 1;
+  // longest rows first over all heads: the kv head and the sequence vary fastest, the query blocks fall
+  const int group = Hq / Hkv;
+  const int tiles = group * (S / 128);
+  const int pairs = (tiles + tiles_per_cta - 1) / tiles_per_cta;
+  const int gb = static_cast<int>(blockIdx.x) % (Hkv * B);
+  const int pair = pairs - 1 - static_cast<int>(blockIdx.x) / (Hkv * B);
+  const int g = gb % Hkv;
+  const int b = gb / Hkv;
+  const int t0 = pair * tiles_per_cta;
+  const bool two = tiles_per_cta == 2 && t0 + 1 < tiles;
+  const int qblk0 = t0 / group, head0 = g * group + t0 % group;
+  const int qblk1 = (t0 + 1) / group, head1 = g * group + (t0 + 1) % group;
+  const int n0 = qblk0 + 1;
+  const int n1 = two ? qblk1 + 1 : 0;           // n1 >= n0 where there are two tiles
+  const int n_blocks = two ? n1 : n0;
   const long long tok0 = static_cast<long long>(b) * S;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars->k_full[i], 1);
-      mbar_init(&bars->k_empty[i], 1);
-      mbar_init(&bars->v_full[i], 1);
-      mbar_init(&bars->v_empty[i], 1);
-      mbar_init(&bars->s_full[i], 1);
-      mbar_init(&bars->s_empty[i], 8);        // one arrival per softmax warp
-      mbar_init(&bars->o_full[i], 1);
-      mbar_init(&bars->o_empty[i], 8);
-      mbar_init(&bars->mx_full[i], 8);
+    for (int i = 0; i < L::STAGES; ++i) {
+      mbar_init(&bars->kv_full[i], 1);
+      mbar_init(&bars->kv_empty[i], 1);
     }
-    mbar_init(&bars->p_full, 8);
-    mbar_init(&bars->p_empty, 1);
-    mbar_init(&bars->l_full, 8);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->s_full[i], 1);
+      mbar_init(&bars->p_full[i][0], 4);        // one arrival per softmax warp
+      mbar_init(&bars->p_full[i][1], 4);
+      mbar_init(&bars->o_done[i], 1);
+    }
     fence_mbar_init();
     tma_prefetch_desc(&tmap);
+    tma_prefetch_desc(&tmap_out);
   }
-  if (warp == 5) {
+  if (warp == 9) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -152,258 +161,231 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, __nv_bfloat16* __restr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
-  const uint32_t tmem_s = tmem_base;          // 2 x 128 columns
-  const uint32_t tmem_o = tmem_base + 256;    // 2 x HD columns
+  // columns: [0,128) S/P of tile A  [128,256) of tile B  [256,256+HD) O of tile A  [384,384+HD) of tile B
 
-  if (warp == 4) {
+  if (warp == 8) {
     // ------------------------------------------------------------- TMA
     if (lane == 0) {
-      mbar_arrive_expect_tx(&bars->q_full, L::TILE);
-      for (int h = 0; h < L::HALVES; ++h)
-        tma_load_2d(smem + L::Q_OFF + h * 16384, &tmap, &bars->q_full, head * HD + 64 * h,
-                    static_cast<int>(tok0) + qblk * 128);
-      // K and V blocks are loaded as soon as their own stage is free, whichever comes first
-      int kj = 0, vj = 0;
-      uint32_t idle = 0;
-      bool ok = true;
-      while ((kj < n_blocks || vj < n_blocks) && ok) {
-        bool progressed = false;
-        if (kj < n_blocks && mbar_test_wait(&bars->k_empty[kj & 1], ((kj >> 1) & 1) ^ 1)) {
-          const int s = kj & 1;
-          mbar_arrive_expect_tx(&bars->k_full[s], L::TILE);
-          for (int h = 0; h < L::HALVES; ++h)
-            tma_load_2d(smem + L::K_OFF + s * L::TILE + h * 16384, &tmap, &bars->k_full[s],
-                        (Hq + g) * HD + 64 * h, static_cast<int>(tok0) + kj * 128);
-          ++kj;
-          progressed = true;
-        }
-        if (vj < n_blocks && mbar_test_wait(&bars->v_empty[vj & 1], ((vj >> 1) & 1) ^ 1)) {
-          const int s = vj & 1;
-          mbar_arrive_expect_tx(&bars->v_full[s], L::TILE);
-          for (int h = 0; h < L::HALVES; ++h)
-            tma_load_2d(smem + L::V_OFF + s * L::TILE + h * 16384, &tmap, &bars->v_full[s],
-                        (Hq + Hkv + g) * HD + 64 * h, static_cast<int>(tok0) + vj * 128);
-          ++vj;
-          progressed = true;
-        }
-        if (progressed) {
-          idle = 0;
-        } else if (++idle > kMaxMbarPolls) {
-          atomicCAS(status, 0, kStatusMbarTimeout);
-          ok = false;
-        } else if ((idle & 1023u) == 0 && *reinterpret_cast<volatile int*>(status) != 0) {
-          ok = false;
-        }
+      mbar_arrive_expect_tx(&bars->q_full, (two ? 2 : 1) * L::TILE);
+      for (int t = 0; t < (two ? 2 : 1); ++t)
+        for (int h = 0; h < L::HALVES; ++h)
+          tma_load_2d(smem + L::Q_OFF + t * L::TILE + h * 16384, &tmap, &bars->q_full,
+                      (t ? head1 : head0) * HD + 64 * h, static_cast<int>(tok0) + (t ? qblk1 : qblk0) * 128);
+      int it = 0, s = 0;
+      uint32_t ph = 1;
+      for (; it < 2 * n_blocks; ++it) {         // even: K of block it / 2, odd: V
+        if (!await(&bars->kv_empty[s], ph, status)) break;
+        mbar_arrive_expect_tx(&bars->kv_full[s], L::TILE);
+        const int col = (Hq + ((it & 1) ? Hkv : 0) + g) * HD;
+        for (int h = 0; h < L::HALVES; ++h)
+          tma_load_2d(smem + L::KV_OFF + s * L::TILE + h * 16384, &tmap, &bars->kv_full[s], col + 64 * h,
+                      static_cast<int>(tok0) + (it >> 1) * 128);
+        if (++s == L::STAGES) { s = 0; ph ^= 1; }
       }
-      if (!ok) {
+      if (it < 2 * n_blocks) {
         // Unwinding after a failed wait: let the copies already issued land
         // before the CTA and its shared memory go away.
         await(&bars->q_full, 0, nullptr);
-        for (int jj = kj - 1; jj >= 0 && jj >= kj - 2; --jj)
-          await(&bars->k_full[jj & 1], (jj >> 1) & 1, nullptr);
-        for (int jj = vj - 1; jj >= 0 && jj >= vj - 2; --jj)
-          await(&bars->v_full[jj & 1], (jj >> 1) & 1, nullptr);
+        for (int jj = it - 1; jj >= 0 && jj >= it - L::STAGES; --jj)
+          await(&bars->kv_full[jj % L::STAGES], (jj / L::STAGES) & 1, nullptr);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == 9) {
     // ------------------------------------------------------------- MMA
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, false, false);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, HD, false, true);
-      const uint32_t q_addr = smem_u32(smem + L::Q_OFF);
-      const uint32_t p_addr = smem_u32(smem + L::P_OFF);
-      // descriptors of the operands that never move (Q, the probability tile), one per k-step: the issuing
-      // thread's instruction count per MMA is what bounds the loops below
-      uint64_t dq[HD / 16], dp[8];
+    // The whole warp walks the loop with uniform values and one elected lane issues: in a divergent single-lane
+    // branch every descriptor has to be moved into uniform registers for each MMA.
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, false, false);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16(128, HD, false, true);
+    const uint64_t dq0 = umma_desc_sw128(smem_u32(smem + L::Q_OFF), 16, 1024);
+    const uint64_t dk_base = umma_desc_sw128(smem_u32(smem + L::KV_OFF), 16, 1024);
+    const uint64_t dv_base = umma_desc_sw128(smem_u32(smem + L::KV_OFF), 16384, 1024);
+
+    auto issue_s = [&](int t, int st) {
+      const uint64_t dq = dq0 + (t * L::TILE >> 4);
+      const uint64_t dk = dk_base + (st * L::TILE >> 4);
 #pragma unroll
-      for (int ks = 0; ks < HD / 16; ++ks)
-        dq[ks] = umma_desc_sw128(q_addr + (ks / 4) * 16384 + (ks % 4) * 32, 16, 1024);
+      for (int ks = 0; ks < HD / 16; ++ks) {
+        const uint32_t off = ((ks / 4) * 16384 + (ks % 4) * 32) >> 4;
+        umma_bf16_ss(tmem_base + t * 128, dq + off, dk + off, idesc_qk, ks > 0 ? 1u : 0u);
+      }
+      umma_commit(&bars->s_full[t]);
+    };
+    auto issue_pv = [&](int t, int st, int half, bool first) {
+      const uint64_t dv = dv_base + (st * L::TILE >> 4);
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        dp[ks] = umma_desc_sw128(p_addr + (ks / 4) * 16384 + (ks % 4) * 32, 16, 1024);
-      bool ok = await(&bars->q_full, 0, status);
-      // Two queues served in whatever order their inputs arrive: S of block s_next (needs K and a free TMEM
-      // stage) and P V of block p_next (needs the probabilities, V and a free output stage).
-      int s_next = 0, p_next = 0;
-      uint32_t idle = 0;
-      while (p_next < n_blocks && ok) {
-        bool progressed = false;
-        if (p_next < s_next) {
-          const int jj = p_next;
-          const int sb = jj & 1;
-          if (mbar_test_wait(&bars->p_full, jj & 1) && mbar_test_wait(&bars->v_full[sb], (jj >> 1) & 1) &&
-              mbar_test_wait(&bars->o_empty[sb], ((jj >> 1) & 1) ^ 1)) {
-            tc_fence_after();
-            const uint64_t dv0 = umma_desc_sw128(smem_u32(smem + L::V_OFF + sb * L::TILE), 16384, 1024);
+      for (int k = 0; k < 4; ++k) {
+        const int ks = half * 4 + k;
+        umma_bf16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + ks * 8, dv + (ks * 2048 >> 4), idesc_pv,
+                     (first && ks == 0) ? 0u : 1u);
+      }
+    };
+    bool ok = await_all(&bars->q_full, 0, status);
+    ok = ok && await_all(&bars->kv_full[0], 0, status);
+    if (ok) {
+      tc_fence_after();
+      if (elect_one()) {
+        issue_s(0, 0);
+        if (two) issue_s(1, 0);
+        umma_commit(&bars->kv_empty[0]);
+      }
+      __syncwarp();
+    }
+    int st = 1;                    // ring slot of V of block j; K of block j + 1 follows it
+    uint32_t ph = 0;
+    for (int j = 0; j < n_blocks && ok; ++j) {
+      const int v_st = st;
+      const uint32_t v_ph = ph;
+      if (++st == L::STAGES) { st = 0; ph ^= 1; }
+      const int k_st = st;
+      const uint32_t k_ph = ph;
+      if (++st == L::STAGES) { st = 0; ph ^= 1; }
+      const bool more = j + 1 < n_blocks;
+      ok = await_all(&bars->kv_full[v_st], v_ph, status);
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-              umma_bf16_ss(tmem_o + sb * HD, dp[ks], dv0 + (ks * 2048 >> 4), idesc_pv, ks > 0 ? 1u : 0u);
-            umma_commit(&bars->p_empty);
-            umma_commit(&bars->o_full[sb]);
-            umma_commit(&bars->v_empty[sb]);
-            ++p_next;
-            progressed = true;
-          }
+      for (int t = 0; t < 2; ++t) {
+        const int nt = t ? n1 : n0;
+        if (!ok || j >= nt) continue;
+        const bool last_user = t == 1 || !two;
+        ok = await_all(&bars->p_full[t][0], j & 1, status);
+        if (!ok) continue;
+        tc_fence_after();
+        if (elect_one()) issue_pv(t, v_st, 0, j == 0);
+        __syncwarp();
+        ok = await_all(&bars->p_full[t][1], j & 1, status);
+        if (!ok) continue;
+        tc_fence_after();
+        if (elect_one()) {
+          issue_pv(t, v_st, 1, false);
+          if (j == nt - 1) umma_commit(&bars->o_done[t]);
+          if (last_user) umma_commit(&bars->kv_empty[v_st]);
         }
-        if (s_next < n_blocks) {
-          const int j = s_next;
-          const int s = j & 1;
-          if (mbar_test_wait(&bars->k_full[s], (j >> 1) & 1) &&
-              mbar_test_wait(&bars->s_empty[s], ((j >> 1) & 1) ^ 1)) {
-            tc_fence_after();
-            const uint64_t dk0 = umma_desc_sw128(smem_u32(smem + L::K_OFF + s * L::TILE), 16, 1024);
-#pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks) {
-              const uint32_t off = (ks / 4) * 16384 + (ks % 4) * 32;
-              umma_bf16_ss(tmem_s + s * 128, dq[ks], dk0 + (off >> 4), idesc_qk, ks > 0 ? 1u : 0u);
-            }
-            umma_commit(&bars->s_full[s]);
-            umma_commit(&bars->k_empty[s]);
-            ++s_next;
-            progressed = true;
+        __syncwarp();
+        if (j + 1 < nt) {
+          // the scores of the next block replace the probabilities just consumed: MMAs execute in issue order
+          ok = await_all(&bars->kv_full[k_st], k_ph, status);
+          if (!ok) continue;
+          tc_fence_after();
+          if (elect_one()) {
+            issue_s(t, k_st);
+            if (last_user) umma_commit(&bars->kv_empty[k_st]);
           }
-        }
-        if (progressed) {
-          idle = 0;
-        } else if (++idle > kMaxMbarPolls) {
-          atomicCAS(status, 0, kStatusMbarTimeout);
-          ok = false;
-        } else if ((idle & 1023u) == 0 && *reinterpret_cast<volatile int*>(status) != 0) {
-          ok = false;
+          __syncwarp();
         }
       }
+      if (!more) break;
     }
-  } else {
+  } else if (warp < 4 || two) {
     // --------------------------------------------------- softmax + output
-    // A warp reaches the TMEM lanes 32*(warp % 4)..+31.  Group wg owns key columns [64*wg, 64*wg + 64) of every
-    // score tile and output columns [wg*HD/2, (wg+1)*HD/2); per tile the groups exchange their row maxima.
-    constexpr int HH = HD / 2;
-    const int wg = warp >= 6 ? 1 : 0;
+    const int t = warp >> 2;
+    const int n_t = t ? n1 : n0;
+    const int qblk = t ? qblk1 : qblk0;
+    const int head = t ? head1 : head0;
     const int row = (warp & 3) * 32 + lane;      // query row == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    float* xbuf = reinterpret_cast<float*>(smem + L::X_OFF);
-    float o_acc[HH];
-#pragma unroll
-    for (int i = 0; i < HH; ++i) o_acc[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f, alpha_prev = 0.f;
+    const uint32_t ts = tmem_base + lane_sel + t * 128;
+    const uint32_t to = tmem_base + lane_sel + 256 + t * 128;
+    float m_run = -INFINITY;
+    float l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_blocks && ok; ++j) {
-      const int s = j & 1;
-      const bool diag = (j == qblk);
-      if (!await_all(&bars->s_full[s], (j >> 1) & 1, status)) { ok = false; break; }
+    for (int j = 0; j < n_t; ++j) {
+      if (!await_all(&bars->s_full[t], j & 1, status)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t ts = tmem_s + lane_sel + s * 128 + wg * 64;
-      uint32_t sv[64];
-      {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(ts, r0);
-        tmem_ld_32x32(ts + 32, r1);
-        tmem_ld_wait();
+      uint32_t sv[4][32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) { sv[i] = r0[i]; sv[32 + i] = r1[i]; }
-      }
-      tc_fence_before();
-      warp_arrive(&bars->s_empty[s], lane);            // the scores live in registers from here on
-      if (diag) {
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, sv[c]);
+      tmem_ld_wait();
+      if (j == qblk) {
         // causal mask, applied once to the registers of the only tile that needs it: a score of -inf then
         // drops out of the maximum and turns into a probability of exactly zero below
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (wg * 64 + i > row) sv[i] = 0xff800000u;
+        for (int i = 0; i < 128; ++i)
+          if (i > row) sv[i / 32][i % 32] = 0xff800000u;
       }
-      float mx = -INFINITY;
+      float mx[4];
 #pragma unroll
-      for (int i = 0; i < 64; i += 2)
-        mx = fmaxf(mx, fmaxf(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])));
-      xbuf[(s * 2 + wg) * 128 + row] = mx;
-      warp_arrive(&bars->mx_full[s], lane);
-      if (!await_all(&bars->mx_full[s], (j >> 1) & 1, status)) { ok = false; break; }
-      mx = fmaxf(mx, xbuf[(s * 2 + (wg ^ 1)) * 128 + row]);
-      const float m_new = fmaxf(m_run, mx);
-      const float alpha = fast_exp2((m_run - m_new) * scale_log2);
-      const float msc = m_new * scale_log2;
-      if (j > 0 && !await_all(&bars->p_empty, (j - 1) & 1, status)) { ok = false; break; }
-      float rs = 0.f;
+      for (int c = 0; c < 4; ++c) {
+        mx[c] = __uint_as_float(sv[c][0]);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+        for (int i = 1; i < 31; i += 2)
+          mx[c] = fmaxf(mx[c], fmaxf(__uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1])));
+        mx[c] = fmaxf(mx[c], __uint_as_float(sv[c][31]));
+      }
+      const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      if (j == 0) {
+        m_run = m_blk;
+      } else if (__any_sync(0xffffffffu, (m_blk - m_run) * scale_log2 > kRescaleLog2)) {
+        const float m_new = fmaxf(m_run, m_blk);
+        const float alpha = fast_exp2((m_run - m_new) * scale_log2);
+        l_run *= alpha;
+        m_run = m_new;
+        // P V of block j - 1 is complete: the commit behind s_full of block j came after it
+#pragma unroll 1
+        for (int c = 0; c < HD / 16; ++c) {
+          uint32_t r[16];
+          tmem_ld_32x16(to + c * 16, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+          tmem_st_32x16(to + c * 16, r);
+        }
+        tmem_st_wait();
+      }
+      const float2 sl2 = make_float2(scale_log2, scale_log2);
+      const float msc = m_run * scale_log2;
+      const float2 nm2 = make_float2(-msc, -msc);
+      float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float p0 = fast_exp2(__uint_as_float(sv[c * 32 + 2 * i]) * scale_log2 - msc);
-          const float p1 = fast_exp2(__uint_as_float(sv[c * 32 + 2 * i + 1]) * scale_log2 - msc);
-          rs += p0 + p1;
-          w[i] = pack_bf16x2(p0, p1);
+          float2 p = fma2(make_float2(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])), sl2, nm2);
+          p.x = fast_exp2(p.x);
+          p.y = fast_exp2(p.y);
+          rs[i & 1] = add2(rs[i & 1], p);
+          w[i] = pack_bf16x2(p.x, p.y);
         }
-        store_row_chunk_sw128(smem + L::P_OFF + wg * 16384, row, c * 4, w);
+        tmem_st_32x16(ts + c * 16, w);
+        if (c & 1) {
+          tmem_st_wait();
+          tc_fence_before();
+          warp_arrive(&bars->p_full[t][c >> 1], lane);
+        }
       }
+      l_run += (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
+    }
+    if (ok && await_all(&bars->o_done[t], 0, status)) {
+      // the tile's Q operand has been read for the last time; its buffer takes the output, 32 rows per warp
+      tc_fence_after();
+      const float inv = 1.f / l_run;
+      uint8_t* obuf = smem + L::Q_OFF + t * L::TILE;
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t r[32], w[16];
+        tmem_ld_32x32(to + c * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+        store_row_chunk_sw128(obuf + (c >> 1) * 16384, row, (c & 1) * 4, w);
+      }
+      lse[(static_cast<long long>(b) * Hq + head) * S + qblk * 128 + row] =
+          m_run * (scale_log2 * 0.6931471805599453f) + logf(l_run);
       fence_proxy_async_smem();
-      warp_arrive(&bars->p_full, lane);
-      if (j > 0) {
-        const int sb = (j - 1) & 1;
-        if (!await_all(&bars->o_full[sb], ((j - 1) >> 1) & 1, status)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t to = tmem_o + lane_sel + sb * HD + wg * HH;
-#pragma unroll
-        for (int c = 0; c < HH / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(to + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            o_acc[c * 32 + i] = o_acc[c * 32 + i] * alpha_prev + __uint_as_float(r[i]);
-        }
-        tc_fence_before();
-        warp_arrive(&bars->o_empty[sb], lane);
-      }
-      l_run = l_run * alpha + rs;
-      m_run = m_new;
-      alpha_prev = alpha;
-    }
-    if (ok) {
-      // total row sum = this group's partial + the other group's
-      xbuf[(4 + wg) * 128 + row] = l_run;
-      warp_arrive(&bars->l_full, lane);
-      ok = await_all(&bars->l_full, 0, status);
-    }
-    if (ok) {
-      const float l_tot = l_run + xbuf[(4 + (wg ^ 1)) * 128 + row];
-      const int jj = n_blocks - 1;
-      const int sb = jj & 1;
-      if (await_all(&bars->o_full[sb], (jj >> 1) & 1, status)) {
-        tc_fence_after();
-        const uint32_t to = tmem_o + lane_sel + sb * HD + wg * HH;
-        const float inv = 1.f / l_tot;
-        const long long tok = tok0 + static_cast<long long>(qblk) * 128 + row;
-        __nv_bfloat16* orow = out + tok * (static_cast<long long>(Hq) * HD) + head * HD + wg * HH;
-#pragma unroll
-        for (int c = 0; c < HH / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(to + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint4 o;
-            uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int e = v * 8 + 2 * i;
-              const float a = (o_acc[c * 32 + e] * alpha_prev + __uint_as_float(r[e])) * inv;
-              const float bb = (o_acc[c * 32 + e + 1] * alpha_prev + __uint_as_float(r[e + 1])) * inv;
-              ow[i] = pack_bf16x2(a, bb);
-            }
-            reinterpret_cast<uint4*>(orow + c * 32)[v] = o;
-          }
-        }
-        if (wg == 0)
-          lse[(static_cast<long long>(b) * Hq + head) * S + qblk * 128 + row] =
-              m_run * (scale_log2 * 0.6931471805599453f) + logf(l_tot);
+      __syncwarp();
+      if (lane == 0) {
+        for (int h = 0; h < L::HALVES; ++h)
+          tma_store_2d_bulk(&tmap_out, obuf + h * 16384 + (warp & 3) * 32 * 128, head * HD + 64 * h,
+                            static_cast<int>(tok0) + qblk * 128 + (warp & 3) * 32);
+        bulk_commit_group();
+        bulk_wait_group<0>();
       }
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) {
+  if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -440,75 +422,59 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   }
 }
 
-// warps 0-3 and 6-9: two groups of 128 threads that split the columns of every S'/dP' tile; warp 4: TMA;
-// warp 5: MMA
+// Both passes stream 64-row tiles through two tensor memory stages.  Warps 0-3 turn the even tiles' scores into
+// probabilities and score gradients, warps 4-7 the odd tiles', so each group has the MMAs of two tiles' time for its
+// work; warp 8: TMA, warp 9: MMA.  P' and dS' (bf16) replace their own fp32 scores in tensor memory and are the A
+// operand of the accumulating MMAs from there: no thread writes shared memory in the loop.  Bound by the MMAs: a
+// 128x64x16 one with both operands in shared memory reads 6 KiB (48 cycles) for 32 cycles of arithmetic.
 constexpr int BWD_THREADS = 320;
 
 template <int HD>
 struct BwdSmem {
   static constexpr int HALVES = HD / 64;
-  static constexpr int X_TILE = 128 * HD * 2;      // stationary tile
+  static constexpr int X_TILE = 128 * HD * 2;      // stationary tile; takes a gradient tile at the end
   static constexpr int Y_TILE = 64 * HD * 2;       // streamed tile
   static constexpr int Y_HALF = 64 * 128;          // one 64x64 box
-  static constexpr int PT_BYTES = 128 * 64 * 2;    // P' or dS' tile (one swizzle row per row)
   static constexpr int X1_OFF = 0;
   static constexpr int X2_OFF = X_TILE;
   static constexpr int Y_STAGES = 4;
-  static constexpr int Y_OFF = 2 * X_TILE;         // Y_STAGES x (Y1, Y2), see y_off
-  // Streamed stages are laid out in pairs: the same 64-column half of the same operand of stages 2p and 2p+1
-  // is one contiguous 128-row tile.  (Issuing S' and dP' of two consecutive tiles as one N = 128 MMA each was
-  // tried on this layout: every MMA costs the issuing thread about 110 cycles whatever its width, but the two
-  // TMEM stages are never free at the same moment in steady state, so the pairs did not form.)
-  static constexpr int HALF_STRIDE = 2 * Y_HALF;   // between the 64-column halves of one stage's operand
-  __host__ __device__ static constexpr int y_off(int st, int operand, int half) {
-    return (st >> 1) * (4 * Y_TILE) + operand * (2 * Y_TILE) + half * HALF_STRIDE + (st & 1) * Y_HALF;
-  }
-  static constexpr int P_OFF = Y_OFF + Y_STAGES * 2 * Y_TILE;
-  static constexpr int DS_OFF = P_OFF + PT_BYTES;
-  static constexpr int VEC_OFF = DS_OFF + PT_BYTES;              // 3 stages x (lse[64], delta[64]) floats
-  static constexpr int BAR_OFF = VEC_OFF + 3 * 2 * 64 * 4;
+  static constexpr int Y_OFF = 2 * X_TILE;         // Y_STAGES x (Y1, Y2)
+  static constexpr int VEC_OFF = Y_OFF + Y_STAGES * 2 * Y_TILE;   // Y_STAGES x (lse[64], delta[64]) floats
+  static constexpr int VEC_BYTES = 64 * 4;
+  static constexpr int BAR_OFF = VEC_OFF + Y_STAGES * 2 * VEC_BYTES;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
 struct BwdBars {
   uint64_t x_full;
   uint64_t y_full[4], y_empty[4];     // streamed tiles (BwdSmem::Y_STAGES)
-  uint64_t s_full[2], s_empty[2];     // S' and dP' pair
-  uint64_t t_full, t_empty;           // P'/dS' shared-memory tiles
-  uint64_t v_full[2];                 // per-column lse/delta vectors (MODE 1)
+  uint64_t s_full[2], dp_full[2];     // S' and dP' of a stage are in tensor memory
+  uint64_t p_full[2];                 // S' has been read; with MODE 1 P' stands in its place
+  uint64_t ds_full[2];                // dS' stands in the place of dP'
   uint64_t acc_full;
   uint32_t tmem_base;
 };
 
-// MODE 0: dQ.  MODE 1: dK, dV.
+// MODE 0: dQ of query head hy, rows of block xb.  MODE 1: dK, dV of kv head hy, rows of block xb.
 template <int HD, int MODE>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 128} over packed qkv
-                const __grid_constant__ CUtensorMap tmap_qkv_y,   // box {64, 64}  over packed qkv
-                const __grid_constant__ CUtensorMap tmap_do_x,    // box {64, 128} over dO [T, Hq*hd]
-                const __grid_constant__ CUtensorMap tmap_do_y,    // box {64, 64}  over dO
-                const float* __restrict__ lse, const float* __restrict__ delta,
-                __nv_bfloat16* __restrict__ d_qkv, int S, int Hq, int Hkv, float scale,
-                float scale_log2, int* status) {
+__device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, const CUtensorMap* tmap_qkv_y,
+                                             const CUtensorMap* tmap_do_x, const CUtensorMap* tmap_do_y,
+                                             const CUtensorMap* tmap_dqkv, const float* __restrict__ lse,
+                                             const float* __restrict__ delta, int xb, int hy, int b, int S, int Hq,
+                                             int Hkv, float scale, float scale_log2, int* status) {
   using L = BwdSmem<HD>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   BwdBars* bars = reinterpret_cast<BwdBars*>(smem + L::BAR_OFF);
-  float* vec = reinterpret_cast<float*>(smem + L::VEC_OFF);
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int group = Hq / Hkv;
-  const int b = blockIdx.z;
-  const long long tok0 = static_cast<long long>(b) * S;
-  const int W = (Hq + 2 * Hkv) * HD;   // packed row width
+  const int tok0 = b * S;
 
-  // Stationary block index and iteration space.
-  //   MODE 0: blockIdx.y = query head; streams kv tiles i in [0, 2*xb + 1].
-  //   MODE 1: blockIdx.y = kv head; for each query head of the group streams
-  //           q tiles i in [2*xb, S/64 - 1].
-  const int xb = (MODE == 0) ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;
-  const int hy = blockIdx.y;
+  // Iteration space.
+  //   MODE 0: streams kv tiles i in [0, 2*xb + 1].
+  //   MODE 1: for each query head of the group streams q tiles i in [2*xb, S/64 - 1].
   const int g = (MODE == 0) ? hy / group : hy;
   const int tiles_per_head = (MODE == 0) ? (2 * xb + 2) : (S / 64 - 2 * xb);
   const int n_iter = (MODE == 0) ? tiles_per_head : tiles_per_head * group;
@@ -521,19 +487,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 12
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->s_full[i], 1);
-      mbar_init(&bars->s_empty[i], 8);        // one arrival per softmax warp
-      mbar_init(&bars->v_full[i], 2);        // warps 0 and 1 write the vectors
+      mbar_init(&bars->dp_full[i], 1);
+      mbar_init(&bars->p_full[i], 4);         // one arrival per softmax warp of the stage
+      mbar_init(&bars->ds_full[i], 4);
     }
-    mbar_init(&bars->t_full, 8);
-    mbar_init(&bars->t_empty, 1);
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
-    tma_prefetch_desc(&tmap_qkv_x);
-    tma_prefetch_desc(&tmap_qkv_y);
-    tma_prefetch_desc(&tmap_do_x);
-    tma_prefetch_desc(&tmap_do_y);
+    tma_prefetch_desc(tmap_qkv_x);
+    tma_prefetch_desc(tmap_qkv_y);
+    tma_prefetch_desc(tmap_do_x);
+    tma_prefetch_desc(tmap_do_y);
+    tma_prefetch_desc(tmap_dqkv);
   }
-  if (warp == 5) {
+  if (warp == 9) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -546,42 +512,47 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 12
   const uint32_t tmem_acc1 = tmem_base + 256;
   const uint32_t tmem_acc2 = tmem_base + 384;
 
-  if (warp == 4) {
+  if (warp == 8) {
     // ------------------------------------------------------------- TMA
     if (lane == 0) {
-      const int xrow = static_cast<int>(tok0) + xb * 128;
+      const int xrow = tok0 + xb * 128;
       mbar_arrive_expect_tx(&bars->x_full, 2 * L::X_TILE);
       for (int h = 0; h < L::HALVES; ++h) {
         if (MODE == 0) {
-          tma_load_2d(smem + L::X1_OFF + h * 16384, &tmap_qkv_x, &bars->x_full, hy * HD + 64 * h, xrow);
-          tma_load_2d(smem + L::X2_OFF + h * 16384, &tmap_do_x, &bars->x_full, hy * HD + 64 * h, xrow);
+          tma_load_2d(smem + L::X1_OFF + h * 16384, tmap_qkv_x, &bars->x_full, hy * HD + 64 * h, xrow);
+          tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_do_x, &bars->x_full, hy * HD + 64 * h, xrow);
         } else {
-          tma_load_2d(smem + L::X1_OFF + h * 16384, &tmap_qkv_x, &bars->x_full,
-                      (Hq + g) * HD + 64 * h, xrow);
-          tma_load_2d(smem + L::X2_OFF + h * 16384, &tmap_qkv_x, &bars->x_full,
-                      (Hq + Hkv + g) * HD + 64 * h, xrow);
+          tma_load_2d(smem + L::X1_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + g) * HD + 64 * h, xrow);
+          tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + Hkv + g) * HD + 64 * h, xrow);
         }
       }
       int it = 0;
+      int hh = (MODE == 0) ? hy : g * group;     // query head and tile of iteration it
+      int ti = (MODE == 0) ? 0 : 2 * xb;
       for (; it < n_iter; ++it) {
         const int st = it % L::Y_STAGES;
         if (!await(&bars->y_empty[st], ((it / L::Y_STAGES) & 1) ^ 1, status)) break;
-        const int hh = (MODE == 0) ? hy : g * group + it / tiles_per_head;   // query head
-        const int ti = (MODE == 0) ? it : 2 * xb + it % tiles_per_head;      // streamed tile index
-        const int yrow = static_cast<int>(tok0) + ti * 64;
-        uint8_t* yb = smem + L::Y_OFF;
-        mbar_arrive_expect_tx(&bars->y_full[st], 2 * L::Y_TILE);
+        const int yrow = tok0 + ti * 64;
+        uint8_t* yb = smem + L::Y_OFF + st * 2 * L::Y_TILE;
+        mbar_arrive_expect_tx(&bars->y_full[st], 2 * L::Y_TILE + (MODE == 1 ? 2 * L::VEC_BYTES : 0));
         for (int h = 0; h < L::HALVES; ++h) {
-          uint8_t* y1 = yb + L::y_off(st, 0, h);
-          uint8_t* y2 = yb + L::y_off(st, 1, h);
+          uint8_t* y1 = yb + h * L::Y_HALF;
+          uint8_t* y2 = y1 + L::Y_TILE;
           if (MODE == 0) {
-            tma_load_2d(y1, &tmap_qkv_y, &bars->y_full[st], (Hq + g) * HD + 64 * h, yrow);
-            tma_load_2d(y2, &tmap_qkv_y, &bars->y_full[st], (Hq + Hkv + g) * HD + 64 * h, yrow);
+            tma_load_2d(y1, tmap_qkv_y, &bars->y_full[st], (Hq + g) * HD + 64 * h, yrow);
+            tma_load_2d(y2, tmap_qkv_y, &bars->y_full[st], (Hq + Hkv + g) * HD + 64 * h, yrow);
           } else {
-            tma_load_2d(y1, &tmap_qkv_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
-            tma_load_2d(y2, &tmap_do_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
+            tma_load_2d(y1, tmap_qkv_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
+            tma_load_2d(y2, tmap_do_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
           }
         }
+        if (MODE == 1) {
+          const long long idx = (static_cast<long long>(b) * Hq + hh) * S + ti * 64;
+          uint8_t* v = smem + L::VEC_OFF + st * 2 * L::VEC_BYTES;
+          bulk_load(v, lse + idx, L::VEC_BYTES, &bars->y_full[st]);
+          bulk_load(v + L::VEC_BYTES, delta + idx, L::VEC_BYTES, &bars->y_full[st]);
+        }
+        if (++ti == S / 64 && MODE == 1) { ti = 2 * xb; ++hh; }
       }
       if (it < n_iter) {
         // Unwinding: wait (bounded) for the copies in flight.
@@ -590,227 +561,250 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 12
           await(&bars->y_full[jj % L::Y_STAGES], (jj / L::Y_STAGES) & 1, nullptr);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == 9) {
     // ------------------------------------------------------------- MMA
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, false, false);
-      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, false, true);
-      const uint32_t x1 = smem_u32(smem + L::X1_OFF);
-      const uint32_t x2 = smem_u32(smem + L::X2_OFF);
-      const uint32_t p_addr = smem_u32(smem + L::P_OFF);
-      const uint32_t ds_addr = smem_u32(smem + L::DS_OFF);
-      uint64_t dx1[HD / 16], dx2[HD / 16];       // descriptors of the stationary operands, fixed for the kernel
+    // Uniform control flow with one elected issuing lane (see the forward kernel).  Order per tile i: P' Y2 of i,
+    // S' of i + 2 into the columns just consumed, dS' Y1 of i, dP' of i + 2.  MMAs execute in issue order.
+    constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, false, false);
+    constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, false, true);
+    const uint64_t dx1 = umma_desc_sw128(smem_u32(smem + L::X1_OFF), 16, 1024);
+    const uint64_t dx2 = umma_desc_sw128(smem_u32(smem + L::X2_OFF), 16, 1024);
+    const uint64_t dyk = umma_desc_sw128(smem_u32(smem + L::Y_OFF), 16, 1024);            // K-major view of a stage
+    const uint64_t dyn = umma_desc_sw128(smem_u32(smem + L::Y_OFF), L::Y_HALF, 1024);     // MN-major view
+    auto issue_scores = [&](uint32_t tmem_d, uint64_t dx, uint64_t dy) {
 #pragma unroll
-      for (int ks = 0; ks < HD / 16; ++ks) {
-        const uint32_t xo = (ks / 4) * 16384 + (ks % 4) * 32;
-        dx1[ks] = umma_desc_sw128(x1 + xo, 16, 1024);
-        dx2[ks] = umma_desc_sw128(x2 + xo, 16, 1024);
+      for (int ks = 0; ks < HD / 16; ++ks)
+        umma_bf16_ss(tmem_d, dx + (((ks / 4) * 16384 + (ks % 4) * 32) >> 4),
+                     dy + (((ks / 4) * L::Y_HALF + (ks % 4) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
+    };
+    auto issue_acc = [&](uint32_t tmem_d, uint32_t tmem_a, uint64_t dy, bool first) {
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)       // contraction over the 64 streamed rows
+        umma_bf16_ts(tmem_d, tmem_a + ks * 8, dy + (ks * 2048 >> 4), idesc_acc, (first && ks == 0) ? 0u : 1u);
+    };
+    bool ok = await_all(&bars->x_full, 0, status);
+    for (int i = 0; i < 2 && i < n_iter && ok; ++i) {
+      ok = await_all(&bars->y_full[i], 0, status);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t y = dyk + (i * 2 * L::Y_TILE >> 4);
+        issue_scores(tmem_base + i * 64, dx1, y);
+        umma_commit(&bars->s_full[i]);
+        issue_scores(tmem_base + 128 + i * 64, dx2, y + (L::Y_TILE >> 4));
+        umma_commit(&bars->dp_full[i]);
       }
-      const uint64_t d_ds = umma_desc_sw128(ds_addr, 16, 1024);
-      const uint64_t d_p = umma_desc_sw128(p_addr, 16, 1024);
-      bool ok = await(&bars->x_full, 0, status);
-      // Two queues served in whatever order their inputs arrive: S'/dP' of tile s_next needs its streamed tile
-      // and a free TMEM stage; the accumulation of tile a_next needs the P'/dS' tiles the threads wrote.  A fixed
-      // order would let a streamed tile that is still in flight hold back the accumulation that frees the
-      // shared-memory stage the next load is waiting for.
-      int s_next = 0, a_next = 0;
-      uint32_t idle = 0;
-      while (a_next < n_iter && ok) {
-        bool progressed = false;
-        if (a_next < s_next && mbar_test_wait(&bars->t_full, a_next & 1)) {
-          const int jt = a_next;
-          const int st = jt % L::Y_STAGES;
-          tc_fence_after();
-          const uint64_t dy1 = umma_desc_sw128(smem_u32(smem + L::Y_OFF + L::y_off(st, 0, 0)), L::HALF_STRIDE, 1024);
-          const uint64_t dy2 = umma_desc_sw128(smem_u32(smem + L::Y_OFF + L::y_off(st, 1, 0)), L::HALF_STRIDE, 1024);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {   // contraction over the 64 streamed rows
-            umma_bf16_ss(tmem_acc1, d_ds + (ks * 32 >> 4), dy1 + (ks * 2048 >> 4), idesc_acc,
-                         (jt > 0 || ks > 0) ? 1u : 0u);
-          }
-          if (MODE == 1) {
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              umma_bf16_ss(tmem_acc2, d_p + (ks * 32 >> 4), dy2 + (ks * 2048 >> 4), idesc_acc,
-                           (jt > 0 || ks > 0) ? 1u : 0u);
-            }
-          }
-          umma_commit(&bars->t_empty);
-          umma_commit(&bars->y_empty[st]);
-          if (jt == n_iter - 1) umma_commit(&bars->acc_full);
-          ++a_next;
-          progressed = true;
-        }
-        if (s_next < n_iter) {
-          const int it = s_next;
-          const int st = it % L::Y_STAGES;
-          const int ss = it & 1;
-          if (mbar_test_wait(&bars->y_full[st], (it / L::Y_STAGES) & 1) &&
-              mbar_test_wait(&bars->s_empty[ss], ((it >> 1) & 1) ^ 1)) {
-            tc_fence_after();
-            const uint32_t y1 = smem_u32(smem + L::Y_OFF + L::y_off(st, 0, 0));
-            const uint32_t y2 = smem_u32(smem + L::Y_OFF + L::y_off(st, 1, 0));
-            constexpr uint32_t idesc = idesc_s;
-            // one descriptor per operand and tile; the k-steps only add a constant to its address field (the
-            // issuing thread's instruction count per MMA is what bounds this loop)
-            const uint64_t dy1 = umma_desc_sw128(y1, 16, 1024);
-            const uint64_t dy2 = umma_desc_sw128(y2, 16, 1024);
-#pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks) {
-              const uint32_t yo = (ks / 4) * L::HALF_STRIDE + (ks % 4) * 32;
-              umma_bf16_ss(tmem_base + ss * 64, dx1[ks], dy1 + (yo >> 4), idesc, ks > 0 ? 1u : 0u);
-            }
-#pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks) {
-              const uint32_t yo = (ks / 4) * L::HALF_STRIDE + (ks % 4) * 32;
-              umma_bf16_ss(tmem_base + 128 + ss * 64, dx2[ks], dy2 + (yo >> 4), idesc, ks > 0 ? 1u : 0u);
-            }
-            umma_commit(&bars->s_full[ss]);
-            ++s_next;
-            progressed = true;
-          }
-        }
-        if (progressed) {
-          idle = 0;
-        } else if (++idle > kMaxMbarPolls) {
-          atomicCAS(status, 0, kStatusMbarTimeout);
-          ok = false;
-        } else if ((idle & 1023u) == 0 && *reinterpret_cast<volatile int*>(status) != 0) {
-          ok = false;
-        }
+      __syncwarp();
+    }
+    for (int i = 0; i < n_iter && ok; ++i) {
+      const int ss = i & 1;
+      const uint32_t ph = (i >> 1) & 1;
+      const int st = i % L::Y_STAGES;
+      const int st2 = (i + 2) % L::Y_STAGES;
+      const bool more = i + 2 < n_iter;
+      const uint64_t yn = dyn + (st * 2 * L::Y_TILE >> 4);
+      const uint64_t yk2 = dyk + (st2 * 2 * L::Y_TILE >> 4);
+      if (!(ok = await_all(&bars->p_full[ss], ph, status))) break;
+      tc_fence_after();
+      if (MODE == 1) {
+        if (elect_one()) issue_acc(tmem_acc2, tmem_base + ss * 64, yn + (L::Y_TILE >> 4), i == 0);
+        __syncwarp();
       }
+      if (more) {
+        if (!(ok = await_all(&bars->y_full[st2], ((i + 2) / L::Y_STAGES) & 1, status))) break;
+        tc_fence_after();
+        if (elect_one()) {
+          issue_scores(tmem_base + ss * 64, dx1, yk2);
+          umma_commit(&bars->s_full[ss]);
+        }
+        __syncwarp();
+      }
+      if (!(ok = await_all(&bars->ds_full[ss], ph, status))) break;
+      tc_fence_after();
+      if (elect_one()) {
+        issue_acc(tmem_acc1, tmem_base + 128 + ss * 64, yn, i == 0);
+        umma_commit(&bars->y_empty[st]);
+        if (more) {
+          issue_scores(tmem_base + 128 + ss * 64, dx2, yk2 + (L::Y_TILE >> 4));
+          umma_commit(&bars->dp_full[ss]);
+        }
+        if (i == n_iter - 1) umma_commit(&bars->acc_full);
+      }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------- P' / dS' tiles + epilogue
-    // A warp reaches the TMEM lanes 32*(warp % 4)..+31; the two groups take columns [0,32) and [32,64).
-    const int wg = warp >= 6 ? 1 : 0;
-    const int row = (warp & 3) * 32 + lane;   // stationary row == TMEM lane
+    const int wg = warp >> 2;                  // tiles wg, wg + 2, ...; tensor memory stage wg
+    const int row = (warp & 3) * 32 + lane;    // stationary row == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t ts = tmem_base + lane_sel + wg * 64;
+    const uint32_t td = ts + 128;
     const int xpos = xb * 128 + row;   // position of this row inside the sequence
-    float row_lse = 0.f, row_delta = 0.f;
+    const float2 sl2 = make_float2(scale_log2, scale_log2);
+    constexpr float kNegLog2e = -1.4426950408889634f;
+    const float2 neg_one = make_float2(-1.f, -1.f);
+    float2 row_nl = make_float2(0.f, 0.f), row_dl = make_float2(0.f, 0.f);
     if (MODE == 0) {
       const long long idx = (static_cast<long long>(b) * Hq + hy) * S + xpos;
-      row_lse = lse[idx] * 1.4426950408889634f;
-      row_delta = delta[idx];
+      row_nl.x = row_nl.y = lse[idx] * kNegLog2e;
+      row_dl.x = row_dl.y = delta[idx];
     }
-    float pre_lse = 0.f, pre_delta = 0.f;      // MODE 1: this thread's lse/delta entries of the next streamed tile
-    if (MODE == 1 && wg == 0 && row < 64 && n_iter > 0) {
-      const long long idx = (static_cast<long long>(b) * Hq + g * group) * S + 2 * xb * 64 + row;
-      pre_lse = lse[idx];
-      pre_delta = delta[idx];
-    }
+    int ti = (MODE == 0) ? wg : 2 * xb + wg;   // tiles_per_head is even: the parity of ti is wg throughout
     bool ok = true;
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int st = it & 1;
-      // lse/delta vectors: three stages, so a stage is rewritten only after every thread has left the
-      // iteration that read it (a thread enters iteration it only after the MMAs of it - 2 have retired)
-      const int vs = it % 3;
-      const int ti = (MODE == 0) ? it : 2 * xb + it % tiles_per_head;
-      if (MODE == 1) {
-        // Per-column lse/delta of the streamed query tile -> shared memory.  The values of the next tile are
-        // requested right away and stay in flight while this tile is processed.
-        if (wg == 0 && row < 64) {
-          vec[vs * 128 + row] = pre_lse * 1.4426950408889634f;
-          vec[vs * 128 + 64 + row] = pre_delta;
-          warp_arrive(&bars->v_full[st], lane);
-          if (it + 1 < n_iter) {
-            const int hn = g * group + (it + 1) / tiles_per_head;
-            const int tn = 2 * xb + (it + 1) % tiles_per_head;
-            const long long idx = (static_cast<long long>(b) * Hq + hn) * S + tn * 64 + row;
-            pre_lse = lse[idx];            // no arithmetic on these until the next iteration: a dependent
-            pre_delta = delta[idx];        // instruction here would stall this warp on the loads right away
-          }
-        }
-        // Bounded wait instead of a named barrier: a thread that gave up on
-        // an earlier wait must not strand the others here.
-        if (!await_all(&bars->v_full[st], (it >> 1) & 1, status)) { ok = false; break; }
-      }
-      if (!await_all(&bars->s_full[st], (it >> 1) & 1, status)) { ok = false; break; }
+    for (int it = wg; it < n_iter; it += 2) {
+      const uint32_t ph = (it >> 1) & 1;
+      const int st = it % L::Y_STAGES;
+      const float4* vl = reinterpret_cast<const float4*>(smem + L::VEC_OFF + st * 2 * L::VEC_BYTES);
+      const float4* vd = vl + L::VEC_BYTES / 16;
+      if (MODE == 1 && !await_all(&bars->y_full[st], (it / L::Y_STAGES) & 1, status)) { ok = false; break; }
+      if (!await_all(&bars->s_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
-      // Causal mask is needed only where the streamed tile overlaps the
-      // stationary rows: element (x row, y col) is kept iff key <= query.
-      const int ypos0 = ti * 64;
-      const bool need_mask = (MODE == 0) ? (ypos0 + 63 > xb * 128) : (ypos0 < xb * 128 + 127);
-      const uint32_t ts = tmem_base + lane_sel + st * 64;
-      {
-        const int c = wg;
-        uint32_t sv[32], dv[32];
-        tmem_ld_32x32(ts + c * 32, sv);
-        tmem_ld_32x32(ts + 128 + c * 32, dv);
-        tmem_ld_wait();
+      uint32_t sv[2][32];
+      tmem_ld_32x32(ts, sv[0]);
+      tmem_ld_32x32(ts + 32, sv[1]);
+      tmem_ld_wait();
+      if (MODE == 0) {
         tc_fence_before();
-        warp_arrive(&bars->s_empty[st], lane);   // S'/dP' of this stage now live in registers
-        if (need_mask) {
-          // causal mask, applied once to the registers of the tiles that cross the diagonal: a score of -inf
-          // turns into a probability (and a score gradient) of exactly zero below
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int col = c * 32 + i;
-            const int qpos = (MODE == 0) ? xpos : ypos0 + col;
-            const int kpos = (MODE == 0) ? ypos0 + col : xpos;
-            if (kpos > qpos) sv[i] = 0xff800000u;
-          }
-        }
-        uint32_t pw[16], dw[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float p[2], d[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int col = c * 32 + 2 * i + e;
-            const float l2 = (MODE == 0) ? row_lse : vec[vs * 128 + col];
-            const float dl = (MODE == 0) ? row_delta : vec[vs * 128 + 64 + col];
-            const float pv = fast_exp2(__uint_as_float(sv[2 * i + e]) * scale_log2 - l2);
-            p[e] = pv;
-            d[e] = pv * (__uint_as_float(dv[2 * i + e]) - dl);
-          }
-          pw[i] = pack_bf16x2(p[0], p[1]);
-          dw[i] = pack_bf16x2(d[0], d[1]);
-        }
-        // the tiles were last read by the MMAs of the previous iteration
-        if (it >= 1 && !await_all(&bars->t_empty, (it - 1) & 1, status)) { ok = false; break; }
-        if (MODE == 1) store_row_chunk_sw128(smem + L::P_OFF, row, c * 4, pw);
-        store_row_chunk_sw128(smem + L::DS_OFF, row, c * 4, dw);
+        warp_arrive(&bars->p_full[wg], lane);   // the scores live in registers from here on
       }
-      fence_proxy_async_smem();
-      warp_arrive(&bars->t_full, lane);
+      // Causal mask, applied once to the registers of the tiles that cross the diagonal (element (x row, y col) is
+      // kept iff key <= query): a score of -inf turns into a probability and a score gradient of exactly zero.
+      const int ypos0 = ti * 64;
+      if ((MODE == 0) ? (ypos0 + 63 > xb * 128) : (ypos0 < xb * 128 + 127)) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          const bool drop = (MODE == 0) ? (ypos0 + i > xpos) : (xpos > ypos0 + i);
+          if (drop) sv[i / 32][i % 32] = 0xff800000u;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t pw[16];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          float2 n0 = row_nl, n1 = row_nl;
+          if (MODE == 1) {
+            const float4 l4 = vl[c * 8 + q];
+            n0 = make_float2(l4.x * kNegLog2e, l4.y * kNegLog2e);
+            n1 = make_float2(l4.z * kNegLog2e, l4.w * kNegLog2e);
+          }
+          uint32_t* v = &sv[c][4 * q];
+          float2 p0 = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, n0);
+          float2 p1 = fma2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl2, n1);
+          p0.x = fast_exp2(p0.x); p0.y = fast_exp2(p0.y);
+          p1.x = fast_exp2(p1.x); p1.y = fast_exp2(p1.y);
+          v[0] = __float_as_uint(p0.x); v[1] = __float_as_uint(p0.y);
+          v[2] = __float_as_uint(p1.x); v[3] = __float_as_uint(p1.y);
+          pw[2 * q] = pack_bf16x2(p0.x, p0.y);
+          pw[2 * q + 1] = pack_bf16x2(p1.x, p1.y);
+        }
+        if (MODE == 1) tmem_st_32x16(ts + c * 16, pw);
+      }
+      if (MODE == 1) {
+        tmem_st_wait();
+        tc_fence_before();
+        warp_arrive(&bars->p_full[wg], lane);
+      }
+      if (!await_all(&bars->dp_full[wg], ph, status)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t dv[2][32];
+      tmem_ld_32x32(td, dv[0]);
+      tmem_ld_32x32(td + 32, dv[1]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t dw[16];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          float2 d0 = row_dl, d1 = row_dl;
+          if (MODE == 1) {
+            const float4 d4 = vd[c * 8 + q];
+            d0 = make_float2(d4.x, d4.y);
+            d1 = make_float2(d4.z, d4.w);
+          }
+          const uint32_t* v = &dv[c][4 * q];
+          const uint32_t* p = &sv[c][4 * q];
+          d0 = fma2(d0, neg_one, make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])));
+          d1 = fma2(d1, neg_one, make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])));
+          d0 = mul2(d0, make_float2(__uint_as_float(p[0]), __uint_as_float(p[1])));
+          d1 = mul2(d1, make_float2(__uint_as_float(p[2]), __uint_as_float(p[3])));
+          dw[2 * q] = pack_bf16x2(d0.x, d0.y);
+          dw[2 * q + 1] = pack_bf16x2(d1.x, d1.y);
+        }
+        tmem_st_32x16(td + c * 16, dw);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      warp_arrive(&bars->ds_full[wg], lane);
+      ti += 2;
+      if (MODE == 1 && ti >= S / 64) ti = 2 * xb + wg;
     }
     if (ok && await_all(&bars->acc_full, 0, status)) {
+      // The stationary operands have been read for the last time; their buffers take the gradient tiles.
+      //   MODE 0: dQ, one 64-column half per warp group.  MODE 1: dK by the first group, dV by the second.
       tc_fence_after();
-      const long long tok = tok0 + xpos;
-      // MODE 0 writes dQ of head hy; MODE 1 writes dK and dV of kv head g.
-      __nv_bfloat16* o1 = d_qkv + tok * W + ((MODE == 0) ? hy * HD : (Hq + g) * HD);
-      __nv_bfloat16* o2 = d_qkv + tok * W + (Hq + Hkv + g) * HD;
+      const int acc = MODE == 0 ? 0 : wg;
+      const uint32_t ta = (acc == 0 ? tmem_acc1 : tmem_acc2) + lane_sel;
+      uint8_t* obuf = smem + (acc == 0 ? L::X1_OFF : L::X2_OFF);
+      const int col0 = (MODE == 0 ? hy : Hq + acc * Hkv + g) * HD;
+      const float sc = acc == 0 ? scale : 1.f;
 #pragma unroll 1
-      for (int a = 0; a < (MODE == 0 ? 1 : 2); ++a) {
-        const uint32_t ta = (a == 0 ? tmem_acc1 : tmem_acc2) + lane_sel;
-        __nv_bfloat16* orow = (a == 0) ? o1 : o2;
-        const float sc = (a == 0) ? scale : 1.f;
-#pragma unroll 1
-        for (int c = wg; c < HD / 32; c += 2) {
-          uint32_t r[32];
-          tmem_ld_32x32(ta + c * 32, r);
+      for (int h = 0; h < L::HALVES; ++h) {
+        if (MODE == 0 && h != wg) continue;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t r[32], w[16];
+          tmem_ld_32x32(ta + h * 64 + c * 32, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint4 o;
-            uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              ow[i] = pack_bf16x2(__uint_as_float(r[v * 8 + 2 * i]) * sc,
-                                  __uint_as_float(r[v * 8 + 2 * i + 1]) * sc);
-            reinterpret_cast<uint4*>(orow + c * 32)[v] = o;
-          }
+          for (int i = 0; i < 16; ++i)
+            w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * sc, __uint_as_float(r[2 * i + 1]) * sc);
+          store_row_chunk_sw128(obuf + h * 16384, row, c * 4, w);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d_bulk(tmap_dqkv, obuf + h * 16384 + (warp & 3) * 32 * 128, col0 + 64 * h,
+                            tok0 + xb * 128 + (warp & 3) * 32);
+          bulk_commit_group();
         }
       }
+      if (lane == 0) bulk_wait_group<0>();
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) {
+  if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// One launch for both passes.  They are independent (dK/dV and dQ go to different columns of d_qkv) and hold a whole
+// SM per CTA; the dK/dV CTAs are few and of very different lengths (with grouped heads up to group x S/64 tiles),
+// so they start first, longest first, and the many shorter dQ CTAs fill the SMs they leave.
+template <int HD>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 128} over packed qkv
+                const __grid_constant__ CUtensorMap tmap_qkv_y,   // box {64, 64}  over packed qkv
+                const __grid_constant__ CUtensorMap tmap_do_x,    // box {64, 128} over dO [T, Hq*hd]
+                const __grid_constant__ CUtensorMap tmap_do_y,    // box {64, 64}  over dO
+                const __grid_constant__ CUtensorMap tmap_dqkv,    // box {64, 32}  over d_qkv
+                const float* __restrict__ lse, const float* __restrict__ delta, int B, int S, int Hq, int Hkv,
+                float scale, float scale_log2, int* status) {
+  const int blocks = S / 128;
+  const int n_kv = blocks * Hkv * B;
+  int idx = blockIdx.x;
+  if (idx < n_kv) {
+    const int hb = idx % (Hkv * B);
+    attn_bwd_cta<HD, 1>(&tmap_qkv_x, &tmap_qkv_y, &tmap_do_x, &tmap_do_y, &tmap_dqkv, lse, delta, idx / (Hkv * B),
+                        hb % Hkv, hb / Hkv, S, Hq, Hkv, scale, scale_log2, status);
+  } else {
+    idx -= n_kv;
+    const int hb = idx % (Hq * B);
+    attn_bwd_cta<HD, 0>(&tmap_qkv_x, &tmap_qkv_y, &tmap_do_x, &tmap_do_y, &tmap_dqkv, lse, delta,
+                        blocks - 1 - idx / (Hq * B), hb % Hq, hb / Hq, S, Hq, Hkv, scale, scale_log2, status);
   }
 }
 
@@ -826,56 +820,39 @@ int set_smem(K kern, int bytes) {
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
+template <int HD>
+static int attn_fwd_impl(const CUtensorMap& tm, const CUtensorMap& to, float* lse, int B, int S, int Hq, int Hkv,
+                         float softmax_scale, int* status, cudaStream_t st) {
+  static bool cfg = false;
+  if (!cfg) {
+    if (set_smem(attn_fwd_kernel<HD>, FwdSmem<HD>::TOTAL)) return -2;
+    cfg = true;
+  }
+  const float scale_log2 = softmax_scale * 1.4426950408889634f;
+  // Two query tiles per CTA overlap the softmax of one with the MMAs of the other.  As long as every tile can have
+  // an SM of its own, one tile per CTA finishes earlier.
+  const long long per_head = static_cast<long long>(Hq / Hkv) * (S / 128);
+  const int tiles_per_cta = per_head * Hkv * B <= 148 ? 1 : 2;
+  const long long ctas = (per_head + tiles_per_cta - 1) / tiles_per_cta * Hkv * B;
+  if (ctas > 0x7fffffffll) return -1;
+  attn_fwd_kernel<HD><<<static_cast<unsigned>(ctas), FWD_THREADS, FwdSmem<HD>::TOTAL, st>>>(
+      tm, to, lse, S, Hq, Hkv, B, tiles_per_cta, scale_log2, status);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 int attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int Hkv, int hd,
              float softmax_scale, int* status, cudaStream_t st) {
   if (S % 128 != 0 || Hq % Hkv != 0 || (hd != 64 && hd != 128)) return -1;
   if (B == 0) return 0;
   const long long T = static_cast<long long>(B) * S;
   const uint64_t W = static_cast<uint64_t>(Hq + 2 * Hkv) * hd;
-  CUtensorMap tm;
+  const uint64_t Wo = static_cast<uint64_t>(Hq) * hd;
+  CUtensorMap tm, to;
   int rc = make_tmap_2d_bf16(&tm, qkv, W, T, W * 2, 64, 128);
   if (rc != 0) return rc;
-  const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  dim3 grid(S / 128, Hq, B);
-  if (hd == 128) {
-    static bool cfg = false;
-    if (!cfg) { if (set_smem(attn_fwd_kernel<128>, FwdSmem<128>::TOTAL)) return -2; cfg = true; }
-    attn_fwd_kernel<128><<<grid, FWD_THREADS, FwdSmem<128>::TOTAL, st>>>(
-        tm, static_cast<__nv_bfloat16*>(out), lse, S, Hq, Hkv, scale_log2, status);
-  } else {
-    static bool cfg = false;
-    if (!cfg) { if (set_smem(attn_fwd_kernel<64>, FwdSmem<64>::TOTAL)) return -2; cfg = true; }
-    attn_fwd_kernel<64><<<grid, FWD_THREADS, FwdSmem<64>::TOTAL, st>>>(
-        tm, static_cast<__nv_bfloat16*>(out), lse, S, Hq, Hkv, scale_log2, status);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-// Side stream and the two events that fork the dK/dV kernel off a caller's stream and join it again; one set
-// per (device, caller stream), created on first use and kept for the life of the process.
-struct BwdFork {
-  cudaStream_t side = nullptr;
-  cudaEvent_t ready = nullptr, done = nullptr;
-};
-
-static bool bwd_fork(cudaStream_t st, BwdFork* out) {
-  static std::mutex mu;
-  static std::map<std::pair<int, cudaStream_t>, BwdFork> forks;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = forks.find({dev, st});
-  if (it == forks.end()) {
-    BwdFork f;
-    int least = 0, greatest = 0;   // the long dK/dV CTAs should win SMs over the dQ CTAs queued behind them
-    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return false;
-    if (cudaStreamCreateWithPriority(&f.side, cudaStreamNonBlocking, greatest) != cudaSuccess) return false;
-    if (cudaEventCreateWithFlags(&f.ready, cudaEventDisableTiming) != cudaSuccess) return false;
-    if (cudaEventCreateWithFlags(&f.done, cudaEventDisableTiming) != cudaSuccess) return false;
-    it = forks.emplace(std::make_pair(dev, st), f).first;
-  }
-  *out = it->second;
-  return true;
+  if ((rc = make_tmap_2d_bf16(&to, out, Wo, T, Wo * 2, 64, 32)) != 0) return rc;
+  return hd == 128 ? attn_fwd_impl<128>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, status, st)
+                   : attn_fwd_impl<64>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, status, st);
 }
 
 template <int HD>
@@ -885,54 +862,29 @@ static int attn_bwd_impl(const void* qkv, const void* out, const void* d_out, co
   const long long T = static_cast<long long>(B) * S;
   const uint64_t W = static_cast<uint64_t>(Hq + 2 * Hkv) * HD;
   const uint64_t Wo = static_cast<uint64_t>(Hq) * HD;
-  CUtensorMap tqx, tqy, tdx, tdy;
+  if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(d_out) | reinterpret_cast<uintptr_t>(lse) |
+        reinterpret_cast<uintptr_t>(delta)) & 15u) != 0)
+    return -1;
+  if (T * Hq >= (1ll << 31)) return -1;
+  CUtensorMap tqx, tqy, tdx, tdy, tdq;
   int rc;
   if ((rc = make_tmap_2d_bf16(&tqx, qkv, W, T, W * 2, 64, 128)) != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&tqy, qkv, W, T, W * 2, 64, 64)) != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&tdx, d_out, Wo, T, Wo * 2, 64, 128)) != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&tdy, d_out, Wo, T, Wo * 2, 64, 64)) != 0) return rc;
+  if ((rc = make_tmap_2d_bf16(&tdq, d_qkv, W, T, W * 2, 64, 32)) != 0) return rc;
   static bool cfg = false;
   if (!cfg) {
-    if (set_smem(attn_bwd_kernel<HD, 0>, BwdSmem<HD>::TOTAL)) return -2;
-    if (set_smem(attn_bwd_kernel<HD, 1>, BwdSmem<HD>::TOTAL)) return -2;
+    if (set_smem(attn_bwd_kernel<HD>, BwdSmem<HD>::TOTAL)) return -2;
     cfg = true;
   }
-  if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(d_out)) & 15u) != 0) return -1;
-  if (T * Hq >= (1ll << 31)) return -1;
   const long long delta_blocks = (T * Hq * (HD / 8) + 255) / 256;
   attn_delta_kernel<HD><<<static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st>>>(
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, T, S, Hq);
-  const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  // The two gradient kernels are independent (dK/dV and dQ go to different columns of d_qkv) and each holds a
-  // whole SM per CTA.  The dK/dV grid is small (S/128 x Hkv CTAs, under two waves for eight KV heads), so its last
-  // wave leaves SMs idle and its longest CTA (the first key tile, visited by every query tile of its head group)
-  // sets its duration.  It is launched first on a high-priority side stream and the dQ CTAs fill the idle SMs
-  // (measured: 0.995 -> 0.751 ms for 32 q / 8 kv heads at S = 4096).  PIPER_ATTN_FORK=0 runs both kernels one
-  // after the other on the caller's stream.
-  static int use_fork = -1;
-  if (use_fork < 0) {
-    const char* env = getenv("PIPER_ATTN_FORK");
-    use_fork = (env != nullptr && env[0] == '0') ? 0 : 1;
-  }
-  BwdFork fork;
-  cudaStream_t kv_stream = st;
-  if (use_fork) {
-    if (!bwd_fork(st, &fork)) return -3;
-    if (cudaEventRecord(fork.ready, st) != cudaSuccess || cudaStreamWaitEvent(fork.side, fork.ready, 0) != cudaSuccess)
-      return -3;
-    kv_stream = fork.side;
-  }
-  attn_bwd_kernel<HD, 1><<<dim3(S / 128, Hkv, B), BWD_THREADS, BwdSmem<HD>::TOTAL, kv_stream>>>(
-      tqx, tqy, tdx, tdy, lse, delta, static_cast<__nv_bfloat16*>(d_qkv), S, Hq, Hkv, softmax_scale,
-      scale_log2, status);
-  const bool kv_ok = cudaGetLastError() == cudaSuccess;
-  if (use_fork && cudaEventRecord(fork.done, fork.side) != cudaSuccess) return -3;
-  attn_bwd_kernel<HD, 0><<<dim3(S / 128, Hq, B), BWD_THREADS, BwdSmem<HD>::TOTAL, st>>>(
-      tqx, tqy, tdx, tdy, lse, delta, static_cast<__nv_bfloat16*>(d_qkv), S, Hq, Hkv, softmax_scale,
-      scale_log2, status);
-  const bool q_ok = cudaGetLastError() == cudaSuccess;
-  if (use_fork && cudaStreamWaitEvent(st, fork.done, 0) != cudaSuccess) return -3;   // the caller's stream owns both
-  return kv_ok && q_ok ? 0 : -3;
+  if (cudaGetLastError() != cudaSuccess) return -3;
+  attn_bwd_kernel<HD><<<static_cast<unsigned>(S / 128 * (Hkv + Hq) * B), BWD_THREADS, BwdSmem<HD>::TOTAL, st>>>(
+      tqx, tqy, tdx, tdy, tdq, lse, delta, B, S, Hq, Hkv, softmax_scale, softmax_scale * 1.4426950408889634f, status);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 int attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,

@@ -281,7 +281,7 @@ void attn_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, const Te
                            delta.data_ptr<float>(), dqkv.data_ptr(), static_cast<int>(B), static_cast<int>(S),
                            static_cast<int>(Hq), static_cast<int>(Hkv), static_cast<int>(hd),
                            static_cast<float>(scale), status.data_ptr<int>(), cur_stream()),
-           "attn_bwd", 3);
+           "attn_bwd", 2);
 }
 
 }  // namespace
