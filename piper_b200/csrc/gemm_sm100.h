@@ -53,7 +53,7 @@ enum : int {
 // zero padding rows, and uses expert g % experts of w [experts, N, K].
 // g_start / g_len live on the device.  rows_capacity is the row count of the
 // row buffers.  out is bf16 [rows_capacity, N] (fwd), bf16 [rows_capacity, K]
-// (dgrad) or fp32 [experts, N, K] (wgrad; accumulate selects += or =).
+// (dgrad) or [experts, N, K] (wgrad; fp32, where accumulate selects += or =, or bf16).
 struct GroupedGemmArgs {
   int mode;
   const void* x;        // [rows_capacity, K]   (fwd, wgrad)
@@ -66,6 +66,7 @@ struct GroupedGemmArgs {
   int N, K;
   long long rows_capacity;
   int accumulate;
+  int out_bf16;         // weight gradient as bf16 instead of fp32 (never accumulates)
   int* status;
 };
 

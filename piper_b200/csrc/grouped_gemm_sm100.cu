@@ -26,18 +26,29 @@ constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 4;
 constexpr int A_STAGE_BYTES = BM * BK * 2;
 constexpr int B_STAGE_BYTES = BN * BK * 2;
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int MN_BOX_BYTES = 64 * BK * 2;
 constexpr int NUM_THREADS = 384;     // TMA, MMA, TMEM-allocation and one idle warp, then eight epilogue warps
 constexpr int MAX_GROUPS = 1024;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + (MAX_GROUPS + 1) * 4;
+constexpr int EPI_WARPS = 8;
+constexpr int C_STAGE_BYTES = 4096;  // weight gradients: one 32-row x 128-byte block per epilogue warp
+
+// The weight gradient contracts over few rows (a few k-blocks per tile) and writes far more than it reads, so it
+// trades one operand stage for staging blocks that leave as TMA stores.
+template <int MODE>
+struct Cfg {
+  static constexpr int STAGES = MODE == kGroupedWgrad ? 3 : 4;
+  static constexpr int C_OFF = STAGES * STAGE_BYTES;
+  static constexpr int BAR_OFF = C_OFF + (MODE == kGroupedWgrad ? EPI_WARPS * C_STAGE_BYTES : 0);
+  static constexpr int TABLE_OFF = BAR_OFF + 256;       // tile_prefix[MAX_GROUPS + 1], start[], len[]
+  static constexpr int SMEM_BYTES = TABLE_OFF + (3 * MAX_GROUPS + 4) * 4 + 1024;
+};
 
 struct Barriers {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[4];
+  uint64_t empty[4];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
@@ -49,7 +60,7 @@ struct GroupedParams {
   int num_groups;        // G = sources * experts
   int experts;           // local experts
   int N, K;              // weight shape per expert [N, K]
-  void* c;               // output
+  void* c;               // output (fwd / dgrad)
   long long ldc;
   int accumulate;
   int* status;
@@ -65,7 +76,7 @@ struct Tile {
 
 template <int MODE>
 __device__ __forceinline__ Tile resolve_tile(int t, const int* tile_prefix, const GroupedParams& p,
-                                             int total_m_tiles, int tiles_n) {
+                                             const int* start, int tiles_n) {
   Tile r;
   r.valid = true;
   if (MODE == kGroupedWgrad) {
@@ -81,7 +92,6 @@ __device__ __forceinline__ Tile resolve_tile(int t, const int* tile_prefix, cons
   // Column tiles of one row tile are consecutive, and row tiles are walked expert by expert (all sources of an
   // expert together): the CTAs of a wave share their A tiles and a few experts' weights through L2, so both
   // operands stream from DRAM once.  (Row tiles fastest re-read every row once per column tile.)
-  (void)total_m_tiles;
   const int mt = t / tiles_n;
   r.n0 = (t % tiles_n) * BN;
   int lo = 0, hi = p.num_groups;          // largest q with tile_prefix[q] <= mt
@@ -92,21 +102,25 @@ __device__ __forceinline__ Tile resolve_tile(int t, const int* tile_prefix, cons
   const int sources = p.num_groups / p.experts;
   r.expert = lo / sources;                 // tile_prefix is ordered (expert, source)
   r.group = (lo % sources) * p.experts + r.expert;
-  r.m0 = p.g_start[r.group] + (mt - tile_prefix[lo]) * BM;
+  r.m0 = start[r.group] + (mt - tile_prefix[lo]) * BM;
   return r;
 }
 
-template <int MODE>
+// OUT_BF16 selects the element type of a weight gradient (fp32 buckets accumulate; a bf16 result is stored).
+template <int MODE, bool OUT_BF16>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                    const GroupedParams p) {
+                    const __grid_constant__ CUtensorMap tmap_c, const GroupedParams p) {
+  constexpr int STAGES = Cfg<MODE>::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + STAGES * STAGE_BYTES);
-  int* tile_prefix = reinterpret_cast<int*>(smem + STAGES * STAGE_BYTES + 256);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + Cfg<MODE>::BAR_OFF);
+  int* tile_prefix = reinterpret_cast<int*>(smem + Cfg<MODE>::TABLE_OFF);
+  int* g_start = tile_prefix + MAX_GROUPS + 1;
+  int* g_len = g_start + MAX_GROUPS;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   constexpr bool A_MN = (MODE == kGroupedWgrad);
   constexpr bool B_MN = (MODE != kGroupedFwd);
@@ -127,12 +141,33 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+  }
+  if (warp == 3) {
+    // Row tiles before each segment, in the order q = expert * sources + source (group = source * experts + expert):
+    // a warp scan, since one thread walking the table pays a memory latency per group in front of every launch.
     int acc = 0;
-    for (int q = 0; q < p.num_groups; ++q) {           // q = expert * sources + source; group = source * experts + expert
-      tile_prefix[q] = acc;
-      acc += p.g_len[(q % sources) * p.experts + q / sources] / BM;
+#pragma unroll 4
+    for (int q0 = 0; q0 < p.num_groups; q0 += 32) {
+      const int q = q0 + lane;
+      const bool in = q < p.num_groups;
+      const int grp = in ? (q % sources) * p.experts + q / sources : 0;
+      const int len = in ? p.g_len[grp] : 0;
+      const int start = in ? p.g_start[grp] : 0;
+      const int n = len / BM;
+      int inc = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (in) {
+        tile_prefix[q] = acc + inc - n;
+        g_start[grp] = start;
+        g_len[grp] = len;
+      }
+      acc += __shfl_sync(0xffffffffu, inc, 31);
     }
-    tile_prefix[p.num_groups] = acc;
+    if (lane == 0) tile_prefix[p.num_groups] = acc;
   }
   if (warp == 2) {
     tmem_alloc(&bars->tmem_base, 2 * BN);
@@ -150,7 +185,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   auto k_blocks_of = [&](const Tile& t) -> int {
     if (MODE != kGroupedWgrad) return (contract + BK - 1) / BK;
     int n = 0;
-    for (int s = 0; s < sources; ++s) n += p.g_len[s * p.experts + t.expert] / BK;
+    for (int s = 0; s < sources; ++s) n += g_len[s * p.experts + t.expert] / BK;
     return n;
   };
 
@@ -159,7 +194,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t it = 0;
       bool ok = true;
       for (int ti = blockIdx.x; ti < num_tiles && ok; ti += gridDim.x) {
-        const Tile t = resolve_tile<MODE>(ti, tile_prefix, p, total_m_tiles, tiles_n);
+        const Tile t = resolve_tile<MODE>(ti, tile_prefix, p, g_start, tiles_n);
         auto issue = [&](int a_x, int a_y, int b_x, int b_y) -> bool {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -191,7 +226,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (MODE == kGroupedWgrad) {
           for (int s = 0; s < sources && ok; ++s) {
             const int g = s * p.experts + t.expert;
-            const int r0 = p.g_start[g], len = p.g_len[g];
+            const int r0 = g_start[g], len = g_len[g];
             for (int r = 0; r < len && ok; r += BK) ok = issue(t.m0, r0 + r, t.n0, r0 + r);
           }
         } else {
@@ -212,38 +247,40 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
-      uint32_t it = 0, local_tile = 0;
-      bool ok = true;
-      for (int ti = blockIdx.x; ti < num_tiles && ok; ti += gridDim.x) {
-        const Tile t = resolve_tile<MODE>(ti, tile_prefix, p, total_m_tiles, tiles_n);
-        const int kb_total = k_blocks_of(t);
-        if (kb_total == 0) continue;
-        const int acc = local_tile & 1;
-        const uint32_t acc_ph = (local_tile >> 1) & 1;
-        ++local_tile;
-        if (!mbar_wait(&bars->acc_empty[acc], acc_ph ^ 1, p.status)) { ok = false; break; }
+    // uniform control flow, one elected lane issues
+    constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
+    const uint64_t da0 = A_MN ? umma_desc_sw128(smem_u32(smem), MN_BOX_BYTES, 1024)
+                              : umma_desc_sw128(smem_u32(smem), 16, 1024);
+    const uint64_t db0 = B_MN ? umma_desc_sw128(smem_u32(smem) + A_STAGE_BYTES, MN_BOX_BYTES, 1024)
+                              : umma_desc_sw128(smem_u32(smem) + A_STAGE_BYTES, 16, 1024);
+    constexpr int a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+    constexpr int b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+    uint32_t local_tile = 0, ph = 0;
+    int s = 0;
+    bool ok = true;
+    for (int ti = blockIdx.x; ti < num_tiles && ok; ti += gridDim.x) {
+      const Tile t = resolve_tile<MODE>(ti, tile_prefix, p, g_start, tiles_n);
+      const int kb_total = k_blocks_of(t);
+      if (kb_total == 0) continue;
+      const int acc = local_tile & 1;
+      const uint32_t acc_ph = (local_tile >> 1) & 1;
+      ++local_tile;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[acc], acc_ph ^ 1, p.status));
+      const uint32_t tmem_d = tmem_base + acc * BN;
+      for (int kb = 0; kb < kb_total && ok; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], ph, p.status));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < kb_total; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&bars->full[s], ph, p.status)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-          const uint32_t sb = sa + A_STAGE_BYTES;
+        if (elect_one()) {
+          const uint64_t da = da0 + (s * STAGE_BYTES >> 4), db = db0 + (s * STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = A_MN ? umma_desc_sw128(sa + k * (UMMA_K * 128), MN_BOX_BYTES, 1024)
-                                     : umma_desc_sw128(sa + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t db = B_MN ? umma_desc_sw128(sb + k * (UMMA_K * 128), MN_BOX_BYTES, 1024)
-                                     : umma_desc_sw128(sb + k * (UMMA_K * 2), 16, 1024);
-            umma_bf16_ss(tmem_d, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_ss(tmem_d, da + k * a_step, db + k * b_step, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit(&bars->empty[s]);
+          if (kb == kb_total - 1) umma_commit(&bars->acc_full[acc]);
         }
-        if (ok) umma_commit(&bars->acc_full[acc]);
+        __syncwarp();
+        if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp >= 4) {
@@ -252,72 +289,88 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t local_tile = 0;
     bool ok = true;
     for (int ti = blockIdx.x; ti < num_tiles && ok; ti += gridDim.x) {
-      const Tile t = resolve_tile<MODE>(ti, tile_prefix, p, total_m_tiles, tiles_n);
+      const Tile t = resolve_tile<MODE>(ti, tile_prefix, p, g_start, tiles_n);
       const int kb_total = k_blocks_of(t);
-      const int row_limit = (MODE == kGroupedWgrad) ? p.N : 0x7fffffff;
       const int row = t.m0 + q * 32 + lane;
-      const long long c_off = (MODE == kGroupedWgrad) ? static_cast<long long>(t.expert) * p.N * p.K : 0;
-      if (kb_total == 0) {
-        // expert without rows: nothing to add; a non-accumulating output tile is zero
-        if (!p.accumulate && row < row_limit) {
-          for (int j = ch * 128; j < ch * 128 + 128 && t.n0 + j < out_cols; ++j) {
-            if (MODE == kGroupedWgrad) reinterpret_cast<float*>(p.c)[c_off + row * p.ldc + t.n0 + j] = 0.f;
-          }
-        }
-        continue;
-      }
+      // expert without rows: nothing to add; a non-accumulating output tile is zero
+      if (kb_total == 0 && (MODE != kGroupedWgrad || p.accumulate)) continue;
       const int acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
-      ++local_tile;
-      if (!mbar_wait(&bars->acc_full[acc], acc_ph, p.status)) { ok = false; break; }
+      if (kb_total > 0) {
+        ++local_tile;
+        if (!__all_sync(0xffffffffu, mbar_wait(&bars->acc_full[acc], acc_ph, p.status))) { ok = false; break; }
+      }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + ch * 128;
+      if (MODE == kGroupedWgrad) {
+        // a warp's 32 rows x 128 bytes at a time through a swizzled block and a TMA store (fp32 accumulation: a TMA
+        // reduce-add, C is never read by the SM); the tensor map clips ragged edges
+        uint8_t* cbuf = smem + Cfg<MODE>::C_OFF + (warp - 4) * C_STAGE_BYTES;
+        constexpr int COLS = OUT_BF16 ? 64 : 32;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = t.n0 + ch * 128 + c * 32;
-        if (row < row_limit && col0 < out_cols) {
-          if (MODE == kGroupedWgrad) {
-            float* crow = reinterpret_cast<float*>(p.c) + c_off + row * p.ldc + col0;
-            if (col0 + 32 <= out_cols) {
+        for (int c = 0; c < 128 / COLS; ++c) {
+          const int col0 = t.n0 + ch * 128 + c * COLS;
+          if (col0 >= out_cols || t.m0 + q * 32 >= p.N) break;
+          uint4 blk[8];
 #pragma unroll
-              for (int v = 0; v < 8; ++v) {
-                float4 o = make_float4(__uint_as_float(r[4 * v + 0]), __uint_as_float(r[4 * v + 1]),
-                                       __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                if (p.accumulate) {
-                  const float4 q = reinterpret_cast<const float4*>(crow)[v];
-                  o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
-                }
-                reinterpret_cast<float4*>(crow)[v] = o;
-              }
+          for (int h = 0; h < COLS / 32; ++h) {
+            uint32_t r[32];
+            if (kb_total > 0) {
+              tmem_ld_32x32(taddr + c * COLS + h * 32, r);
+              tmem_ld_wait();
             } else {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {      // constant indices keep r[] in registers
-                if (col0 + j < out_cols) {
-                  const float x = __uint_as_float(r[j]);
-                  crow[j] = p.accumulate ? crow[j] + x : x;
-                }
-              }
+              for (int i = 0; i < 32; ++i) r[i] = 0;
             }
-          } else {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.c) + row * p.ldc + col0;
-            if (col0 + 32 <= out_cols) {
+            if (OUT_BF16) {
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
-                uint4 o;
-                o.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
-                o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
-                o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
-                o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
-                reinterpret_cast<uint4*>(crow)[v] = o;
+                uint32_t* o = reinterpret_cast<uint32_t*>(&blk[h * 4 + v]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  o[i] = pack_bf16x2(__uint_as_float(r[8 * v + 2 * i]), __uint_as_float(r[8 * v + 2 * i + 1]));
               }
             } else {
 #pragma unroll
-              for (int j = 0; j < 32; ++j)        // constant indices keep r[] in registers
-                if (col0 + j < out_cols) crow[j] = __float2bfloat16(__uint_as_float(r[j]));
+              for (int v = 0; v < 8; ++v) blk[v] = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
             }
+          }
+          if (lane == 0) bulk_wait_group_read<0>();      // the previous block has left the buffer
+          __syncwarp();
+#pragma unroll
+          for (int v = 0; v < 8; ++v) reinterpret_cast<uint4*>(cbuf + lane * 128)[v ^ (lane & 7)] = blk[v];
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (p.accumulate) tma_reduce_add_3d_bulk(&tmap_c, cbuf, col0, t.m0 + q * 32, t.expert);
+            else tma_store_3d_bulk(&tmap_c, cbuf, col0, t.m0 + q * 32, t.expert);
+            bulk_commit_group();
+          }
+        }
+        if (kb_total == 0) continue;
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + c * 32, r);
+          tmem_ld_wait();
+          const int col0 = t.n0 + ch * 128 + c * 32;
+          if (col0 >= out_cols) continue;
+          __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.c) + row * p.ldc + col0;
+          if (col0 + 32 <= out_cols) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              uint4 o;
+              o.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
+              o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
+              o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
+              o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
+              reinterpret_cast<uint4*>(crow)[v] = o;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)        // constant indices keep r[] in registers
+              if (col0 + j < out_cols) crow[j] = __float2bfloat16(__uint_as_float(r[j]));
           }
         }
       }
@@ -325,6 +378,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
     }
+    if (MODE == kGroupedWgrad && lane == 0) bulk_wait_group<0>();   // staged blocks leave before the CTA does
   }
 
   tc_fence_before();
@@ -340,8 +394,9 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                               CUtensorMapFloatOOBfill);
 
-int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                      uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1) {
+int make_tmap_3d(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
+                      uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1,
+                      CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
   static EncodeFn fn = nullptr;
   if (fn == nullptr) {
     void* ptr = nullptr;
@@ -361,22 +416,23 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t 
   const cuuint32_t box[3] = {b0, b1, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r =
-      fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+      fn(out, type, 3, const_cast<void*>(base), dims, strides, box, estr,
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int MODE>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GroupedParams& p, int num_sms, cudaStream_t st) {
-  auto kern = grouped_gemm_kernel<MODE>;
+template <int MODE, bool OUT_BF16>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GroupedParams& p, int num_sms,
+           cudaStream_t st) {
+  auto kern = grouped_gemm_kernel<MODE, OUT_BF16>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<MODE>::SMEM_BYTES) != cudaSuccess)
       return -2;
     configured = true;
   }
-  kern<<<num_sms, NUM_THREADS, SMEM_BYTES, st>>>(ta, tb, p);
+  kern<<<num_sms, NUM_THREADS, Cfg<MODE>::SMEM_BYTES, st>>>(ta, tb, tc, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -389,7 +445,7 @@ int grouped_gemm_launch(const GroupedGemmArgs& g, int num_sms, cudaStream_t st) 
     // A rank can receive no rows at all (every token routed to experts of other ranks): nothing to multiply.
     // The weight gradient of such a step is zero.
     if (g.mode == kGroupedWgrad && !g.accumulate) {
-      const size_t bytes = static_cast<size_t>(g.experts) * g.N * g.K * sizeof(float);
+      const size_t bytes = static_cast<size_t>(g.experts) * g.N * g.K * (g.out_bf16 ? 2 : 4);
       if (cudaMemsetAsync(g.out, 0, bytes, st) != cudaSuccess) return -3;
     }
     return 0;
@@ -411,22 +467,28 @@ int grouped_gemm_launch(const GroupedGemmArgs& g, int num_sms, cudaStream_t st) 
   if (g.mode == kGroupedFwd) {
     // A = X [R, K] K-major; B = W [E, N, K] K-major; C = Y [R, N]
     if ((rc = make_tmap_2d_bf16(&ta, g.x, K, R, K * 2, BK, BM)) != 0) return rc;
-    if ((rc = make_tmap_3d_bf16(&tb, g.w, K, N, E, K * 2, N * K * 2, BK, BN)) != 0) return rc;
+    if ((rc = make_tmap_3d(&tb, g.w, K, N, E, K * 2, N * K * 2, BK, BN)) != 0) return rc;
     p.ldc = g.N;
-    return launch<kGroupedFwd>(ta, tb, p, num_sms, st);
+    return launch<kGroupedFwd, true>(ta, tb, ta, p, num_sms, st);
   }
   if (g.mode == kGroupedDgrad) {
     // A = dY [R, N] K-major (contraction N); B = W [E, N, K] read MN-major; C = dX [R, K]
     if ((rc = make_tmap_2d_bf16(&ta, g.dy, N, R, N * 2, BK, BM)) != 0) return rc;
-    if ((rc = make_tmap_3d_bf16(&tb, g.w, K, N, E, K * 2, N * K * 2, 64, BK)) != 0) return rc;
+    if ((rc = make_tmap_3d(&tb, g.w, K, N, E, K * 2, N * K * 2, 64, BK)) != 0) return rc;
     p.ldc = g.K;
-    return launch<kGroupedDgrad>(ta, tb, p, num_sms, st);
+    return launch<kGroupedDgrad, true>(ta, tb, ta, p, num_sms, st);
   }
-  // wgrad: A = dY [R, N] MN-major, B = X [R, K] MN-major, C = dW [E, N, K] fp32
+  // wgrad: A = dY [R, N] MN-major, B = X [R, K] MN-major, C = dW [E, N, K] fp32 or bf16
   if ((rc = make_tmap_2d_bf16(&ta, g.dy, N, R, N * 2, 64, BK)) != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&tb, g.x, K, R, K * 2, 64, BK)) != 0) return rc;
+  CUtensorMap tc;
+  const uint64_t es = g.out_bf16 ? 2 : 4;
+  if ((rc = make_tmap_3d(&tc, g.out, K, N, E, K * es, N * K * es, 128 / es, 32,
+                         g.out_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32)) != 0)
+    return rc;
   p.ldc = g.K;
-  return launch<kGroupedWgrad>(ta, tb, p, num_sms, st);
+  return g.out_bf16 ? launch<kGroupedWgrad, true>(ta, tb, tc, p, num_sms, st)
+                    : launch<kGroupedWgrad, false>(ta, tb, tc, p, num_sms, st);
 }
 
 }  // namespace piper

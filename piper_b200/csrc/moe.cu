@@ -28,10 +28,11 @@ constexpr int MAX_K = 8;
 
 // Softmax probabilities of one token, E/32 values per lane (expert e lives in
 // lane e % 32, slot e / 32).
-__device__ __forceinline__ void token_softmax(const __nv_bfloat16* row, int E, int lane, float (&p)[MAX_PER_LANE]) {
+template <int SLOTS>
+__device__ __forceinline__ void token_softmax(const __nv_bfloat16* row, int E, int lane, float (&p)[SLOTS]) {
   float mx = -INFINITY;
 #pragma unroll
-  for (int s = 0; s < MAX_PER_LANE; ++s) {
+  for (int s = 0; s < SLOTS; ++s) {
     const int e = s * 32 + lane;
     p[s] = (e < E) ? __bfloat162float(row[e]) : -INFINITY;
     mx = fmaxf(mx, p[s]);
@@ -39,54 +40,52 @@ __device__ __forceinline__ void token_softmax(const __nv_bfloat16* row, int E, i
   mx = warp_max(mx);
   float sum = 0.f;
 #pragma unroll
-  for (int s = 0; s < MAX_PER_LANE; ++s) {
+  for (int s = 0; s < SLOTS; ++s) {
     p[s] = (s * 32 + lane < E) ? __expf(p[s] - mx) : 0.f;
     sum += p[s];
   }
   sum = warp_sum(sum);
   const float inv = 1.f / sum;
 #pragma unroll
-  for (int s = 0; s < MAX_PER_LANE; ++s) p[s] *= inv;
+  for (int s = 0; s < SLOTS; ++s) p[s] *= inv;
 }
 
+// Bound by the serial chain of k arg-max rounds: probabilities are compared as integers (same order for values >= 0,
+// and a NaN stays selectable instead of selecting nothing), so a round is two warp reductions in hardware; lane j
+// keeps the j-th choice and the k results are written, and counted, at once.
+template <int SLOTS>
 __global__ void route_kernel(const __nv_bfloat16* __restrict__ logits, float* __restrict__ weights,
                              int* __restrict__ idx, int* __restrict__ counts, long long T, int E, int k,
                              int renorm) {
   const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
-  float p[MAX_PER_LANE];
-  token_softmax(logits + t * E, E, lane, p);
-  float sel_w[MAX_K];
-  int sel_e[MAX_K];
-  float total = 0.f;
+  float p[SLOTS];
+  token_softmax<SLOTS>(logits + t * E, E, lane, p);
+  int key[SLOTS];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) key[s] = s * 32 + lane < E ? (__float_as_int(p[s]) & 0x7fffffff) : -1;
+  float my_w = 0.f, total = 0.f;
+  int my_e = 0;
   for (int j = 0; j < k; ++j) {
     // arg-max over the remaining probabilities; ties go to the lower expert index
-    float best = -1.f;
-    int best_e = 0x7fffffff;
+    int best = key[0], slot = 0;
 #pragma unroll
-    for (int s = 0; s < MAX_PER_LANE; ++s) {
-      const int e = s * 32 + lane;
-      if (e < E && (p[s] > best || (p[s] == best && e < best_e))) { best = p[s]; best_e = e; }
-    }
+    for (int s = 1; s < SLOTS; ++s)
+      if (key[s] > best) { best = key[s]; slot = s; }
+    const int top = __reduce_max_sync(0xffffffffu, best);
+    const int e = __reduce_min_sync(0xffffffffu, best == top ? slot * 32 + lane : 0x7fffffff);
+    const float w = __int_as_float(top);
+    total += w;
+    if (lane == j) { my_w = w; my_e = e; }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
-    sel_w[j] = best;
-    sel_e[j] = best_e;
-    total += best;
-    if ((best_e & 31) == lane) p[best_e >> 5] = -1.f;   // remove from further rounds
+    for (int s = 0; s < SLOTS; ++s)
+      if (s * 32 + lane == e) key[s] = -1;     // remove from further rounds
   }
-  if (lane == 0) {
-    const float scale = renorm ? 1.f / total : 1.f;
-    for (int j = 0; j < k; ++j) {
-      weights[t * k + j] = sel_w[j] * scale;
-      idx[t * k + j] = sel_e[j];
-      atomicAdd(counts + sel_e[j], 1);
-    }
+  if (lane < k) {
+    weights[t * k + lane] = my_w * (renorm ? 1.f / total : 1.f);
+    idx[t * k + lane] = my_e;
+    atomicAdd(counts + my_e, 1);
   }
 }
 
@@ -98,7 +97,7 @@ __global__ void route_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
   float p[MAX_PER_LANE], dp[MAX_PER_LANE];
-  token_softmax(logits + t * E, E, lane, p);
+  token_softmax<MAX_PER_LANE>(logits + t * E, E, lane, p);
 #pragma unroll
   for (int s = 0; s < MAX_PER_LANE; ++s) dp[s] = 0.f;
   float S = 1.f, dot_w = 0.f;
@@ -127,167 +126,224 @@ __global__ void route_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const
   }
 }
 
+// One warp: a scan over each source's segments (one thread walking 128 groups took 5 us of dependent loads).
 __global__ void group_table_kernel(const int* __restrict__ counts, int num_groups, int experts,
                                    const int* __restrict__ row_base, int* __restrict__ g_start,
                                    int* __restrict__ g_len, int* __restrict__ total) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const int lane = threadIdx.x;
   int run = 0, last = 0;
-  for (int g = 0; g < num_groups; ++g) {
-    if (row_base != nullptr && g % experts == 0) run = row_base[g / experts];
-    const int len = (counts[g] + 127) / 128 * 128;
-    g_start[g] = run;
-    g_len[g] = len;
-    run += len;
-    if (run > last) last = run;
-  }
-  total[0] = last;
-}
-
-struct alignas(16) vec16 { uint4 v; };
-
-// One warp per token: claims a row per entry, copies the token row there.
-__global__ void permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx,
-                               const int* __restrict__ g_start, int* __restrict__ cursor, int* __restrict__ pos,
-                               __nv_bfloat16* __restrict__ rows, long long T, int D, int k, int E, long long rows_cap,
-                               int* status) {
-  const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= T) return;
-  const uint4* src = reinterpret_cast<const uint4*>(x + t * D);
-  for (int j = 0; j < k; ++j) {
-    int r = -1;
-    if (lane == 0) {
-      const int e = idx[t * k + j];
-      if (e >= 0 && e < E) r = g_start[e] + atomicAdd(cursor + e, 1);
-      if (r < 0 || r >= rows_cap) {             // rejected: recorded, the copy is skipped
-        report_bad_argument(status, 31, e, r);
-        r = -1;
+  for (int s0 = 0; s0 < num_groups; s0 += experts) {
+    if (row_base != nullptr) run = row_base[s0 / experts];
+    const int n = min(experts, num_groups - s0);
+#pragma unroll 4
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int g = s0 + e0 + lane;
+      const bool in = e0 + lane < n;
+      const int len = in ? (counts[g] + 127) / 128 * 128 : 0;
+      int inc = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
       }
-      pos[t * k + j] = r < 0 ? 0 : r;
+      if (in) {
+        g_start[g] = run + inc - len;
+        g_len[g] = len;
+      }
+      run += __shfl_sync(0xffffffffu, inc, 31);
+      if (run > last) last = run;
     }
-    r = __shfl_sync(0xffffffffu, r, 0);
-    if (r < 0) continue;
-    uint4* dst = reinterpret_cast<uint4*>(rows + static_cast<long long>(r) * D);
-    for (int i = lane; i < D / 8; i += 32) dst[i] = src[i];
   }
+  if (lane == 0) total[0] = last;
 }
 
-// Zeroes rows [g_start + counts, g_start + g_len) of every group.
-__global__ void zero_padding_kernel(__nv_bfloat16* __restrict__ rows, const int* __restrict__ g_start,
-                                    const int* __restrict__ g_len, const int* __restrict__ counts, int D,
-                                    long long rows_cap, int* status) {
-  const int g = blockIdx.x;
+constexpr int ROW_THREADS = 128;      // four tokens per CTA: enough CTAs for the small token counts
+constexpr int PAD_CTAS = 4;           // CTAs that clear the padding of one group
+
+// Zeroes part `part` of rows [g_start + counts, g_start + g_len) of group g.
+__device__ __forceinline__ void zero_padding(__nv_bfloat16* __restrict__ rows, const int* __restrict__ g_start,
+                                             const int* __restrict__ g_len, const int* __restrict__ counts, int g,
+                                             int part, int D, long long rows_cap, int* status) {
   const int first = g_start[g] + counts[g];
   const int last = g_start[g] + g_len[g];
   if (counts[g] < 0 || g_start[g] < 0 || last < first || last > rows_cap) {
-    if (threadIdx.x == 0) report_bad_argument(status, 35, g, last);
+    if (threadIdx.x == 0 && part == 0) report_bad_argument(status, 35, g, last);
     return;                                   // a segment outside the buffer is left alone
   }
   const uint4 z = make_uint4(0, 0, 0, 0);
   const long long nvec = static_cast<long long>(last - first) * (D / 8);
   uint4* base = reinterpret_cast<uint4*>(rows + static_cast<long long>(first) * D);
-  for (long long i = threadIdx.x; i < nvec; i += blockDim.x) base[i] = z;
+  for (long long i = part * ROW_THREADS + threadIdx.x; i < nvec; i += PAD_CTAS * ROW_THREADS) base[i] = z;
 }
 
-__global__ void permute_bwd_kernel(const __nv_bfloat16* __restrict__ drows, const int* __restrict__ pos,
-                                   __nv_bfloat16* __restrict__ dx, long long T, int D, int k, long long rows_cap,
-                                   int* status) {
-  const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+// One warp per token: the first k lanes claim the rows of its entries together, then the token row is read once and
+// written k times; the CTAs behind the tokens' clear the padding rows of the segments.
+__global__ void __launch_bounds__(ROW_THREADS)
+permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx, const int* __restrict__ g_start,
+               const int* __restrict__ g_len, const int* __restrict__ counts, int* __restrict__ cursor,
+               int* __restrict__ pos, __nv_bfloat16* __restrict__ rows, long long T, int D, int k, int E,
+               long long rows_cap, unsigned token_ctas, int* status) {
+  if (blockIdx.x >= token_ctas) {
+    const int b = static_cast<int>(blockIdx.x - token_ctas);
+    zero_padding(rows, g_start, g_len, counts, b / PAD_CTAS, b % PAD_CTAS, D, rows_cap, status);
+    return;
+  }
+  const long long t = (static_cast<long long>(blockIdx.x) * ROW_THREADS + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
-  for (int i = lane; i < D / 8; i += 32) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j = 0; j < k; ++j) {
-      const long long r = pos[t * k + j];
-      if (r < 0 || r >= rows_cap) {             // a row outside the buffer contributes nothing
-        report_bad_argument(status, 32, t, r);
-        continue;
+  const uint4* src = reinterpret_cast<const uint4*>(x + t * D);
+  const int nvec = D / 8;
+  for (int j0 = 0; j0 < k; j0 += 32) {
+    const int kk = min(32, k - j0);
+    int mine = -1;
+    if (lane < kk) {
+      const long long slot = t * k + j0 + lane;
+      const int e = idx[slot];
+      if (e >= 0 && e < E) mine = g_start[e] + atomicAdd(cursor + e, 1);
+      if (mine < 0 || mine >= rows_cap) {       // rejected: recorded, the copy is skipped
+        report_bad_argument(status, 31, e, mine);
+        mine = -1;
       }
-      const uint4 q = reinterpret_cast<const uint4*>(drows + r * D)[i];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+      pos[slot] = mine < 0 ? 0 : mine;
+    }
+    for (int i0 = 0; i0 < nvec; i0 += 128) {
+      uint4 v[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float2 f = __bfloat1622float2(h[c]);
-        acc[2 * c] += f.x;
-        acc[2 * c + 1] += f.y;
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u * 32 + lane < nvec) v[u] = src[i0 + u * 32 + lane];
+      for (int j = 0; j < kk; ++j) {
+        const int r = __shfl_sync(0xffffffffu, mine, j);
+        if (r < 0) continue;
+        uint4* dst = reinterpret_cast<uint4*>(rows + static_cast<long long>(r) * D);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i0 + u * 32 + lane < nvec) dst[i0 + u * 32 + lane] = v[u];
       }
     }
-    uint4 o;
-    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) oh[c] = __floats2bfloat162_rn(acc[2 * c], acc[2 * c + 1]);
-    reinterpret_cast<uint4*>(dx + t * D)[i] = o;
   }
 }
 
-__global__ void combine_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ pos,
-                               const float* __restrict__ weights, __nv_bfloat16* __restrict__ out, long long T,
-                               int D, int k, long long rows_cap, int* status) {
-  const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= T) return;
-  for (int i = lane; i < D / 8; i += 32) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j = 0; j < k; ++j) {
-      const float w = weights[t * k + j];
-      const long long r = pos[t * k + j];
-      if (r < 0 || r >= rows_cap) {
-        report_bad_argument(status, 33, t, r);
-        continue;
-      }
-      const uint4 q = reinterpret_cast<const uint4*>(rows + r * D)[i];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float2 f = __bfloat1622float2(h[c]);
-        acc[2 * c] += w * f.x;
-        acc[2 * c + 1] += w * f.y;
-      }
+// The rows of a token's entries [j0, j0 + K), one per lane, then broadcast: the gather loops below keep K loads in
+// flight per lane instead of one that waits for its own index.  A row outside the buffer is reported and becomes -1.
+template <int K>
+__device__ __forceinline__ void token_rows(const int* __restrict__ pos, long long t, int k, int j0, int lane,
+                                           long long rows_cap, int tag, int* status, int (&r)[K]) {
+  int mine = -1;
+  if (lane < K && j0 + lane < k) {
+    mine = pos[t * k + j0 + lane];
+    if (mine < 0 || mine >= rows_cap) {
+      report_bad_argument(status, tag, t, mine);
+      mine = -1;
     }
-    uint4 o;
-    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) oh[c] = __floats2bfloat162_rn(acc[2 * c], acc[2 * c + 1]);
-    reinterpret_cast<uint4*>(out + t * D)[i] = o;
   }
+#pragma unroll
+  for (int j = 0; j < K; ++j) r[j] = __shfl_sync(0xffffffffu, mine, j);
 }
 
-__global__ void combine_bwd_kernel(const __nv_bfloat16* __restrict__ rows, const __nv_bfloat16* __restrict__ dout,
-                                   const int* __restrict__ pos, const float* __restrict__ weights,
-                                   __nv_bfloat16* __restrict__ drows, float* __restrict__ dweights, long long T,
-                                   int D, int k, long long rows_cap, int* status) {
-  const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+// out[t] = sum_j weights[t, j] * rows[pos[t, j]] (weights == nullptr: plain sum); K entries at a time, any k.
+template <int K>
+__global__ void __launch_bounds__(ROW_THREADS)
+gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ pos,
+                  const float* __restrict__ weights, __nv_bfloat16* __restrict__ out, long long T, int D, int k,
+                  long long rows_cap, int tag, int* status) {
+  const long long t = (static_cast<long long>(blockIdx.x) * ROW_THREADS + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
-  for (int j = 0; j < k; ++j) {
-    const float w = weights[t * k + j];
-    const long long r = pos[t * k + j];
-    if (r < 0 || r >= rows_cap) {
-      if (lane == 0) {
-        report_bad_argument(status, 34, t, r);
-        dweights[t * k + j] = 0.f;
+  int r[K];
+  float w[K];
+  auto load_entries = [&](int j0) {
+    token_rows<K>(pos, t, k, j0, lane, rows_cap, tag, status, r);
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[j] = weights == nullptr ? 1.f : j0 + j < k ? weights[t * k + j0 + j] : 0.f;
+  };
+  load_entries(0);
+  for (int i0 = 0; i0 < D / 8; i0 += 32) {
+    const int i = i0 + lane;
+    const bool in = i < D / 8;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int j0 = 0; j0 < k; j0 += K) {
+      if (k > K) load_entries(j0);
+      uint4 q[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j)
+        if (in && r[j] >= 0) q[j] = reinterpret_cast<const uint4*>(rows + static_cast<long long>(r[j]) * D)[i];
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (!in || r[j] < 0) continue;
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q[j]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 f = __bfloat1622float2(h[c]);
+          acc[2 * c] += w[j] * f.x;
+          acc[2 * c + 1] += w[j] * f.y;
+        }
       }
-      continue;
     }
-    float dot = 0.f;
-    for (int i = lane; i < D / 8; i += 32) {
-      const uint4 g = reinterpret_cast<const uint4*>(dout + t * D)[i];
-      const uint4 q = reinterpret_cast<const uint4*>(rows + r * D)[i];
-      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g);
-      const __nv_bfloat162* qh = reinterpret_cast<const __nv_bfloat162*>(&q);
+    if (in) {
       uint4 o;
       __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float2 gf = __bfloat1622float2(gh[c]);
-        const float2 qf = __bfloat1622float2(qh[c]);
-        dot += gf.x * qf.x + gf.y * qf.y;
-        oh[c] = __floats2bfloat162_rn(w * gf.x, w * gf.y);
-      }
-      reinterpret_cast<uint4*>(drows + r * D)[i] = o;
+      for (int c = 0; c < 4; ++c) oh[c] = __floats2bfloat162_rn(acc[2 * c], acc[2 * c + 1]);
+      reinterpret_cast<uint4*>(out + t * D)[i] = o;
     }
-    dot = warp_sum(dot);
-    if (lane == 0) dweights[t * k + j] = dot;
+  }
+}
+
+// drows[pos[t, j]] = weights[t, j] * dout[t], dweights[t, j] = <rows[pos[t, j]], dout[t]>; K entries share one read
+// of dout.  The CTAs behind the tokens' clear the padding rows of drows.
+template <int K>
+__global__ void __launch_bounds__(ROW_THREADS)
+combine_bwd_kernel(const __nv_bfloat16* __restrict__ rows, const __nv_bfloat16* __restrict__ dout,
+                   const int* __restrict__ pos, const float* __restrict__ weights,
+                   __nv_bfloat16* __restrict__ drows, float* __restrict__ dweights,
+                   const int* __restrict__ g_start, const int* __restrict__ g_len, const int* __restrict__ counts,
+                   long long T, int D, int k, long long rows_cap, unsigned token_ctas, int* status) {
+  if (blockIdx.x >= token_ctas) {
+    const int b = static_cast<int>(blockIdx.x - token_ctas);
+    zero_padding(drows, g_start, g_len, counts, b / PAD_CTAS, b % PAD_CTAS, D, rows_cap, status);
+    return;
+  }
+  const long long t = (static_cast<long long>(blockIdx.x) * ROW_THREADS + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t >= T) return;
+  for (int j0 = 0; j0 < k; j0 += K) {
+    int r[K];
+    float w[K], dot[K];
+    token_rows<K>(pos, t, k, j0, lane, rows_cap, 34, status, r);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      w[j] = j0 + j < k ? weights[t * k + j0 + j] : 0.f;
+      dot[j] = 0.f;
+    }
+#pragma unroll 1
+    for (int i = lane; i < D / 8; i += 32) {
+      const uint4 g = reinterpret_cast<const uint4*>(dout + t * D)[i];
+      uint4 q[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j)
+        if (r[j] >= 0) q[j] = reinterpret_cast<const uint4*>(rows + static_cast<long long>(r[j]) * D)[i];
+      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g);
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (r[j] < 0) continue;
+        const __nv_bfloat162* qh = reinterpret_cast<const __nv_bfloat162*>(&q[j]);
+        uint4 o;
+        __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 gf = __bfloat1622float2(gh[c]);
+          const float2 qf = __bfloat1622float2(qh[c]);
+          dot[j] += gf.x * qf.x + gf.y * qf.y;
+          oh[c] = __floats2bfloat162_rn(w[j] * gf.x, w[j] * gf.y);
+        }
+        reinterpret_cast<uint4*>(drows + static_cast<long long>(r[j]) * D)[i] = o;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const float d = warp_sum(dot[j]);
+      if (lane == 0 && j0 + j < k) dweights[t * k + j0 + j] = d;
+    }
   }
 }
 
@@ -303,8 +359,9 @@ int moe_route(const void* logits, float* weights, int* idx, int* counts, long lo
               cudaStream_t st) {
   if (E > 32 * MAX_PER_LANE || k > MAX_K || k > E || k < 1) return -1;
   if (T == 0) return 0;
-  route_kernel<<<warps_grid(T, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), weights, idx, counts,
-                                                   T, E, k, renorm);
+  auto kern = E <= 32 ? route_kernel<1> : E <= 64 ? route_kernel<2> : E <= 128 ? route_kernel<4> : route_kernel<8>;
+  kern<<<warps_grid(T, ROW_THREADS), ROW_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), weights, idx,
+                                                           counts, T, E, k, renorm);
   return PIPER_LAUNCH_OK();
 }
 
@@ -329,43 +386,47 @@ int moe_permute(const void* x, const int* idx, const int* g_start, const int* g_
                 int* pos, void* rows, long long T, int D, int E, int k, long long rows_cap, int* status,
                 cudaStream_t st) {
   if (D % 8 != 0) return -1;
-  if (T > 0)
-    permute_kernel<<<warps_grid(T, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), idx, g_start, cursor,
-                                                       pos, static_cast<__nv_bfloat16*>(rows), T, D, k, E, rows_cap,
-                                                       status);
-  zero_padding_kernel<<<E, 256, 0, st>>>(static_cast<__nv_bfloat16*>(rows), g_start, g_len, counts, D, rows_cap, status);
+  const unsigned token_ctas = warps_grid(T, ROW_THREADS);
+  permute_kernel<<<token_ctas + E * PAD_CTAS, ROW_THREADS, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(x), idx, g_start, g_len, counts, cursor, pos, static_cast<__nv_bfloat16*>(rows),
+      T, D, k, E, rows_cap, token_ctas, status);
+  return PIPER_LAUNCH_OK();
+}
+
+// Entries per pass: all of them where k is 1, 2, 4 or 8, else passes of eight.
+static int gather_sum(const void* rows, const int* pos, const float* weights, void* out, long long T, int D, int k,
+                      long long rows_cap, int tag, int* status, cudaStream_t st) {
+  if (D % 8 != 0) return -1;
+  if (T == 0) return 0;
+  auto kern = k == 1 ? gather_sum_kernel<1> : k == 2 ? gather_sum_kernel<2> : k <= 4 ? gather_sum_kernel<4>
+                                                                                      : gather_sum_kernel<8>;
+  kern<<<warps_grid(T, ROW_THREADS), ROW_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(rows), pos, weights,
+                                                           static_cast<__nv_bfloat16*>(out), T, D, k, rows_cap, tag,
+                                                           status);
   return PIPER_LAUNCH_OK();
 }
 
 int moe_permute_bwd(const void* drows, const int* pos, void* dx, long long T, int D, int k, long long rows_cap,
                     int* status, cudaStream_t st) {
-  if (D % 8 != 0) return -1;
-  if (T == 0) return 0;
-  permute_bwd_kernel<<<warps_grid(T, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(drows), pos,
-                                                         static_cast<__nv_bfloat16*>(dx), T, D, k, rows_cap, status);
-  return PIPER_LAUNCH_OK();
+  return gather_sum(drows, pos, nullptr, dx, T, D, k, rows_cap, 32, status, st);
 }
 
 int moe_combine(const void* rows, const int* pos, const float* weights, void* out, long long T, int D, int k,
                 long long rows_cap, int* status, cudaStream_t st) {
-  if (D % 8 != 0) return -1;
-  if (T == 0) return 0;
-  combine_kernel<<<warps_grid(T, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(rows), pos, weights,
-                                                     static_cast<__nv_bfloat16*>(out), T, D, k, rows_cap, status);
-  return PIPER_LAUNCH_OK();
+  return gather_sum(rows, pos, weights, out, T, D, k, rows_cap, 33, status, st);
 }
 
 int moe_combine_bwd(const void* rows, const void* dout, const int* pos, const float* weights, void* drows,
                     float* dweights, const int* g_start, const int* g_len, const int* counts, int num_groups,
                     long long T, int D, int k, long long rows_cap, int* status, cudaStream_t st) {
   if (D % 8 != 0) return -1;
-  if (T > 0)
-    combine_bwd_kernel<<<warps_grid(T, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(rows),
-                                                           static_cast<const __nv_bfloat16*>(dout), pos, weights,
-                                                           static_cast<__nv_bfloat16*>(drows), dweights, T, D, k,
-                                                           rows_cap, status);
-  zero_padding_kernel<<<num_groups, 256, 0, st>>>(static_cast<__nv_bfloat16*>(drows), g_start, g_len, counts, D,
-                                                  rows_cap, status);
+  const unsigned token_ctas = warps_grid(T, ROW_THREADS);
+  if (token_ctas + num_groups == 0) return 0;
+  auto kern = k == 1 ? combine_bwd_kernel<1> : k == 2 ? combine_bwd_kernel<2> : k <= 4 ? combine_bwd_kernel<4>
+                                                                                        : combine_bwd_kernel<8>;
+  kern<<<token_ctas + num_groups * PAD_CTAS, ROW_THREADS, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(rows), static_cast<const __nv_bfloat16*>(dout), pos, weights,
+      static_cast<__nv_bfloat16*>(drows), dweights, g_start, g_len, counts, T, D, k, rows_cap, token_ctas, status);
   return PIPER_LAUNCH_OK();
 }
 

@@ -230,9 +230,9 @@ def _grouped_wgrad(rows: Tensor, dy: Tensor, w: Tensor, g_start: Tensor, g_len: 
         if sink is not None:
             _grouped(2, rows, dy, None, sink, g_start, g_len, E, N, K, accumulate=True)
             return None
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
-        _grouped(2, rows, dy, None, dw, g_start, g_len, E, N, K, accumulate=False)
-        return dw.to(w.dtype)
+        # every tile of dW is written once (zeros for an expert without rows), rounded from the fp32 accumulator
+        dw = torch.empty(w.shape, dtype=w.dtype, device=w.device)
+        return _grouped(2, rows, dy, None, dw, g_start, g_len, E, N, K, accumulate=False)
     dw = torch.zeros(w.shape, dtype=torch.float32)
     for g, a, b in _grouped_ref_segments(g_start, g_len):
         dw[g % E] += dy[a:b].float().t() @ rows[a:b].float()

@@ -74,6 +74,82 @@ def test_dispatch_grouped_mlp_combine(T, D, E, k, F):
     assert _rel(w2.grad, w2r.grad) < 3e-2
 
 
+@pytest.mark.parametrize("E,k", [(8, 8), (33, 3), (64, 1), (256, 8)])
+def test_router_expert_counts(E, k):
+    """One to eight probability slots per lane, the last one partly filled, and the smallest and largest k."""
+    from piper_b200.ops import moe as M
+
+    torch.manual_seed(2)
+    rank = torch.rand(130, E, device="cuda").argsort(1)
+    logits = (torch.linspace(-4, 4, E, device="cuda")[rank]).to(torch.bfloat16)
+    w, idx, counts = M.moe_route(logits, k, True)
+    p = torch.softmax(logits.float(), dim=-1)
+    wr, _ = torch.topk(p, k, dim=-1)
+    assert torch.allclose(torch.gather(p, 1, idx.long()), wr, rtol=1e-6)
+    assert all(len(set(r)) == k for r in idx.cpu().tolist())
+    assert _rel(w, wr / wr.sum(-1, keepdim=True)) < 1e-5       # fp32 softmax with __expf
+    assert torch.equal(counts, torch.bincount(idx.reshape(-1).long(), minlength=E).to(torch.int32))
+
+
+@pytest.mark.parametrize("T,D,E,k", [(5, 72, 4, 1), (130, 264, 8, 3), (33, 1032, 48, 12), (64, 256, 40, 33)])
+def test_permute_and_combine_entry_counts(T, D, E, k):
+    """Entry counts with a gather of their own, between them, above eight and above a warp; rows that are no multiple
+    of 32 vectors; experts without rows."""
+    from piper_b200.ops import moe as M, native
+
+    torch.manual_seed(3)
+    x = torch.randn(T, D, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    idx = torch.rand(T, E, device="cuda").argsort(1)[:, :k].to(torch.int32).contiguous()
+    counts = torch.bincount(idx.reshape(-1).long(), minlength=E).to(torch.int32)
+    weights = torch.rand(T, k, device="cuda", requires_grad=True)
+    rows, pos, g_start, g_len, _ = M.moe_dispatch(x, idx, counts)
+    end = g_start + g_len
+    assert torch.equal(g_start[1:], end[:-1]) and torch.equal(g_len, (counts + 127) // 128 * 128)
+    assert torch.equal(rows.detach()[pos.long()], x.detach().repeat_interleave(k, dim=0))
+    used = torch.zeros(rows.shape[0], dtype=torch.bool, device="cuda")
+    used[pos.long()] = True
+    assert not rows.detach()[: int(end[-1])][~used[: int(end[-1])]].any()          # padding rows are zero
+    out = M.moe_combine(rows * 1.0, pos, weights, g_start, g_len, counts)
+    g = torch.randn_like(out)
+    out.backward(g)
+    xr, wr = x.detach().double(), weights.detach().double()
+    gd = g.double()
+    assert _rel(out, xr * wr.sum(1, keepdim=True)) < 1e-2
+    assert _rel(x.grad, gd * wr.sum(1, keepdim=True)) < 1e-2
+    assert _rel(weights.grad, (xr * gd).sum(1, keepdim=True).expand(T, k)) < 1e-2
+    native.check_status()
+
+
+@pytest.mark.parametrize("N,K,sources", [(128, 256, 1), (136, 72, 2), (200, 328, 1), (512, 264, 2)])
+def test_grouped_weight_gradient(N, K, sources):
+    """bf16 result and fp32 bucket (stored, then accumulated), ragged edges of both dimensions, more than one row
+    segment per expert and experts without rows."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(4)
+    E = 6
+    lens = torch.tensor([[128, 0, 256, 384, 0, 128], [256, 0, 0, 128, 128, 0]][:sources], dtype=torch.int32)
+    g_len = lens.reshape(-1).cuda()
+    g_start = (torch.cumsum(g_len, 0) - g_len).to(torch.int32)
+    R = int(g_len.sum())
+    x = torch.randn(R, K, device="cuda").to(torch.bfloat16)
+    dy = torch.randn(R, N, device="cuda").to(torch.bfloat16)
+    want = torch.zeros(E, N, K, dtype=torch.float64, device="cuda")
+    for gi, (s, n) in enumerate(zip(g_start.tolist(), g_len.tolist())):
+        want[gi % E] += dy[s:s + n].double().t() @ x[s:s + n].double()
+    lib, st = native.lib(), native.status_tensor()
+    b16 = torch.full((E, N, K), 7.0, device="cuda", dtype=torch.bfloat16)
+    lib.grouped_gemm(2, x, dy, None, b16, g_start, g_len, E, N, K, False, st)
+    f32 = torch.full((E, N, K), 7.0, device="cuda")
+    lib.grouped_gemm(2, x, dy, None, f32, g_start, g_len, E, N, K, False, st)
+    scale = want.abs().max()
+    assert ((f32.double() - want).abs().max() / scale) < 1e-5          # fp32 sums of up to 512 products
+    assert torch.equal(b16, f32.to(torch.bfloat16))                     # the same accumulators, rounded once
+    lib.grouped_gemm(2, x, dy, None, f32, g_start, g_len, E, N, K, True, st)
+    assert ((f32.double() - 2 * want).abs().max() / scale) < 2e-5
+    native.check_status()
+
+
 def test_qwen3_moe_model_trains_on_one_gpu():
     from piper_b200 import piper_exec_dag, piper_setup
     from piper_b200.models.qwen3 import PiperQwen3Model, Qwen3Config
