@@ -202,6 +202,24 @@ void embedding_bwd(const Tensor& tokens, const Tensor& dout, Tensor dtable) {
            "embedding_bwd");
 }
 
+void embedding_bwd_bf16(const Tensor& tokens, const Tensor& dout, Tensor owner, Tensor acc, Tensor dtable) {
+  check_bf16(dout, "dout");
+  check_bf16(dtable, "dtable");
+  TORCH_CHECK(tokens.scalar_type() == at::kLong && tokens.is_contiguous(), "tokens must be contiguous int64");
+  TORCH_CHECK(owner.scalar_type() == at::kInt && owner.numel() == dtable.size(0), "owner must be int32 [V]");
+  TORCH_CHECK(acc.scalar_type() == at::kFloat && acc.numel() == tokens.numel() * dtable.size(1),
+              "acc must be fp32 [T, D]");
+  TORCH_CHECK(dout.is_contiguous() && acc.is_contiguous() && dtable.is_contiguous() && dout.numel() == acc.numel(),
+              "embedding_bwd_bf16 expects contiguous tensors");
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(dout.data_ptr()) | reinterpret_cast<uintptr_t>(acc.data_ptr()) |
+                reinterpret_cast<uintptr_t>(dtable.data_ptr())) & 15u) == 0,
+              "embedding_bwd_bf16 expects 16-byte aligned tensors");
+  check_rc(piper::embedding_bwd_bf16(reinterpret_cast<const long long*>(tokens.data_ptr<int64_t>()), dout.data_ptr(),
+                                     owner.data_ptr<int>(), acc.data_ptr<float>(), dtable.data_ptr(), tokens.numel(),
+                                     static_cast<int>(dtable.size(1)), static_cast<int>(dtable.size(0)), cur_stream()),
+           "embedding_bwd_bf16", 3);
+}
+
 void ce_fwd(const Tensor& logits, const Tensor& labels, Tensor loss, Tensor lse, int64_t ignore_index) {
   check_bf16(logits, "logits");
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1, "logits must be [T, V] with unit inner stride");
@@ -302,6 +320,7 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd", &embedding_bwd);
+  m.def("embedding_bwd_bf16", &embedding_bwd_bf16);
   m.def("ce_fwd", &ce_fwd);
   m.def("ce_bwd", &ce_bwd);
   m.def("adam_flat", &adam_flat);

@@ -682,6 +682,47 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ tokens,
   for (int i = threadIdx.x; i < D; i += blockDim.x) atomicAdd(dst + i, __bfloat162float(src[i]));
 }
 
+// Embedding gradient straight into a bf16 table, cleared first: rows of one token value are summed in fp32 in a compact
+// [T, D] buffer at the position of its first occurrence (owner[v], the lowest position), then rounded once into the
+// table.  The fp32 table it replaces cost a clear, a read and a conversion of V rows for the T that are touched.
+__global__ void embedding_owner_kernel(const long long* __restrict__ tokens, int* __restrict__ owner, int T, int V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= T) return;
+  const long long tok = tokens[i];
+  if (tok >= 0 && tok < V) atomicMin(owner + tok, i);
+}
+
+__global__ void __launch_bounds__(128)
+embedding_compact_kernel(const long long* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout,
+                         const int* __restrict__ owner, float* __restrict__ acc, int D, int V) {
+  const long long row = blockIdx.x;
+  const long long tok = tokens[row];
+  if (tok < 0 || tok >= V) return;
+  const bf16x8* src = reinterpret_cast<const bf16x8*>(dout + row * D);
+  float4* dst = reinterpret_cast<float4*>(acc + static_cast<long long>(owner[tok]) * D);
+  for (int i = threadIdx.x; i < D / 8; i += blockDim.x) {
+    float f[8];
+    unpack8(src[i], f);
+    atomicAdd(dst + 2 * i, make_float4(f[0], f[1], f[2], f[3]));
+    atomicAdd(dst + 2 * i + 1, make_float4(f[4], f[5], f[6], f[7]));
+  }
+}
+
+__global__ void __launch_bounds__(128)
+embedding_scatter_kernel(const long long* __restrict__ tokens, const int* __restrict__ owner,
+                         const float* __restrict__ acc, __nv_bfloat16* __restrict__ dtable, int D, int V) {
+  const long long row = blockIdx.x;
+  const long long tok = tokens[row];
+  if (tok < 0 || tok >= V || owner[tok] != row) return;
+  const float4* src = reinterpret_cast<const float4*>(acc + row * D);
+  bf16x8* dst = reinterpret_cast<bf16x8*>(dtable + tok * D);
+  for (int i = threadIdx.x; i < D / 8; i += blockDim.x) {
+    const float4 a = src[2 * i], b = src[2 * i + 1];
+    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    dst[i] = pack8(f);
+  }
+}
+
 // ------------------------------------------------------------ cross-entropy
 // One CTA per row of bf16 logits [T, V]: online max / sum-exp, per-token loss
 // and log-sum-exp.  ignore_index rows produce loss 0.
@@ -980,6 +1021,18 @@ int embedding_bwd(const long long* tokens, const void* dout, float* dtable, long
   if (T == 0) return 0;
   embedding_bwd_kernel<<<static_cast<unsigned>(T), 256, 0, st>>>(
       tokens, static_cast<const __nv_bfloat16*>(dout), dtable, T, D, V);
+  return PIPER_LAUNCH_OK();
+}
+
+int embedding_bwd_bf16(const long long* tokens, const void* dout, int* owner, float* acc, void* dtable, long long T,
+                       int D, int V, cudaStream_t st) {
+  if (D % 8 != 0 || T >= (1ll << 31)) return -1;
+  if (cudaMemsetAsync(dtable, 0, static_cast<size_t>(V) * D * 2, st) != cudaSuccess) return -3;
+  if (T == 0) return 0;
+  const unsigned n = static_cast<unsigned>(T);
+  embedding_owner_kernel<<<(n + 255) / 256, 256, 0, st>>>(tokens, owner, static_cast<int>(T), V);
+  embedding_compact_kernel<<<n, 128, 0, st>>>(tokens, static_cast<const __nv_bfloat16*>(dout), owner, acc, D, V);
+  embedding_scatter_kernel<<<n, 128, 0, st>>>(tokens, owner, acc, static_cast<__nv_bfloat16*>(dtable), D, V);
   return PIPER_LAUNCH_OK();
 }
 

@@ -40,6 +40,9 @@ int embedding_bwd(const long long* tokens, const void* dout, float* dtable, long
                   cudaStream_t st);
 
 // Per-row loss and log-sum-exp of bf16 logits [T, V] with row stride ld.
+// owner [V] int32 filled with a value >= T, acc [T, D] fp32 zeroed by the caller; D % 8 == 0.
+int embedding_bwd_bf16(const long long* tokens, const void* dout, int* owner, float* acc, void* dtable, long long T,
+                       int D, int V, cudaStream_t st);
 int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long T, int V,
            long long ld, long long ignore_index, cudaStream_t st);
 // out = (softmax - onehot) * gscale[0] * row_scale; out may alias logits.

@@ -656,8 +656,19 @@ def _embedding_backward(ctx, dout):
     tokens, table = ctx.saved_tensors
     sink = grad_sinks.get(table)
     if _is_native(table):
+        T, (V, D) = tokens.numel(), table.shape
+        dout = dout.contiguous()
+        if sink is None and T < V and D % 8 == 0 and dout.dtype == torch.bfloat16 and dout.data_ptr() % 16 == 0:
+            # Fewer tokens than table rows: sums of the touched rows in a compact fp32 buffer and one pass over a
+            # bf16 table (T >= V would make that buffer the larger one).  2048 tokens, 128256 x 2048 table: the
+            # fp32 table's clear and conversion took 375 us.
+            d_table = torch.empty_like(table, memory_format=torch.contiguous_format)
+            owner = torch.full((V,), T, dtype=torch.int32, device=table.device)
+            acc = torch.zeros((T, D), dtype=torch.float32, device=table.device)
+            native.lib().embedding_bwd_bf16(tokens.contiguous(), dout, owner, acc, d_table)
+            return None, d_table
         buf = sink if sink is not None else torch.zeros(table.shape, dtype=torch.float32, device=table.device)
-        native.lib().embedding_bwd(tokens.contiguous(), dout.contiguous(), buf)
+        native.lib().embedding_bwd(tokens.contiguous(), dout, buf)
         return None, (None if sink is not None else buf.to(table.dtype))
     g = torch.zeros(table.shape, dtype=torch.float32, device=table.device)
     g.index_add_(0, tokens.reshape(-1), dout.reshape(-1, table.shape[1]).float())

@@ -194,6 +194,22 @@ def test_attention_fwd_bwd(B, S, Hq, Hkv, hd):
     assert _close(gq[:, (Hq + Hkv) * hd:], gr[:, (Hq + Hkv) * hd:], 3e-2)   # dV
 
 
+@pytest.mark.parametrize("T,V,D", [(64, 1000, 264), (300, 301, 256), (0, 16, 64), (77, 40, 256)])
+def test_embedding_gradient(T, V, D):
+    """Compact accumulation into a bf16 table (T < V) and the fp32 table (T >= V); many repeated tokens."""
+    from piper_b200 import ops
+
+    torch.manual_seed(17)
+    table = torch.randn(V, D, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    tok = torch.randint(0, max(1, V // 4), (T,), device="cuda")
+    out = ops.embedding(tok, table)
+    g = torch.randn_like(out)
+    out.backward(g)
+    ref = torch.zeros(V, D, device="cuda").index_add_(0, tok, g.float())
+    assert table.grad.dtype == torch.bfloat16
+    assert torch.allclose(table.grad.float(), ref, rtol=2 ** -8, atol=1e-5)     # one rounding of an fp32 sum
+
+
 @pytest.mark.parametrize("T,F", [(9000, 776), (5000, 14336)])
 def test_swiglu_grid_stride_walk(T, F):
     """More vectors than the grid has threads, with a row length that the grid stride does not divide."""
