@@ -3,27 +3,17 @@
 // sequence a multiple of 128 long).  All matrix products run on tcgen05 with
 // accumulators in tensor memory; operands arrive by TMA (no multicast) in
 // 128-byte-swizzled tiles, and the probability / score-gradient tiles the
-// threads produce are written to shared memory in the same swizzled layout so
-// that they can feed the next tcgen05.mma directly.
+// threads produce go back to tensor memory, from where they feed the next
+// tcgen05.mma.
 //
-// Forward (attn_fwd_kernel): one CTA per (128 query rows, head).  Warps 0-3
-// own one query row per thread (row == TMEM lane), warp 4 issues TMA, warp 5
-// issues MMAs.  S = Q K^T is double-buffered in TMEM so the next block's
-// scores are computed while the threads run the online softmax; each P V
-// product lands in a fresh TMEM buffer and is folded into fp32 registers with
-// the running rescale factor, so TMEM is never rewritten by threads.
+// Forward (attn_fwd_kernel): one CTA per two query tiles of 128 rows; online softmax, P and O in tensor memory.
 //
-// Backward (attn_bwd_kernel<MODE>): one template for both passes.
-//   MODE 0 (dQ):  stationary tile = 128 query rows of one head (Q, dO);
-//                 streams 64-row K/V tiles; accumulates dQ.
-//   MODE 1 (dKV): stationary tile = 128 key rows of one kv head (K, V);
-//                 streams 64-row Q/dO tiles of every query head in the group;
-//                 accumulates dK and dV.
-// In both, S' = X1 Y1^T and dP' = X2 Y2^T are recomputed into double-buffered
-// TMEM, threads form P' = exp(S' - lse) and dS' = P' (dP' - delta) as bf16
-// tiles in shared memory, and acc1 += dS' Y1 (acc2 += P' Y2 in MODE 1) reuses
-// the streamed tiles as MN-major operands.  Nothing is reduced with atomics,
-// so gradients are reproducible.
+// Backward (attn_bwd_kernel): S and dP are recomputed; threads form P = exp(S - lse) and dS = P (dP - delta) as bf16
+// in tensor memory.  Two kinds of CTA in one launch:
+//   dK/dV: stationary tile = 128 key rows of one kv head (K, V); streams 64-row Q/dO tiles of every query head in
+//          the group; accumulates dK = dS^T Q and dV = P^T dO.
+//   dQ:    stationary tile = 128 query rows of one head (Q, dO); streams 128-row K and V blocks; dQ = dS K.
+// Nothing is reduced with atomics, so gradients are reproducible.
 //
 // Every mbarrier wait is bounded (see ptx.cuh); on expiry a status code is
 // recorded and the CTA unwinds and frees its TMEM.
@@ -422,11 +412,13 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   }
 }
 
-// Both passes stream 64-row tiles through two tensor memory stages.  Warps 0-3 turn the even tiles' scores into
-// probabilities and score gradients, warps 4-7 the odd tiles', so each group has the MMAs of two tiles' time for its
-// work; warp 8: TMA, warp 9: MMA.  P' and dS' (bf16) replace their own fp32 scores in tensor memory and are the A
-// operand of the accumulating MMAs from there: no thread writes shared memory in the loop.  Bound by the MMAs: a
-// 128x64x16 one with both operands in shared memory reads 6 KiB (48 cycles) for 32 cycles of arithmetic.
+// The dK/dV pass streams 64-row tiles through two tensor memory stages (dK, dV and two 64-wide pairs of S' and dP' fill
+// it).  Warps 0-3 turn the even tiles' scores into probabilities and score gradients, warps 4-7 the odd tiles', so
+// each group has the MMAs of two tiles' time for its work; warp 8: TMA, warp 9: MMA.  P' and dS' (bf16) replace their
+// own fp32 scores in tensor memory and are the A operand of the accumulating MMAs from there: no thread writes shared
+// memory in the loop.  Bound by the MMAs: a 128x64x16 one with both operands in shared memory reads 6 KiB (48 cycles)
+// for 32 cycles of arithmetic.  Both passes with probabilities through shared memory, two launches on two streams:
+// 751 us at S = 4096, 32 q / 8 kv heads x 128.
 constexpr int BWD_THREADS = 320;
 
 template <int HD>
@@ -449,19 +441,19 @@ struct BwdBars {
   uint64_t x_full;
   uint64_t y_full[4], y_empty[4];     // streamed tiles (BwdSmem::Y_STAGES)
   uint64_t s_full[2], dp_full[2];     // S' and dP' of a stage are in tensor memory
-  uint64_t p_full[2];                 // S' has been read; with MODE 1 P' stands in its place
+  uint64_t p_full[2];                 // P' stands in the place of S'
   uint64_t ds_full[2];                // dS' stands in the place of dP'
   uint64_t acc_full;
   uint32_t tmem_base;
 };
 
-// MODE 0: dQ of query head hy, rows of block xb.  MODE 1: dK, dV of kv head hy, rows of block xb.
-template <int HD, int MODE>
-__device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, const CUtensorMap* tmap_qkv_y,
-                                             const CUtensorMap* tmap_do_x, const CUtensorMap* tmap_do_y,
-                                             const CUtensorMap* tmap_dqkv, const float* __restrict__ lse,
-                                             const float* __restrict__ delta, int xb, int hy, int b, int S, int Hq,
-                                             int Hkv, float scale, float scale_log2, int* status) {
+// dK and dV of key block xb of kv head g.
+template <int HD>
+__device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, const CUtensorMap* tmap_qkv_y,
+                                             const CUtensorMap* tmap_do_y, const CUtensorMap* tmap_dqkv,
+                                             const float* __restrict__ lse, const float* __restrict__ delta, int xb,
+                                             int g, int b, int S, int Hq, int Hkv, float scale, float scale_log2,
+                                             int* status) {
   using L = BwdSmem<HD>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -472,12 +464,9 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
   const int group = Hq / Hkv;
   const int tok0 = b * S;
 
-  // Iteration space.
-  //   MODE 0: streams kv tiles i in [0, 2*xb + 1].
-  //   MODE 1: for each query head of the group streams q tiles i in [2*xb, S/64 - 1].
-  const int g = (MODE == 0) ? hy / group : hy;
-  const int tiles_per_head = (MODE == 0) ? (2 * xb + 2) : (S / 64 - 2 * xb);
-  const int n_iter = (MODE == 0) ? tiles_per_head : tiles_per_head * group;
+  // for each query head of the group streams q tiles i in [2*xb, S/64 - 1]
+  const int tiles_per_head = S / 64 - 2 * xb;
+  const int n_iter = tiles_per_head * group;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->x_full, 1);
@@ -495,7 +484,6 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
     fence_mbar_init();
     tma_prefetch_desc(tmap_qkv_x);
     tma_prefetch_desc(tmap_qkv_y);
-    tma_prefetch_desc(tmap_do_x);
     tma_prefetch_desc(tmap_do_y);
     tma_prefetch_desc(tmap_dqkv);
   }
@@ -518,41 +506,28 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
       const int xrow = tok0 + xb * 128;
       mbar_arrive_expect_tx(&bars->x_full, 2 * L::X_TILE);
       for (int h = 0; h < L::HALVES; ++h) {
-        if (MODE == 0) {
-          tma_load_2d(smem + L::X1_OFF + h * 16384, tmap_qkv_x, &bars->x_full, hy * HD + 64 * h, xrow);
-          tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_do_x, &bars->x_full, hy * HD + 64 * h, xrow);
-        } else {
-          tma_load_2d(smem + L::X1_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + g) * HD + 64 * h, xrow);
-          tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + Hkv + g) * HD + 64 * h, xrow);
-        }
+        tma_load_2d(smem + L::X1_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + g) * HD + 64 * h, xrow);
+        tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + Hkv + g) * HD + 64 * h, xrow);
       }
       int it = 0;
-      int hh = (MODE == 0) ? hy : g * group;     // query head and tile of iteration it
-      int ti = (MODE == 0) ? 0 : 2 * xb;
+      int hh = g * group, ti = 2 * xb;           // query head and tile of iteration it
       for (; it < n_iter; ++it) {
         const int st = it % L::Y_STAGES;
         if (!await(&bars->y_empty[st], ((it / L::Y_STAGES) & 1) ^ 1, status)) break;
         const int yrow = tok0 + ti * 64;
         uint8_t* yb = smem + L::Y_OFF + st * 2 * L::Y_TILE;
-        mbar_arrive_expect_tx(&bars->y_full[st], 2 * L::Y_TILE + (MODE == 1 ? 2 * L::VEC_BYTES : 0));
+        mbar_arrive_expect_tx(&bars->y_full[st], 2 * L::Y_TILE + 2 * L::VEC_BYTES);
         for (int h = 0; h < L::HALVES; ++h) {
           uint8_t* y1 = yb + h * L::Y_HALF;
           uint8_t* y2 = y1 + L::Y_TILE;
-          if (MODE == 0) {
-            tma_load_2d(y1, tmap_qkv_y, &bars->y_full[st], (Hq + g) * HD + 64 * h, yrow);
-            tma_load_2d(y2, tmap_qkv_y, &bars->y_full[st], (Hq + Hkv + g) * HD + 64 * h, yrow);
-          } else {
-            tma_load_2d(y1, tmap_qkv_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
-            tma_load_2d(y2, tmap_do_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
-          }
+          tma_load_2d(y1, tmap_qkv_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
+          tma_load_2d(y2, tmap_do_y, &bars->y_full[st], hh * HD + 64 * h, yrow);
         }
-        if (MODE == 1) {
-          const long long idx = (static_cast<long long>(b) * Hq + hh) * S + ti * 64;
-          uint8_t* v = smem + L::VEC_OFF + st * 2 * L::VEC_BYTES;
-          bulk_load(v, lse + idx, L::VEC_BYTES, &bars->y_full[st]);
-          bulk_load(v + L::VEC_BYTES, delta + idx, L::VEC_BYTES, &bars->y_full[st]);
-        }
-        if (++ti == S / 64 && MODE == 1) { ti = 2 * xb; ++hh; }
+        const long long idx = (static_cast<long long>(b) * Hq + hh) * S + ti * 64;
+        uint8_t* v = smem + L::VEC_OFF + st * 2 * L::VEC_BYTES;
+        bulk_load(v, lse + idx, L::VEC_BYTES, &bars->y_full[st]);
+        bulk_load(v + L::VEC_BYTES, delta + idx, L::VEC_BYTES, &bars->y_full[st]);
+        if (++ti == S / 64) { ti = 2 * xb; ++hh; }
       }
       if (it < n_iter) {
         // Unwinding: wait (bounded) for the copies in flight.
@@ -606,10 +581,8 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
       const uint64_t yk2 = dyk + (st2 * 2 * L::Y_TILE >> 4);
       if (!(ok = await_all(&bars->p_full[ss], ph, status))) break;
       tc_fence_after();
-      if (MODE == 1) {
-        if (elect_one()) issue_acc(tmem_acc2, tmem_base + ss * 64, yn + (L::Y_TILE >> 4), i == 0);
-        __syncwarp();
-      }
+      if (elect_one()) issue_acc(tmem_acc2, tmem_base + ss * 64, yn + (L::Y_TILE >> 4), i == 0);
+      __syncwarp();
       if (more) {
         if (!(ok = await_all(&bars->y_full[st2], ((i + 2) / L::Y_STAGES) & 1, status))) break;
         tc_fence_after();
@@ -643,51 +616,36 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
     const float2 sl2 = make_float2(scale_log2, scale_log2);
     constexpr float kNegLog2e = -1.4426950408889634f;
     const float2 neg_one = make_float2(-1.f, -1.f);
-    float2 row_nl = make_float2(0.f, 0.f), row_dl = make_float2(0.f, 0.f);
-    if (MODE == 0) {
-      const long long idx = (static_cast<long long>(b) * Hq + hy) * S + xpos;
-      row_nl.x = row_nl.y = lse[idx] * kNegLog2e;
-      row_dl.x = row_dl.y = delta[idx];
-    }
-    int ti = (MODE == 0) ? wg : 2 * xb + wg;   // tiles_per_head is even: the parity of ti is wg throughout
+    int ti = 2 * xb + wg;   // tiles_per_head is even: the parity of ti is wg throughout
     bool ok = true;
     for (int it = wg; it < n_iter; it += 2) {
       const uint32_t ph = (it >> 1) & 1;
       const int st = it % L::Y_STAGES;
       const float4* vl = reinterpret_cast<const float4*>(smem + L::VEC_OFF + st * 2 * L::VEC_BYTES);
       const float4* vd = vl + L::VEC_BYTES / 16;
-      if (MODE == 1 && !await_all(&bars->y_full[st], (it / L::Y_STAGES) & 1, status)) { ok = false; break; }
+      if (!await_all(&bars->y_full[st], (it / L::Y_STAGES) & 1, status)) { ok = false; break; }
       if (!await_all(&bars->s_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
       uint32_t sv[2][32];
       tmem_ld_32x32(ts, sv[0]);
       tmem_ld_32x32(ts + 32, sv[1]);
       tmem_ld_wait();
-      if (MODE == 0) {
-        tc_fence_before();
-        warp_arrive(&bars->p_full[wg], lane);   // the scores live in registers from here on
-      }
       // Causal mask, applied once to the registers of the tiles that cross the diagonal (element (x row, y col) is
       // kept iff key <= query): a score of -inf turns into a probability and a score gradient of exactly zero.
       const int ypos0 = ti * 64;
-      if ((MODE == 0) ? (ypos0 + 63 > xb * 128) : (ypos0 < xb * 128 + 127)) {
+      if (ypos0 < xb * 128 + 127) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          const bool drop = (MODE == 0) ? (ypos0 + i > xpos) : (xpos > ypos0 + i);
-          if (drop) sv[i / 32][i % 32] = 0xff800000u;
-        }
+        for (int i = 0; i < 64; ++i)
+          if (xpos > ypos0 + i) sv[i / 32][i % 32] = 0xff800000u;
       }
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t pw[16];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          float2 n0 = row_nl, n1 = row_nl;
-          if (MODE == 1) {
-            const float4 l4 = vl[c * 8 + q];
-            n0 = make_float2(l4.x * kNegLog2e, l4.y * kNegLog2e);
-            n1 = make_float2(l4.z * kNegLog2e, l4.w * kNegLog2e);
-          }
+          const float4 l4 = vl[c * 8 + q];
+          const float2 n0 = make_float2(l4.x * kNegLog2e, l4.y * kNegLog2e);
+          const float2 n1 = make_float2(l4.z * kNegLog2e, l4.w * kNegLog2e);
           uint32_t* v = &sv[c][4 * q];
           float2 p0 = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, n0);
           float2 p1 = fma2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl2, n1);
@@ -698,13 +656,11 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
           pw[2 * q] = pack_bf16x2(p0.x, p0.y);
           pw[2 * q + 1] = pack_bf16x2(p1.x, p1.y);
         }
-        if (MODE == 1) tmem_st_32x16(ts + c * 16, pw);
+        tmem_st_32x16(ts + c * 16, pw);
       }
-      if (MODE == 1) {
-        tmem_st_wait();
-        tc_fence_before();
-        warp_arrive(&bars->p_full[wg], lane);
-      }
+      tmem_st_wait();
+      tc_fence_before();
+      warp_arrive(&bars->p_full[wg], lane);
       if (!await_all(&bars->dp_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
       uint32_t dv[2][32];
@@ -716,12 +672,8 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
         uint32_t dw[16];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          float2 d0 = row_dl, d1 = row_dl;
-          if (MODE == 1) {
-            const float4 d4 = vd[c * 8 + q];
-            d0 = make_float2(d4.x, d4.y);
-            d1 = make_float2(d4.z, d4.w);
-          }
+          const float4 d4 = vd[c * 8 + q];
+          float2 d0 = make_float2(d4.x, d4.y), d1 = make_float2(d4.z, d4.w);
           const uint32_t* v = &dv[c][4 * q];
           const uint32_t* p = &sv[c][4 * q];
           d0 = fma2(d0, neg_one, make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])));
@@ -737,20 +689,18 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
       tc_fence_before();
       warp_arrive(&bars->ds_full[wg], lane);
       ti += 2;
-      if (MODE == 1 && ti >= S / 64) ti = 2 * xb + wg;
+      if (ti >= S / 64) ti = 2 * xb + wg;
     }
     if (ok && await_all(&bars->acc_full, 0, status)) {
       // The stationary operands have been read for the last time; their buffers take the gradient tiles.
-      //   MODE 0: dQ, one 64-column half per warp group.  MODE 1: dK by the first group, dV by the second.
+      // dK by the first warp group, dV by the second.
       tc_fence_after();
-      const int acc = MODE == 0 ? 0 : wg;
-      const uint32_t ta = (acc == 0 ? tmem_acc1 : tmem_acc2) + lane_sel;
-      uint8_t* obuf = smem + (acc == 0 ? L::X1_OFF : L::X2_OFF);
-      const int col0 = (MODE == 0 ? hy : Hq + acc * Hkv + g) * HD;
-      const float sc = acc == 0 ? scale : 1.f;
+      const uint32_t ta = (wg == 0 ? tmem_acc1 : tmem_acc2) + lane_sel;
+      uint8_t* obuf = smem + (wg == 0 ? L::X1_OFF : L::X2_OFF);
+      const int col0 = (Hq + wg * Hkv + g) * HD;
+      const float sc = wg == 0 ? scale : 1.f;
 #pragma unroll 1
       for (int h = 0; h < L::HALVES; ++h) {
-        if (MODE == 0 && h != wg) continue;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t r[32], w[16];
@@ -781,6 +731,248 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmap_qkv_x, cons
   }
 }
 
+// The dQ pass: one query tile of one head against 128-key blocks.  With no dV product the scores need not stay in
+// tensor memory, so there is room for 128-wide tiles: S double-buffered, dP whose columns take dS, dQ.  A 128x128x16
+// MMA with both operands in shared memory runs at the arithmetic rate (64 cycles) where two 128x64x16 ones take 96.
+// The MMAs of a block are dQ of i, dP of i + 1, S of i + 2; the two warp groups halve the columns of every block, and
+// the exponentials of block i + 1 run under dQ of i and dP of i + 1.
+template <int HD>
+struct DqSmem {
+  static constexpr int HALVES = HD / 64;
+  static constexpr int TILE = 128 * HD * 2;
+  static constexpr int K_STAGES = 3;               // K is read by S and, two blocks of MMAs later, by dQ
+  static constexpr int X1_OFF = 0;                 // Q; takes the dQ tile at the end
+  static constexpr int X2_OFF = TILE;              // dO
+  static constexpr int K_OFF = 2 * TILE;
+  static constexpr int V_OFF = K_OFF + K_STAGES * TILE;    // 2 stages
+  static constexpr int BAR_OFF = V_OFF + 2 * TILE;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+};
+
+struct DqBars {
+  uint64_t x_full;
+  uint64_t k_full[3], k_empty[3], v_full[2], v_empty[2];
+  uint64_t s_full[2], dp_full, ds_full;
+  uint64_t acc_full;
+  uint32_t tmem_base;
+};
+
+template <int HD>
+__device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const CUtensorMap* tmap_do_x,
+                                            const CUtensorMap* tmap_dqkv, const float* __restrict__ lse,
+                                            const float* __restrict__ delta, int xb, int hy, int b, int S, int Hq,
+                                            int Hkv, float scale, float scale_log2, int* status) {
+  using L = DqSmem<HD>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  DqBars* bars = reinterpret_cast<DqBars*>(smem + L::BAR_OFF);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  const int lane = threadIdx.x & 31;
+  const int g = hy / (Hq / Hkv);
+  const int tok0 = b * S;
+  const int n_blocks = xb + 1;
+
+  if (threadIdx.x == 0) {
+    mbar_init(&bars->x_full, 1);
+    for (int i = 0; i < L::K_STAGES; ++i) {
+      mbar_init(&bars->k_full[i], 1);
+      mbar_init(&bars->k_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->v_full[i], 1);
+      mbar_init(&bars->v_empty[i], 1);
+      mbar_init(&bars->s_full[i], 1);
+    }
+    mbar_init(&bars->dp_full, 1);
+    mbar_init(&bars->ds_full, 8);              // one arrival per softmax warp
+    mbar_init(&bars->acc_full, 1);
+    fence_mbar_init();
+    tma_prefetch_desc(tmap_qkv_x);
+    tma_prefetch_desc(tmap_do_x);
+    tma_prefetch_desc(tmap_dqkv);
+  }
+  if (warp == 9) {
+    tmem_alloc(&bars->tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  // columns: [0,128) S even  [128,256) S odd  [256,384) dP, dS  [384,384+HD) dQ
+
+  if (warp == 8) {
+    // ------------------------------------------------------------- TMA
+    if (lane == 0) {
+      mbar_arrive_expect_tx(&bars->x_full, 2 * L::TILE);
+      for (int h = 0; h < L::HALVES; ++h) {
+        tma_load_2d(smem + L::X1_OFF + h * 16384, tmap_qkv_x, &bars->x_full, hy * HD + 64 * h, tok0 + xb * 128);
+        tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_do_x, &bars->x_full, hy * HD + 64 * h, tok0 + xb * 128);
+      }
+      int kj = 0, vj = 0;
+      for (; vj < n_blocks; ++vj) {
+        if (!await(&bars->k_empty[kj % L::K_STAGES], ((kj / L::K_STAGES) & 1) ^ 1, status)) break;
+        const int ks = kj % L::K_STAGES;
+        mbar_arrive_expect_tx(&bars->k_full[ks], L::TILE);
+        for (int h = 0; h < L::HALVES; ++h)
+          tma_load_2d(smem + L::K_OFF + ks * L::TILE + h * 16384, tmap_qkv_x, &bars->k_full[ks],
+                      (Hq + g) * HD + 64 * h, tok0 + kj * 128);
+        ++kj;
+        if (!await(&bars->v_empty[vj & 1], ((vj >> 1) & 1) ^ 1, status)) break;
+        mbar_arrive_expect_tx(&bars->v_full[vj & 1], L::TILE);
+        for (int h = 0; h < L::HALVES; ++h)
+          tma_load_2d(smem + L::V_OFF + (vj & 1) * L::TILE + h * 16384, tmap_qkv_x, &bars->v_full[vj & 1],
+                      (Hq + Hkv + g) * HD + 64 * h, tok0 + vj * 128);
+      }
+      if (vj < n_blocks) {
+        // Unwinding: wait (bounded) for the copies in flight.
+        await(&bars->x_full, 0, nullptr);
+        for (int j = kj - 1; j >= 0 && j >= kj - L::K_STAGES; --j)
+          await(&bars->k_full[j % L::K_STAGES], (j / L::K_STAGES) & 1, nullptr);
+        for (int j = vj - 1; j >= 0 && j >= vj - 2; --j) await(&bars->v_full[j & 1], (j >> 1) & 1, nullptr);
+      }
+    }
+  } else if (warp == 9) {
+    // ------------------------------------------------------------- MMA
+    constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);
+    constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, false, true);
+    const uint64_t dq = umma_desc_sw128(smem_u32(smem + L::X1_OFF), 16, 1024);
+    const uint64_t ddo = umma_desc_sw128(smem_u32(smem + L::X2_OFF), 16, 1024);
+    const uint64_t dk = umma_desc_sw128(smem_u32(smem + L::K_OFF), 16, 1024);
+    const uint64_t dkn = umma_desc_sw128(smem_u32(smem + L::K_OFF), 16384, 1024);     // MN-major view
+    const uint64_t dv = umma_desc_sw128(smem_u32(smem + L::V_OFF), 16, 1024);
+    auto issue_scores = [&](uint32_t tmem_d, uint64_t dx, uint64_t dy) {
+#pragma unroll
+      for (int ks = 0; ks < HD / 16; ++ks) {
+        const uint32_t off = ((ks / 4) * 16384 + (ks % 4) * 32) >> 4;
+        umma_bf16_ss(tmem_d, dx + off, dy + off, idesc_s, ks > 0 ? 1u : 0u);
+      }
+    };
+    auto s_block = [&](int j) -> bool {
+      const int st = j % L::K_STAGES;
+      if (!await_all(&bars->k_full[st], (j / L::K_STAGES) & 1, status)) return false;
+      tc_fence_after();
+      if (elect_one()) {
+        issue_scores(tmem_base + (j & 1) * 128, dq, dk + (st * L::TILE >> 4));
+        umma_commit(&bars->s_full[j & 1]);
+      }
+      __syncwarp();
+      return true;
+    };
+    auto dp_block = [&](int j) -> bool {
+      if (!await_all(&bars->v_full[j & 1], (j >> 1) & 1, status)) return false;
+      tc_fence_after();
+      if (elect_one()) {
+        issue_scores(tmem_base + 256, ddo, dv + ((j & 1) * L::TILE >> 4));
+        umma_commit(&bars->dp_full);
+        umma_commit(&bars->v_empty[j & 1]);
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = await_all(&bars->x_full, 0, status) && s_block(0) && dp_block(0) && (n_blocks == 1 || s_block(1));
+    for (int i = 0; i < n_blocks && ok; ++i) {
+      ok = await_all(&bars->ds_full, i & 1, status);     // and the scores of block i have been read
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t kn = dkn + ((i % L::K_STAGES) * L::TILE >> 4);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)     // dS of keys 0-63 at columns 256.., of keys 64-127 at 320..
+          umma_bf16_ts(tmem_base + 384, tmem_base + 256 + (ks / 4) * 64 + (ks % 4) * 8, kn + (ks * 2048 >> 4), idesc_acc,
+                       (i == 0 && ks == 0) ? 0u : 1u);
+        umma_commit(&bars->k_empty[i % L::K_STAGES]);
+        if (i == n_blocks - 1) umma_commit(&bars->acc_full);
+      }
+      __syncwarp();
+      if (i + 1 < n_blocks) ok = dp_block(i + 1);
+      if (i + 2 < n_blocks) ok = ok && s_block(i + 2);
+    }
+  } else {
+    // --------------------------------------------------- dS blocks + epilogue
+    const int wg = warp >> 2;                  // key columns [64 wg, 64 wg + 64) of every block
+    const int row = (warp & 3) * 32 + lane;    // query row == TMEM lane
+    const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t td = tmem_base + lane_sel + 256 + wg * 64;
+    const float2 sl2 = make_float2(scale_log2, scale_log2);
+    const long long idx = (static_cast<long long>(b) * Hq + hy) * S + xb * 128 + row;
+    const float nl = lse[idx] * -1.4426950408889634f, ndl = -delta[idx];
+    const float2 nl2 = make_float2(nl, nl), ndl2 = make_float2(ndl, ndl);
+    bool ok = true;
+    for (int j = 0; j < n_blocks; ++j) {
+      if (!await_all(&bars->s_full[j & 1], (j >> 1) & 1, status)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t sv[2][32];
+      tmem_ld_32x32(tmem_base + lane_sel + (j & 1) * 128 + wg * 64, sv[0]);
+      tmem_ld_32x32(tmem_base + lane_sel + (j & 1) * 128 + wg * 64 + 32, sv[1]);
+      tmem_ld_wait();
+      if (j == xb) {
+        // causal mask: a score of -inf turns into a probability and a score gradient of exactly zero
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (wg * 64 + i > row) sv[i / 32][i % 32] = 0xff800000u;
+      }
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        uint32_t* v = &sv[i / 32][i % 32];
+        float2 p = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, nl2);
+        v[0] = __float_as_uint(fast_exp2(p.x));
+        v[1] = __float_as_uint(fast_exp2(p.y));
+      }
+      if (!await_all(&bars->dp_full, j & 1, status)) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t dv[32], dw[16];
+        tmem_ld_32x32(td + c * 32, dv);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float2 d = add2(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), ndl2);
+          d = mul2(d, make_float2(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])));
+          dw[i] = pack_bf16x2(d.x, d.y);
+        }
+        tmem_st_32x16(td + c * 16, dw);        // over columns this thread has already read
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      warp_arrive(&bars->ds_full, lane);
+    }
+    if (ok && wg < L::HALVES && await_all(&bars->acc_full, 0, status)) {
+      // Q has been read for the last time; its buffer takes the dQ tile, one 64-column half per warp group
+      tc_fence_after();
+      const uint32_t ta = tmem_base + lane_sel + 384 + wg * 64;
+      uint8_t* obuf = smem + L::X1_OFF + wg * 16384;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[32], w[16];
+        tmem_ld_32x32(ta + c * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * scale, __uint_as_float(r[2 * i + 1]) * scale);
+        store_row_chunk_sw128(obuf, row, c * 4, w);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d_bulk(tmap_dqkv, obuf + (warp & 3) * 32 * 128, hy * HD + 64 * wg,
+                          tok0 + xb * 128 + (warp & 3) * 32);
+        bulk_commit_group();
+        bulk_wait_group<0>();
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
 // One launch for both passes.  They are independent (dK/dV and dQ go to different columns of d_qkv) and hold a whole
 // SM per CTA; the dK/dV CTAs are few and of very different lengths (with grouped heads up to group x S/64 tiles),
 // so they start first, longest first, and the many shorter dQ CTAs fill the SMs they leave.
@@ -798,13 +990,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 12
   int idx = blockIdx.x;
   if (idx < n_kv) {
     const int hb = idx % (Hkv * B);
-    attn_bwd_cta<HD, 1>(&tmap_qkv_x, &tmap_qkv_y, &tmap_do_x, &tmap_do_y, &tmap_dqkv, lse, delta, idx / (Hkv * B),
-                        hb % Hkv, hb / Hkv, S, Hq, Hkv, scale, scale_log2, status);
+    attn_dkv_cta<HD>(&tmap_qkv_x, &tmap_qkv_y, &tmap_do_y, &tmap_dqkv, lse, delta, idx / (Hkv * B), hb % Hkv, hb / Hkv,
+                     S, Hq, Hkv, scale, scale_log2, status);
   } else {
     idx -= n_kv;
     const int hb = idx % (Hq * B);
-    attn_bwd_cta<HD, 0>(&tmap_qkv_x, &tmap_qkv_y, &tmap_do_x, &tmap_do_y, &tmap_dqkv, lse, delta,
-                        blocks - 1 - idx / (Hq * B), hb % Hq, hb / Hq, S, Hq, Hkv, scale, scale_log2, status);
+    attn_dq_cta<HD>(&tmap_qkv_x, &tmap_do_x, &tmap_dqkv, lse, delta, blocks - 1 - idx / (Hq * B), hb % Hq, hb / Hq, S,
+                    Hq, Hkv, scale, scale_log2, status);
   }
 }
 
@@ -873,16 +1065,17 @@ static int attn_bwd_impl(const void* qkv, const void* out, const void* d_out, co
   if ((rc = make_tmap_2d_bf16(&tdx, d_out, Wo, T, Wo * 2, 64, 128)) != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&tdy, d_out, Wo, T, Wo * 2, 64, 64)) != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&tdq, d_qkv, W, T, W * 2, 64, 32)) != 0) return rc;
+  constexpr int smem = DqSmem<HD>::TOTAL > BwdSmem<HD>::TOTAL ? DqSmem<HD>::TOTAL : BwdSmem<HD>::TOTAL;
   static bool cfg = false;
   if (!cfg) {
-    if (set_smem(attn_bwd_kernel<HD>, BwdSmem<HD>::TOTAL)) return -2;
+    if (set_smem(attn_bwd_kernel<HD>, smem)) return -2;
     cfg = true;
   }
   const long long delta_blocks = (T * Hq * (HD / 8) + 255) / 256;
   attn_delta_kernel<HD><<<static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st>>>(
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, T, S, Hq);
   if (cudaGetLastError() != cudaSuccess) return -3;
-  attn_bwd_kernel<HD><<<static_cast<unsigned>(S / 128 * (Hkv + Hq) * B), BWD_THREADS, BwdSmem<HD>::TOTAL, st>>>(
+  attn_bwd_kernel<HD><<<static_cast<unsigned>(S / 128 * (Hkv + Hq) * B), BWD_THREADS, smem, st>>>(
       tqx, tqy, tdx, tdy, tdq, lse, delta, B, S, Hq, Hkv, softmax_scale, softmax_scale * 1.4426950408889634f, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -564,6 +564,8 @@ def _attention_backward(ctx, dout, _dlse):
     qkv, out, lse = ctx.saved_tensors
     if _is_native(qkv):
         qc = qkv.contiguous()
+        if lse.data_ptr() % 16:            # the kernels copy pieces of it in bulk
+            lse = lse.clone()
         dqkv = torch.empty_like(qc)
         delta = torch.empty((B, Hq, S), dtype=torch.float32, device=qkv.device)
         native.lib().attn_bwd(qc, out, dout.contiguous(), lse, delta, dqkv, B, S, Hq, Hkv, hd, scale,

@@ -194,6 +194,32 @@ def test_attention_fwd_bwd(B, S, Hq, Hkv, hd):
     assert _close(gq[:, (Hq + Hkv) * hd:], gr[:, (Hq + Hkv) * hd:], 3e-2)   # dV
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,hd,growth", [(1, 640, 32, 32, 64, 0.0), (2, 640, 24, 8, 128, 0.0),
+                                                  (1, 768, 32, 8, 128, 40.0), (3, 256, 32, 4, 64, 40.0)])
+def test_attention_paired_tiles(B, S, Hq, Hkv, hd, growth):
+    """More query tiles than SMs, so a CTA takes two: odd tile counts per head (a last CTA with one tile), pairs of
+    heads and pairs of neighbouring query blocks.  ``growth`` makes later keys' scores larger by far more than the
+    rescale threshold, so the accumulated output is rescaled in most blocks."""
+    from piper_b200 import ops
+    from piper_b200.ops.core import _attention_ref
+
+    torch.manual_seed(15)
+    qkv = torch.randn(B * S, (Hq + 2 * Hkv) * hd, device="cuda")
+    ramp = 1.0 + growth * (torch.arange(B * S, device="cuda") % S) / S
+    qkv[:, Hq * hd: (Hq + Hkv) * hd] *= ramp.unsqueeze(1)
+    qkv = qkv.to(torch.bfloat16).requires_grad_(True)
+    out = ops.attention(qkv, B, S, Hq, Hkv, hd)
+    g = torch.randn_like(out)
+    out.backward(g)
+    q2 = qkv.detach().float().requires_grad_(True)
+    ref, _ = _attention_ref(q2, B, S, Hq, Hkv, hd, 1.0 / math.sqrt(hd))
+    ref.backward(g.float())
+    assert _close(out, ref, 2e-2)
+    nq, nk = Hq * hd, Hkv * hd
+    for lo, hi in ((0, nq), (nq, nq + nk), (nq + nk, nq + 2 * nk)):
+        assert _close(qkv.grad[:, lo:hi], q2.grad[:, lo:hi], 3e-2), (lo, hi)
+
+
 @pytest.mark.parametrize("T,V,D", [(64, 1000, 264), (300, 301, 256), (0, 16, 64), (77, 40, 256)])
 def test_embedding_gradient(T, V, D):
     """Compact accumulation into a bf16 table (T < V) and the fp32 table (T >= V); many repeated tokens."""
