@@ -417,12 +417,16 @@ static int forced_tile() {
 int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 0;
   {
-    // 256x256 tiles move a third fewer operand bytes per flop.  Measured on B200: they win for bf16 outputs once
-    // there is at least one tile per SM, and for fp32 (weight-gradient) outputs that are at least as tall as
-    // wide; wide fp32 outputs do a little better with 128x256 tiles and their double-buffered accumulators.
+    // 256x256 tiles move a third fewer operand bytes per flop: measured on B200, they keep the tensor pipe 81 % busy
+    // where 128x256 tiles reach 74 %.  They also come in fewer, larger pieces.  The time is taken as rounds of tiles
+    // over the SMs times the cost of a tile (1 against 0.5 x 81 / 74), and the smaller one runs: 128 big tiles are one
+    // round where 256 small ones are two, and 320 big ones are three where 640 small ones are five.  Wide fp32
+    // (weight-gradient) outputs always take the small tiles: their double-buffered accumulators hide the reduce-adds.
     const int tile = g.tile != 0 ? g.tile : forced_tile();
-    const long long tiles256 = static_cast<long long>((g.M + 255) / 256) * ((g.N + 255) / 256);
-    const bool fits = g.M >= 256 && g.N >= 256 && tiles256 >= num_sms;
+    const long long n_tiles = (g.N + 255) / 256;
+    const long long rounds256 = ((g.M + 255) / 256 * n_tiles + num_sms - 1) / num_sms;
+    const long long rounds128 = ((g.M + 127) / 128 * n_tiles + num_sms - 1) / num_sms;
+    const bool fits = g.M >= 256 && g.N >= 256 && rounds256 * 1000 < rounds128 * 547;
     const bool pays = g.epilogue == kEpiStoreBf16 || g.M >= g.N;
     if (tile == 256 || (tile == 0 && fits && pays))
       return gemm256_bf16_launch(g, num_sms, next_sched_slot(), stream);
