@@ -1,6 +1,6 @@
 """``torch.ops.piper.*``: the traced compute ops of the bundled models.
 
-Each op is a ``torch.library.custom_op`` so that TorchDynamo records it as a
+Each op is registered with the dispatcher (``registry.py``) so that TorchDynamo records it as a
 single FX node (the graph splitter and the schedule see whole ops, never their
 internals), with
 
@@ -35,6 +35,7 @@ import torch
 from torch import Tensor
 
 from . import native
+from .registry import custom_op
 
 # --------------------------------------------------------------------------
 # runtime state consulted by backward formulas
@@ -119,7 +120,7 @@ def _gemm(a: Tensor, b: Tensor, out: Tensor, a_mn: bool, b_mn: bool, accumulate:
     return out
 
 
-@torch.library.custom_op("piper::linear", mutates_args=())
+@custom_op("piper::linear")
 def linear(x: Tensor, w: Tensor) -> Tensor:
     """y[..., N] = x[..., K] @ w[N, K]^T."""
     if _is_native(x):
@@ -176,6 +177,9 @@ def _linear_wgrad(x2: Tensor, dy2: Tensor, w: Tensor) -> Optional[Tensor]:
 # step on one GPU: 3,227 ms (0), 3,180 ms (1), 3,066 ms (2), identical losses.
 _GEMM_FORK = int(os.environ.get("PIPER_GEMM_FORK", "2") or 0)
 _side_streams: dict = {}
+# The fork costs the host two event waits and two stream switches (about 45 us of Python); below this many
+# multiply-adds (some 12 us of GEMM) there is no idle round of tiles worth that.
+_FORK_MIN_MACS = 1 << 33
 
 
 class deferred_join:
@@ -219,7 +223,8 @@ def _linear_backward(ctx, dy):
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     deferred = wgrad_store.active is not None
-    if (_GEMM_FORK and ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and not deferred and _is_native(dy2)):
+    if (_GEMM_FORK and ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and not deferred and _is_native(dy2)
+            and x2.shape[0] * w.numel() >= _FORK_MIN_MACS):
         cur = torch.cuda.current_stream(dy2.device)
         side = _side_stream(cur)
         dw_out = None if grad_sinks.get(w) is not None else torch.empty_like(w)   # allocated on the current stream
@@ -258,7 +263,7 @@ linear.register_autograd(_linear_backward, setup_context=_linear_setup)
 # --------------------------------------------------------------------------
 
 
-@torch.library.custom_op("piper::rmsnorm_fwd", mutates_args=())
+@custom_op("piper::rmsnorm_fwd")
 def rmsnorm_fwd(x: Tensor, w: Tensor, eps: float) -> tuple[Tensor, Tensor]:
     """Returns (y, rstd) with y = x * rsqrt(mean(x^2) + eps) * w computed in fp32."""
     if _is_native(x):
@@ -319,7 +324,7 @@ def _rmsnorm_setup(ctx, inputs, output):
 
 def _rmsnorm_backward(ctx, dy, _drstd):
     x, w, rstd = ctx.saved_tensors
-    dx, dw = _rmsnorm_bwd_impl(dy, x, w, rstd, None)
+    dx, dw = _rmsnorm_bwd_impl(torch.zeros_like(x) if dy is None else dy, x, w, rstd, None)
     return dx, dw, None
 
 
@@ -330,7 +335,7 @@ def rmsnorm(x: Tensor, w: Tensor, eps: float = 1e-6) -> Tensor:
     return rmsnorm_fwd(x, w, eps)[0]
 
 
-@torch.library.custom_op("piper::add_rmsnorm_fwd", mutates_args=())
+@custom_op("piper::add_rmsnorm_fwd")
 def add_rmsnorm_fwd(x: Tensor, res: Tensor, w: Tensor, eps: float) -> tuple[Tensor, Tensor, Tensor]:
     """h = x + res; y = rmsnorm(h) * w.  Returns (y, h, rstd)."""
     if _is_native(x):
@@ -363,7 +368,7 @@ def _add_rmsnorm_setup(ctx, inputs, output):
 def _add_rmsnorm_backward(ctx, dy, dh, _drstd):
     h, w, rstd = ctx.saved_tensors
     if dy is None:
-        return dh, dh, None, None
+        dy = torch.zeros_like(h)
     dres = None if dh is None else dh.contiguous()
     dx, dw = _rmsnorm_bwd_impl(dy, h, w, rstd, dres)
     return dx, dx, dw, None
@@ -378,7 +383,7 @@ def add_rmsnorm(x: Tensor, res: Tensor, w: Tensor, eps: float = 1e-6) -> tuple[T
     return y, h
 
 
-@torch.library.custom_op("piper::residual_add", mutates_args=())
+@custom_op("piper::residual_add")
 def residual_add(a: Tensor, b: Tensor) -> Tensor:
     """a + b for two activations of the same shape (the residual add that is not fused into a norm)."""
     if _is_native(a) and a.dtype == torch.bfloat16 and a.numel() % 8 == 0:
@@ -433,7 +438,7 @@ def _qk_rope_ref(qkv, cos, sin, qw, kw, S, Hq, Hkv, hd, interleaved, eps, sign=1
     return out.reshape(qkv.shape).to(qkv.dtype)
 
 
-@torch.library.custom_op("piper::qk_rope", mutates_args=())
+@custom_op("piper::qk_rope")
 def qk_rope(qkv: Tensor, cos: Tensor, sin: Tensor, qw: Optional[Tensor], kw: Optional[Tensor], S: int,
             Hq: int, Hkv: int, hd: int, interleaved: bool, eps: float) -> Tensor:
     """Applies optional per-head RMSNorm and rotary embedding to the q and k heads of packed qkv."""
@@ -533,7 +538,7 @@ def _attention_ref(qkv: Tensor, B: int, S: int, Hq: int, Hkv: int, hd: int, scal
     return o.transpose(1, 2).reshape(B * S, Hq * hd), lse
 
 
-@torch.library.custom_op("piper::attention_fwd", mutates_args=())
+@custom_op("piper::attention_fwd")
 def attention_fwd(qkv: Tensor, B: int, S: int, Hq: int, Hkv: int, hd: int, scale: float) -> tuple[Tensor, Tensor]:
     """Causal grouped-query attention.  qkv: [B*S, (Hq+2Hkv)*hd] -> (out [B*S, Hq*hd], lse [B,Hq,S])."""
     if _is_native(qkv):
@@ -562,6 +567,8 @@ def _attention_setup(ctx, inputs, output):
 def _attention_backward(ctx, dout, _dlse):
     B, S, Hq, Hkv, hd, scale = ctx.cfg
     qkv, out, lse = ctx.saved_tensors
+    if dout is None:
+        dout = torch.zeros_like(out)
     if _is_native(qkv):
         qc = qkv.contiguous()
         if lse.data_ptr() % 16:            # the kernels copy pieces of it in bulk
@@ -590,7 +597,7 @@ def attention(qkv: Tensor, B: int, S: int, Hq: int, Hkv: int, hd: int, scale: Op
 # --------------------------------------------------------------------------
 
 
-@torch.library.custom_op("piper::swiglu", mutates_args=())
+@custom_op("piper::swiglu")
 def swiglu(h13: Tensor) -> Tensor:
     """act = silu(h13[..., :F]) * h13[..., F:]."""
     F = h13.shape[-1] // 2
@@ -634,7 +641,7 @@ swiglu.register_autograd(_swiglu_backward, setup_context=_swiglu_setup)
 # --------------------------------------------------------------------------
 
 
-@torch.library.custom_op("piper::embedding", mutates_args=())
+@custom_op("piper::embedding")
 def embedding(tokens: Tensor, table: Tensor) -> Tensor:
     if _is_native(table):
         _require_bf16(table)
@@ -687,7 +694,7 @@ embedding.register_autograd(_embedding_backward, setup_context=_embedding_setup)
 # --------------------------------------------------------------------------
 
 
-@torch.library.custom_op("piper::cross_entropy_fwd", mutates_args=())
+@custom_op("piper::cross_entropy_fwd")
 def cross_entropy_fwd(logits: Tensor, labels: Tensor, ignore_index: int) -> tuple[Tensor, Tensor]:
     """Per-token loss [T] (fp32) and log-sum-exp [T] of logits [T, V]."""
     if _is_native(logits):
@@ -719,6 +726,8 @@ def _ce_setup(ctx, inputs, output):
 
 def _ce_backward(ctx, dloss, _dlse):
     logits, labels, lse = ctx.saved_tensors
+    if dloss is None:
+        dloss = torch.zeros_like(lse)
     if _is_native(logits):
         # The kernel takes one scalar scale; per-token upstream gradients other
         # than a broadcast scalar take the PyTorch expression below.
@@ -751,3 +760,14 @@ def cross_entropy(logits: Tensor, labels: Tensor, ignore_index: int = -100, redu
         return loss.sum()
     n = (lb != ignore_index).sum().clamp(min=1)
     return loss.sum() / n
+
+# The registered overloads are what programs call and tracers record.
+linear = linear.overload
+rmsnorm_fwd = rmsnorm_fwd.overload
+add_rmsnorm_fwd = add_rmsnorm_fwd.overload
+residual_add = residual_add.overload
+qk_rope = qk_rope.overload
+attention_fwd = attention_fwd.overload
+swiglu = swiglu.overload
+embedding = embedding.overload
+cross_entropy_fwd = cross_entropy_fwd.overload

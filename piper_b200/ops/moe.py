@@ -21,6 +21,7 @@ import torch
 from torch import Tensor
 
 from . import core, native
+from .registry import custom_op
 from .core import _is_native, _require_bf16, grad_sinks, wgrad_store
 
 PAD = 128
@@ -44,7 +45,7 @@ def row_capacity(tokens: int, k: int, experts: int) -> int:
 
 
 # ------------------------------------------------------------------ router
-@torch.library.custom_op("piper::moe_route", mutates_args=())
+@custom_op("piper::moe_route")
 def moe_route(logits: Tensor, k: int, renorm: bool) -> tuple[Tensor, Tensor, Tensor]:
     """softmax over experts, top-k, optional renormalisation -> (weights fp32 [T,k], idx int32 [T,k], counts int32 [E])."""
     T, E = logits.shape
@@ -98,7 +99,7 @@ moe_route.register_autograd(_route_backward, setup_context=_route_setup)
 
 
 # -------------------------------------------------------------- group table
-@torch.library.custom_op("piper::moe_group_table", mutates_args=())
+@custom_op("piper::moe_group_table")
 def moe_group_table(counts: Tensor, expert_weights: Tensor) -> tuple[Tensor, Tensor]:
     """counts [G] int32 (source-major) -> (g_start, g_len): padded segments laid out back to back.
 
@@ -125,7 +126,7 @@ def _(counts, expert_weights):
 
 
 # ---------------------------------------------------------------- dispatch
-@torch.library.custom_op("piper::moe_dispatch", mutates_args=())
+@custom_op("piper::moe_dispatch")
 def moe_dispatch(x: Tensor, idx: Tensor, counts: Tensor) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
     """x [T, D] -> (rows [cap, D], pos int32 [T*k], g_start int32 [E], g_len int32 [E], ep_counts int32 [E]).
 
@@ -204,7 +205,7 @@ def _grouped_ref_segments(g_start: Tensor, g_len: Tensor):
     return [(g, s, s + n) for g, (s, n) in enumerate(zip(gs, gl)) if n > 0]
 
 
-@torch.library.custom_op("piper::grouped_linear", mutates_args=())
+@custom_op("piper::grouped_linear")
 def grouped_linear(rows: Tensor, w: Tensor, g_start: Tensor, g_len: Tensor) -> Tensor:
     """out[r] = rows[r] @ w[expert(group of r)]^T for w [experts, N, K]; rows outside every group are undefined."""
     E, N, K = w.shape
@@ -291,7 +292,7 @@ grouped_linear.register_autograd(_glinear_backward, setup_context=_glinear_setup
 
 
 # ----------------------------------------------------------------- combine
-@torch.library.custom_op("piper::moe_combine", mutates_args=())
+@custom_op("piper::moe_combine")
 def moe_combine(rows: Tensor, pos: Tensor, weights: Tensor, g_start: Tensor, g_len: Tensor, counts: Tensor) -> Tensor:
     """out[t] = sum_j weights[t, j] * rows[pos[t*k + j]]."""
     T, k = weights.shape
@@ -333,3 +334,10 @@ def _combine_backward(ctx, dout):
 
 
 moe_combine.register_autograd(_combine_backward, setup_context=_combine_setup)
+
+# The registered overloads are what programs call and tracers record.
+moe_route = moe_route.overload
+moe_group_table = moe_group_table.overload
+moe_dispatch = moe_dispatch.overload
+grouped_linear = grouped_linear.overload
+moe_combine = moe_combine.overload

@@ -1,0 +1,58 @@
+"""The op registration against what programs rely on: dispatch modes, fake tensors, saved-tensor hooks, keyword calls,
+gradients of single outputs."""
+import pytest
+import torch
+
+from piper_b200 import ops
+from piper_b200.ops import core, moe
+
+
+def test_ops_are_single_dispatcher_calls_and_hooks_see_their_saved_tensors():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    seen = []
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    x, w = torch.randn(4, 16, requires_grad=True), torch.randn(8, 16, requires_grad=True)
+    packed = []
+    with Mode(), torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t.shape), t)[1], lambda t: t):
+        y = ops.linear(x=x, w=w)
+    assert seen.count("piper.linear.default") == 1 and packed == [x.shape, w.shape]
+    y.sum().backward()
+    assert torch.allclose(w.grad, x.detach().sum(0).expand(8, 16)) and x.grad is not None
+    with torch.no_grad():
+        assert not ops.linear(x, w).requires_grad
+    torch.library.opcheck(torch.ops.piper.linear.default, (x, w))
+    torch.library.opcheck(torch.ops.piper.rmsnorm_fwd.default, (x, torch.randn(16, requires_grad=True), 1e-5))
+
+
+def test_full_graph_capture_records_the_op():
+    x, w = torch.randn(4, 16, requires_grad=True), torch.randn(16)
+    for backend in ("eager", "aot_eager"):
+        f = torch.compile(lambda a: ops.rmsnorm(a, w, 1e-5).sum(), backend=backend, fullgraph=True)
+        assert torch.allclose(f(x), ops.rmsnorm(x, w, 1e-5).sum())
+
+
+@pytest.mark.parametrize("pick", [0, 1, 2])
+def test_gradients_of_one_output_alone(pick):
+    """Outputs that a program did not use send no gradient: the formula sees zeros in their place."""
+    x, r, w = torch.randn(4, 16, requires_grad=True), torch.randn(4, 16), torch.randn(16)
+    out = core.add_rmsnorm_fwd(x, r, w, 1e-5)[pick]
+    (g,) = torch.autograd.grad(out.sum(), x)
+    h = (x.detach() + r).requires_grad_(True)
+    rstd = torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-5)
+    want = torch.autograd.grad([h * rstd * w, h][pick].sum(), h)[0] if pick < 2 else torch.zeros_like(x)
+    assert torch.allclose(g, want, atol=1e-5)
+    qkv = torch.randn(128, 3 * 64, requires_grad=True)
+    o, lse = core.attention_fwd(qkv, 1, 128, 1, 1, 64, 0.125)
+    assert torch.isfinite(torch.autograd.grad((o if pick else lse).sum(), qkv)[0]).all()
+
+
+def test_integer_outputs_carry_no_gradient():
+    counts = torch.tensor([3, 5], dtype=torch.int32)
+    start, length = moe.moe_group_table(counts, torch.randn(2, 4, 4, requires_grad=True))
+    assert not start.requires_grad and length.tolist() == [128, 128]
