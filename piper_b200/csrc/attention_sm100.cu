@@ -72,7 +72,8 @@ __device__ __forceinline__ void store_row_chunk_sw128(uint8_t* tile, int row, in
 // row maximum has grown by more than 2^kRescaleLog2 (the row sums use the same, possibly stale, maximum).
 // Tiles of one kv head are numbered query block major, so a pair is two heads of the group on the same rows where
 // the group is even, and neighbouring query blocks otherwise.
-// One CTA per 128 query rows, probabilities through shared memory: 254 us at S = 4096, 32 q / 8 kv heads.
+// S = 4096, 32 q / 8 kv heads x 128: 254 us with one CTA per 128 query rows and probabilities through shared memory,
+// 122 us so (tensor pipe 58 % busy).
 //
 // Warps 0-3: softmax of tile A, 4-7: of tile B (one query row per thread, row == TMEM lane); 8: TMA; 9: MMA.
 constexpr int FWD_THREADS = 320;
@@ -417,8 +418,8 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 // each group has the MMAs of two tiles' time for its work; warp 8: TMA, warp 9: MMA.  P' and dS' (bf16) replace their
 // own fp32 scores in tensor memory and are the A operand of the accumulating MMAs from there: no thread writes shared
 // memory in the loop.  Bound by the MMAs: a 128x64x16 one with both operands in shared memory reads 6 KiB (48 cycles)
-// for 32 cycles of arithmetic.  Both passes with probabilities through shared memory, two launches on two streams:
-// 751 us at S = 4096, 32 q / 8 kv heads x 128.
+// for 32 cycles of arithmetic.  Both passes at S = 4096, 32 q / 8 kv heads x 128: 751 us with probabilities through
+// shared memory in two launches on two streams, 427 us so with dQ on 64-row tiles as well, 379 us with dQ as below.
 constexpr int BWD_THREADS = 320;
 
 template <int HD>

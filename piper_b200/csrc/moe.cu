@@ -52,7 +52,8 @@ __device__ __forceinline__ void token_softmax(const __nv_bfloat16* row, int E, i
 
 // Bound by the serial chain of k arg-max rounds: probabilities are compared as integers (same order for values >= 0,
 // and a NaN stays selectable instead of selecting nothing), so a round is two warp reductions in hardware; lane j
-// keeps the j-th choice and the k results are written, and counted, at once.
+// keeps the j-th choice and the k results are written, and counted, at once.  4096 tokens, 128 experts, top 8:
+// 17 us with ten shuffles a round and one lane writing, 10 us so.
 template <int SLOTS>
 __global__ void route_kernel(const __nv_bfloat16* __restrict__ logits, float* __restrict__ weights,
                              int* __restrict__ idx, int* __restrict__ counts, long long T, int E, int k,
@@ -177,7 +178,8 @@ __device__ __forceinline__ void zero_padding(__nv_bfloat16* __restrict__ rows, c
 }
 
 // One warp per token: the first k lanes claim the rows of its entries together, then the token row is read once and
-// written k times; the CTAs behind the tokens' clear the padding rows of the segments.
+// written k times; the CTAs behind the tokens' clear the padding rows of the segments.  4096 tokens x 2048, top 8 of 128:
+// 33 us + 10 us of clearing in a launch of its own, 39 us together (170 MB written).
 __global__ void __launch_bounds__(ROW_THREADS)
 permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx, const int* __restrict__ g_start,
                const int* __restrict__ g_len, const int* __restrict__ counts, int* __restrict__ cursor,
@@ -241,6 +243,7 @@ __device__ __forceinline__ void token_rows(const int* __restrict__ pos, long lon
 }
 
 // out[t] = sum_j weights[t, j] * rows[pos[t, j]] (weights == nullptr: plain sum); K entries at a time, any k.
+// 4096 tokens x 2048, top 8: 50 us with one row in flight per lane, 32 us (4.7 TB/s) with eight.
 template <int K>
 __global__ void __launch_bounds__(ROW_THREADS)
 gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ pos,
@@ -290,7 +293,8 @@ gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict_
 }
 
 // drows[pos[t, j]] = weights[t, j] * dout[t], dweights[t, j] = <rows[pos[t, j]], dout[t]>; K entries share one read
-// of dout.  The CTAs behind the tokens' clear the padding rows of drows.
+// of dout.  The CTAs behind the tokens' clear the padding rows of drows.  4096 tokens x 2048, top 8: 59 us + 10 us of
+// clearing with one row at a time, 49 us together.
 template <int K>
 __global__ void __launch_bounds__(ROW_THREADS)
 combine_bwd_kernel(const __nv_bfloat16* __restrict__ rows, const __nv_bfloat16* __restrict__ dout,
