@@ -120,6 +120,40 @@ def test_linear_op_autograd():
     assert _close(w.grad, wr.grad, 1e-2)
 
 
+@pytest.mark.parametrize("M,N,K", [(2048, 4096, 128), (4096, 5120, 64), (1000, 8192, 72), (257, 256, 64)])
+def test_gemm_tile_choice_does_not_change_the_result(M, N, K):
+    """Shapes on both sides of the tile rule (one round of big tiles, three rounds against five, ragged, tiny): the
+    chosen kernel gives the bits of either tile, in both output types."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(19)
+    lib, st = native.lib(), native.status_tensor()
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    for dtype in (torch.bfloat16, torch.float32):
+        auto, small, big = (torch.empty(M, N, device="cuda", dtype=dtype) for _ in range(3))
+        lib.gemm(a, b, auto, False, False, False, st)
+        lib.gemm_tiled(a, b, small, False, False, False, st, 128)
+        lib.gemm_tiled(a, b, big, False, False, False, st, 256)
+        assert torch.equal(auto, small) and torch.equal(auto, big)
+
+
+@pytest.mark.parametrize("T", [4095, 4096])
+def test_linear_gradients_around_the_fork_threshold(T):
+    """2048 x 1024 weights: 4096 rows are the first size whose weight-gradient GEMM runs on the side stream."""
+    from piper_b200 import ops
+    from piper_b200.ops import core
+
+    assert (T * 2048 * 1024 >= core._FORK_MIN_MACS) == (T == 4096)
+    torch.manual_seed(20)
+    x = torch.randn(T, 1024, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    w = (torch.randn(2048, 1024, device="cuda", dtype=torch.bfloat16) * 0.05).requires_grad_(True)
+    g = torch.randn(T, 2048, device="cuda", dtype=torch.bfloat16)
+    ops.linear(x, w).backward(g)
+    assert _close(x.grad, g.float() @ w.detach().float(), 1e-2)
+    assert _close(w.grad, g.float().t() @ x.detach().float(), 1e-2)
+
+
 @pytest.mark.parametrize("T,D", [(300, 256), (300, 2048), (1000, 4096), (300, 8192), (7, 4096)])
 def test_rmsnorm_and_residual(T, D):
     from piper_b200 import ops
