@@ -80,6 +80,8 @@ def _route_setup(ctx, inputs, output):
 
 def _route_backward(ctx, dw, _didx, _dcounts):
     logits, idx, w = ctx.saved_tensors
+    if dw is None:
+        dw = torch.zeros_like(w)
     if _is_native(logits):
         d = torch.empty_like(logits, memory_format=torch.contiguous_format)
         native.lib().moe_route_bwd(logits.contiguous(), idx, w, dw.contiguous().float(), d, ctx.renorm)
@@ -175,13 +177,15 @@ def _(x, idx, counts):
 def _dispatch_setup(ctx, inputs, output):
     x, idx, _counts = inputs
     ctx.k = idx.shape[1]
-    ctx.xshape = x.shape
+    ctx.xshape, ctx.xdtype = x.shape, x.dtype
     ctx.save_for_backward(output[1])
 
 
 def _dispatch_backward(ctx, drows, _dpos, _dgs, _dgl, _dec):
     (pos,) = ctx.saved_tensors
     T, D = ctx.xshape
+    if drows is None:
+        return torch.zeros((T, D), dtype=ctx.xdtype, device=pos.device), None, None
     if _is_native(drows):
         dx = torch.empty((T, D), dtype=drows.dtype, device=drows.device)
         native.lib().moe_permute_bwd(drows.contiguous(), pos, dx, ctx.k)

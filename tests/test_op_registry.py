@@ -2,6 +2,7 @@
 gradients of single outputs."""
 import pytest
 import torch
+import torch.utils.checkpoint
 
 from piper_b200 import ops
 from piper_b200.ops import core, moe
@@ -57,3 +58,56 @@ def test_integer_outputs_carry_no_gradient():
     counts = torch.tensor([3, 5], dtype=torch.int32)
     start, length = moe.moe_group_table(counts, torch.randn(2, 4, 4, requires_grad=True))
     assert not start.requires_grad and length.tolist() == [128, 128]
+
+
+class _Drop(torch.autograd.Function):
+    """A consumer that sends no gradient back."""
+
+    @staticmethod
+    def forward(ctx, y):
+        return y.sum() * 0.0
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def _one_output_calls():
+    T, E, k, D = 6, 4, 2, 16
+    idx = torch.rand(T, E).argsort(1)[:, :k].to(torch.int32).contiguous()
+    counts = torch.bincount(idx.reshape(-1).long(), minlength=E).to(torch.int32)
+    rows, pos, g_start, g_len, _ = moe.moe_dispatch(torch.randn(T, D), idx, counts)
+    cos, sin = torch.randn(T, 32), torch.randn(T, 32)
+    return {
+        "linear": (core.linear, [(T, D), (8, D)]),
+        "rmsnorm": (lambda x, w: core.rmsnorm_fwd(x, w, 1e-5)[0], [(T, D), (D,)]),
+        "add_rmsnorm": (lambda x, r, w: core.add_rmsnorm_fwd(x, r, w, 1e-5)[0], [(T, D), (T, D), (D,)]),
+        "residual_add": (core.residual_add, [(T, D), (T, D)]),
+        "qk_rope": (lambda x, q, k_: core.qk_rope(x, cos, sin, q, k_, T, 1, 1, 64, False, 1e-5),
+                    [(T, 192), (64,), (64,)]),
+        "attention": (lambda x: core.attention_fwd(x, 1, 128, 1, 1, 64, 0.1)[0], [(128, 192)]),
+        "swiglu": (core.swiglu, [(T, D)]),
+        "embedding": (lambda t: core.embedding(torch.arange(T), t), [(9, D)]),
+        "cross_entropy": (lambda x: core.cross_entropy_fwd(x, torch.zeros(T, dtype=torch.long), -100)[0], [(T, D)]),
+        "moe_route": (lambda x: moe.moe_route(x, k, True)[0], [(T, E)]),
+        "moe_dispatch": (lambda x: moe.moe_dispatch(x, idx, counts)[0], [(T, D)]),
+        "grouped_linear": (lambda r, w: moe.grouped_linear(r, w, g_start, g_len), [tuple(rows.shape), (E, 8, D)]),
+        "moe_combine": (lambda r, w: moe.moe_combine(r, pos, w, g_start, g_len, counts), [tuple(rows.shape), (T, k)]),
+    }
+
+
+@pytest.mark.parametrize("name", sorted(_one_output_calls()))
+def test_a_gradient_that_does_not_arrive_counts_as_zeros(name):
+    fn, shapes = _one_output_calls()[name]
+    args = [torch.randn(s, requires_grad=True) for s in shapes]
+    _Drop.apply(fn(*args)).backward()
+    for a in args:
+        assert a.grad is not None and a.grad.shape == a.shape and a.grad.dtype == a.dtype and not a.grad.any()
+
+
+def test_reentrant_checkpoint_over_a_block_that_only_detaches_its_input():
+    x, w = torch.randn(4, 16, requires_grad=True), torch.randn(8, 16, requires_grad=True)
+    q = torch.randn(3, requires_grad=True)
+    out = torch.utils.checkpoint.checkpoint(lambda y, z: z * 2 + y.detach().sum(), core.linear(x, w), q, use_reentrant=True)
+    out.sum().backward()
+    assert not x.grad.any() and not w.grad.any() and torch.equal(q.grad, torch.full((3,), 2.0))
