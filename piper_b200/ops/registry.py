@@ -13,29 +13,42 @@ without a gradient in every pass, filling them all would cost launches, so its f
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Callable, Optional
 
 import torch
 
-_lib = torch.library.Library("piper", "FRAGMENT")
 _below_autograd = torch._C._AutoDispatchBelowAutograd
+# One library per op, kept over a reload of this module: defining an op again replaces it.
+_libs: dict = globals().get("_libs", {})
 
 
 class Op:
-    """What ``custom_op`` returns: callable like the op, with the registration decorators."""
+    """What ``custom_op`` returns.  The registration methods of ``torch.library.custom_op`` objects are also attributes of
+    ``overload``, the callable that the op modules export."""
 
     def __init__(self, name: str, body: Callable) -> None:
-        self.name = name
-        schema = torch.library.infer_schema(body, mutates_args=())
-        _lib.define(name + schema, tags=(torch.Tag.pt2_compliant_tag,))
+        self.name, self.qualname = name, "piper::" + name
+        self._kernels: dict = {}
+        self._formula: Optional[Callable] = None
+        stale = _libs.pop(name, None)
+        if stale is not None:
+            stale._destroy()
+        self._lib = _libs[name] = torch.library.Library("piper", "FRAGMENT")
+        self._body = body
+        self._lib.define(name + torch.library.infer_schema(body, mutates_args=()),
+                         tags=(torch.Tag.pt2_compliant_tag,))
+        self._lib.impl(name, body, "CompositeExplicitAutograd")
         self.overload = getattr(torch.ops.piper, name).default
-        _lib.impl(name, body, "CompositeExplicitAutograd")
+        for method in ("register_autocast", "register_autograd", "register_effect", "register_fake", "register_kernel",
+                       "register_torch_dispatch", "register_vmap", "set_kernel_enabled"):
+            setattr(self.overload, method, getattr(self, method))
 
     def register_fake(self, fn: Callable) -> Callable:
-        torch.library.register_fake("piper::" + self.name, fn, lib=_lib)
+        torch.library.register_fake(self.qualname, fn, lib=self._lib, allow_override=True)
         return fn
 
-    def register_autograd(self, backward: Callable, setup_context: Optional[Callable] = None) -> None:
+    def register_autograd(self, backward: Callable, *, setup_context: Optional[Callable] = None) -> None:
         """``backward(ctx, *grads)`` returns a gradient per input; see above for gradients that did not arrive."""
         overload = self.overload
         one_output = len(overload._schema.returns) == 1
@@ -53,15 +66,56 @@ class Op:
 
         Formula.backward = staticmethod(backward)
         Formula.__name__ = Formula.__qualname__ = f"piper_{self.name}"
-        apply = Formula.apply
+        registered, self._formula = self._formula is not None, Formula.apply
+        if registered:
+            return
 
         def autograd(*args):
             if torch.is_grad_enabled() and any(isinstance(a, torch.Tensor) and a.requires_grad for a in args):
-                return apply(*args)
+                return self._formula(*args)
             with _below_autograd():
                 return overload(*args)
 
-        _lib.impl(self.name, autograd, "Autograd")
+        self._lib.impl(self.name, autograd, "Autograd")
+
+    def register_kernel(self, device_types, func: Optional[Callable] = None) -> Callable:
+        """A body for one device type, several, or (None) all, in place of the general one."""
+        if func is None:
+            return lambda f: self.register_kernel(device_types, f)
+        if device_types is None or isinstance(device_types, str):
+            device_types = ("cpu", "cuda") if device_types is None else (device_types,)
+        for device in device_types:
+            known = device in self._kernels
+            self._kernels[device] = func
+            if not known:
+                torch.library.register_kernel(
+                    self.overload, device, lambda *args, _d=device: (self._kernels[_d] or self._body)(*args),
+                    lib=self._lib)
+        return func
+
+    @contextlib.contextmanager
+    def set_kernel_enabled(self, device_type: str, enabled: bool = True):
+        """Scope in which a device's registered kernel is used or the general body in its place."""
+        before = self._kernels.get(device_type)
+        if before is not None and not enabled:
+            self._kernels[device_type] = None
+        try:
+            yield
+        finally:
+            if before is not None:
+                self._kernels[device_type] = before
+
+    def register_vmap(self, func: Optional[Callable] = None):
+        return torch.library.register_vmap(self.overload, func, lib=self._lib)
+
+    def register_torch_dispatch(self, torch_dispatch_class, fn: Optional[Callable] = None):
+        return torch.library.register_torch_dispatch(self.qualname, torch_dispatch_class, fn, lib=self._lib)
+
+    def register_autocast(self, device_type: str, cast_inputs: torch.dtype):
+        return torch.library.register_autocast(self.overload, device_type, cast_inputs, lib=self._lib)
+
+    def register_effect(self, effect) -> None:
+        torch.library._register_effectful_op(self.qualname, effect)
 
 
 def custom_op(qualname: str) -> Callable[[Callable], Op]:

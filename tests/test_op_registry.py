@@ -1,5 +1,8 @@
 """The op registration against what programs rely on: dispatch modes, fake tensors, saved-tensor hooks, keyword calls,
 gradients of single outputs."""
+import subprocess
+import sys
+
 import pytest
 import torch
 import torch.utils.checkpoint
@@ -111,3 +114,47 @@ def test_reentrant_checkpoint_over_a_block_that_only_detaches_its_input():
     out = torch.utils.checkpoint.checkpoint(lambda y, z: z * 2 + y.detach().sum(), core.linear(x, w), q, use_reentrant=True)
     out.sum().backward()
     assert not x.grad.any() and not w.grad.any() and torch.equal(q.grad, torch.full((3,), 2.0))
+
+
+_MODULE_CHANGES = """
+import importlib, torch
+from piper_b200 import ops
+from piper_b200.ops import core, moe, registry
+x, w = torch.randn(4, 16, requires_grad=True), torch.randn(8, 16, requires_grad=True)
+want = (x @ w.t()).detach()
+before = ops.linear
+for module in (registry, core, moe):
+    importlib.reload(module)
+for f in (before, core.linear, torch.ops.piper.linear):
+    x.grad = None
+    y = f(x, w)
+    y.sum().backward()
+    assert torch.allclose(y, want) and torch.allclose(x.grad, w.detach().sum(0).expand(4, 16))
+start, length = moe.moe_group_table(torch.tensor([3, 5], dtype=torch.int32), torch.randn(2, 4, 4))
+assert length.tolist() == [128, 128]
+
+op = core.linear
+op.register_kernel("cpu", lambda a, b: a @ b.t() + 1)
+assert torch.allclose(op(x, w), want + 1)
+with op.set_kernel_enabled("cpu", False):
+    assert torch.allclose(op(x, w), want)
+op.register_kernel(None)(lambda a, b: a @ b.t() + 2)
+assert torch.allclose(op(x, w), want + 2)
+op.register_autocast("cpu", torch.bfloat16)
+with torch.autocast("cpu", dtype=torch.bfloat16):
+    assert op(x, w).dtype == torch.bfloat16
+op.register_vmap(lambda info, dims, a, b: (a * 3, dims[0]))
+assert torch.equal(torch.func.vmap(op, in_dims=(0, None))(x.detach()[None], w.detach()), x.detach()[None] * 3)
+op.register_fake(lambda a, b: a.new_empty(7))
+with torch._subclasses.FakeTensorMode():
+    assert op(torch.empty(4, 16), torch.empty(8, 16)).shape == (7,)
+op.register_autograd(lambda ctx, g: (torch.full((4, 16), 5.0), None))
+x.grad = None
+op(x, w).sum().backward()
+assert (x.grad == 5).all()
+"""
+
+
+def test_op_modules_reload_and_ops_take_further_registrations():
+    """In a process of its own: both change the ops for everything after them."""
+    subprocess.run([sys.executable, "-c", _MODULE_CHANGES], check=True, timeout=300)
