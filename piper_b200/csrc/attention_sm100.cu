@@ -68,16 +68,17 @@ __device__ __forceinline__ void store_row_chunk_sw128(uint8_t* tile, int row, in
 // cycles of MMA and 1,024 cycles of ex2 (16 per cycle and SM).  A CTA therefore works on two query tiles (A, B) that
 // share one K/V stream: while four softmax warps turn the scores of one tile into probabilities, the MMAs of the
 // other tile run.  The probabilities go back to the tensor memory columns of their scores and feed P V from there, so
-// no thread writes shared memory in the loop; the output accumulates in tensor memory and is rescaled only when a
-// row maximum has grown by more than 2^kRescaleLog2 (the row sums use the same, possibly stale, maximum).
+// no thread writes shared memory in the loop; the output accumulates in tensor memory and is rescaled in every block in
+// which a row maximum of the warp has grown.  (Letting the maximum go stale until it has grown by 2^8 saves 8-15 % of
+// the time, but the largest probability of a row is then rounded to bf16 where it is exactly 1 otherwise: error against
+// 64 bits 2.05e-3 -> 2.09e-3 at S = 4096.)
 // Tiles of one kv head are numbered query block major, so a pair is two heads of the group on the same rows where
 // the group is even, and neighbouring query blocks otherwise.
-// S = 4096, 32 q / 8 kv heads x 128: 254 us with one CTA per 128 query rows and probabilities through shared memory,
-// 122 us so (tensor pipe 58 % busy).
+// S = 4096, 32 q / 8 kv heads x 128: 237 us with one CTA per 128 query rows and probabilities through shared memory,
+// 127 us so; S = 8192, 32 / 8 x 64: 745 and 421 us.
 //
 // Warps 0-3: softmax of tile A, 4-7: of tile B (one query row per thread, row == TMEM lane); 8: TMA; 9: MMA.
 constexpr int FWD_THREADS = 320;
-constexpr float kRescaleLog2 = 8.f;      // probabilities stay below 2^8 of the stale maximum: no range is lost
 
 template <int HD>
 struct FwdSmem {
@@ -302,24 +303,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         mx[c] = fmaxf(mx[c], __uint_as_float(sv[c][31]));
       }
       const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      float alpha = 1.f;
+      bool grown = false;
       if (j == 0) {
         m_run = m_blk;
-      } else if (__any_sync(0xffffffffu, (m_blk - m_run) * scale_log2 > kRescaleLog2)) {
+      } else if ((grown = __any_sync(0xffffffffu, m_blk > m_run))) {
         const float m_new = fmaxf(m_run, m_blk);
-        const float alpha = fast_exp2((m_run - m_new) * scale_log2);
+        alpha = fast_exp2((m_run - m_new) * scale_log2);
         l_run *= alpha;
         m_run = m_new;
-        // P V of block j - 1 is complete: the commit behind s_full of block j came after it
-#pragma unroll 1
-        for (int c = 0; c < HD / 16; ++c) {
-          uint32_t r[16];
-          tmem_ld_32x16(to + c * 16, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-          tmem_st_32x16(to + c * 16, r);
-        }
-        tmem_st_wait();
       }
       const float2 sl2 = make_float2(scale_log2, scale_log2);
       const float msc = m_run * scale_log2;
@@ -337,6 +329,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
           w[i] = pack_bf16x2(p.x, p.y);
         }
         tmem_st_32x16(ts + c * 16, w);
+        if (c == 1 && grown) {
+          // Here rather than before the exponentials: half of the scores' registers are free for the loads, and the
+          // first half of the probabilities waits for it in any case.  P V of block j - 1 is complete: the commit
+          // behind s_full of block j came after it.
+#pragma unroll 1
+          for (int h = 0; h < HD / 64; ++h) {
+            uint32_t r[2][32];
+            tmem_ld_32x32(to + h * 64, r[0]);
+            tmem_ld_32x32(to + h * 64 + 32, r[1]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 64; ++i) r[i / 32][i % 32] = __float_as_uint(__uint_as_float(r[i / 32][i % 32]) * alpha);
+            tmem_st_32x32(to + h * 64, r[0]);
+            tmem_st_32x32(to + h * 64 + 32, r[1]);
+          }
+        }
         if (c & 1) {
           tmem_st_wait();
           tc_fence_before();

@@ -232,8 +232,8 @@ def test_attention_fwd_bwd(B, S, Hq, Hkv, hd):
                                                   (1, 768, 32, 8, 128, 40.0), (3, 256, 32, 4, 64, 40.0)])
 def test_attention_paired_tiles(B, S, Hq, Hkv, hd, growth):
     """More query tiles than SMs, so a CTA takes two: odd tile counts per head (a last CTA with one tile), pairs of
-    heads and pairs of neighbouring query blocks.  ``growth`` makes later keys' scores larger by far more than the
-    rescale threshold, so the accumulated output is rescaled in most blocks."""
+    heads and pairs of neighbouring query blocks.  ``growth`` makes later keys' scores larger, so the accumulated output
+    is rescaled by small factors in most blocks."""
     from piper_b200 import ops
     from piper_b200.ops.core import _attention_ref
 
@@ -252,6 +252,31 @@ def test_attention_paired_tiles(B, S, Hq, Hkv, hd, growth):
     nq, nk = Hq * hd, Hkv * hd
     for lo, hi in ((0, nq), (nq, nq + nk), (nq + nk, nq + 2 * nk)):
         assert _close(qkv.grad[:, lo:hi], q2.grad[:, lo:hi], 3e-2), (lo, hi)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_largest_probability_is_exact(hd):
+    """One key of the second block beats every earlier one by 2^0.1 to 2^7.9 and alone has a value, so a row is v / l.
+    With the row's own maximum its probability is 1 and only l's fp32 sums (1e-6) and the output's rounding to bf16 are
+    left: one element in 2,000 at most falls on the other side.  A probability that is itself rounded to bf16 moves
+    the result by up to 2^-9, half of its last place."""
+    from piper_b200.ops import core
+
+    S, Hq = 256, 4
+    torch.manual_seed(16)
+    g = torch.linspace(0.1, 7.9, 128 * Hq)[torch.randperm(128 * Hq)].view(128, Hq) * math.log(2.0) * math.sqrt(hd)
+    q, k, v = torch.zeros(S, Hq, hd), torch.zeros(S, hd), torch.zeros(S, hd)
+    q[128:, :, 0] = g
+    k[128, 0] = 1.0
+    v[128] = torch.randn(hd)
+    qkv = torch.cat([q.reshape(S, Hq * hd), k, v], dim=1).to(torch.bfloat16).cuda()
+    out, lse = core.attention_fwd(qkv, 1, S, Hq, 1, hd, 1.0 / math.sqrt(hd))
+    s = qkv[128:, : Hq * hd].view(128, Hq, hd)[:, :, 0].double() / math.sqrt(hd)
+    others = torch.arange(128, 256, device="cuda", dtype=torch.float64).view(128, 1)     # earlier keys have score 0
+    l = 1.0 + others * torch.exp(-s)
+    want = (qkv[128, (Hq + 1) * hd:].double() / l.unsqueeze(-1)).to(torch.bfloat16)
+    assert (out[128:].view(128, Hq, hd) != want).float().mean() < 0.01
+    assert torch.allclose(lse[0, :, 128:].t().double(), s + torch.log(l), rtol=1e-5)
 
 
 @pytest.mark.parametrize("T,V,D", [(64, 1000, 264), (300, 301, 256), (0, 16, 64), (77, 40, 256)])
