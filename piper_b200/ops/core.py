@@ -178,8 +178,14 @@ def _linear_wgrad(x2: Tensor, dy2: Tensor, w: Tensor) -> Optional[Tensor]:
 _GEMM_FORK = int(os.environ.get("PIPER_GEMM_FORK", "2") or 0)
 _side_streams: dict = {}
 # The fork costs the host two event waits and two stream switches (about 45 us of Python); below this many
-# multiply-adds (some 12 us of GEMM) there is no idle round of tiles worth that.
+# multiply-adds (some 12 us of GEMM) there is no idle round of tiles worth that.  A small GEMM whose bucket the side
+# stream is still adding to follows it there all the same: the sums of a weight that is used several times keep one
+# order, and with it their bits.
 _FORK_MIN_MACS = 1 << 33
+
+
+def _forks(macs: int, sink: Optional[Tensor]) -> bool:
+    return macs >= _FORK_MIN_MACS or (sink is not None and sink.data_ptr() in deferred_join.buckets)
 
 
 class deferred_join:
@@ -187,6 +193,7 @@ class deferred_join:
 
     depth = 0
     pending: dict = {}
+    buckets: set = set()      # addresses of the gradient sinks that the side streams add to in this scope
 
     def __enter__(self):
         deferred_join.depth += 1
@@ -198,6 +205,7 @@ class deferred_join:
             for cur, side in deferred_join.pending.values():
                 cur.wait_stream(side)
             deferred_join.pending.clear()
+            deferred_join.buckets.clear()
         return False
 
 
@@ -224,10 +232,11 @@ def _linear_backward(ctx, dy):
         x2 = x2.contiguous()
     deferred = wgrad_store.active is not None
     if (_GEMM_FORK and ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and not deferred and _is_native(dy2)
-            and x2.shape[0] * w.numel() >= _FORK_MIN_MACS):
+            and _forks(x2.shape[0] * w.numel(), grad_sinks.get(w))):
+        sink = grad_sinks.get(w)
         cur = torch.cuda.current_stream(dy2.device)
         side = _side_stream(cur)
-        dw_out = None if grad_sinks.get(w) is not None else torch.empty_like(w)   # allocated on the current stream
+        dw_out = None if sink is not None else torch.empty_like(w)   # allocated on the current stream
         side.wait_stream(cur)
         with torch.cuda.stream(side):
             if dw_out is None:
@@ -240,6 +249,7 @@ def _linear_backward(ctx, dy):
             x2.record_stream(side)
             dy2.record_stream(side)
             deferred_join.pending[(cur.device.index, cur.cuda_stream)] = (cur, side)
+            deferred_join.buckets.add(sink.data_ptr())
         else:
             cur.wait_stream(side)   # everything later on this stream, frees of x and dy included, follows both GEMMs
         return dx, dw_out

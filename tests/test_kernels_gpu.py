@@ -138,20 +138,52 @@ def test_gemm_tile_choice_does_not_change_the_result(M, N, K):
         assert torch.equal(auto, small) and torch.equal(auto, big)
 
 
-@pytest.mark.parametrize("T", [4095, 4096])
-def test_linear_gradients_around_the_fork_threshold(T):
-    """2048 x 1024 weights: 4096 rows are the first size whose weight-gradient GEMM runs on the side stream."""
+@pytest.mark.parametrize("sizes,forked", [((4095,), []), ((4096,), [4096]), ((4096, 4095), [4096, 4095]),
+                                          ((4095, 4096), [4096])])
+def test_linear_gradients_around_the_fork_threshold(sizes, forked, monkeypatch):
+    """2048 x 1024 weights: 4096 rows are the first size whose weight-gradient GEMM runs on the side stream.  Two uses of
+    one weight in one scope add to its bucket in the order of their backward passes (a small one behind a forked one is
+    forked too), so every repetition gives the same bits."""
     from piper_b200 import ops
     from piper_b200.ops import core
 
-    assert (T * 2048 * 1024 >= core._FORK_MIN_MACS) == (T == 4096)
+    assert core._GEMM_FORK == 2 and 4096 * 2048 * 1024 == core._FORK_MIN_MACS
     torch.manual_seed(20)
-    x = torch.randn(T, 1024, device="cuda", dtype=torch.bfloat16, requires_grad=True)
     w = (torch.randn(2048, 1024, device="cuda", dtype=torch.bfloat16) * 0.05).requires_grad_(True)
-    g = torch.randn(T, 2048, device="cuda", dtype=torch.bfloat16)
-    ops.linear(x, w).backward(g)
-    assert _close(x.grad, g.float() @ w.detach().float(), 1e-2)
-    assert _close(w.grad, g.float().t() @ x.detach().float(), 1e-2)
+    xs = [torch.randn(T, 1024, device="cuda", dtype=torch.bfloat16, requires_grad=True) for T in sizes]
+    gs = [torch.randn(T, 2048, device="cuda", dtype=torch.bfloat16) for T in sizes]
+    seen, rows = [], []
+    side_stream = core._side_stream
+    monkeypatch.setattr(core, "_side_stream", lambda cur: (seen.append(rows[-1]), side_stream(cur))[1])
+
+    def backward():
+        seen.clear()
+        for x, g in zip(xs, gs):
+            x.grad = None
+            rows.append(x.shape[0])
+            ops.linear(x, w).backward(g)
+
+    want = sum(g.float().t() @ x.detach().float() for x, g in zip(xs, gs))
+    backward()                                                # no bucket: every fork is joined, no order to keep
+    assert seen == [T for T in sizes if T == 4096]
+    for x, g in zip(xs, gs):
+        assert _close(x.grad, g.float() @ w.detach().float(), 1e-2)
+    assert _close(w.grad, want, 1e-2)
+    held = torch.randn(2048, 1024, device="cuda")            # what the bucket holds already: the order shows in the bits
+    sink = torch.empty_like(held)
+    core.grad_sinks.register(w, sink)
+    try:
+        results = []
+        for _ in range(5):
+            sink.copy_(held)
+            with core.deferred_join():
+                backward()
+                assert seen == forked
+            results.append(sink.clone())
+        assert not core.deferred_join.buckets and not core.deferred_join.pending
+    finally:
+        core.grad_sinks.unregister(w)
+    assert _close(results[0], want + held, 1e-4) and all(torch.equal(r, results[0]) for r in results)
 
 
 @pytest.mark.parametrize("T,D", [(300, 256), (300, 2048), (1000, 4096), (300, 8192), (7, 4096)])
