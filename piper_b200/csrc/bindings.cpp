@@ -107,6 +107,11 @@ void gemm(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool
   gemm_tiled(a, b, c, a_mn, b_mn, accumulate, status, 0);
 }
 
+int64_t gemm_tile_rows(int64_t M, int64_t N, int64_t K, bool f32_out, int64_t sms) {
+  return piper::gemm_tile_rows(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), f32_out,
+                               static_cast<int>(sms));
+}
+
 void rmsnorm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, Tensor y, const OptTensor& h_out,
                  Tensor rstd, double eps) {
   check_bf16(x, "x");
@@ -311,6 +316,7 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("kernel_launch_count", &kernel_launch_count);
   m.def("gemm", &gemm);
   m.def("gemm_tiled", &gemm_tiled);
+  m.def("gemm_tile_rows", &gemm_tile_rows);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd_num_partials", &rmsnorm_bwd_num_partials);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);

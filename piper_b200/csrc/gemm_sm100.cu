@@ -414,23 +414,32 @@ static int forced_tile() {
   return v;
 }
 
+// 256x256 tiles move a third fewer operand bytes per flop: measured on B200, they keep the tensor pipe 81 % busy where
+// 128x256 tiles reach 74 %.  They also come in fewer, larger pieces.  The time is taken as rounds of tiles over the SMs
+// times the cost of a tile (1 against 0.5 x 81 / 74 = 0.547), and the smaller one runs: of 640 small tiles in five rounds
+// and 320 big ones in three, the small ones (2.74 < 3; 137 against 167 us for 4096 x 5120 x 4096).
+// A single round of big tiles hides neither its first loads nor its epilogue, where two rounds of small ones overlap
+// both, and a second round that is nearly empty runs faster than a full one.  So it is taken only for long contractions
+// over well-filled SMs: at 128 tiles on 148 SMs big against small tiles measured 0.92-0.96 as fast for K = 512,
+// 0.98-1.00 for 2048, 1.00-1.06 for 4096 and 1.10-1.11 for 8192; at 76 to 98 tiles 0.97-1.00 for 4096, 1.03-1.09 for 8192.
+// Wide fp32 (weight-gradient) outputs always take the small tiles: their double-buffered accumulators hide the
+// reduce-adds.
+int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms) {
+  const long long n_tiles = (N + 255) / 256;
+  const long long tiles256 = (M + 255) / 256 * n_tiles;
+  const long long rounds256 = (tiles256 + num_sms - 1) / num_sms;
+  const long long rounds128 = ((M + 127) / 128 * n_tiles + num_sms - 1) / num_sms;
+  const bool fits = M >= 256 && N >= 256 && rounds256 * 1000 < rounds128 * 547;
+  const bool fills = tiles256 >= num_sms || tiles256 * K >= 3072ll * num_sms;
+  const bool pays = !f32_out || M >= N;
+  return fits && fills && pays ? 256 : 128;
+}
+
 int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 0;
-  {
-    // 256x256 tiles move a third fewer operand bytes per flop: measured on B200, they keep the tensor pipe 81 % busy
-    // where 128x256 tiles reach 74 %.  They also come in fewer, larger pieces.  The time is taken as rounds of tiles
-    // over the SMs times the cost of a tile (1 against 0.5 x 81 / 74), and the smaller one runs: 128 big tiles are one
-    // round where 256 small ones are two, and 320 big ones are three where 640 small ones are five.  Wide fp32
-    // (weight-gradient) outputs always take the small tiles: their double-buffered accumulators hide the reduce-adds.
-    const int tile = g.tile != 0 ? g.tile : forced_tile();
-    const long long n_tiles = (g.N + 255) / 256;
-    const long long rounds256 = ((g.M + 255) / 256 * n_tiles + num_sms - 1) / num_sms;
-    const long long rounds128 = ((g.M + 127) / 128 * n_tiles + num_sms - 1) / num_sms;
-    const bool fits = g.M >= 256 && g.N >= 256 && rounds256 * 1000 < rounds128 * 547;
-    const bool pays = g.epilogue == kEpiStoreBf16 || g.M >= g.N;
-    if (tile == 256 || (tile == 0 && fits && pays))
-      return gemm256_bf16_launch(g, num_sms, next_sched_slot(), stream);
-  }
+  int tile = g.tile != 0 ? g.tile : forced_tile();
+  if (tile == 0) tile = gemm_tile_rows(g.M, g.N, g.K, g.epilogue != kEpiStoreBf16, num_sms);
+  if (tile == 256) return gemm256_bf16_launch(g, num_sms, next_sched_slot(), stream);
   CUtensorMap ta, tb;
   int rc;
   // K-major operand: dims {K, rows}, box {64, tile rows}.

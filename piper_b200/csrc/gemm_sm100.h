@@ -37,6 +37,9 @@ struct GemmArgs {
 // CUresult of a failed tensor-map encode.
 int gemm_bf16_launch(const GemmArgs& args, int num_sms, cudaStream_t stream);
 
+// The CTA tile height (128 or 256) that gemm_bf16_launch chooses for an [M, N] output and a contraction over K.
+int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms);
+
 // Same contract with 256x256 tiles per CTA (gemm256_sm100.cu).  sched: two zeroed ints of device memory for the
 // dynamic tile scheduler (rearmed by the kernel), or null for static tile striding.  gemm_bf16_launch picks
 // between the two tile shapes; PIPER_GEMM_TILE=128 or 256 forces one.

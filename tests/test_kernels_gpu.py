@@ -120,17 +120,20 @@ def test_linear_op_autograd():
     assert _close(w.grad, wr.grad, 1e-2)
 
 
-@pytest.mark.parametrize("M,N,K", [(2048, 4096, 128), (4096, 5120, 64), (1000, 8192, 72), (257, 256, 64)])
-def test_gemm_tile_choice_does_not_change_the_result(M, N, K):
-    """Shapes on both sides of the tile rule (one round of big tiles, three rounds against five, ragged, tiny): the
-    chosen kernel gives the bits of either tile, in both output types."""
+@pytest.mark.parametrize("M,N,K,bf16_tile,f32_tile", [(2048, 4096, 4096, 256, 128), (4096, 5120, 64, 128, 128),
+                                                      (1000, 8192, 72, 128, 128), (8192, 1000, 4104, 256, 256),
+                                                      (4096, 4352, 72, 256, 128), (257, 256, 64, 128, 128)])
+def test_gemm_tile_choice_does_not_change_the_result(M, N, K, bf16_tile, f32_tile):
+    """Shapes on both sides of the tile rule (one round of big tiles against two with long and short contractions, three
+    against five, two against four, ragged, tall and wide fp32, tiny): the chosen kernel gives the bits of either tile, in both output types."""
     from piper_b200.ops import native
 
     torch.manual_seed(19)
     lib, st = native.lib(), native.status_tensor()
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
-    for dtype in (torch.bfloat16, torch.float32):
+    for dtype, tile in ((torch.bfloat16, bf16_tile), (torch.float32, f32_tile)):
+        assert lib.gemm_tile_rows(M, N, K, dtype == torch.float32, 148) == tile
         auto, small, big = (torch.empty(M, N, device="cuda", dtype=dtype) for _ in range(3))
         lib.gemm(a, b, auto, False, False, False, st)
         lib.gemm_tiled(a, b, small, False, False, False, st, 128)

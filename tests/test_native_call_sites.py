@@ -50,3 +50,23 @@ def test_native_op_call_sites_match_the_registered_schemas():
                                 f"its schema takes {required}..{len(args)}")
     assert not problems, "\n".join(problems)
     assert checked > 100
+
+
+@pytest.mark.parametrize("M,N,K,f32,sms,rows", [
+    (2048, 4096, 4096, False, 148, 256),      # 128 big tiles in one round, 256 small ones in two
+    (2048, 4096, 2048, False, 148, 128),      # the same with too short a contraction
+    (1184, 6400, 64, False, 100, 128),        # 125 in two, 250 in three
+    (4096, 5120, 8192, False, 148, 128),      # 320 in three, 640 in five
+    (9472, 8192, 64, False, 148, 256),        # 1184 in eight, 2368 in sixteen
+    (2048, 4096, 64, False, 64, 256),         # two rounds against four
+    (2048, 4096, 8192, False, 256, 128),      # one round either way
+    (2048, 4096, 4096, True, 148, 128), (4096, 2048, 4096, True, 148, 256),      # wide and tall fp32
+    (255, 65536, 4096, False, 148, 128), (65536, 255, 4096, False, 148, 128),    # narrower than a big tile
+    (65536, 256, 64, False, 148, 256),
+])
+def test_gemm_tile_rule(M, N, K, f32, sms, rows):
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    assert native.lib().gemm_tile_rows(M, N, K, f32, sms) == rows
