@@ -1021,19 +1021,28 @@ int set_smem(K kern, int bytes) {
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
+// Two query tiles per CTA overlap the softmax of one with the MMAs of the other, but last 1.1 to 1.3 times as long as
+// the longer of the two alone.  As long as every tile has an SM of its own, or the SMs get through all key blocks of all
+// tiles (longest first) before a longest tile and a block have passed, one tile per CTA finishes earlier.  One against
+// two on 148 SMs, head dimension 64 / 128: 16 key blocks, 256 tiles 29.0 against 35.1 / 35.0 against 37.1 us, 320
+// tiles 37.3 / 35.1 and 44.7 / 37.2; 4 blocks, 152 tiles 11.0 / 12.6 and 12.6 / 14.7, 208 tiles 14.6 / 12.9 and 16.7 / 14.7;
+// with one block two tiles are never slower.
+int attn_tiles_per_cta(int B, int S, int Hq, int num_sms) {
+  const long long blocks = S / 128, tiles = static_cast<long long>(B) * Hq * blocks;
+  return tiles <= num_sms || tiles * (blocks + 1) / 2 <= (blocks - 1) * num_sms ? 1 : 2;
+}
+
 template <int HD>
 static int attn_fwd_impl(const CUtensorMap& tm, const CUtensorMap& to, float* lse, int B, int S, int Hq, int Hkv,
-                         float softmax_scale, int* status, cudaStream_t st) {
+                         float softmax_scale, int num_sms, int* status, cudaStream_t st) {
   static bool cfg = false;
   if (!cfg) {
     if (set_smem(attn_fwd_kernel<HD>, FwdSmem<HD>::TOTAL)) return -2;
     cfg = true;
   }
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  // Two query tiles per CTA overlap the softmax of one with the MMAs of the other.  As long as every tile can have
-  // an SM of its own, one tile per CTA finishes earlier.
   const long long per_head = static_cast<long long>(Hq / Hkv) * (S / 128);
-  const int tiles_per_cta = per_head * Hkv * B <= 148 ? 1 : 2;
+  const int tiles_per_cta = attn_tiles_per_cta(B, S, Hq, num_sms);
   const long long ctas = (per_head + tiles_per_cta - 1) / tiles_per_cta * Hkv * B;
   if (ctas > 0x7fffffffll) return -1;
   attn_fwd_kernel<HD><<<static_cast<unsigned>(ctas), FWD_THREADS, FwdSmem<HD>::TOTAL, st>>>(
@@ -1042,7 +1051,7 @@ static int attn_fwd_impl(const CUtensorMap& tm, const CUtensorMap& to, float* ls
 }
 
 int attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int Hkv, int hd,
-             float softmax_scale, int* status, cudaStream_t st) {
+             float softmax_scale, int num_sms, int* status, cudaStream_t st) {
   if (S % 128 != 0 || Hq % Hkv != 0 || (hd != 64 && hd != 128)) return -1;
   if (B == 0) return 0;
   const long long T = static_cast<long long>(B) * S;
@@ -1052,8 +1061,8 @@ int attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int H
   int rc = make_tmap_2d_bf16(&tm, qkv, W, T, W * 2, 64, 128);
   if (rc != 0) return rc;
   if ((rc = make_tmap_2d_bf16(&to, out, Wo, T, Wo * 2, 64, 32)) != 0) return rc;
-  return hd == 128 ? attn_fwd_impl<128>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, status, st)
-                   : attn_fwd_impl<64>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, status, st);
+  return hd == 128 ? attn_fwd_impl<128>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, num_sms, status, st)
+                   : attn_fwd_impl<64>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, num_sms, status, st);
 }
 
 template <int HD>

@@ -11,7 +11,10 @@ namespace piper {
 
 // out [B*S, Hq*hd] bf16, lse [B, Hq, S] fp32 (natural log).
 int attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int Hkv, int hd,
-             float softmax_scale, int* status, cudaStream_t st);
+             float softmax_scale, int num_sms, int* status, cudaStream_t st);
+
+// Query tiles (1 or 2) that a CTA of attn_fwd works on.
+int attn_tiles_per_cta(int B, int S, int Hq, int num_sms);
 
 // d_qkv has the layout of qkv and is fully overwritten.  delta is scratch of
 // B*Hq*S floats provided by the caller.

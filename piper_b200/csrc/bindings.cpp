@@ -289,9 +289,13 @@ void attn_fwd(const Tensor& qkv, Tensor out, Tensor lse, int64_t B, int64_t S, i
   TORCH_CHECK(qkv.numel() == B * S * (Hq + 2 * Hkv) * hd, "qkv has the wrong size");
   check_rc(piper::attn_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), static_cast<int>(B),
                            static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(Hkv),
-                           static_cast<int>(hd), static_cast<float>(scale), status.data_ptr<int>(),
+                           static_cast<int>(hd), static_cast<float>(scale), num_sms(), status.data_ptr<int>(),
                            cur_stream()),
            "attn_fwd");
+}
+
+int64_t attn_tiles_per_cta(int64_t B, int64_t S, int64_t Hq, int64_t sms) {
+  return piper::attn_tiles_per_cta(static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(sms));
 }
 
 void attn_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, const Tensor& lse, Tensor delta,
@@ -335,6 +339,7 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("add_bf16", &add_bf16);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
+  m.def("attn_tiles_per_cta", &attn_tiles_per_cta);
   register_moe_ops(m);
   register_fused_ops(m);
 }

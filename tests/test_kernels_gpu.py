@@ -263,15 +263,18 @@ def test_attention_fwd_bwd(B, S, Hq, Hkv, hd):
     assert _close(gq[:, (Hq + Hkv) * hd:], gr[:, (Hq + Hkv) * hd:], 3e-2)   # dV
 
 
-@pytest.mark.parametrize("B,S,Hq,Hkv,hd,growth", [(1, 640, 32, 32, 64, 0.0), (2, 640, 24, 8, 128, 0.0),
-                                                  (1, 768, 32, 8, 128, 40.0), (3, 256, 32, 4, 64, 40.0)])
-def test_attention_paired_tiles(B, S, Hq, Hkv, hd, growth):
-    """More query tiles than SMs, so a CTA takes two: odd tile counts per head (a last CTA with one tile), pairs of
-    heads and pairs of neighbouring query blocks.  ``growth`` makes later keys' scores larger, so the accumulated output
+@pytest.mark.parametrize("B,S,Hq,Hkv,hd,growth,tiles", [(1, 640, 40, 40, 64, 0.0, 2), (2, 640, 24, 8, 128, 0.0, 2),
+                                                        (1, 768, 40, 8, 128, 40.0, 2), (3, 256, 32, 4, 64, 40.0, 2),
+                                                        (1, 640, 32, 32, 64, 0.0, 1), (1, 768, 32, 8, 128, 40.0, 1)])
+def test_attention_paired_tiles(B, S, Hq, Hkv, hd, growth, tiles):
+    """More query tiles than SMs, so a CTA takes two (one where the longest tile covers the rest): odd tile counts per
+    head (a last CTA with one tile), pairs of heads and pairs of neighbouring query blocks.  ``growth`` makes later keys' scores larger, so the accumulated output
     is rescaled by small factors in most blocks."""
     from piper_b200 import ops
+    from piper_b200.ops import native
     from piper_b200.ops.core import _attention_ref
 
+    assert native.lib().attn_tiles_per_cta(B, S, Hq, 148) == tiles
     torch.manual_seed(15)
     qkv = torch.randn(B * S, (Hq + 2 * Hkv) * hd, device="cuda")
     ramp = 1.0 + growth * (torch.arange(B * S, device="cuda") % S) / S

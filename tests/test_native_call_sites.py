@@ -70,3 +70,17 @@ def test_gemm_tile_rule(M, N, K, f32, sms, rows):
     if not native.lib_path().exists():
         pytest.skip("the native library has not been built")
     assert native.lib().gemm_tile_rows(M, N, K, f32, sms) == rows
+
+
+@pytest.mark.parametrize("B,S,Hq,sms,tiles", [
+    (1, 128, 148, 148, 1), (1, 128, 149, 148, 2),         # an SM for every tile, and one too few (one block each)
+    (1, 512, 44, 148, 1), (1, 512, 45, 148, 2),           # 440 of 444 block times in which the longest tile is done
+    (1, 2048, 16, 148, 1), (2, 2048, 8, 148, 1), (1, 2048, 17, 148, 2),
+    (1, 2048, 16, 64, 2), (8, 4096, 32, 148, 2),
+])
+def test_attention_tiles_per_cta_rule(B, S, Hq, sms, tiles):
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    assert native.lib().attn_tiles_per_cta(B, S, Hq, sms) == tiles
