@@ -207,21 +207,22 @@ void embedding_bwd(const Tensor& tokens, const Tensor& dout, Tensor dtable) {
            "embedding_bwd");
 }
 
-void embedding_bwd_bf16(const Tensor& tokens, const Tensor& dout, Tensor owner, Tensor acc, Tensor dtable) {
+void embedding_bwd_bf16(const Tensor& tokens, const Tensor& dout, Tensor scratch, Tensor dtable) {
   check_bf16(dout, "dout");
   check_bf16(dtable, "dtable");
   TORCH_CHECK(tokens.scalar_type() == at::kLong && tokens.is_contiguous(), "tokens must be contiguous int64");
-  TORCH_CHECK(owner.scalar_type() == at::kInt && owner.numel() == dtable.size(0), "owner must be int32 [V]");
-  TORCH_CHECK(acc.scalar_type() == at::kFloat && acc.numel() == tokens.numel() * dtable.size(1),
-              "acc must be fp32 [T, D]");
-  TORCH_CHECK(dout.is_contiguous() && acc.is_contiguous() && dtable.is_contiguous() && dout.numel() == acc.numel(),
+  const int64_t T = tokens.numel(), V = dtable.size(0), D = dtable.size(1);
+  TORCH_CHECK(dout.is_contiguous() && dtable.is_contiguous() && dout.numel() == T * D,
               "embedding_bwd_bf16 expects contiguous tensors");
-  TORCH_CHECK(((reinterpret_cast<uintptr_t>(dout.data_ptr()) | reinterpret_cast<uintptr_t>(acc.data_ptr()) |
+  TORCH_CHECK(scratch.scalar_type() == at::kInt && scratch.is_contiguous() &&
+                  scratch.numel() >= piper::embedding_bwd_scratch(T, static_cast<int>(D), static_cast<int>(V)),
+              "scratch must hold an owner per row and the sums");
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(dout.data_ptr()) | reinterpret_cast<uintptr_t>(scratch.data_ptr()) |
                 reinterpret_cast<uintptr_t>(dtable.data_ptr())) & 15u) == 0,
               "embedding_bwd_bf16 expects 16-byte aligned tensors");
   check_rc(piper::embedding_bwd_bf16(reinterpret_cast<const long long*>(tokens.data_ptr<int64_t>()), dout.data_ptr(),
-                                     owner.data_ptr<int>(), acc.data_ptr<float>(), dtable.data_ptr(), tokens.numel(),
-                                     static_cast<int>(dtable.size(1)), static_cast<int>(dtable.size(0)), cur_stream()),
+                                     scratch.data_ptr<int>(), dtable.data_ptr(), T, static_cast<int>(D),
+                                     static_cast<int>(V), cur_stream()),
            "embedding_bwd_bf16", 3);
 }
 

@@ -683,23 +683,24 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ tokens,
 }
 
 // Embedding gradient straight into a bf16 table, cleared first: rows of one token value are summed in fp32 in a compact
-// [T, D] buffer at the position of its first occurrence (owner[v], the lowest position), then rounded once into the
-// table.  The fp32 table it replaces cost a clear, a read and a conversion of V rows for the T that are touched.
+// [T, D] buffer at the position of its first occurrence, then rounded once into the table.  The fp32 table it replaces
+// cost a clear, a read and a conversion of V rows for the T that are touched.
+// owner[v] = T - (lowest position of v), 0 for a value that does not occur: cleared by the same memset as the sums.
 __global__ void embedding_owner_kernel(const long long* __restrict__ tokens, int* __restrict__ owner, int T, int V) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T) return;
   const long long tok = tokens[i];
-  if (tok >= 0 && tok < V) atomicMin(owner + tok, i);
+  if (tok >= 0 && tok < V) atomicMax(owner + tok, T - i);
 }
 
 __global__ void __launch_bounds__(128)
 embedding_compact_kernel(const long long* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout,
-                         const int* __restrict__ owner, float* __restrict__ acc, int D, int V) {
+                         const int* __restrict__ owner, float* __restrict__ acc, int T, int D, int V) {
   const long long row = blockIdx.x;
   const long long tok = tokens[row];
   if (tok < 0 || tok >= V) return;
   const bf16x8* src = reinterpret_cast<const bf16x8*>(dout + row * D);
-  float4* dst = reinterpret_cast<float4*>(acc + static_cast<long long>(owner[tok]) * D);
+  float4* dst = reinterpret_cast<float4*>(acc + static_cast<long long>(T - owner[tok]) * D);
   for (int i = threadIdx.x; i < D / 8; i += blockDim.x) {
     float f[8];
     unpack8(src[i], f);
@@ -710,10 +711,10 @@ embedding_compact_kernel(const long long* __restrict__ tokens, const __nv_bfloat
 
 __global__ void __launch_bounds__(128)
 embedding_scatter_kernel(const long long* __restrict__ tokens, const int* __restrict__ owner,
-                         const float* __restrict__ acc, __nv_bfloat16* __restrict__ dtable, int D, int V) {
+                         const float* __restrict__ acc, __nv_bfloat16* __restrict__ dtable, int T, int D, int V) {
   const long long row = blockIdx.x;
   const long long tok = tokens[row];
-  if (tok < 0 || tok >= V || owner[tok] != row) return;
+  if (tok < 0 || tok >= V || T - owner[tok] != row) return;
   const float4* src = reinterpret_cast<const float4*>(acc + row * D);
   bf16x8* dst = reinterpret_cast<bf16x8*>(dtable + tok * D);
   for (int i = threadIdx.x; i < D / 8; i += blockDim.x) {
@@ -1024,15 +1025,21 @@ int embedding_bwd(const long long* tokens, const void* dout, float* dtable, long
   return PIPER_LAUNCH_OK();
 }
 
-int embedding_bwd_bf16(const long long* tokens, const void* dout, int* owner, float* acc, void* dtable, long long T,
-                       int D, int V, cudaStream_t st) {
+long long embedding_bwd_scratch(long long T, int D, int V) { return (V + 3ll) / 4 * 4 + T * D; }
+
+int embedding_bwd_bf16(const long long* tokens, const void* dout, int* scratch, void* dtable, long long T, int D, int V,
+                       cudaStream_t st) {
   if (D % 8 != 0 || T >= (1ll << 31)) return -1;
   if (cudaMemsetAsync(dtable, 0, static_cast<size_t>(V) * D * 2, st) != cudaSuccess) return -3;
   if (T == 0) return 0;
+  const long long words = embedding_bwd_scratch(T, D, V);
+  if (cudaMemsetAsync(scratch, 0, static_cast<size_t>(words) * 4, st) != cudaSuccess) return -3;
+  float* acc = reinterpret_cast<float*>(scratch + (words - T * D));
   const unsigned n = static_cast<unsigned>(T);
-  embedding_owner_kernel<<<(n + 255) / 256, 256, 0, st>>>(tokens, owner, static_cast<int>(T), V);
-  embedding_compact_kernel<<<n, 128, 0, st>>>(tokens, static_cast<const __nv_bfloat16*>(dout), owner, acc, D, V);
-  embedding_scatter_kernel<<<n, 128, 0, st>>>(tokens, owner, acc, static_cast<__nv_bfloat16*>(dtable), D, V);
+  const int t = static_cast<int>(T);
+  embedding_owner_kernel<<<(n + 255) / 256, 256, 0, st>>>(tokens, scratch, t, V);
+  embedding_compact_kernel<<<n, 128, 0, st>>>(tokens, static_cast<const __nv_bfloat16*>(dout), scratch, acc, t, D, V);
+  embedding_scatter_kernel<<<n, 128, 0, st>>>(tokens, scratch, acc, static_cast<__nv_bfloat16*>(dtable), t, D, V);
   return PIPER_LAUNCH_OK();
 }
 

@@ -39,10 +39,13 @@ int embedding_fwd(const long long* tokens, const void* table, void* out, long lo
 int embedding_bwd(const long long* tokens, const void* dout, float* dtable, long long T, int D, int V,
                   cudaStream_t st);
 
+// The same into a bf16 table that need not be cleared; D % 8 == 0.  scratch: embedding_bwd_scratch() 32-bit words, 16-byte
+// aligned (an owner per table row, then fp32 sums [T, D]).
+long long embedding_bwd_scratch(long long T, int D, int V);
+int embedding_bwd_bf16(const long long* tokens, const void* dout, int* scratch, void* dtable, long long T, int D, int V,
+                       cudaStream_t st);
+
 // Per-row loss and log-sum-exp of bf16 logits [T, V] with row stride ld.
-// owner [V] int32 filled with a value >= T, acc [T, D] fp32 zeroed by the caller; D % 8 == 0.
-int embedding_bwd_bf16(const long long* tokens, const void* dout, int* owner, float* acc, void* dtable, long long T,
-                       int D, int V, cudaStream_t st);
 int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long T, int V,
            long long ld, long long ignore_index, cudaStream_t st);
 // out = (softmax - onehot) * gscale[0] * row_scale; out may alias logits.
