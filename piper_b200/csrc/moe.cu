@@ -260,12 +260,14 @@ gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict_
     for (int j = 0; j < K; ++j) w[j] = weights == nullptr ? 1.f : j0 + j < k ? weights[t * k + j0 + j] : 0.f;
   };
   load_entries(0);
+  // one or two entries: the launcher passes k == K, and the loads of four or two vectors go out together
+#pragma unroll (K >= 4 ? 1 : 4 / K)
   for (int i0 = 0; i0 < D / 8; i0 += 32) {
     const int i = i0 + lane;
     const bool in = i < D / 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j0 = 0; j0 < k; j0 += K) {
-      if (k > K) load_entries(j0);
+    for (int j0 = 0; j0 < (K >= 4 ? k : K); j0 += K) {
+      if (K >= 4 && k > K) load_entries(j0);
       uint4 q[K];
 #pragma unroll
       for (int j = 0; j < K; ++j)
