@@ -178,19 +178,21 @@ __device__ __forceinline__ void zero_padding(__nv_bfloat16* __restrict__ rows, c
 }
 
 // One warp per token: the first k lanes claim the rows of its entries together, then the token row is read once and
-// written k times; the CTAs behind the tokens' clear the padding rows of the segments.  4096 tokens x 2048, top 8 of 128:
-// 33 us + 10 us of clearing in a launch of its own, 39 us together (170 MB written).
+// written k times; the first CTAs clear the padding rows of the segments (behind the tokens' they would be a tail of long
+// CTAs: 8192 x 2048 over 64 experts, top 8, 91.3 us behind and 88.6 us in front).  4096 tokens x 2048, top 8 of 128: 47 us with
+// the clearing in a launch of its own, 46 us together; 4096 x 4096, top 2 of 8: 41 and 21 us.
 __global__ void __launch_bounds__(ROW_THREADS)
 permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx, const int* __restrict__ g_start,
                const int* __restrict__ g_len, const int* __restrict__ counts, int* __restrict__ cursor,
                int* __restrict__ pos, __nv_bfloat16* __restrict__ rows, long long T, int D, int k, int E,
                long long rows_cap, unsigned token_ctas, int* status) {
-  if (blockIdx.x >= token_ctas) {
-    const int b = static_cast<int>(blockIdx.x - token_ctas);
+  const unsigned pad_ctas = E * PAD_CTAS;
+  if (blockIdx.x < pad_ctas) {
+    const int b = static_cast<int>(blockIdx.x);
     zero_padding(rows, g_start, g_len, counts, b / PAD_CTAS, b % PAD_CTAS, D, rows_cap, status);
     return;
   }
-  const long long t = (static_cast<long long>(blockIdx.x) * ROW_THREADS + threadIdx.x) >> 5;
+  const long long t = (static_cast<long long>(blockIdx.x - pad_ctas) * ROW_THREADS + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
   const uint4* src = reinterpret_cast<const uint4*>(x + t * D);
