@@ -11,10 +11,10 @@
 //                  contraction over all row segments of expert e)
 //
 // The structure is that of the dense kernel (gemm_sm100.cu): persistent
-// CTAs, TMA producer warp, single-thread tcgen05.mma issuer, two TMEM
-// accumulators, eight epilogue warps; only the tile -> coordinate mapping
-// differs and is computed on the device from the group table, because the
-// row counts are produced by the router on the GPU.  Expert weights are read
+// CTAs, TMA producer warp, tcgen05.mma issued by one elected lane of a warp
+// that walks the loop uniformly, two TMEM accumulators, eight epilogue warps;
+// the tile -> coordinate mapping is computed on the device from the group
+// table, because the row counts are produced by the router on the GPU.  Expert weights are read
 // through a 3-D tensor map (k, n, expert).  No multicast; bounded waits.
 #include "gemm_sm100.h"
 #include "ptx.cuh"
