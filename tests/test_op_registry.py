@@ -2,6 +2,7 @@
 gradients of single outputs."""
 import subprocess
 import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -157,4 +158,5 @@ assert (x.grad == 5).all()
 
 def test_op_modules_reload_and_ops_take_further_registrations():
     """In a process of its own: both change the ops for everything after them."""
-    subprocess.run([sys.executable, "-c", _MODULE_CHANGES], check=True, timeout=300)
+    root = Path(__file__).resolve().parent.parent
+    subprocess.run([sys.executable, "-c", _MODULE_CHANGES], check=True, timeout=300, cwd=root)
