@@ -426,8 +426,9 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 // each group has the MMAs of two tiles' time for its work; warp 8: TMA, warp 9: MMA.  P' and dS' (bf16) replace their
 // own fp32 scores in tensor memory and are the A operand of the accumulating MMAs from there: no thread writes shared
 // memory in the loop.  Bound by the MMAs: a 128x64x16 one with both operands in shared memory reads 6 KiB (48 cycles)
-// for 32 cycles of arithmetic.  Both passes at S = 4096, 32 q / 8 kv heads x 128: 751 us with probabilities through
-// shared memory in two launches on two streams, 427 us so with dQ on 64-row tiles as well, 379 us with dQ as below.
+// for 32 cycles of arithmetic.  Both passes and the delta kernel at S = 4096, 32 q / 8 kv heads x 128: 653 us with
+// probabilities through shared memory in two launches, 391 us so (this kernel alone 379 us, and 427 us with dQ on
+// 64-row tiles as well).
 constexpr int BWD_THREADS = 320;
 
 template <int HD>

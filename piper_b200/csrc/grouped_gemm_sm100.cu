@@ -108,7 +108,8 @@ __device__ __forceinline__ Tile resolve_tile(int t, const int* tile_prefix, cons
 
 // Measured at 4096 tokens, 128 experts, top 8, 2048 x 768 (two projections each): forward 378 -> 361 us and input
 // gradient 377 -> 357 us with the group table scanned by a warp; weight gradient 473 us into bf16, against 1206 us for
-// direct fp32 stores plus 836 us that cleared and converted the fp32 tensor.  No unit is above 60 % busy there.
+// direct fp32 stores plus 836 us that cleared and converted the fp32 tensor.  No unit is above 62 % busy (64 experts,
+// top 4); what fills the rest has not been measured.
 // OUT_BF16 selects the element type of a weight gradient (fp32 buckets accumulate; a bf16 result is stored).
 template <int MODE, bool OUT_BF16>
 __global__ void __launch_bounds__(NUM_THREADS, 1)

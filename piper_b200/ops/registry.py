@@ -4,8 +4,8 @@ An op is a schema, one body for all devices, a fake (meta) body and an autograd 
 plain ``torch.autograd.Function`` around a call of the same op below autograd, so dispatch modes, fake tensors and
 saved-tensor hooks see the op and its saved tensors as with ``torch.library.custom_op``; what is left out is that
 wrapper's own work per call, which is host time in front of every launch.  Measured with the kernels of a B200 behind
-them, forward and backward: a residual norm 145 us a pass through the wrapper and 118 us through this one (its kernels
-take 63 us); the attention layer on 4 x 128 tokens, with its small GEMMs no longer forked, 671 and 332 us.
+them, forward and backward: a residual norm 150 us a pass through the wrapper and 120 us through this one (its kernels
+take 63 us); the attention layer on 4 x 128 tokens, whose small GEMMs are no longer forked either, 604 and 350 us.
 
 Gradients that did not arrive (a consumer's backward returned None, or a reentrant checkpoint did not use its input):
 the formula of an op with one output is handed zeros in their place.  Where an op has several outputs, most of them
