@@ -58,8 +58,8 @@ float* opt_f32(const OptTensor& t) {
 // C[M,N] = A * B^T.  a: [M,K] (a_mn=false) or [K,M] (a_mn=true); b: [N,K]
 // (b_mn=false) or [K,N] (b_mn=true).  c bf16 -> store; c fp32 -> store or
 // accumulate.
-void gemm_tiled(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
-                int64_t tile) {
+void gemm_shaped(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
+                 int64_t tile, int64_t width) {
   check_bf16(a, "a");
   check_bf16(b, "b");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm expects 2-D tensors");
@@ -100,16 +100,28 @@ void gemm_tiled(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn
   g.status = status.data_ptr<int>();
   TORCH_CHECK(tile == 0 || tile == 128 || tile == 256, "gemm tile must be 0 (auto), 128 or 256");
   g.tile = static_cast<int>(tile);
+  g.width = static_cast<int>(width);
   check_rc(piper::gemm_bf16_launch(g, num_sms(), cur_stream()), "gemm");
 }
 
+void gemm_tiled(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
+                int64_t tile) {
+  gemm_shaped(a, b, c, a_mn, b_mn, accumulate, status, tile, 0);
+}
+
 void gemm(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status) {
-  gemm_tiled(a, b, c, a_mn, b_mn, accumulate, status, 0);
+  gemm_shaped(a, b, c, a_mn, b_mn, accumulate, status, 0, 0);
 }
 
 int64_t gemm_tile_rows(int64_t M, int64_t N, int64_t K, bool f32_out, int64_t sms) {
   return piper::gemm_tile_rows(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), f32_out,
                                static_cast<int>(sms));
+}
+
+std::tuple<int64_t, int64_t> gemm_shape(int64_t M, int64_t N, int64_t K, bool b_mn, bool f32_out, int64_t sms) {
+  const piper::GemmShape s = piper::gemm_shape(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), b_mn,
+                                               f32_out, static_cast<int>(sms));
+  return {s.ctas, s.width};
 }
 
 void rmsnorm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, Tensor y, const OptTensor& h_out,
@@ -321,7 +333,9 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("kernel_launch_count", &kernel_launch_count);
   m.def("gemm", &gemm);
   m.def("gemm_tiled", &gemm_tiled);
+  m.def("gemm_shaped", &gemm_shaped);
   m.def("gemm_tile_rows", &gemm_tile_rows);
+  m.def("gemm_shape", &gemm_shape);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd_num_partials", &rmsnorm_bwd_num_partials);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);

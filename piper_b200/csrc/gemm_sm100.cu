@@ -1,27 +1,35 @@
 // Dense bf16 GEMM for sm_100a: C[M,N] = A[M,K] * B[N,K]^T with fp32
 // accumulation in tensor memory.
 //
-// One persistent CTA per SM walks 128x256 output tiles.  Roles by warp:
-//   warp 0      TMA producer: fills a 4-stage shared-memory ring with
-//               128-byte-swizzled operand tiles (cp.async.bulk.tensor, no
-//               multicast).
-//   warp 1      MMA issuer: one lane issues tcgen05.mma (128x256x16) into one
-//               of two 256-column TMEM accumulators and commits to mbarriers.
+// Persistent CTAs walk output tiles of 128 rows and a width chosen per launch (32 to 256 columns), either each CTA
+// by itself or in pairs on two neighbouring SMs (tcgen05 cta_group::2: 256-row tiles, each CTA holds 128 rows of A and
+// half of B's rows in shared memory, its tensor memory takes its 128 rows of C).  Roles by warp:
+//   warp 0      TMA producer: fills a ring of shared-memory stages with 128-byte-swizzled operand tiles
+//               (cp.async.bulk.tensor, no multicast); the first CTA of a pair also hands out the tiles.
+//   warp 1      MMA issuer (first CTA of a pair, for both): tcgen05.mma into one of two 256-column accumulators.
+//               The warp walks the loop uniformly and one elected lane issues: in a single-lane branch every descriptor
+//               has to be moved into uniform registers, about 100 cycles per MMA.
 //   warp 2      TMEM allocator / deallocator.
-//   warps 4-7   epilogue: tcgen05.ld the finished accumulator (32 lanes per
-//               warp), convert and store, while the MMA warp already works on
-//               the next tile in the other accumulator.
+//   warps 4-11  epilogue: tcgen05.ld of the finished accumulator, conversion, staging in shared memory, TMA store (or
+//               TMA reduce-add), while the MMAs of the next tile run in the other accumulator.
+//
+// What bounds it: an SM fills shared memory from L2 at about 80 bytes per cycle.  A k-block of a 128 x w tile is
+// (128 + w) x 128 bytes for 2w cycles of MMA, 614 cycles of fill against 512 at w = 256; in a pair each SM loads half
+// of B's rows, (128 + w / 2) x 128 bytes, 410 cycles of fill, and reads half as much of B from shared memory.
 //
 // Each operand can be K-major (contraction index contiguous in memory) or
 // MN-major (row index contiguous), which covers forward (X W^T), input
 // gradient (dY W) and weight gradient (dY^T X) of a linear layer without any
 // transposed copy.  The epilogue either stores bf16 or adds into an fp32
-// buffer (gradient accumulation into the flat fp32 bucket).
+// buffer (gradient accumulation into the flat fp32 bucket).  Every output element is the sum of the same products in
+// the same order whatever the tile shape, so results do not depend on it.
 //
 // All mbarrier waits are bounded; on expiry the kernel records a status code,
 // drains its TMA copies, frees TMEM and returns.
 #include "gemm_sm100.h"
 
+#include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "ptx.cuh"
@@ -29,269 +37,298 @@
 namespace piper {
 namespace {
 
-constexpr int BM = 128;
-constexpr int BN = 256;
-constexpr int BK = 64;            // 64 bf16 = one 128-byte swizzle row
+constexpr int BM = 128;                        // rows of a CTA
+constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 4;
-constexpr int ACC_BUFS = 2;
-constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KiB
-constexpr int B_STAGE_BYTES = BN * BK * 2;   // 32 KiB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-constexpr int MN_BOX_BYTES = 64 * BK * 2;    // one MN-major TMA box: 64 k-rows x 128 B
-constexpr int NUM_THREADS = 256;
-constexpr int C_STAGE_BYTES = 32 * 32 * 4;   // fp32 epilogue: one 32x32 block per warp, two buffers per warp
-constexpr int C_STAGING_BYTES = 4 * 2 * C_STAGE_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int SMEM_BYTES_F32 = STAGES * STAGE_BYTES + 1024 /*align*/ + 1024 /*barriers, padded*/ + C_STAGING_BYTES;
+constexpr int A_STAGE_BYTES = BM * BK * 2;
+constexpr int MN_BOX_BYTES = 64 * BK * 2;
+constexpr int MAX_STAGES = 8;
+constexpr int OPERAND_BYTES = 196608;          // 4 stages of 128 x 256 operands, 6 of a CTA pair
+constexpr int EPI_WARPS = 8;
+constexpr int NUM_THREADS = 128 + 32 * EPI_WARPS;
+constexpr int C_STAGE_BYTES = 4096;            // per epilogue warp: two bf16 or one fp32 block of 32 x 32
+constexpr int BAR_OFF = OPERAND_BYTES + EPI_WARPS * C_STAGE_BYTES;
+constexpr int SMEM_BYTES = BAR_OFF + 512 + 1024;
+constexpr int RING = 16;                       // tiles handed out ahead: at most the stages + 2 accumulators + 1
 
-struct Barriers {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
-  uint64_t acc_full[ACC_BUFS];
-  uint64_t acc_empty[ACC_BUFS];
+struct Bars {
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
+  uint64_t tile_full[RING];
+  int tile[RING];
   uint32_t tmem_base;
-  int tile_ring[8];          // producer -> MMA warp: tile index of the n-th local tile (-1 = no more tiles)
-  int acc_tile[ACC_BUFS];    // MMA warp -> epilogue: tile index held by each accumulator (-1 = no more tiles)
+};
+static_assert(sizeof(Bars) <= 512, "barriers");
+
+struct Params {
+  int M, N, K;
+  int width;          // columns of a tile
+  int stages;
+  int accumulate;
+  int c_bufs;         // staging buffers per epilogue warp; the second ones take the room of operand stages
+  int band;           // tiles of the faster dimension that are walked together
+  int* status;
+  int* sched;
 };
 
-template <bool A_MN, bool B_MN, int EPI>
+template <int CTAS, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-            const __grid_constant__ CUtensorMap tmap_c, void* __restrict__ c_ptr, long long ldc, int M, int N,
-            int K, int accumulate, int* status, int* sched) {
+                 const __grid_constant__ CUtensorMap tmap_c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + STAGES * STAGE_BYTES);
-
-  const int warp = threadIdx.x >> 5;
+  uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+  Bars* bars = reinterpret_cast<Bars*>(smem + BAR_OFF);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
-  const int tiles_m = (M + BM - 1) / BM;
-  const int tiles_n = (N + BN - 1) / BN;
+  const uint32_t rank = CTAS == 2 ? cluster_rank() : 0;
+  const int width = p.width;
+  const int b_rows = width / CTAS;                                       // rows of B that this CTA loads
+  const int b_boxes = (b_rows + 63) / 64;
+  const int stage_bytes = A_STAGE_BYTES + (B_MN ? b_boxes * MN_BOX_BYTES : b_rows * BK * 2);
+  const int stages = p.stages;
+  const int tiles_m = (p.M + BM * CTAS - 1) / (BM * CTAS);
+  const int tiles_n = (p.N + width - 1) / width;
   const int num_tiles = tiles_m * tiles_n;
-  const int k_blocks = (K + BK - 1) / BK;
-  // Tiles that run at the same time should share operands: walk the dimension with fewer tiles fastest, so a
-  // wave of CTAs covers all of it and the operand of the long dimension streams through L2 once.
+  const int k_blocks = (p.K + BK - 1) / BK;
   const bool n_fast = tiles_n < tiles_m;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < MAX_STAGES; ++s) {
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->empty[s], 1);
     }
-    for (int a = 0; a < ACC_BUFS; ++a) {
-      mbar_init(&bars->acc_full[a], 2);    // tcgen05.commit + the MMA thread's own arrive (publishes acc_tile)
-      mbar_init(&bars->acc_empty[a], 4);   // one arrive per epilogue warp
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&bars->acc_full[a], 1);
+      mbar_init(&bars->acc_empty[a], EPI_WARPS * CTAS);
     }
+    for (int i = 0; i < RING; ++i) mbar_init(&bars->tile_full[i], 1);
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    tma_prefetch_desc(&tmap_c);
   }
   if (warp == 2) {
-    tmem_alloc(&bars->tmem_base, ACC_BUFS * BN);
-    tmem_relinquish();
+    tmem_alloc_n<CTAS>(&bars->tmem_base, 512);
+    tmem_relinquish_n<CTAS>();
   }
   tc_fence_before();
-  __syncthreads();
+  if (CTAS == 2) cluster_sync(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
+  // Tiles that run at the same time share operands: the dimension with fewer tiles is walked fastest, so that a wave
+  // covers all of it and the operand of the other dimension streams through L2 once; in bands, where the operand of the
+  // faster dimension would not stay in L2 from one wave to the next.
+  auto coords = [&](int tile, int& tm, int& tn) {
+    const int fast = n_fast ? tiles_n : tiles_m, slow = n_fast ? tiles_m : tiles_n;
+    const int b = tile / (p.band * slow), f0 = b * p.band;
+    const int bw = min(p.band, fast - f0), r = tile - f0 * slow;
+    const int f = f0 + r % bw, sl = r / bw;
+    tm = n_fast ? sl : f;
+    tn = n_fast ? f : sl;
+  };
+  // The n-th tile of this CTA (or pair), -1 behind the last one.
+  auto tile_at = [&](uint32_t n, int& tile) -> bool {
+    const bool got = CTAS == 2 ? mbar_wait_cluster(&bars->tile_full[n % RING], (n / RING) & 1, p.status)
+                               : mbar_wait(&bars->tile_full[n % RING], (n / RING) & 1, p.status);
+    if (!__all_sync(0xffffffffu, got)) return false;
+    tile = *reinterpret_cast<volatile int*>(&bars->tile[n % RING]);
+    return true;
+  };
+
   if (warp == 0) {
-    // ------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0, n_local = 0;
-      bool ok = true;
-      while (ok) {
-        // Tiles are handed out dynamically (one atomic per tile) so that a CTA that reaches the SM late,
-        // or shares the GPU with communication kernels, simply processes fewer tiles.
-        const int tile = sched != nullptr ? atomicAdd(&sched[0], 1)
-                                          : static_cast<int>(blockIdx.x + n_local * gridDim.x);
-        const bool none_left = tile >= num_tiles;
-        bars->tile_ring[n_local & 7] = none_left ? -1 : tile;
-        if (none_left) {
-          // pass the end marker to the MMA warp through the next stage's barrier (no bytes expected)
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (mbar_wait(&bars->empty[s], ph ^ 1, status)) mbar_arrive(&bars->full[s]);
-          break;
+    // ------------------------------------------------------ TMA producer (both CTAs of a pair load their own halves)
+    uint32_t n = 0;
+    int s = 0;
+    uint32_t ph = 0, fills = 0;
+    bool ok = true;
+    for (;; ++n) {
+      if (rank == 0 && elect_one()) {
+        int next = p.sched != nullptr ? atomicAdd(&p.sched[0], 1)
+                                      : static_cast<int>(blockIdx.x / CTAS + n * (gridDim.x / CTAS));
+        if (next >= num_tiles) next = -1;
+        bars->tile[n % RING] = next;
+        if (CTAS == 2) {
+          st_cluster_u32(mapa_u32(smem_u32(&bars->tile[n % RING]), 1), static_cast<uint32_t>(next));
+          mbar_arrive_cluster(mapa_u32(smem_u32(&bars->tile_full[n % RING]), 1));
         }
-        const int m0 = (n_fast ? tile / tiles_n : tile % tiles_m) * BM;
-        const int n0 = (n_fast ? tile % tiles_n : tile / tiles_m) * BN;
-        ++n_local;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&bars->empty[s], ph ^ 1, status)) { ok = false; break; }
-          uint8_t* sa = smem + s * STAGE_BYTES;
+        mbar_arrive(&bars->tile_full[n % RING]);
+      }
+      __syncwarp();
+      int tile;
+      if (!(ok = tile_at(n, tile)) || tile < 0) break;
+      int tm, tn;
+      coords(tile, tm, tn);
+      const int m0 = tm * (BM * CTAS) + static_cast<int>(rank) * BM;
+      const int n0 = tn * width + static_cast<int>(rank) * b_rows;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->empty[s], ph ^ 1, p.status)))) break;
+        if (elect_one()) {
+          uint8_t* sa = smem + s * stage_bytes;
           uint8_t* sb = sa + A_STAGE_BYTES;
-          mbar_arrive_expect_tx(&bars->full[s], STAGE_BYTES);
+          if (rank == 0) mbar_arrive_expect_tx(&bars->full[s], CTAS * stage_bytes);
           const int k0 = kb * BK;
           if (A_MN) {
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(sa + j * MN_BOX_BYTES, &tmap_a, &bars->full[s], m0 + 64 * j, k0);
+            tma_load_2d_n<CTAS>(sa, &tmap_a, &bars->full[s], m0, k0);
+            tma_load_2d_n<CTAS>(sa + MN_BOX_BYTES, &tmap_a, &bars->full[s], m0 + 64, k0);
           } else {
-            tma_load_2d(sa, &tmap_a, &bars->full[s], k0, m0);
+            tma_load_2d_n<CTAS>(sa, &tmap_a, &bars->full[s], k0, m0);
           }
           if (B_MN) {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * MN_BOX_BYTES, &tmap_b, &bars->full[s], n0 + 64 * j, k0);
+            for (int j = 0; j < b_boxes; ++j)
+              tma_load_2d_n<CTAS>(sb + j * MN_BOX_BYTES, &tmap_b, &bars->full[s], n0 + 64 * j, k0);
           } else {
-            tma_load_2d(sb, &tmap_b, &bars->full[s], k0, n0);
+            tma_load_2d_n<CTAS>(sb, &tmap_b, &bars->full[s], k0, n0);
           }
         }
+        __syncwarp();
+        ++fills;
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
-      if (!ok) {
-        // Unwinding: let the copies already issued land before the CTA (and
-        // its shared memory) goes away.  Stage s was last filled by iteration
-        // it_s = largest value < it congruent to s.
-        for (int s = 0; s < STAGES; ++s) {
-          if (it <= static_cast<uint32_t>(s)) continue;
-          const uint32_t fills = (it - 1 - s) / STAGES + 1;
-          mbar_wait(&bars->full[s], (fills - 1) & 1, nullptr);
-        }
+      if (!ok) break;
+    }
+    if (ok) {
+      // every stage handed back before the CTA may leave: no commit is still on its way to these barriers
+      for (int i = 0; i < stages && ok; ++i) {
+        ok = mbar_wait(&bars->empty[s], ph ^ 1, p.status);
+        if (++s == stages) { s = 0; ph ^= 1; }
+      }
+    } else if (rank == 0) {
+      for (int i = 0; i < stages; ++i) {         // let the copies already issued land
+        if (fills <= static_cast<uint32_t>(i)) continue;
+        mbar_wait(&bars->full[i], ((fills - 1 - i) / stages) & 1, nullptr);
       }
     }
   } else if (warp == 1) {
-    // -------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
-      uint32_t it = 0;
-      uint32_t local_tile = 0;
+    // -------------------------------------------------------- MMA issuer (first CTA of a pair, for both)
+    if (rank == 0) {
+      const uint32_t idesc = umma_idesc_bf16(BM * CTAS, width, A_MN, B_MN);
+      const uint64_t da0 = umma_desc_sw128(smem_u32(smem), A_MN ? MN_BOX_BYTES : 16, 1024);
+      const uint64_t db0 = umma_desc_sw128(smem_u32(smem) + A_STAGE_BYTES, B_MN ? MN_BOX_BYTES : 16, 1024);
+      constexpr int a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+      constexpr int b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+      int s = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      while (ok) {
-        const int acc = local_tile & 1;
-        const uint32_t acc_ph = (local_tile >> 1) & 1;
-        // the first stage of a tile also tells which tile it is
-        {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&bars->full[s], ph, status)) { ok = false; break; }
-        }
-        const int tile = *reinterpret_cast<volatile int*>(&bars->tile_ring[local_tile & 7]);
-        if (!mbar_wait(&bars->acc_empty[acc], acc_ph ^ 1, status)) { ok = false; break; }
-        if (tile < 0) {
-          // no more tiles: release the epilogue warps (both arrivals of the accumulator barrier)
-          bars->acc_tile[acc] = -1;
-          mbar_arrive(&bars->acc_full[acc]);
-          mbar_arrive(&bars->acc_full[acc]);
+      for (uint32_t n = 0; ok; ++n) {
+        int tile;
+        if (!(ok = tile_at(n, tile)) || tile < 0) break;
+        const uint32_t acc = n & 1;
+        if (!(ok = __all_sync(0xffffffffu, CTAS == 2 ? mbar_wait_cluster(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status)
+                                                     : mbar_wait(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status))))
           break;
-        }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (kb > 0 && !mbar_wait(&bars->full[s], ph, status)) { ok = false; break; }
+        const uint32_t tmem_d = tmem_base + acc * 256;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], ph, p.status)))) break;
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-          const uint32_t sb = sa + A_STAGE_BYTES;
-          // one descriptor per operand and stage; a k-step only adds a constant to its address field, which
-          // keeps the issuing thread's instruction count per MMA low
-          const uint64_t da0 = A_MN ? umma_desc_sw128(sa, MN_BOX_BYTES, 1024) : umma_desc_sw128(sa, 16, 1024);
-          const uint64_t db0 = B_MN ? umma_desc_sw128(sb, MN_BOX_BYTES, 1024) : umma_desc_sw128(sb, 16, 1024);
+          if (elect_one()) {
+            const uint64_t da = da0 + (static_cast<uint32_t>(s * stage_bytes) >> 4);
+            const uint64_t db = db0 + (static_cast<uint32_t>(s * stage_bytes) >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = da0 + ((A_MN ? k * (UMMA_K * 128) : k * (UMMA_K * 2)) >> 4);
-            const uint64_t db = db0 + ((B_MN ? k * (UMMA_K * 128) : k * (UMMA_K * 2)) >> 4);
-            umma_bf16_ss(tmem_d, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16_ss_n<CTAS>(tmem_d, da + k * a_step, db + k * b_step, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit_n<CTAS>(&bars->empty[s]);
+            if (kb == k_blocks - 1) umma_commit_n<CTAS>(&bars->acc_full[acc]);
           }
-          umma_commit(&bars->empty[s]);       // frees the smem stage when the MMAs retire
+          __syncwarp();
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
-        if (ok) {
-          bars->acc_tile[acc] = tile;
-          mbar_arrive(&bars->acc_full[acc]);  // publishes acc_tile
-          umma_commit(&bars->acc_full[acc]);  // arrives when the accumulator is complete
-        }
-        ++local_tile;
       }
     }
   } else if (warp >= 4) {
     // ---------------------------------------------------------- epilogue
-    const int ew = warp - 4;                  // == warp % 4: TMEM lanes [32*ew, 32*ew+32)
-    uint32_t local_tile = 0;
-    bool ok = true;
-    for (;; ++local_tile) {
-      const int acc = local_tile & 1;
-      const uint32_t acc_ph = (local_tile >> 1) & 1;
-      if (!mbar_wait(&bars->acc_full[acc], acc_ph, status)) { ok = false; break; }
-      const int tile = *reinterpret_cast<volatile int*>(&bars->acc_tile[acc]);
-      if (tile < 0) break;
-      const int m0 = (n_fast ? tile / tiles_n : tile % tiles_m) * BM;
-      const int n0 = (n_fast ? tile % tiles_n : tile / tiles_m) * BN;
+    const int q = warp & 3;                     // TMEM lanes [32q, 32q + 32)
+    const int half = (warp - 4) >> 2;           // odd or even 32-column chunks
+    uint8_t* const stage0 = smem + BAR_OFF - (warp - 3) * C_STAGE_BYTES * p.c_bufs;
+    uint8_t* stage = stage0;
+    for (uint32_t n = 0;; ++n) {
+      int tile;
+      if (!tile_at(n, tile) || tile < 0) break;
+      const uint32_t acc = n & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->acc_full[acc], (n >> 1) & 1, p.status))) break;
+      int tm, tn;
+      coords(tile, tm, tn);
+      const int row0 = tm * (BM * CTAS) + static_cast<int>(rank) * BM + q * 32;
+      const int n0 = tn * width;
       tc_fence_after();
-      const int row = m0 + ew * 32 + lane;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + acc * BN;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * 256;
+      // chunks of 32 columns: two in flight for bf16 (2 KiB staged each), one for fp32 (4 KiB)
+      constexpr int CHUNKS = EPI == kEpiStoreBf16 ? 2 : 1;
+      constexpr int BLOCK = C_STAGE_BYTES / CHUNKS;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c * 32, r);
+      for (int c = half; c < width / 32; c += 2 * CHUNKS) {
+        if (row0 >= p.M || n0 + c * 32 >= p.N) break;
+        uint32_t r[CHUNKS][32];
+#pragma unroll
+        for (int j = 0; j < CHUNKS; ++j)
+          if (j == 0 || c + 2 * j < width / 32) tmem_ld_32x32(taddr + (c + 2 * j) * 32, r[j]);
         tmem_ld_wait();
-        const int col0 = n0 + c * 32;
-        if (row < M && col0 < N) {
+        if (lane == 0) {                               // the previous blocks have left the buffer
+          if (p.c_bufs == 2) bulk_wait_group_read<1>();
+          else bulk_wait_group_read<0>();
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < CHUNKS; ++j) {
+          uint8_t* blk = stage + j * BLOCK;
           if (EPI == kEpiStoreBf16) {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(c_ptr) + row * ldc + col0;
-            if (col0 + 32 <= N) {
+            // 64-byte rows, 16-byte chunks XOR-swizzled by the row pair
 #pragma unroll
-              for (int v = 0; v < 4; ++v) {
-                uint4 o;
-                o.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
-                o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
-                o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
-                o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
-                reinterpret_cast<uint4*>(crow)[v] = o;
-              }
-            } else {
-              #pragma unroll
-                for (int j = 0; j < 32; ++j)   // constant indices keep r[] in registers
-                  if (col0 + j < N) crow[j] = __float2bfloat16(__uint_as_float(r[j]));
+            for (int v = 0; v < 4; ++v) {
+              const uint32_t* x = &r[j][8 * v];
+              uint4 o;
+              o.x = pack_bf16x2(__uint_as_float(x[0]), __uint_as_float(x[1]));
+              o.y = pack_bf16x2(__uint_as_float(x[2]), __uint_as_float(x[3]));
+              o.z = pack_bf16x2(__uint_as_float(x[4]), __uint_as_float(x[5]));
+              o.w = pack_bf16x2(__uint_as_float(x[6]), __uint_as_float(x[7]));
+              reinterpret_cast<uint4*>(blk + lane * 64)[v ^ ((lane >> 1) & 3)] = o;
             }
-          }
-        }
-        if (EPI == kEpiAccumF32 && m0 + ew * 32 < M && col0 < N) {
-          // fp32 output: the warp's 32x32 block goes through shared memory (128-byte rows, 16-byte chunks
-          // XOR-swizzled by row so that the 32 row-writes of one instruction spread over all banks) and leaves
-          // as one TMA store, or one TMA reduce-add when accumulating: C is never read into the SM, the stores
-          // are full lines, and the tensor map clips ragged edges.
-          float* cbuf = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + 1024 +
-                                                 (ew * 2 + (c & 1)) * C_STAGE_BYTES);
-          bulk_wait_group_read<1>();               // the store that last used this buffer has read it
-          __syncwarp();
+          } else {
+            // 128-byte rows, 16-byte chunks XOR-swizzled by row
 #pragma unroll
-          for (int v = 0; v < 8; ++v) {
-            const float4 o = make_float4(__uint_as_float(r[4 * v + 0]), __uint_as_float(r[4 * v + 1]),
-                                         __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-            reinterpret_cast<float4*>(cbuf + lane * 32)[v ^ (lane & 7)] = o;
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (accumulate) tma_reduce_add_2d_bulk(&tmap_c, cbuf, col0, m0 + ew * 32);
-            else tma_store_2d_bulk(&tmap_c, cbuf, col0, m0 + ew * 32);
-            bulk_commit_group();
+            for (int v = 0; v < 8; ++v)
+              reinterpret_cast<uint4*>(blk + lane * 128)[v ^ (lane & 7)] =
+                  make_uint4(r[j][4 * v], r[j][4 * v + 1], r[j][4 * v + 2], r[j][4 * v + 3]);
           }
         }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          // the tensor map clips ragged edges; a reduce-add never reads C into the SM
+#pragma unroll
+          for (int j = 0; j < CHUNKS; ++j) {
+            const int col0 = n0 + (c + 2 * j) * 32;
+            if (j > 0 && (c + 2 * j >= width / 32 || col0 >= p.N)) continue;
+            if (EPI == kEpiAccumF32 && p.accumulate) tma_reduce_add_2d_bulk(&tmap_c, stage + j * BLOCK, col0, row0);
+            else tma_store_2d_bulk(&tmap_c, stage + j * BLOCK, col0, row0);
+          }
+          bulk_commit_group();
+        }
+        if (p.c_bufs == 2) stage = stage == stage0 ? stage0 + C_STAGE_BYTES : stage0;
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
+      if (lane == 0) {
+        if (CTAS == 2) mbar_arrive_cluster(mapa_u32(smem_u32(&bars->acc_empty[acc]), 0));
+        else mbar_arrive(&bars->acc_empty[acc]);
+      }
     }
-    if (EPI == kEpiAccumF32 && lane == 0) bulk_wait_group<0>();   // staged blocks must leave before the CTA does
+    if (lane == 0) bulk_wait_group<0>();         // staged blocks must leave before the CTA does
   }
 
   tc_fence_before();
-  __syncthreads();
+  if (CTAS == 2) cluster_sync(); else __syncthreads();
   if (warp == 2) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, ACC_BUFS * BN);
+    tmem_dealloc_n<CTAS>(tmem_base, 512);
   }
-  if (sched != nullptr && threadIdx.x == 0) {
-    // the last CTA to leave rearms the scheduler slot for its next use
-    if (atomicAdd(&sched[1], 1) == static_cast<int>(gridDim.x) - 1) {
-      sched[0] = 0;
-      sched[1] = 0;
+  if (p.sched != nullptr && threadIdx.x == 0) {
+    if (atomicAdd(&p.sched[1], 1) == static_cast<int>(gridDim.x) - 1) {   // last CTA rearms the scheduler slot
+      p.sched[0] = 0;
+      p.sched[1] = 0;
       __threadfence();
     }
   }
@@ -302,26 +339,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 constexpr int kSchedSlots = 4096;
 
 int* next_sched_slot() {
-  static int* pool = nullptr;
-  static unsigned long long counter = 0;
-  static bool disabled = false;
-  if (disabled) return nullptr;
-  if (pool == nullptr) {
+  static int* const pool = []() -> int* {
     const char* env = getenv("PIPER_GEMM_STATIC_TILES");
-    if (env != nullptr && env[0] == '1') {
-      disabled = true;
+    if (env != nullptr && env[0] == '1') return nullptr;
+    int* p = nullptr;
+    if (cudaMalloc(&p, kSchedSlots * 2 * sizeof(int)) != cudaSuccess ||
+        cudaMemset(p, 0, kSchedSlots * 2 * sizeof(int)) != cudaSuccess)
       return nullptr;
-    }
-    if (cudaMalloc(&pool, kSchedSlots * 2 * sizeof(int)) != cudaSuccess ||
-        cudaMemset(pool, 0, kSchedSlots * 2 * sizeof(int)) != cudaSuccess) {
-      pool = nullptr;
-      disabled = true;
-      return nullptr;
-    }
-  }
-  return pool + 2 * (counter++ % kSchedSlots);
+    return p;
+  }();
+  static std::atomic<unsigned long long> counter{0};
+  return pool == nullptr ? nullptr : pool + 2 * (counter++ % kSchedSlots);
 }
 
+// cuTensorMapEncodeTiled through the runtime's driver entry point, so the
+// library does not link against libcuda directly.
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
 // library does not link against libcuda directly.
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -380,27 +412,60 @@ int make_tmap_c_f32(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <bool A_MN, bool B_MN, int EPI>
-static int launch(const GemmArgs& g, const CUtensorMap& ta, const CUtensorMap& tb, int num_sms,
+// bf16 tensor map of C with 32x32 boxes and 64-byte swizzle.
+static int make_tmap_c_bf16(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t row_stride_bytes) {
+  EncodeFn fn = get_encode_fn();
+  if (fn == nullptr) return -1;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {row_stride_bytes};
+  const cuuint32_t box[2] = {32, 32};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+
+template <int CTAS, bool A_MN, bool B_MN, int EPI>
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int num_sms,
                   cudaStream_t stream) {
-  auto kern = gemm_kernel<A_MN, B_MN, EPI>;
-  constexpr int smem_bytes = EPI == kEpiAccumF32 ? SMEM_BYTES_F32 : SMEM_BYTES;
+  auto kern = gemm_kernel<CTAS, A_MN, B_MN, EPI>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
-      return -2;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -2;
     configured = true;
   }
-  CUtensorMap tc = ta;      // unused by the bf16 epilogue
-  if (EPI == kEpiAccumF32) {
-    const int rc = make_tmap_c_f32(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 4);
-    if (rc != 0) return rc;
+  const int tiles = ((p.M + BM * CTAS - 1) / (BM * CTAS)) * ((p.N + p.width - 1) / p.width);
+  const int units = num_sms / CTAS;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(CTAS * (tiles < units ? tiles : units)));
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CTAS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p) == cudaSuccess ? 0 : -3;
+}
+
+template <int CTAS>
+static int launch_layout(const GemmArgs& g, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
+                         const Params& p, int num_sms, cudaStream_t stream) {
+  const int key = (g.a_mn_major ? 4 : 0) | (g.b_mn_major ? 2 : 0) | (g.epilogue == kEpiAccumF32 ? 1 : 0);
+  switch (key) {
+    case 0: return launch<CTAS, false, false, kEpiStoreBf16>(ta, tb, tc, p, num_sms, stream);
+    case 1: return launch<CTAS, false, false, kEpiAccumF32>(ta, tb, tc, p, num_sms, stream);
+    case 2: return launch<CTAS, false, true, kEpiStoreBf16>(ta, tb, tc, p, num_sms, stream);
+    case 3: return launch<CTAS, false, true, kEpiAccumF32>(ta, tb, tc, p, num_sms, stream);
+    case 4: return launch<CTAS, true, false, kEpiStoreBf16>(ta, tb, tc, p, num_sms, stream);
+    case 5: return launch<CTAS, true, false, kEpiAccumF32>(ta, tb, tc, p, num_sms, stream);
+    case 6: return launch<CTAS, true, true, kEpiStoreBf16>(ta, tb, tc, p, num_sms, stream);
+    default: return launch<CTAS, true, true, kEpiAccumF32>(ta, tb, tc, p, num_sms, stream);
   }
-  const int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
-  const int grid = tiles < num_sms ? tiles : num_sms;
-  kern<<<grid, NUM_THREADS, smem_bytes, stream>>>(ta, tb, tc, g.c, g.ldc, g.M, g.N, g.K, g.accumulate,
-                                                  g.status, next_sched_slot());
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 // 0: choose by shape, 128 / 256: forced by PIPER_GEMM_TILE
@@ -414,53 +479,103 @@ static int forced_tile() {
   return v;
 }
 
-// 256x256 tiles move a third fewer operand bytes per flop: measured on B200, they keep the tensor pipe 81 % busy where
-// 128x256 tiles reach 74 %.  They also come in fewer, larger pieces.  The time is taken as rounds of tiles over the SMs
-// times the cost of a tile (1 against 0.5 x 81 / 74 = 0.547), and the smaller one runs: of 640 small tiles in five rounds
-// and 320 big ones in three, the small ones (2.74 < 3; 137 against 167 us for 4096 x 5120 x 4096).
-// A single round of big tiles hides neither its first loads nor its epilogue, where two rounds of small ones overlap
-// both, and a second round that is nearly empty runs faster than a full one.  So it is taken only for long contractions
-// over well-filled SMs: at 128 tiles on 148 SMs big against small tiles measured 0.92-0.96 as fast for K = 512,
-// 0.98-1.00 for 2048, 1.00-1.06 for 4096 and 1.10-1.11 for 8192; at 76 to 98 tiles 0.97-1.00 for 4096, 1.03-1.09 for 8192.
-// Wide fp32 (weight-gradient) outputs always take the small tiles: their double-buffered accumulators hide the
-// reduce-adds.
+// The height of a tile of full width: 256 rows by a CTA pair or 128 by one CTA.  Pairs load a third fewer operand bytes
+// per flop and draw less power (4096 x 28672 x 4096 in a long loop 733 us with one CTA per tile, 690 us in pairs), but
+// every tile costs the pair a hand-over between the SMs (1.5 us more for one small tile, 1024 x 4096 x 4096 25.5 and 27.6
+// us).  So they are taken where there are rounds enough: by the number of rounds if all SMs had a 256 x 256 tile each, and
+// in a single such round for long contractions over well-filled SMs.  Wide fp32 outputs (weight gradients that add into
+// a bucket) of fewer than two rounds take the small tiles.
 int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms) {
   const long long n_tiles = (N + 255) / 256;
   const long long tiles256 = (M + 255) / 256 * n_tiles;
   const long long rounds256 = (tiles256 + num_sms - 1) / num_sms;
   const long long rounds128 = ((M + 127) / 128 * n_tiles + num_sms - 1) / num_sms;
-  const bool fits = M >= 256 && N >= 256 && rounds256 * 1000 < rounds128 * 547;
+  const bool fits = M >= 256 && N >= 256 && rounds256 * 1000 < rounds128 * 599;
   const bool fills = tiles256 >= num_sms || tiles256 * K >= 3072ll * num_sms;
-  const bool pays = !f32_out || M >= N;
+  const bool pays = !f32_out || M >= N || tiles256 >= 2 * num_sms;
   return fits && fills && pays ? 256 : 128;
+}
+
+// Cycles of a launch, up to what all shapes have in common: rounds of tiles over the SMs (or pairs), each as long as the
+// MMAs of its k-blocks, the fill of their operands from L2 (65 bytes per cycle and SM) or the epilogue of the tile
+// before it, and the last epilogue and the start, which is longer for a pair.  The constants are fitted to 89 launches
+// in all widths by one CTA and by two (outputs from 100 x 688 to 28672 x 4096, K from 64 to 32000, all layouts, bf16 and
+// fp32): the shape it picks is 1.4 % behind the fastest of the sixteen on average, 13 % at most (few tiles over a long
+// contraction), where 256 columns throughout are 18 % behind in pairs and 22 % by single CTAs.  Narrower tiles even out the last round: 4096 x 5120 x
+// 2048 in 23 x 16 tiles of 224 columns 60.8 us, in 20 x 16 of 256 columns 62.9 us; 1000 x 3072 x 8192 in 64 tiles of 192 columns
+// 43.3 us, in 48 of 256 columns 49.8 us; and a small problem covers more SMs: 512 x 768 x 256 8.1 and 10.0 us.
+static double gemm_cost(int M, int N, int K, bool b_mn, bool f32_out, int ctas, int width, int num_sms) {
+  const double k_blocks = (K + BK - 1) / BK;
+  const long long tiles = static_cast<long long>((M + BM * ctas - 1) / (BM * ctas)) * ((N + width - 1) / width);
+  const long long units = num_sms / ctas;
+  const double rounds = static_cast<double>((tiles + units - 1) / units);
+  const int b_rows = b_mn ? (width / ctas + 63) / 64 * 64 : width / ctas;
+  const double block = std::max(2.0 * width, (BM + b_rows) * 128 / 65.0);
+  const double epilogue = 1500 + (f32_out ? 12 : 8) * width;
+  return rounds * std::max(k_blocks * block, epilogue) + epilogue + (ctas == 2 ? 4000 : 2000);
+}
+
+GemmShape gemm_shape(int M, int N, int K, bool b_mn, bool f32_out, int num_sms) {
+  GemmShape best[2] = {{1, 256}, {2, 256}};
+  double cost[2];
+  for (int i = 0; i < 2; ++i) {
+    for (int width = 256; width >= 32; width -= 32) {
+      const double c = num_sms <= i ? 1e300 : gemm_cost(M, N, K, b_mn, f32_out, i + 1, width, num_sms);
+      if (width == 256 || c < cost[i]) {
+        cost[i] = c;
+        best[i].width = width;
+      }
+    }
+  }
+  // within 3 % of one another the model does not tell them apart
+  const bool close = std::max(cost[0], cost[1]) < 1.03 * std::min(cost[0], cost[1]);
+  const bool pair = close ? gemm_tile_rows(M, N, K, f32_out, num_sms) == 256 : cost[1] < cost[0];
+  return best[pair ? 1 : 0];
 }
 
 int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 0;
-  int tile = g.tile != 0 ? g.tile : forced_tile();
-  if (tile == 0) tile = gemm_tile_rows(g.M, g.N, g.K, g.epilogue != kEpiStoreBf16, num_sms);
-  if (tile == 256) return gemm256_bf16_launch(g, num_sms, next_sched_slot(), stream);
-  CUtensorMap ta, tb;
+  const int tile = g.tile != 0 ? g.tile : forced_tile();
+  GemmShape shape = {tile / 128, g.width != 0 ? g.width : 256};
+  if (tile == 0) shape = gemm_shape(g.M, g.N, g.K, g.b_mn_major != 0, g.epilogue != kEpiStoreBf16, num_sms);
+  if (shape.ctas < 1 || shape.ctas > 2 || shape.width < 32 || shape.width > 256 || shape.width % 32 != 0) return -1;
+  if (num_sms < 2) shape.ctas = 1;
+  const uint32_t b_rows = shape.width / shape.ctas;
+  CUtensorMap ta, tb, tc;
   int rc;
-  // K-major operand: dims {K, rows}, box {64, tile rows}.
-  // MN-major operand: dims {rows, K}, box {64, 64}.
+  // K-major operand: dims {K, rows}, box {64, rows of a CTA}; MN-major operand: dims {rows, K}, box {64, 64}.
   rc = g.a_mn_major ? make_tmap_2d_bf16(&ta, g.a, g.M, g.K, g.lda * 2, 64, BK)
                     : make_tmap_2d_bf16(&ta, g.a, g.K, g.M, g.lda * 2, BK, BM);
   if (rc != 0) return rc;
   rc = g.b_mn_major ? make_tmap_2d_bf16(&tb, g.b, g.N, g.K, g.ldb * 2, 64, BK)
-                    : make_tmap_2d_bf16(&tb, g.b, g.K, g.N, g.ldb * 2, BK, BN);
+                    : make_tmap_2d_bf16(&tb, g.b, g.K, g.N, g.ldb * 2, BK, b_rows);
   if (rc != 0) return rc;
-  const int key = (g.a_mn_major ? 4 : 0) | (g.b_mn_major ? 2 : 0) | (g.epilogue == kEpiAccumF32 ? 1 : 0);
-  switch (key) {
-    case 0: return launch<false, false, kEpiStoreBf16>(g, ta, tb, num_sms, stream);
-    case 1: return launch<false, false, kEpiAccumF32>(g, ta, tb, num_sms, stream);
-    case 2: return launch<false, true, kEpiStoreBf16>(g, ta, tb, num_sms, stream);
-    case 3: return launch<false, true, kEpiAccumF32>(g, ta, tb, num_sms, stream);
-    case 4: return launch<true, false, kEpiStoreBf16>(g, ta, tb, num_sms, stream);
-    case 5: return launch<true, false, kEpiAccumF32>(g, ta, tb, num_sms, stream);
-    case 6: return launch<true, true, kEpiStoreBf16>(g, ta, tb, num_sms, stream);
-    default: return launch<true, true, kEpiAccumF32>(g, ta, tb, num_sms, stream);
-  }
+  rc = g.epilogue == kEpiAccumF32 ? make_tmap_c_f32(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 4)
+                                  : make_tmap_c_bf16(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 2);
+  if (rc != 0) return rc;
+  const int stage = A_STAGE_BYTES + (g.b_mn_major ? (b_rows + 63) / 64 * MN_BOX_BYTES : b_rows * BK * 2);
+  Params p;
+  // Contractions over a few k-blocks wait for their epilogues, above all for fp32 reduce-adds; two blocks in flight per
+  // warp cost a stage or two that they do not fill (3840 x 5760 x 152 into fp32 26.1 and 23.4 us).
+  p.c_bufs = g.epilogue == kEpiAccumF32 && g.K <= 8 * BK ? 2 : 1;
+  const int fit = (OPERAND_BYTES - (p.c_bufs - 1) * EPI_WARPS * C_STAGE_BYTES) / stage;
+  p.M = g.M;
+  p.N = g.N;
+  p.K = g.K;
+  p.width = shape.width;
+  p.stages = fit < MAX_STAGES ? fit : MAX_STAGES;
+  p.accumulate = g.accumulate;
+  const int tiles_m = (g.M + BM * shape.ctas - 1) / (BM * shape.ctas), tiles_n = (g.N + shape.width - 1) / shape.width;
+  // An operand that stays in L2 (126 MB) is best read whole by every wave (4096 x 28672 x 4096: 701 us, in bands of 8
+  // 717 us); one that does not is read from DRAM again by each, and bands of 8 tiles make the wave square (4096 x 4096 x
+  // 28672: 799 and 761 us, x 14336: 389 and 381 us).
+  const bool n_fast = tiles_n < tiles_m;
+  const long long fast_bytes = 2ll * (n_fast ? g.N : g.M) * g.K;
+  p.band = fast_bytes > (96ll << 20) ? 8 : (n_fast ? tiles_n : tiles_m);
+  p.status = g.status;
+  p.sched = next_sched_slot();
+  return shape.ctas == 2 ? launch_layout<2>(g, ta, tb, tc, p, num_sms, stream)
+                         : launch_layout<1>(g, ta, tb, tc, p, num_sms, stream);
 }
 
 }  // namespace piper

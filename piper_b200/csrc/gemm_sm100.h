@@ -30,20 +30,22 @@ struct GemmArgs {
   int epilogue;     // kEpi*
   int accumulate;   // only for kEpiAccumF32
   int* status;      // device int, 0 = ok (see ptx.cuh)
-  int tile = 0;     // 0: chosen by shape (or PIPER_GEMM_TILE); 128 / 256: that CTA tile height
+  int tile = 0;     // 0: chosen by shape (or PIPER_GEMM_TILE); 128: one CTA per tile, 256: a CTA pair
+  int width = 0;    // with tile != 0: columns of a tile, a multiple of 32 up to 256 (0: 256)
 };
 
 // Returns 0 on success, a negative code for a launch/set-up failure, or the
 // CUresult of a failed tensor-map encode.
 int gemm_bf16_launch(const GemmArgs& args, int num_sms, cudaStream_t stream);
 
-// The CTA tile height (128 or 256) that gemm_bf16_launch chooses for an [M, N] output and a contraction over K.
+// The tile height (128: one CTA, 256: a CTA pair) that suits an [M, N] output in tiles of full width.
 int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms);
 
-// Same contract with 256x256 tiles per CTA (gemm256_sm100.cu).  sched: two zeroed ints of device memory for the
-// dynamic tile scheduler (rearmed by the kernel), or null for static tile striding.  gemm_bf16_launch picks
-// between the two tile shapes; PIPER_GEMM_TILE=128 or 256 forces one.
-int gemm256_bf16_launch(const GemmArgs& args, int num_sms, int* sched, cudaStream_t stream);
+// The tile shape that gemm_bf16_launch chooses: CTAs per tile (1 or 2, 128 rows each) and columns.
+struct GemmShape {
+  int ctas, width;
+};
+GemmShape gemm_shape(int M, int N, int K, bool b_mn_major, bool f32_out, int num_sms);
 
 enum : int {
   kGroupedFwd = 0,     // Y[rows, N]  = X[rows, K] * W[e]^T

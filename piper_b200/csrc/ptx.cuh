@@ -288,6 +288,116 @@ __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// ------------------------------------------------------ CTA pairs
+// A pair is a cluster of two CTAs on neighbouring SMs that share one tcgen05.mma (cta_group::2): rows 0-127 of A and D
+// and the first half of B's rows belong to the CTA of rank 0, which issues, the rest to the other.  Loads into either
+// CTA report to the barrier of rank 0; commits arrive at the same barrier of both.  The _n<CTAS> forms are the plain
+// ones for CTAS == 1.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Address of `smem_addr` of this CTA in the shared memory of the cluster's CTA `rank`.
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  return a;
+}
+
+__device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
+// mbar_wait on a barrier of this CTA that threads of the other CTA arrive at.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status) {
+  for (uint32_t i = 0; i < kMaxMbarPolls; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((i & 1023u) == 1023u && status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) return false;
+  }
+  if (status != nullptr) atomicCAS(status, 0, kStatusMbarTimeout);
+  return false;
+}
+
+template <int CTAS>
+__device__ __forceinline__ void tma_load_2d_n(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
+  if (CTAS == 1) {
+    tma_load_2d(smem_dst, m, bar, x, y);
+  } else {
+    // bit 24 of a shared::cluster address selects the CTA of the pair: cleared, the barrier is that of rank 0
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar) & 0xFEFFFFFFu), "r"(x), "r"(y)
+        : "memory");
+  }
+}
+
+template <int CTAS>
+__device__ __forceinline__ void tmem_alloc_n(uint32_t* smem_result, uint32_t ncols) {
+  if (CTAS == 1)
+    tmem_alloc(smem_result, ncols);
+  else
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
+                 "r"(ncols)
+                 : "memory");
+}
+
+template <int CTAS>
+__device__ __forceinline__ void tmem_relinquish_n() {
+  if (CTAS == 1) tmem_relinquish();
+  else asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+template <int CTAS>
+__device__ __forceinline__ void tmem_dealloc_n(uint32_t taddr, uint32_t ncols) {
+  if (CTAS == 1) tmem_dealloc(taddr, ncols);
+  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+template <int CTAS>
+__device__ __forceinline__ void umma_bf16_ss_n(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                               uint32_t accumulate) {
+  if (CTAS == 1)
+    umma_bf16_ss(tmem_d, desc_a, desc_b, idesc, accumulate);
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+template <int CTAS>
+__device__ __forceinline__ void umma_commit_n(uint64_t* bar) {
+  if (CTAS == 1)
+    umma_commit(bar);
+  else
+    asm volatile(
+        "{\n\t.reg .b16 both;\n\tmov.b16 both, 3;\n\t"
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n\t}"
+        ::"r"(smem_u32(bar))
+        : "memory");
+}
+
 // ------------------------------------------------------ UMMA descriptors
 // 64-bit shared-memory matrix descriptor for the 128-byte-swizzle layouts.
 //   K-major operand : rows of 128 B (64 bf16 along K), 8-row groups 1024 B

@@ -41,7 +41,7 @@ def main(argv=None):
     ap.add_argument("--iters", type=int, default=10)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--no-cublas", action="store_true", help="skip the library GEMM comparison")
-    ap.add_argument("--tile", type=int, default=0, choices=(0, 128, 256), help="force the GEMM CTA tile height")
+    ap.add_argument("--tile", type=int, default=0, choices=(0, 128, 256), help="force the GEMM tile height (256: a CTA pair)")
     args = ap.parse_args(argv)
     global _time
     _base_time = _time

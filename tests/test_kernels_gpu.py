@@ -141,6 +141,38 @@ def test_gemm_tile_choice_does_not_change_the_result(M, N, K, bf16_tile, f32_til
         assert torch.equal(auto, small) and torch.equal(auto, big)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 40, 24), (129, 72, 8), (256, 256, 64), (513, 1000, 1000), (2304, 4608, 192)])
+@pytest.mark.parametrize("tile", [128, 256])
+def test_gemm_shapes_give_the_same_bits(M, N, K, tile):
+    """Every tile width by one CTA and by a pair, in every operand layout and both output types (K = 192 and less: two
+    staging blocks per fp32 epilogue warp, K = 1000: one): less than a tile, remainders of rows (a pair whose second CTA
+    has none), columns and k-blocks, more tiles than SMs.  fp32 sums of K bf16 products: 2^-8 covers the rounding of the
+    bf16 result, and all shapes add in one order."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(21)
+    lib, st = native.lib(), native.status_tensor()
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    layouts = [(x, xm, y, ym) for x, xm in ((a, False), (a.t().contiguous(), True))
+               for y, ym in ((b, False), (b.t().contiguous(), True)) if not xm or M % 8 == 0]
+    ref = a.float() @ b.float().t()
+    held = torch.randn(M, N, device="cuda")
+    first = None
+    for x, xm, y, ym in layouts:
+        for width in range(32, 257, 32):
+            outs = (torch.full((M, N + 8), 7.0, device="cuda", dtype=torch.bfloat16), torch.full((M, N + 8), 7.0, device="cuda"),
+                    torch.nn.functional.pad(held, (0, 8), value=7.0))
+            for out, add in zip(outs, (False, False, True)):
+                lib.gemm_shaped(x, y, out[:, :N], xm, ym, add, st, tile, width)
+                assert (out[:, N:] == 7).all()                 # nothing beyond the last column
+            if first is None:
+                first = outs
+                assert _close(outs[0][:, :N], ref, 2 ** -8) and _close(outs[1][:, :N], ref, 1e-5)
+                assert _close(outs[2][:, :N], ref + held, 1e-5)
+            assert all(torch.equal(o, f) for o, f in zip(outs, first)), (xm, ym, width)
+
+
 @pytest.mark.parametrize("sizes,forked", [((4095,), []), ((4096,), [4096]), ((4096, 4095), [4096, 4095]),
                                           ((4095, 4096), [4096])])
 def test_linear_gradients_around_the_fork_threshold(sizes, forked, monkeypatch):

@@ -72,6 +72,26 @@ def test_gemm_tile_rule(M, N, K, f32, sms, rows):
     assert native.lib().gemm_tile_rows(M, N, K, f32, sms) == rows
 
 
+@pytest.mark.parametrize("M,N,K,b_mn,f32,sms,shape", [
+    (1, 8, 8, False, False, 148, (1, 32)),                    # one tile: the narrowest
+    (512, 768, 256, False, False, 148, (1, 32)),              # 96 tiles on as many SMs
+    (128, 16384, 2048, False, False, 148, (1, 128)),          # 128 tiles in one round
+    (200, 8192, 3072, False, False, 148, (2, 128)),           # the same with two rows of tiles: pairs
+    (1000, 3072, 8192, False, False, 148, (2, 192)),          # 64 pairs of 192 columns in one round, 48 of 256 in one
+    (1000, 8192, 3072, True, False, 148, (2, 224)),           # 148 pairs in two rounds exactly
+    (4096, 28672, 4096, False, False, 148, (2, 256)), (28672, 4096, 4096, True, True, 148, (2, 256)),
+    (4096, 28672, 4096, False, False, 1, (1, 256)),           # no pairs on a single SM
+    (2048, 2048, 576, False, False, 148, (1, 256)),           # near ties: by gemm_tile_rows, which has 128 rows here
+    (8192, 8192, 320, False, False, 148, (2, 256)),           # and 256 here
+])
+def test_gemm_shape_rule(M, N, K, b_mn, f32, sms, shape):
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    assert tuple(native.lib().gemm_shape(M, N, K, b_mn, f32, sms)) == shape
+
+
 @pytest.mark.parametrize("B,S,Hq,sms,tiles", [
     (1, 128, 148, 148, 1), (1, 128, 149, 148, 2),         # an SM for every tile, and one too few (one block each)
     (1, 512, 44, 148, 1), (1, 512, 45, 148, 2),           # 440 of 444 block times in which the longest tile is done
