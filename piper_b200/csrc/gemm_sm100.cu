@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <cstdlib>
 
 #include "ptx.cuh"
@@ -48,7 +49,7 @@ constexpr int EPI_WARPS = 8;
 constexpr int NUM_THREADS = 128 + 32 * EPI_WARPS;
 constexpr int C_STAGE_BYTES = 4096;            // per epilogue warp: two bf16 or one fp32 block of 32 x 32
 constexpr int BAR_OFF = OPERAND_BYTES + EPI_WARPS * C_STAGE_BYTES;
-constexpr int SMEM_BYTES = BAR_OFF + 512 + 1024;
+constexpr int SMEM_BYTES = BAR_OFF + 768 + 1024;
 constexpr int RING = 16;                       // tiles handed out ahead: at most the stages + 2 accumulators + 1
 
 struct Bars {
@@ -57,10 +58,10 @@ struct Bars {
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t tile_full[RING];
-  int tile[RING];
+  int tile[RING][4];         // the tile's number in the first word
   uint32_t tmem_base;
 };
-static_assert(sizeof(Bars) <= 512, "barriers");
+static_assert(sizeof(Bars) <= 768 && offsetof(Bars, tile) % 16 == 0 && SMEM_BYTES <= 232448, "shared memory");
 
 struct Params {
   int M, N, K;
@@ -131,9 +132,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   };
   // The n-th tile of this CTA (or pair), -1 behind the last one.
   auto tile_at = [&](uint32_t n, int& tile) -> bool {
-    const bool got = CTAS == 2 ? mbar_wait_cluster(&bars->tile_full[n % RING], (n / RING) & 1, p.status)
-                               : mbar_wait(&bars->tile_full[n % RING], (n / RING) & 1, p.status);
-    if (!__all_sync(0xffffffffu, got)) return false;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bars->tile_full[n % RING], (n / RING) & 1, p.status))) return false;
     tile = *reinterpret_cast<volatile int*>(&bars->tile[n % RING]);
     return true;
   };
@@ -146,15 +145,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     bool ok = true;
     for (;; ++n) {
       if (rank == 0 && elect_one()) {
-        int next = p.sched != nullptr ? atomicAdd(&p.sched[0], 1)
-                                      : static_cast<int>(blockIdx.x / CTAS + n * (gridDim.x / CTAS));
+        // the first tile is the number of the CTA (or pair), the next ones come from a counter
+        const int units = static_cast<int>(gridDim.x) / CTAS;
+        int next = n == 0 || p.sched == nullptr || num_tiles <= units
+                       ? static_cast<int>(blockIdx.x) / CTAS + static_cast<int>(n) * units
+                       : units + atomicAdd(&p.sched[0], 1);
         if (next >= num_tiles) next = -1;
-        bars->tile[n % RING] = next;
-        if (CTAS == 2) {
-          st_cluster_u32(mapa_u32(smem_u32(&bars->tile[n % RING]), 1), static_cast<uint32_t>(next));
-          mbar_arrive_cluster(mapa_u32(smem_u32(&bars->tile_full[n % RING]), 1));
-        }
+        bars->tile[n % RING][0] = next;
+        if (CTAS == 2)
+          st_async_v4(mapa_u32(smem_u32(&bars->tile[n % RING]), 1), mapa_u32(smem_u32(&bars->tile_full[n % RING]), 1),
+                      next, 0, 0, 0);
         mbar_arrive(&bars->tile_full[n % RING]);
+      } else if (rank == 1 && elect_one()) {
+        mbar_arrive_expect_tx(&bars->tile_full[n % RING], 16);
       }
       __syncwarp();
       int tile;
@@ -216,9 +219,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         int tile;
         if (!(ok = tile_at(n, tile)) || tile < 0) break;
         const uint32_t acc = n & 1;
-        if (!(ok = __all_sync(0xffffffffu, CTAS == 2 ? mbar_wait_cluster(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status)
-                                                     : mbar_wait(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status))))
-          break;
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status)))) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * 256;
         for (int kb = 0; kb < k_blocks; ++kb) {
@@ -334,24 +335,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   }
 }
 
-// Pool of tile-scheduler slots (next tile, finished CTAs), one slot per launch in rotation.  It is the only
-// device memory this library allocates by itself: 32 KiB, once per process.
-constexpr int kSchedSlots = 4096;
-
-int* next_sched_slot() {
-  static int* const pool = []() -> int* {
-    const char* env = getenv("PIPER_GEMM_STATIC_TILES");
-    if (env != nullptr && env[0] == '1') return nullptr;
-    int* p = nullptr;
-    if (cudaMalloc(&p, kSchedSlots * 2 * sizeof(int)) != cudaSuccess ||
-        cudaMemset(p, 0, kSchedSlots * 2 * sizeof(int)) != cudaSuccess)
-      return nullptr;
-    return p;
-  }();
-  static std::atomic<unsigned long long> counter{0};
-  return pool == nullptr ? nullptr : pool + 2 * (counter++ % kSchedSlots);
-}
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
 // library does not link against libcuda directly.
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
@@ -375,6 +358,24 @@ EncodeFn get_encode_fn() {
 }
 
 }  // namespace
+
+// Pool of tile-scheduler slots (next tile, finished CTAs), one slot per launch in rotation.  It is the only
+// device memory this library allocates by itself: 32 KiB, once per process.
+constexpr int kSchedSlots = 4096;
+
+int* gemm_sched_slot() {
+  static int* const pool = []() -> int* {
+    const char* env = getenv("PIPER_GEMM_STATIC_TILES");
+    if (env != nullptr && env[0] == '1') return nullptr;
+    int* p = nullptr;
+    if (cudaMalloc(&p, kSchedSlots * 2 * sizeof(int)) != cudaSuccess ||
+        cudaMemset(p, 0, kSchedSlots * 2 * sizeof(int)) != cudaSuccess)
+      return nullptr;
+    return p;
+  }();
+  static std::atomic<unsigned long long> counter{0};
+  return pool == nullptr ? nullptr : pool + 2 * (counter++ % kSchedSlots);
+}
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer) {
@@ -481,8 +482,8 @@ static int forced_tile() {
 
 // The height of a tile of full width: 256 rows by a CTA pair or 128 by one CTA.  Pairs load a third fewer operand bytes
 // per flop and draw less power (4096 x 28672 x 4096 in a long loop 733 us with one CTA per tile, 690 us in pairs), but
-// every tile costs the pair a hand-over between the SMs (1.5 us more for one small tile, 1024 x 4096 x 4096 25.5 and 27.6
-// us).  So they are taken where there are rounds enough: by the number of rounds if all SMs had a 256 x 256 tile each, and
+// a pair starts later and hands every tile over between its SMs (512 x 768 x 256 5.2 us and 6.0 us, 1024 x 4096 x 4096
+// 25.8 and 26.4 us).  So they are taken where there are rounds enough: by the number of rounds if all SMs had a 256 x 256 tile each, and
 // in a single such round for long contractions over well-filled SMs.  Wide fp32 outputs (weight gradients that add into
 // a bucket) of fewer than two rounds take the small tiles.
 int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms) {
@@ -500,10 +501,10 @@ int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms) {
 // MMAs of its k-blocks, the fill of their operands from L2 (65 bytes per cycle and SM) or the epilogue of the tile
 // before it, and the last epilogue and the start, which is longer for a pair.  The constants are fitted to 89 launches
 // in all widths by one CTA and by two (outputs from 100 x 688 to 28672 x 4096, K from 64 to 32000, all layouts, bf16 and
-// fp32): the shape it picks is 1.4 % behind the fastest of the sixteen on average, 13 % at most (few tiles over a long
-// contraction), where 256 columns throughout are 18 % behind in pairs and 22 % by single CTAs.  Narrower tiles even out the last round: 4096 x 5120 x
-// 2048 in 23 x 16 tiles of 224 columns 60.8 us, in 20 x 16 of 256 columns 62.9 us; 1000 x 3072 x 8192 in 64 tiles of 192 columns
-// 43.3 us, in 48 of 256 columns 49.8 us; and a small problem covers more SMs: 512 x 768 x 256 8.1 and 10.0 us.
+// fp32): the shape it picks is 1.1 % behind the fastest of the sixteen on average, 14 % at most (few tiles over a long
+// contraction), where 256 columns throughout are 17 % behind in pairs and 25 % by single CTAs.  Narrower tiles even out the last round: 4096 x 5120 x
+// 2048 in 23 x 16 tiles of 224 columns 56.3 us, in 20 x 16 of 256 columns 58.8 us; 1000 x 3072 x 8192 in 64 tiles of 192 columns
+// 37.6 us, in 48 of 256 columns 44.6 us; and a small problem covers more SMs: 512 x 768 x 256 5.2 and 7.2 us.
 static double gemm_cost(int M, int N, int K, bool b_mn, bool f32_out, int ctas, int width, int num_sms) {
   const double k_blocks = (K + BK - 1) / BK;
   const long long tiles = static_cast<long long>((M + BM * ctas - 1) / (BM * ctas)) * ((N + width - 1) / width);
@@ -511,8 +512,8 @@ static double gemm_cost(int M, int N, int K, bool b_mn, bool f32_out, int ctas, 
   const double rounds = static_cast<double>((tiles + units - 1) / units);
   const int b_rows = b_mn ? (width / ctas + 63) / 64 * 64 : width / ctas;
   const double block = std::max(2.0 * width, (BM + b_rows) * 128 / 65.0);
-  const double epilogue = 1500 + (f32_out ? 12 : 8) * width;
-  return rounds * std::max(k_blocks * block, epilogue) + epilogue + (ctas == 2 ? 4000 : 2000);
+  const double epilogue = 2000 + (f32_out ? 15 : 10) * width;
+  return rounds * std::max(k_blocks * block, epilogue) + epilogue + (ctas == 2 ? 2500 : 2000);
 }
 
 GemmShape gemm_shape(int M, int N, int K, bool b_mn, bool f32_out, int num_sms) {
@@ -573,7 +574,7 @@ int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
   const long long fast_bytes = 2ll * (n_fast ? g.N : g.M) * g.K;
   p.band = fast_bytes > (96ll << 20) ? 8 : (n_fast ? tiles_n : tiles_m);
   p.status = g.status;
-  p.sched = next_sched_slot();
+  p.sched = gemm_sched_slot();
   return shape.ctas == 2 ? launch_layout<2>(g, ta, tb, tc, p, num_sms, stream)
                          : launch_layout<1>(g, ta, tb, tc, p, num_sms, stream);
 }

@@ -77,6 +77,10 @@ struct GroupedGemmArgs {
 
 int grouped_gemm_launch(const GroupedGemmArgs& args, int num_sms, cudaStream_t stream);
 
+// Two zeroed ints of device memory for the dynamic tile scheduler of one launch (next tile, finished CTAs; rearmed by the
+// kernel), or null for static tile striding.
+int* gemm_sched_slot();
+
 constexpr int kMaxPeers = 8;
 
 // Y[M, N] = X[M, K] * W[N, K]^T with W sharded by rows: w_shards[p] points at

@@ -81,8 +81,8 @@ def test_gemm_tile_rule(M, N, K, f32, sms, rows):
     (1000, 8192, 3072, True, False, 148, (2, 224)),           # 148 pairs in two rounds exactly
     (4096, 28672, 4096, False, False, 148, (2, 256)), (28672, 4096, 4096, True, True, 148, (2, 256)),
     (4096, 28672, 4096, False, False, 1, (1, 256)),           # no pairs on a single SM
-    (2048, 2048, 576, False, False, 148, (1, 256)),           # near ties: by gemm_tile_rows, which has 128 rows here
-    (8192, 8192, 320, False, False, 148, (2, 256)),           # and 256 here
+    (2048, 2048, 448, False, False, 148, (1, 256)),           # near ties, by gemm_tile_rows: 128 rows where pairs cost less
+    (4096, 4096, 256, False, False, 148, (2, 256)),           # and 256 rows where they cost more
 ])
 def test_gemm_shape_rule(M, N, K, b_mn, f32, sms, shape):
     from piper_b200.ops import native
