@@ -150,6 +150,34 @@ def test_grouped_weight_gradient(N, K, sources):
     native.check_status()
 
 
+@pytest.mark.parametrize("E,N,K,sources", [(40, 520, 72, 1), (40, 264, 712, 2), (3, 128, 64, 2), (5, 72, 520, 1)])
+def test_grouped_products_by_pairs_and_single_ctas(E, N, K, sources):
+    """Forty experts take CTA pairs, a few single CTAs.  Ragged features on both sides, segments of no rows, one half
+    token tile, whole ones and both; rows outside every segment are left alone.  fp32 sums rounded once to bf16."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(5)
+    units = torch.tensor([0, 1, 2, 3, 5, 4])[torch.arange(E * sources) % 6]
+    g_len = (units * 128).to(torch.int32).cuda()
+    g_start = (torch.cumsum(g_len, 0) - g_len).to(torch.int32)
+    used, R = int(g_len.sum()), int(g_len.sum()) + 128
+    x = torch.randn(R, K, device="cuda").to(torch.bfloat16)
+    dy = torch.randn(R, N, device="cuda").to(torch.bfloat16)
+    w = torch.randn(E, N, K, device="cuda").to(torch.bfloat16)
+    y = torch.full((R, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    dx = torch.full((R, K), 7.0, device="cuda", dtype=torch.bfloat16)
+    lib, st = native.lib(), native.status_tensor()
+    lib.grouped_gemm(0, x, None, w, y, g_start, g_len, E, N, K, False, st)
+    lib.grouped_gemm(1, None, dy, w, dx, g_start, g_len, E, N, K, False, st)
+    native.check_status()
+    assert (y[used:] == 7).all() and (dx[used:] == 7).all()
+    for gi, (s, n) in enumerate(zip(g_start.tolist(), g_len.tolist())):
+        if n:
+            for got, want in ((y[s:s + n], x[s:s + n].double() @ w[gi % E].double().t()),
+                              (dx[s:s + n], dy[s:s + n].double() @ w[gi % E].double())):
+                assert ((got.double() - want).abs().max() / want.abs().max()) < 2 ** -8
+
+
 def test_qwen3_moe_model_trains_on_one_gpu():
     from piper_b200 import piper_exec_dag, piper_setup
     from piper_b200.models.qwen3 import PiperQwen3Model, Qwen3Config
