@@ -328,6 +328,7 @@ void attn_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, const Te
 
 #include "bindings_moe.inc"
 #include "bindings_fused.inc"
+#include "bindings_ops.inc"
 
 TORCH_LIBRARY(piper_c, m) {
   m.def("kernel_launch_count", &kernel_launch_count);
@@ -357,4 +358,5 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("attn_tiles_per_cta", &attn_tiles_per_cta);
   register_moe_ops(m);
   register_fused_ops(m);
+  register_native_ops(m);
 }

@@ -35,7 +35,7 @@ import torch
 from torch import Tensor
 
 from . import native
-from .registry import custom_op
+from .registry import custom_op, host_op
 
 # --------------------------------------------------------------------------
 # runtime state consulted by backward formulas
@@ -43,33 +43,55 @@ from .registry import custom_op
 
 
 class GradSinks:
-    """Maps a parameter's storage address to the fp32 buffer its gradient accumulates into."""
+    """Maps a parameter's storage address to the fp32 buffer its gradient accumulates into.  The native library keeps a
+    copy of this module's map for the formulas it runs."""
 
     def __init__(self) -> None:
         self._sinks: dict[int, Tensor] = {}
 
+    def _native(self):
+        return torch.ops.piper_c if native.loaded() and globals().get("grad_sinks") is self else None
+
     def register(self, param: Tensor, sink: Tensor) -> None:
         assert sink.dtype == torch.float32 and sink.numel() == param.numel()
-        self._sinks[param.data_ptr()] = sink.view(param.shape)
+        address = param.data_ptr()
+        self._sinks[address] = sink.view(param.shape)
+        if (lib := self._native()) is not None:
+            lib.sink_set.default(address, self._sinks[address])
 
     def unregister(self, param: Tensor) -> None:
-        self._sinks.pop(param.data_ptr(), None)
+        address = param.data_ptr()
+        if self._sinks.pop(address, None) is not None and (lib := self._native()) is not None:
+            lib.sink_unset.default(address)
 
     def get(self, param: Tensor) -> Optional[Tensor]:
         return self._sinks.get(param.data_ptr())
 
     def clear(self) -> None:
         self._sinks.clear()
+        if (lib := self._native()) is not None:
+            lib.sink_clear()
 
 
 grad_sinks = GradSinks()
+grad_sinks.clear()          # after a reload, the library's copy too
 
 
 class WgradStore:
     """Queue of deferred weight-gradient GEMMs of one backward-input pass: (thunk returning dW or None, weight)."""
 
     def __init__(self) -> None:
-        self.active: Optional[list] = None
+        self.active = None
+
+    @property
+    def active(self) -> Optional[list]:
+        return self._active
+
+    @active.setter
+    def active(self, queue: Optional[list]) -> None:
+        self._active = queue
+        if globals().get("wgrad_store", self) is self:
+            native.set_flag(native.DEFER_WGRAD, queue is not None)
 
     def begin(self) -> list:
         self.active = []
@@ -93,11 +115,37 @@ class WgradStore:
 
 
 wgrad_store = WgradStore()
+wgrad_store.active = None
+
+
+class _GatherGemms(dict):
+    """A dict that tells the native library whether it holds anything."""
+
+    def _changed(self) -> None:
+        if globals().get("gather_gemms") is self:
+            native.set_flag(native.GATHER_GEMMS, len(self) > 0)
+
+
+def _telling(name: str):
+    method = getattr(dict, name)
+
+    def changing(self, *args, **kwargs):
+        try:
+            return method(self, *args, **kwargs)
+        finally:
+            self._changed()
+
+    return changing
+
+
+for _name in ("__setitem__", "__delitem__", "pop", "popitem", "clear", "update", "setdefault", "__ior__"):
+    setattr(_GatherGemms, _name, _telling(_name))
 
 # ZeRO-3 with the fused lowering: weight address -> launcher of the GEMM that gathers that weight's rows from the
 # data-parallel peers while it multiplies by them (registered by ``parallel/fused.py`` when the parameters of a
 # segment are materialised, consumed by the first ``linear`` that uses the weight).
-gather_gemms: dict = {}
+gather_gemms: dict = _GatherGemms()
+gather_gemms.clear()
 
 
 def _is_native(t: Tensor) -> bool:
@@ -136,6 +184,9 @@ def linear(x: Tensor, w: Tensor) -> Tensor:
             _gemm(x2, w, y, False, False)
         return y.view(*x.shape[:-1], w.shape[0])
     return torch.nn.functional.linear(x, w)
+
+
+host_op("linear_host", linear._body)
 
 
 @linear.register_fake
@@ -206,6 +257,7 @@ class deferred_join:
                 cur.wait_stream(side)
             deferred_join.pending.clear()
             deferred_join.buckets.clear()
+            native.set_flag(native.FORK_PENDING, False)
         return False
 
 
@@ -250,6 +302,7 @@ def _linear_backward(ctx, dy):
             dy2.record_stream(side)
             deferred_join.pending[(cur.device.index, cur.cuda_stream)] = (cur, side)
             deferred_join.buckets.add(sink.data_ptr())
+            native.set_flag(native.FORK_PENDING, True)
         else:
             cur.wait_stream(side)   # everything later on this stream, frees of x and dy included, follows both GEMMs
         return dx, dw_out
@@ -267,6 +320,34 @@ def _linear_backward(ctx, dy):
 
 
 linear.register_autograd(_linear_backward, setup_context=_linear_setup)
+
+
+class HostContext:
+    """The context of a formula that the native library hands over."""
+
+    def __init__(self, saved_tensors, needs_input_grad) -> None:
+        self.saved_tensors, self.needs_input_grad = saved_tensors, needs_input_grad
+
+
+def _linear_backward_host(dy: Tensor, x: Tensor, w: Tensor, need_x: bool, need_w: bool) -> tuple[Tensor, Tensor]:
+    dx, dw = _linear_backward(HostContext((x, w), (need_x, need_w)), dy)
+    none = torch.empty(0)
+    return none if dx is None else dx, none if dw is None else dw
+
+
+host_op("linear_backward_host", _linear_backward_host)
+
+
+def _hand_over(lib) -> None:
+    lib.set_fork_macs(_FORK_MIN_MACS)
+    lib.sink_clear()
+    for address, sink in grad_sinks._sinks.items():
+        lib.sink_set(address, sink)
+
+
+native.on_load["core"] = _hand_over
+if native.loaded():
+    _hand_over(native.lib())
 
 # --------------------------------------------------------------------------
 # RMSNorm (optionally fused with the residual add)

@@ -21,7 +21,7 @@ import torch
 from torch import Tensor
 
 from . import core, native
-from .registry import custom_op
+from .registry import custom_op, host_op
 from .core import _is_native, _require_bf16, grad_sinks, wgrad_store
 
 PAD = 128
@@ -37,6 +37,7 @@ _EP_TABLE = None
 def set_ep_context(runtime, table) -> None:
     global _EP_RUNTIME, _EP_TABLE
     _EP_RUNTIME, _EP_TABLE = runtime, table
+    native.set_flag(native.EXPERT_RUNTIME, runtime is not None or table is not None)
 
 
 def row_capacity(tokens: int, k: int, experts: int) -> int:
@@ -122,6 +123,9 @@ def moe_group_table(counts: Tensor, expert_weights: Tensor) -> tuple[Tensor, Ten
     return g_start.to(torch.int32), g_len.to(torch.int32)
 
 
+host_op("moe_group_table_host", moe_group_table._body)
+
+
 @moe_group_table.register_fake
 def _(counts, expert_weights):
     return torch.empty_like(counts), torch.empty_like(counts)
@@ -164,6 +168,9 @@ def moe_dispatch(x: Tensor, idx: Tensor, counts: Tensor) -> tuple[Tensor, Tensor
     rows = torch.zeros((cap, D), dtype=x.dtype)
     rows[pos.long()] = x.repeat_interleave(k, dim=0)
     return rows, pos, g_start, g_len.to(torch.int32), counts.clone()
+
+
+host_op("moe_dispatch_host", moe_dispatch._body)
 
 
 @moe_dispatch.register_fake
@@ -293,6 +300,16 @@ def _glinear_backward(ctx, dy):
 
 
 grouped_linear.register_autograd(_glinear_backward, setup_context=_glinear_setup)
+
+
+def _glinear_backward_host(dy: Tensor, rows: Tensor, w: Tensor, g_start: Tensor, g_len: Tensor, need_rows: bool,
+                           need_w: bool) -> tuple[Tensor, Tensor]:
+    drows, dw, _, _ = _glinear_backward(core.HostContext((rows, w, g_start, g_len), (need_rows, need_w)), dy)
+    none = torch.empty(0)
+    return none if drows is None else drows, none if dw is None else dw
+
+
+host_op("grouped_linear_backward_host", _glinear_backward_host)
 
 
 # ----------------------------------------------------------------- combine

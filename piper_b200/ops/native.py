@@ -10,12 +10,19 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from pathlib import Path
 
 import torch
 
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libpiper_b200.so"
 _loaded = False
+_load_lock = threading.RLock()
+# What the op bodies and formulas in the library look at besides the gradient buckets: each flag sends the calls that it
+# concerns to the Python body or formula.
+DEFER_WGRAD, FORK_PENDING, GATHER_GEMMS, EXPERT_RUNTIME = range(4)
+_flags = [False] * 4
+on_load: dict = {}         # module -> function that hands its state to the library once that is loaded
 _status: dict[int, torch.Tensor] = {}
 _status_detail: dict[int, torch.Tensor] = {}
 _cdll = None
@@ -44,10 +51,22 @@ def available() -> bool:
     return _LIB_PATH.exists()
 
 
+def loaded() -> bool:
+    return _loaded
+
+
 def lib():
     """Load the native library once and return the ``torch.ops.piper_c`` namespace."""
-    global _loaded
     if not _loaded:
+        _load()
+    return torch.ops.piper_c
+
+
+def _load() -> None:
+    global _loaded
+    with _load_lock:
+        if _loaded:
+            return
         if not _LIB_PATH.exists():
             raise RuntimeError(
                 f"native library {_LIB_PATH} is missing; build it with `python -m piper_b200.build` "
@@ -55,7 +74,17 @@ def lib():
             )
         torch.ops.load_library(str(_LIB_PATH))
         _loaded = True
-    return torch.ops.piper_c
+        for i, on in enumerate(_flags):
+            torch.ops.piper_c.set_op_flag(i, on)
+        for hand_over in list(on_load.values()):
+            hand_over(torch.ops.piper_c)
+
+
+def set_flag(flag: int, on: bool) -> None:
+    if _flags[flag] != on:
+        _flags[flag] = on
+        if _loaded:
+            torch.ops.piper_c.set_op_flag.default(flag, on)
 
 
 def cdll() -> ctypes.CDLL:
@@ -74,9 +103,8 @@ def status_tensor(device: torch.device | None = None) -> torch.Tensor:
     t = _status.get(idx)
     if t is None:
         # word 0 is the status; a peer wait that runs out leaves (tag, flag index, wanted value) in words 1..3
-        _status_detail[idx] = torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", idx))
+        _status_detail[idx] = lib().status_words(idx)
         t = _status[idx] = _status_detail[idx][:1]
-        lib().set_status_word(t)          # kernels whose bindings take no status argument report into it too
     return t
 
 

@@ -7,6 +7,10 @@ wrapper's own work per call, which is host time in front of every launch.  Measu
 them, forward and backward: a residual norm 150 us a pass through the wrapper and 120 us through this one (its kernels
 take 63 us); the attention layer on 4 x 128 tokens, whose small GEMMs are no longer forked either, 604 and 350 us.
 
+On CUDA tensors both kernels of an op are replaced by those of ``csrc/bindings_ops.inc`` once the native library is
+loaded: the same bodies and formulas without Python in front of every launch.  A program that registers a formula or a
+CUDA kernel of its own gets the Python ones back for that op.
+
 Gradients that did not arrive (a consumer's backward returned None, or a reentrant checkpoint did not use its input):
 the formula of an op with one output is handed zeros in their place.  Where an op has several outputs, most of them
 without a gradient in every pass, filling them all would cost launches, so its formula gets None and treats it as zeros.
@@ -18,9 +22,36 @@ from typing import Callable, Optional
 
 import torch
 
+from . import native
+
 _below_autograd = torch._C._AutoDispatchBelowAutograd
 # One library per op, kept over a reload of this module: defining an op again replaces it.
 _libs: dict = globals().get("_libs", {})
+_ops: dict = globals().get("_ops", {})
+
+
+def _library(name: str) -> torch.library.Library:
+    stale = _libs.pop(name, None)
+    if stale is not None:
+        stale._destroy()
+    _libs[name] = torch.library.Library("piper", "FRAGMENT")
+    return _libs[name]
+
+
+def host_op(name: str, body: Callable) -> None:
+    """Makes a Python function callable from the library as ``piper::<name>``."""
+    library = _library(name)
+    library.define(name + torch.library.infer_schema(body, mutates_args=()))
+    library.impl(name, body, "CompositeExplicitAutograd")
+
+
+def _install_native(lib) -> None:
+    for op in list(_ops.values()):
+        if op._use_native:
+            lib.native_op_install(op.name)
+
+
+native.on_load["registry"] = _install_native
 
 
 class Op:
@@ -31,10 +62,8 @@ class Op:
         self.name, self.qualname = name, "piper::" + name
         self._kernels: dict = {}
         self._formula: Optional[Callable] = None
-        stale = _libs.pop(name, None)
-        if stale is not None:
-            stale._destroy()
-        self._lib = _libs[name] = torch.library.Library("piper", "FRAGMENT")
+        self._use_native = True
+        self._lib = _library(name)
         self._body = body
         self._lib.define(name + torch.library.infer_schema(body, mutates_args=()),
                          tags=(torch.Tag.pt2_compliant_tag,))
@@ -43,6 +72,14 @@ class Op:
         for method in ("register_autocast", "register_autograd", "register_effect", "register_fake", "register_kernel",
                        "register_torch_dispatch", "register_vmap", "set_kernel_enabled"):
             setattr(self.overload, method, getattr(self, method))
+        _ops[name] = self
+        if native.loaded():
+            native.lib().native_op_install(name)
+
+    def _drop_native(self) -> None:
+        self._use_native = False
+        if native.loaded():
+            native.lib().native_op_remove(self.name)
 
     def register_fake(self, fn: Callable) -> Callable:
         torch.library.register_fake(self.qualname, fn, lib=self._lib, allow_override=True)
@@ -68,6 +105,7 @@ class Op:
         Formula.__name__ = Formula.__qualname__ = f"piper_{self.name}"
         registered, self._formula = self._formula is not None, Formula.apply
         if registered:
+            self._drop_native()
             return
 
         def autograd(*args):
@@ -84,6 +122,8 @@ class Op:
             return lambda f: self.register_kernel(device_types, f)
         if device_types is None or isinstance(device_types, str):
             device_types = ("cpu", "cuda") if device_types is None else (device_types,)
+        if any(torch.device(device).type == "cuda" for device in device_types):
+            self._drop_native()
         for device in device_types:
             known = device in self._kernels
             self._kernels[device] = func

@@ -160,3 +160,165 @@ def test_op_modules_reload_and_ops_take_further_registrations():
     """In a process of its own: both change the ops for everything after them."""
     root = Path(__file__).resolve().parent.parent
     subprocess.run([sys.executable, "-c", _MODULE_CHANGES], check=True, timeout=300, cwd=root)
+
+
+def _cuda_calls():
+    """Calls on CUDA tensors, with the arguments that take gradients."""
+    def rn(*shape):
+        return torch.randn(*shape, device="cuda").to(torch.bfloat16)
+
+    E, k, T = 8, 2, 4
+    idx = torch.arange(T * k, device="cuda", dtype=torch.int32).view(T, k)          # one row per expert: a fixed order
+    counts = torch.ones(E, device="cuda", dtype=torch.int32)
+    cos, sin = torch.randn(128, 32, device="cuda"), torch.randn(128, 32, device="cuda")
+    with torch.no_grad():
+        rows, pos, g_start, g_len, _ = moe.moe_dispatch(rn(T, 64), idx, counts)
+    rows = rows[: int((g_start + g_len)[-1])].clone()
+    labels, tokens = torch.randint(0, 64, (6,), device="cuda"), torch.tensor([7, 0, 3, 1, 8, 5], device="cuda")
+    return {
+        "linear": (core.linear, [rn(3, 2, 64), rn(8, 64)]),
+        "rmsnorm_fwd": (lambda x, w: core.rmsnorm_fwd(x, w, 1e-5), [rn(3, 2, 256), rn(256)]),
+        "add_rmsnorm_fwd": (lambda x, r, w: core.add_rmsnorm_fwd(x, r, w, 1e-5), [rn(6, 256), rn(6, 256), rn(256)]),
+        "residual_add": (core.residual_add, [rn(6, 64), rn(6, 64)]),
+        "qk_rope": (lambda x: core.qk_rope(x, cos, sin, None, None, 128, 2, 1, 64, True, 1e-5), [rn(128, 256)]),
+        "qk_rope normed": (lambda x, q, w: core.qk_rope(x, cos, sin, q, w, 128, 2, 1, 64, False, 1e-5),
+                           [rn(128, 256), rn(64), rn(64)]),
+        "attention_fwd": (lambda x: core.attention_fwd(x, 1, 128, 2, 1, 64, 0.125), [rn(128, 256)]),
+        "swiglu": (core.swiglu, [rn(2, 3, 64)]),
+        "embedding": (lambda t: core.embedding(tokens, t), [rn(9, 64)]),
+        "cross_entropy_fwd": (lambda x: core.cross_entropy_fwd(x, labels, -100), [rn(6, 64)]),
+        "moe_route": (lambda x: moe.moe_route(x, k, True), [rn(T, E)]),
+        "moe_group_table": (lambda w: moe.moe_group_table(counts, w), [rn(E, 8, 8)]),
+        "moe_dispatch": (lambda x: moe.moe_dispatch(x, idx, counts), [rn(T, 64)]),
+        "grouped_linear": (lambda r, w: moe.grouped_linear(r, w, g_start, g_len), [rows, rn(E, 72, 64)]),
+        "moe_combine": (lambda r, w: moe.moe_combine(r, pos, w, g_start, g_len, counts),
+                        [rows, torch.rand(T, k, device="cuda")]),
+    }
+
+
+def _one_pass(fn, args, form):
+    """Outputs, gradients, buckets of one pass in some form of the call."""
+    torch.manual_seed(7)
+    if form == "strided":
+        args = [torch.stack((args[0], args[0]), -1)[..., 0], *args[1:]]
+    leaves = [a.detach().requires_grad_(form != "first only" or i == 0) for i, a in enumerate(args)]
+    sinks = {}
+    if form in ("sinks", "deferred"):
+        sinks = {i: torch.randn(a.shape, device="cuda") for i, a in enumerate(leaves) if i > 0}
+    for i, sink in sinks.items():
+        core.grad_sinks.register(leaves[i], sink)
+    queue = core.wgrad_store.begin() if form == "deferred" else []
+    try:
+        with torch.set_grad_enabled(form != "no grad"):
+            out = fn(*leaves)
+        outs = list(out) if isinstance(out, tuple) else [out]
+        heads = [o for o in outs if o.requires_grad][:1 if form == "first output" else None]
+        if heads and form == "dropped":
+            _Drop.apply(heads[0]).backward()
+        elif heads:
+            torch.autograd.backward(heads, [torch.full((), 0.5, device="cuda", dtype=o.dtype).expand_as(o)
+                                            if form == "broadcast" else torch.randn_like(o) for o in heads])
+        core.wgrad_store.end()
+        assert not core.wgrad_store.drain(queue)             # every weight that defers has a bucket here
+    finally:
+        core.wgrad_store.end()
+        for i in sinks:
+            core.grad_sinks.unregister(leaves[i])
+    return [o.detach() for o in outs], [a.grad for a in leaves], list(sinks.values()), [o.requires_grad for o in outs]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "no grad", "first only", "first output", "strided", "broadcast", "dropped", "sinks",
+                                  "deferred"])
+def test_native_formulas_do_what_the_python_ones_do(form):
+    """Every op on CUDA tensors by its C++ kernels and by the Python ones, in the forms in which programs call them: the
+    same bits, the same absent gradients, the same sums in the buckets (of norm weights of rotary heads, which atomics add
+    up in any order, to fp32 rounding of 128 x 2 summands)."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(6)
+    lib = native.lib()
+    for name, (fn, args) in _cuda_calls().items():
+        op = name.split()[0]
+        if form == "strided" and op in ("grouped_linear", "moe_combine"):
+            continue                                         # rows come from dispatch, whole
+        got = _one_pass(fn, args, form)
+        lib.native_op_remove(op)
+        try:
+            want = _one_pass(fn, args, form)
+        finally:
+            lib.native_op_install(op)
+        assert got[3] == want[3], name
+        for part, (a, b) in enumerate(zip(got[:3], want[:3])):
+            assert len(a) == len(b)
+            for i, (x, y) in enumerate(zip(a, b)):
+                assert (x is None) == (y is None), (name, part, i)
+                if x is None:
+                    continue
+                assert x.dtype == y.dtype and x.shape == y.shape and x.stride() == y.stride(), (name, part, i)
+                if name == "qk_rope normed" and (part == 2 or part == 1 and i > 0):
+                    assert torch.allclose(x.float(), y.float(), rtol=1e-2, atol=1e-3), (name, part, i)
+                elif not (op == "moe_dispatch" and part == 0 and i == 0):       # rows behind the last segment are undefined
+                    assert torch.equal(x, y), (name, part, i)
+    native.check_status()
+
+
+_CUDA_CHANGES = """
+import importlib, torch
+from piper_b200 import ops
+from piper_b200.ops import core, moe, native, registry
+def rn(*s): return torch.randn(*s, device="cuda").to(torch.bfloat16)
+x, w = rn(8, 64).requires_grad_(True), rn(16, 64)
+want = ops.linear(x, w).detach()
+sink = torch.zeros(16, 64, device="cuda")
+core.grad_sinks.register(w, sink)
+for module in (registry, core, moe):
+    importlib.reload(module)
+for f in (ops.linear, core.linear, torch.ops.piper.linear):
+    assert torch.equal(f(x, w), want)
+w.requires_grad_(True)
+core.linear(x, w).sum().backward()
+assert w.grad is not None and not sink.any()           # the buckets of the module before are forgotten
+for bad in (x.detach().float(), x.detach().half()):
+    try:
+        core.linear(bad, w)
+        raise SystemExit("accepted " + str(bad.dtype))
+    except TypeError as e:
+        assert str(bad.dtype) in str(e)
+core.gather_gemms[w.data_ptr()] = lambda x2, y: y.fill_(3)
+assert (core.linear(x, w) == 3).all() and torch.equal(core.linear(x, w), want)     # used once
+moe.set_ep_context(None, (torch.tensor([1, 2], device="cuda", dtype=torch.int32),) * 2)
+counts = torch.tensor([3, 5], device="cuda", dtype=torch.int32)
+assert moe.moe_group_table(counts, rn(2, 8, 8))[0].tolist() == [1, 2]
+moe.set_ep_context(None, None)
+assert moe.moe_group_table(counts, rn(2, 8, 8))[0].tolist() == [0, 128]
+seen = []
+with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.shape), t)[1], lambda t: t):
+    core.linear(x, w)
+assert seen == [x.shape, w.shape]
+op = core.linear
+op.register_autograd(lambda ctx, g: (torch.full((8, 64), 5.0, device="cuda", dtype=torch.bfloat16), None))
+x.grad = None
+op(x, w).sum().backward()
+assert (x.grad == 5).all()
+op = core.swiglu
+op.register_kernel("cuda", lambda h: h[..., :1] * 0 + 2)
+assert (op(x) == 2).all()
+with op.set_kernel_enabled("cuda", False):
+    assert not (op(x) == 2).all()
+with torch._subclasses.FakeTensorMode():
+    h = torch.empty(4, 32, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    assert core.rmsnorm_fwd(h, torch.empty(32, device="cuda", dtype=torch.bfloat16), 1e-5)[0].shape == (4, 32)
+try:
+    torch.func.grad(lambda a: core.residual_add(a, a).sum())(x.detach())
+    raise SystemExit("functorch transforms were refused before")
+except RuntimeError:
+    pass
+native.check_status()
+"""
+
+
+@pytest.mark.gpu
+def test_native_formulas_give_way_to_python_state_and_registrations():
+    root = Path(__file__).resolve().parent.parent
+    subprocess.run([sys.executable, "-c", _CUDA_CHANGES], check=True, timeout=300, cwd=root)
