@@ -11,9 +11,9 @@
 // Backward (attn_bwd_kernel): S and dP are recomputed; threads form P = exp(S - lse) and dS = P (dP - delta) as bf16
 // in tensor memory.  Two kinds of CTA in one launch:
 //   dK/dV: stationary tile = 128 key rows of one kv head (K, V); streams 64-row Q/dO tiles of every query head in
-//          the group; accumulates dK = dS^T Q and dV = P^T dO.
+//          the group, or of some where the group is split over several CTAs; accumulates dK = dS^T Q and dV = P^T dO.
 //   dQ:    stationary tile = 128 query rows of one head (Q, dO); streams 128-row K and V blocks; dQ = dS K.
-// Nothing is reduced with atomics, so gradients are reproducible.
+// No gradient is reduced with atomics, so they are reproducible.
 //
 // Every mbarrier wait is bounded (see ptx.cuh); on expiry a status code is
 // recorded and the CTA unwinds and frees its TMEM.
@@ -395,7 +395,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
 template <int HD>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                  float* __restrict__ delta, long long T, int S, int Hq) {
+                  float* __restrict__ delta, int* __restrict__ arrived, int n_arrived, long long T, int S, int Hq) {
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n_arrived; i += gridDim.x * 256) arrived[i] = 0;
   constexpr int LANES = HD / 8;
   const int wl = threadIdx.x & 31;
   const int lane = wl & (LANES - 1);
@@ -422,14 +423,15 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 }
 
 // The dK/dV pass streams 64-row tiles through two tensor memory stages (dK, dV and two 64-wide pairs of S' and dP' fill
-// it).  Warps 0-3 turn the even tiles' scores into probabilities and score gradients, warps 4-7 the odd tiles', so
-// each group has the MMAs of two tiles' time for its work; warp 8: TMA, warp 9: MMA.  P' and dS' (bf16) replace their
+// it).  Warps 0-7 turn the even tiles' scores into probabilities and score gradients, warps 8-15 the odd tiles' (four warps
+// per 32 columns), so each group has the MMAs of two tiles' time for its work; warp 16: TMA, warp 17: MMA.  P' and dS' (bf16) replace their
 // own fp32 scores in tensor memory and are the A operand of the accumulating MMAs from there: no thread writes shared
 // memory in the loop.  Bound by the MMAs: a 128x64x16 one with both operands in shared memory reads 6 KiB (48 cycles)
 // for 32 cycles of arithmetic.  Both passes and the delta kernel at S = 4096, 32 q / 8 kv heads x 128: 653 us with
 // probabilities through shared memory in two launches, 391 us so (this kernel alone 379 us, and 427 us with dQ on
-// 64-row tiles as well).
-constexpr int BWD_THREADS = 320;
+// 64-row tiles as well).  With eight softmax warps instead of sixteen: 376 and 374 us, 3 x 1408, 32 / 8 x 64 142 and 138 us.
+constexpr int BWD_THREADS = 576;
+constexpr int BWD_TMA_WARP = 16, BWD_MMA_WARP = 17;
 
 template <int HD>
 struct BwdSmem {
@@ -455,15 +457,19 @@ struct BwdBars {
   uint64_t ds_full[2];                // dS' stands in the place of dP'
   uint64_t acc_full;
   uint32_t tmem_base;
+  int last;                           // this CTA has to add the parts
 };
 
-// dK and dV of key block xb of kv head g.
+// dK and dV of key block xb of kv head g.  The query heads of the group may be split over `parts` CTAs; each accumulates over
+// its own and leaves its sums in `partial` ([part][slice of 64 columns][column][row]), and the one that finishes last
+// (by `arrived`, no CTA waits) adds them in the order of the parts, so the gradients are reproducible.
 template <int HD>
 __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, const CUtensorMap* tmap_qkv_y,
                                              const CUtensorMap* tmap_do_y, const CUtensorMap* tmap_dqkv,
                                              const float* __restrict__ lse, const float* __restrict__ delta, int xb,
-                                             int g, int b, int S, int Hq, int Hkv, float scale, float scale_log2,
-                                             int* status) {
+                                             int g, int b, int part, int parts, float* __restrict__ partial,
+                                             int* __restrict__ arrived, int S, int Hq, int Hkv, float scale,
+                                             float scale_log2, int* status) {
   using L = BwdSmem<HD>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -471,12 +477,13 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
   BwdBars* bars = reinterpret_cast<BwdBars*>(smem + L::BAR_OFF);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
-  const int group = Hq / Hkv;
+  const int heads = Hq / Hkv / parts;          // query heads of this CTA
+  const int head0 = g * (Hq / Hkv) + part * heads;
   const int tok0 = b * S;
 
-  // for each query head of the group streams q tiles i in [2*xb, S/64 - 1]
+  // for each of its query heads streams q tiles i in [2*xb, S/64 - 1]
   const int tiles_per_head = S / 64 - 2 * xb;
-  const int n_iter = tiles_per_head * group;
+  const int n_iter = tiles_per_head * heads;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->x_full, 1);
@@ -487,8 +494,8 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->s_full[i], 1);
       mbar_init(&bars->dp_full[i], 1);
-      mbar_init(&bars->p_full[i], 4);         // one arrival per softmax warp of the stage
-      mbar_init(&bars->ds_full[i], 4);
+      mbar_init(&bars->p_full[i], 8);         // one arrival per softmax warp of the stage
+      mbar_init(&bars->ds_full[i], 8);
     }
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
@@ -497,7 +504,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     tma_prefetch_desc(tmap_do_y);
     tma_prefetch_desc(tmap_dqkv);
   }
-  if (warp == 9) {
+  if (warp == BWD_MMA_WARP) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -509,8 +516,9 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
   //          [256,256+HD) acc1   [384,384+HD) acc2
   const uint32_t tmem_acc1 = tmem_base + 256;
   const uint32_t tmem_acc2 = tmem_base + 384;
+  bool done = false;                           // (softmax warps) the gradients are complete
 
-  if (warp == 8) {
+  if (warp == BWD_TMA_WARP) {
     // ------------------------------------------------------------- TMA
     if (lane == 0) {
       const int xrow = tok0 + xb * 128;
@@ -520,7 +528,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
         tma_load_2d(smem + L::X2_OFF + h * 16384, tmap_qkv_x, &bars->x_full, (Hq + Hkv + g) * HD + 64 * h, xrow);
       }
       int it = 0;
-      int hh = g * group, ti = 2 * xb;           // query head and tile of iteration it
+      int hh = head0, ti = 2 * xb;           // query head and tile of iteration it
       for (; it < n_iter; ++it) {
         const int st = it % L::Y_STAGES;
         if (!await(&bars->y_empty[st], ((it / L::Y_STAGES) & 1) ^ 1, status)) break;
@@ -546,7 +554,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
           await(&bars->y_full[jj % L::Y_STAGES], (jj / L::Y_STAGES) & 1, nullptr);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == BWD_MMA_WARP) {
     // ------------------------------------------------------------- MMA
     // Uniform control flow with one elected issuing lane (see the forward kernel).  Order per tile i: P' Y2 of i,
     // S' of i + 2 into the columns just consumed, dS' Y1 of i, dP' of i + 2.  MMAs execute in issue order.
@@ -565,7 +573,8 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     auto issue_acc = [&](uint32_t tmem_d, uint32_t tmem_a, uint64_t dy, bool first) {
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)       // contraction over the 64 streamed rows
-        umma_bf16_ts(tmem_d, tmem_a + ks * 8, dy + (ks * 2048 >> 4), idesc_acc, (first && ks == 0) ? 0u : 1u);
+        umma_bf16_ts(tmem_d, tmem_a + (ks / 2) * 32 + (ks % 2) * 8, dy + (ks * 2048 >> 4), idesc_acc,
+                     (first && ks == 0) ? 0u : 1u);
     };
     bool ok = await_all(&bars->x_full, 0, status);
     for (int i = 0; i < 2 && i < n_iter && ok; ++i) {
@@ -617,10 +626,11 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     }
   } else {
     // ------------------------------------------- P' / dS' tiles + epilogue
-    const int wg = warp >> 2;                  // tiles wg, wg + 2, ...; tensor memory stage wg
+    const int wg = warp >> 3;                  // tiles wg, wg + 2, ...; tensor memory stage wg
+    const int ch = (warp >> 2) & 1;            // columns [32 ch, 32 ch + 32) of every tile
     const int row = (warp & 3) * 32 + lane;    // stationary row == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t ts = tmem_base + lane_sel + wg * 64;
+    const uint32_t ts = tmem_base + lane_sel + wg * 64 + ch * 32;
     const uint32_t td = ts + 128;
     const int xpos = xb * 128 + row;   // position of this row inside the sequence
     const float2 sl2 = make_float2(scale_log2, scale_log2);
@@ -631,111 +641,135 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     for (int it = wg; it < n_iter; it += 2) {
       const uint32_t ph = (it >> 1) & 1;
       const int st = it % L::Y_STAGES;
-      const float4* vl = reinterpret_cast<const float4*>(smem + L::VEC_OFF + st * 2 * L::VEC_BYTES);
+      const float4* vl = reinterpret_cast<const float4*>(smem + L::VEC_OFF + st * 2 * L::VEC_BYTES) + ch * 8;
       const float4* vd = vl + L::VEC_BYTES / 16;
       if (!await_all(&bars->y_full[st], (it / L::Y_STAGES) & 1, status)) { ok = false; break; }
       if (!await_all(&bars->s_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
-      uint32_t sv[2][32];
-      tmem_ld_32x32(ts, sv[0]);
-      tmem_ld_32x32(ts + 32, sv[1]);
+      uint32_t sv[32], w[16];
+      tmem_ld_32x32(ts, sv);
       tmem_ld_wait();
       // Causal mask, applied once to the registers of the tiles that cross the diagonal (element (x row, y col) is
       // kept iff key <= query): a score of -inf turns into a probability and a score gradient of exactly zero.
-      const int ypos0 = ti * 64;
+      const int ypos0 = ti * 64 + ch * 32;
       if (ypos0 < xb * 128 + 127) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (xpos > ypos0 + i) sv[i / 32][i % 32] = 0xff800000u;
+        for (int i = 0; i < 32; ++i)
+          if (xpos > ypos0 + i) sv[i] = 0xff800000u;
       }
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t pw[16];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 l4 = vl[c * 8 + q];
-          const float2 n0 = make_float2(l4.x * kNegLog2e, l4.y * kNegLog2e);
-          const float2 n1 = make_float2(l4.z * kNegLog2e, l4.w * kNegLog2e);
-          uint32_t* v = &sv[c][4 * q];
-          float2 p0 = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, n0);
-          float2 p1 = fma2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl2, n1);
-          p0.x = fast_exp2(p0.x); p0.y = fast_exp2(p0.y);
-          p1.x = fast_exp2(p1.x); p1.y = fast_exp2(p1.y);
-          v[0] = __float_as_uint(p0.x); v[1] = __float_as_uint(p0.y);
-          v[2] = __float_as_uint(p1.x); v[3] = __float_as_uint(p1.y);
-          pw[2 * q] = pack_bf16x2(p0.x, p0.y);
-          pw[2 * q + 1] = pack_bf16x2(p1.x, p1.y);
-        }
-        tmem_st_32x16(ts + c * 16, pw);
+      for (int q = 0; q < 8; ++q) {
+        const float4 l4 = vl[q];
+        const float2 n0 = make_float2(l4.x * kNegLog2e, l4.y * kNegLog2e);
+        const float2 n1 = make_float2(l4.z * kNegLog2e, l4.w * kNegLog2e);
+        uint32_t* v = &sv[4 * q];
+        float2 p0 = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, n0);
+        float2 p1 = fma2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl2, n1);
+        p0.x = fast_exp2(p0.x); p0.y = fast_exp2(p0.y);
+        p1.x = fast_exp2(p1.x); p1.y = fast_exp2(p1.y);
+        v[0] = __float_as_uint(p0.x); v[1] = __float_as_uint(p0.y);
+        v[2] = __float_as_uint(p1.x); v[3] = __float_as_uint(p1.y);
+        w[2 * q] = pack_bf16x2(p0.x, p0.y);
+        w[2 * q + 1] = pack_bf16x2(p1.x, p1.y);
       }
+      tmem_st_32x16(ts, w);                    // over columns this thread has already read
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&bars->p_full[wg], lane);
       if (!await_all(&bars->dp_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
-      uint32_t dv[2][32];
-      tmem_ld_32x32(td, dv[0]);
-      tmem_ld_32x32(td + 32, dv[1]);
+      uint32_t dv[32];
+      tmem_ld_32x32(td, dv);
       tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t dw[16];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 d4 = vd[c * 8 + q];
-          float2 d0 = make_float2(d4.x, d4.y), d1 = make_float2(d4.z, d4.w);
-          const uint32_t* v = &dv[c][4 * q];
-          const uint32_t* p = &sv[c][4 * q];
-          d0 = fma2(d0, neg_one, make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])));
-          d1 = fma2(d1, neg_one, make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])));
-          d0 = mul2(d0, make_float2(__uint_as_float(p[0]), __uint_as_float(p[1])));
-          d1 = mul2(d1, make_float2(__uint_as_float(p[2]), __uint_as_float(p[3])));
-          dw[2 * q] = pack_bf16x2(d0.x, d0.y);
-          dw[2 * q + 1] = pack_bf16x2(d1.x, d1.y);
-        }
-        tmem_st_32x16(td + c * 16, dw);
+      for (int q = 0; q < 8; ++q) {
+        const float4 d4 = vd[q];
+        float2 d0 = make_float2(d4.x, d4.y), d1 = make_float2(d4.z, d4.w);
+        const uint32_t* v = &dv[4 * q];
+        const uint32_t* p = &sv[4 * q];
+        d0 = fma2(d0, neg_one, make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])));
+        d1 = fma2(d1, neg_one, make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])));
+        d0 = mul2(d0, make_float2(__uint_as_float(p[0]), __uint_as_float(p[1])));
+        d1 = mul2(d1, make_float2(__uint_as_float(p[2]), __uint_as_float(p[3])));
+        w[2 * q] = pack_bf16x2(d0.x, d0.y);
+        w[2 * q + 1] = pack_bf16x2(d1.x, d1.y);
       }
+      tmem_st_32x16(td, w);
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&bars->ds_full[wg], lane);
       ti += 2;
       if (ti >= S / 64) ti = 2 * xb + wg;
     }
-    if (ok && await_all(&bars->acc_full, 0, status)) {
-      // The stationary operands have been read for the last time; their buffers take the gradient tiles.
-      // dK by the first warp group, dV by the second.
+    done = ok && await_all(&bars->acc_full, 0, status);
+  }
+
+  // The gradients leave in slices of 64 columns, of dK first, of dV behind them, four warps per slice.
+  constexpr int SLICES = 2 * L::HALVES;
+  const int slice = warp >> 2, row = (warp & 3) * 32 + lane;
+  const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const uint32_t ta = (slice < L::HALVES ? tmem_acc1 : tmem_acc2 - L::HALVES * 64) + slice * 64 + lane_sel;
+  bool works = warp < 4 * SLICES && done;
+  if (parts > 1) {
+    if (works) {
       tc_fence_after();
-      const uint32_t ta = (wg == 0 ? tmem_acc1 : tmem_acc2) + lane_sel;
-      uint8_t* obuf = smem + (wg == 0 ? L::X1_OFF : L::X2_OFF);
-      const int col0 = (Hq + wg * Hkv + g) * HD;
-      const float sc = wg == 0 ? scale : 1.f;
+      float* mine = partial + (part * SLICES + slice) * 8192 + row;
 #pragma unroll 1
-      for (int h = 0; h < L::HALVES; ++h) {
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32(ta + c * 32, r);
+        tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t r[32], w[16];
-          tmem_ld_32x32(ta + h * 64 + c * 32, r);
-          tmem_ld_wait();
+        for (int i = 0; i < 32; ++i) __stcg(mine + (c * 32 + i) * 128, __uint_as_float(r[i]));
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) bars->last = atomicAdd(arrived, 1) == parts - 1;
+    __syncthreads();
+    works = works && bars->last;
+    __threadfence();
+  }
+  if (works) {
+    // The stationary operands have been read for the last time; their buffers take the gradient tiles.
+    tc_fence_after();
+    const bool is_k = slice < L::HALVES;
+    const int h = is_k ? slice : slice - L::HALVES;
+    uint8_t* obuf = smem + (is_k ? L::X1_OFF : L::X2_OFF) + h * 16384;
+    const float sc = is_k ? scale : 1.f;
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {
+      uint32_t r[32], w[16];
+      if (parts == 1) {
+        tmem_ld_32x32(ta + c * 32, r);
+        tmem_ld_wait();
+      } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * sc, __uint_as_float(r[2 * i + 1]) * sc);
-          store_row_chunk_sw128(obuf + h * 16384, row, c * 4, w);
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_2d_bulk(tmap_dqkv, obuf + h * 16384 + (warp & 3) * 32 * 128, col0 + 64 * h,
-                            tok0 + xb * 128 + (warp & 3) * 32);
-          bulk_commit_group();
+        for (int i = 0; i < 32; ++i) r[i] = 0;
+        for (int p = 0; p < parts; ++p) {
+          const float* share = partial + (p * SLICES + slice) * 8192 + c * 32 * 128 + row;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldcg(share + i * 128));
         }
       }
-      if (lane == 0) bulk_wait_group<0>();
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * sc, __uint_as_float(r[2 * i + 1]) * sc);
+      store_row_chunk_sw128(obuf, row, c * 4, w);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d_bulk(tmap_dqkv, obuf + (warp & 3) * 32 * 128, (Hq + (is_k ? 0 : Hkv) + g) * HD + 64 * h,
+                        tok0 + xb * 128 + (warp & 3) * 32);
+      bulk_commit_group();
+      bulk_wait_group<0>();
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == BWD_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -744,7 +778,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
 // The dQ pass: one query tile of one head against 128-key blocks.  With no dV product the scores need not stay in
 // tensor memory, so there is room for 128-wide tiles: S double-buffered, dP whose columns take dS, dQ.  A 128x128x16
 // MMA with both operands in shared memory runs at the arithmetic rate (64 cycles) where two 128x64x16 ones take 96.
-// The MMAs of a block are dQ of i, dP of i + 1, S of i + 2; the two warp groups halve the columns of every block, and
+// The MMAs of a block are dQ of i, dP of i + 1, S of i + 2; four groups of warps share the columns of every block, and
 // the exponentials of block i + 1 run under dQ of i and dP of i + 1.
 template <int HD>
 struct DqSmem {
@@ -795,14 +829,14 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
       mbar_init(&bars->s_full[i], 1);
     }
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->ds_full, 8);              // one arrival per softmax warp
+    mbar_init(&bars->ds_full, 16);             // one arrival per softmax warp
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
     tma_prefetch_desc(tmap_qkv_x);
     tma_prefetch_desc(tmap_do_x);
     tma_prefetch_desc(tmap_dqkv);
   }
-  if (warp == 9) {
+  if (warp == BWD_MMA_WARP) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -812,7 +846,7 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
   // columns: [0,128) S even  [128,256) S odd  [256,384) dP, dS  [384,384+HD) dQ
 
-  if (warp == 8) {
+  if (warp == BWD_TMA_WARP) {
     // ------------------------------------------------------------- TMA
     if (lane == 0) {
       mbar_arrive_expect_tx(&bars->x_full, 2 * L::TILE);
@@ -843,7 +877,7 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
         for (int j = vj - 1; j >= 0 && j >= vj - 2; --j) await(&bars->v_full[j & 1], (j >> 1) & 1, nullptr);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == BWD_MMA_WARP) {
     // ------------------------------------------------------------- MMA
     constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);
     constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, false, true);
@@ -889,8 +923,8 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
       if (elect_one()) {
         const uint64_t kn = dkn + ((i % L::K_STAGES) * L::TILE >> 4);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)     // dS of keys 0-63 at columns 256.., of keys 64-127 at 320..
-          umma_bf16_ts(tmem_base + 384, tmem_base + 256 + (ks / 4) * 64 + (ks % 4) * 8, kn + (ks * 2048 >> 4), idesc_acc,
+        for (int ks = 0; ks < 8; ++ks)     // dS of 32 keys each at columns 256, 288, 320, 352
+          umma_bf16_ts(tmem_base + 384, tmem_base + 256 + (ks / 2) * 32 + (ks % 2) * 8, kn + (ks * 2048 >> 4), idesc_acc,
                        (i == 0 && ks == 0) ? 0u : 1u);
         umma_commit(&bars->k_empty[i % L::K_STAGES]);
         if (i == n_blocks - 1) umma_commit(&bars->acc_full);
@@ -901,10 +935,10 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
     }
   } else {
     // --------------------------------------------------- dS blocks + epilogue
-    const int wg = warp >> 2;                  // key columns [64 wg, 64 wg + 64) of every block
+    const int wg = warp >> 2;                  // key columns [32 wg, 32 wg + 32) of every block
     const int row = (warp & 3) * 32 + lane;    // query row == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t td = tmem_base + lane_sel + 256 + wg * 64;
+    const uint32_t td = tmem_base + lane_sel + 256 + wg * 32;
     const float2 sl2 = make_float2(scale_log2, scale_log2);
     const long long idx = (static_cast<long long>(b) * Hq + hy) * S + xb * 128 + row;
     const float nl = lse[idx] * -1.4426950408889634f, ndl = -delta[idx];
@@ -913,38 +947,33 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
     for (int j = 0; j < n_blocks; ++j) {
       if (!await_all(&bars->s_full[j & 1], (j >> 1) & 1, status)) { ok = false; break; }
       tc_fence_after();
-      uint32_t sv[2][32];
-      tmem_ld_32x32(tmem_base + lane_sel + (j & 1) * 128 + wg * 64, sv[0]);
-      tmem_ld_32x32(tmem_base + lane_sel + (j & 1) * 128 + wg * 64 + 32, sv[1]);
+      uint32_t sv[32];
+      tmem_ld_32x32(tmem_base + lane_sel + (j & 1) * 128 + wg * 32, sv);
       tmem_ld_wait();
       if (j == xb) {
         // causal mask: a score of -inf turns into a probability and a score gradient of exactly zero
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (wg * 64 + i > row) sv[i / 32][i % 32] = 0xff800000u;
+        for (int i = 0; i < 32; ++i)
+          if (wg * 32 + i > row) sv[i] = 0xff800000u;
       }
 #pragma unroll
-      for (int i = 0; i < 64; i += 2) {
-        uint32_t* v = &sv[i / 32][i % 32];
-        float2 p = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, nl2);
-        v[0] = __float_as_uint(fast_exp2(p.x));
-        v[1] = __float_as_uint(fast_exp2(p.y));
+      for (int i = 0; i < 32; i += 2) {
+        float2 p = fma2(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2, nl2);
+        sv[i] = __float_as_uint(fast_exp2(p.x));
+        sv[i + 1] = __float_as_uint(fast_exp2(p.y));
       }
       if (!await_all(&bars->dp_full, j & 1, status)) { ok = false; break; }
       tc_fence_after();
+      uint32_t dv[32], dw[16];
+      tmem_ld_32x32(td, dv);
+      tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t dv[32], dw[16];
-        tmem_ld_32x32(td + c * 32, dv);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float2 d = add2(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), ndl2);
-          d = mul2(d, make_float2(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])));
-          dw[i] = pack_bf16x2(d.x, d.y);
-        }
-        tmem_st_32x16(td + c * 16, dw);        // over columns this thread has already read
+      for (int i = 0; i < 16; ++i) {
+        float2 d = add2(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), ndl2);
+        d = mul2(d, make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])));
+        dw[i] = pack_bf16x2(d.x, d.y);
       }
+      tmem_st_32x16(td, dw);                   // over columns this thread has already read
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&bars->ds_full, lane);
@@ -977,7 +1006,7 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == BWD_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -994,14 +1023,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv_x,   // box {64, 12
                 const __grid_constant__ CUtensorMap tmap_do_y,    // box {64, 64}  over dO
                 const __grid_constant__ CUtensorMap tmap_dqkv,    // box {64, 32}  over d_qkv
                 const float* __restrict__ lse, const float* __restrict__ delta, int B, int S, int Hq, int Hkv,
-                float scale, float scale_log2, int* status) {
+                int parts, float* __restrict__ partial, int* __restrict__ arrived, float scale, float scale_log2,
+                int* status) {
   const int blocks = S / 128;
-  const int n_kv = blocks * Hkv * B;
+  const int n_kv = blocks * Hkv * B * parts;
   int idx = blockIdx.x;
   if (idx < n_kv) {
+    const int part = idx % parts;
+    idx /= parts;
     const int hb = idx % (Hkv * B);
     attn_dkv_cta<HD>(&tmap_qkv_x, &tmap_qkv_y, &tmap_do_y, &tmap_dqkv, lse, delta, idx / (Hkv * B), hb % Hkv, hb / Hkv,
-                     S, Hq, Hkv, scale, scale_log2, status);
+                     part, parts, partial + static_cast<long long>(idx) * parts * HD * 256, arrived + idx, S, Hq, Hkv,
+                     scale, scale_log2, status);
   } else {
     idx -= n_kv;
     const int hb = idx % (Hq * B);
@@ -1066,10 +1099,30 @@ int attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int H
                    : attn_fwd_impl<64>(tm, to, lse, B, S, Hq, Hkv, softmax_scale, num_sms, status, st);
 }
 
+// CTAs that share the query heads of a key block in the dK/dV pass.  The launch takes the work over the SMs (about 5,800
+// cycles per 128 x 128 tile of both passes and 6,000 per CTA) or its longest CTA (1,600 cycles per 64 query rows of each of
+// its heads in the first key block, and the exchange of the parts' sums), whichever is longer; splitting has to shorten
+// that by 3 %.  One CTA per key block against the split, on 148 SMs: 1 x 5120, 16 q / 2 kv heads x 128 540 and 289 us in two; 1 x
+// 4096, 32 / 4 x 128 442 and 374 us in two; 2 x 2048, 32 / 4 x 128 231 and 219 us in two; 1 x 512, 32 / 4 x 128 70 and 37 us in four;
+// not split: 1 x 4096, 32 / 8 x 128 368 and 393 us, 8 x 1024, 16 / 2 x 64 124 and 132 us, 8 x 128, 16 / 4 x 128 13.3 and 15.8 us.
+int attn_bwd_parts(int B, int S, int Hq, int Hkv, int num_sms) {
+  const long long blocks = S / 128, group = Hkv > 0 ? Hq / Hkv : 1;
+  auto cost = [&](long long parts) {
+    const long long tiles = B * Hq * blocks * (blocks + 1) / 2, ctas = B * blocks * (Hkv * parts + Hq);
+    const long long work = (tiles * 5800 + ctas * 6000) / num_sms;
+    const long long longest = group / parts * 2 * blocks * 1600 + 6000 + (parts > 1 ? 3000 + 3000 * parts : 0);
+    return work > longest ? work : longest;
+  };
+  int best = 1;
+  for (int parts = 2; parts <= 8 && group % parts == 0; parts *= 2)
+    if (cost(parts) * 100 < cost(best) * 97) best = parts;
+  return best;
+}
+
 template <int HD>
 static int attn_bwd_impl(const void* qkv, const void* out, const void* d_out, const float* lse,
-                         float* delta, void* d_qkv, int B, int S, int Hq, int Hkv, float softmax_scale,
-                         int* status, cudaStream_t st) {
+                         float* delta, float* scratch, void* d_qkv, int B, int S, int Hq, int Hkv,
+                         float softmax_scale, int num_sms, int* status, cudaStream_t st) {
   const long long T = static_cast<long long>(B) * S;
   const uint64_t W = static_cast<uint64_t>(Hq + 2 * Hkv) * HD;
   const uint64_t Wo = static_cast<uint64_t>(Hq) * HD;
@@ -1090,23 +1143,36 @@ static int attn_bwd_impl(const void* qkv, const void* out, const void* d_out, co
     if (set_smem(attn_bwd_kernel<HD>, smem)) return -2;
     cfg = true;
   }
+  // scratch: a counter per key block, padded to 16 bytes, and the parts' sums
+  const int parts = scratch == nullptr ? 1 : attn_bwd_parts(B, S, Hq, Hkv, num_sms);
+  const int n_kv = S / 128 * Hkv * B;
+  int* arrived = reinterpret_cast<int*>(scratch);
+  float* partial = scratch == nullptr ? nullptr : scratch + (n_kv + 3) / 4 * 4;
   const long long delta_blocks = (T * Hq * (HD / 8) + 255) / 256;
   attn_delta_kernel<HD><<<static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, T, S, Hq);
+      static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, arrived,
+      parts > 1 ? n_kv : 0, T, S, Hq);
   if (cudaGetLastError() != cudaSuccess) return -3;
-  attn_bwd_kernel<HD><<<static_cast<unsigned>(S / 128 * (Hkv + Hq) * B), BWD_THREADS, smem, st>>>(
-      tqx, tqy, tdx, tdy, tdq, lse, delta, B, S, Hq, Hkv, softmax_scale, softmax_scale * 1.4426950408889634f, status);
+  attn_bwd_kernel<HD><<<static_cast<unsigned>(n_kv * parts + S / 128 * Hq * B), BWD_THREADS, smem, st>>>(
+      tqx, tqy, tdx, tdy, tdq, lse, delta, B, S, Hq, Hkv, parts, partial, arrived, softmax_scale,
+      softmax_scale * 1.4426950408889634f, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-int attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,
-             void* d_qkv, int B, int S, int Hq, int Hkv, int hd, float softmax_scale, int* status,
+long long attn_bwd_scratch(int B, int S, int Hq, int Hkv, int hd, int num_sms) {
+  const int parts = attn_bwd_parts(B, S, Hq, Hkv, num_sms);
+  const long long n_kv = static_cast<long long>(S / 128) * Hkv * B;
+  return parts == 1 ? 0 : (n_kv + 3) / 4 * 4 + n_kv * parts * hd * 256;
+}
+
+int attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta, float* scratch,
+             void* d_qkv, int B, int S, int Hq, int Hkv, int hd, float softmax_scale, int num_sms, int* status,
              cudaStream_t st) {
   if (S % 128 != 0 || Hq % Hkv != 0 || (hd != 64 && hd != 128)) return -1;
   if (B == 0) return 0;
   if (hd == 128)
-    return attn_bwd_impl<128>(qkv, out, d_out, lse, delta, d_qkv, B, S, Hq, Hkv, softmax_scale, status, st);
-  return attn_bwd_impl<64>(qkv, out, d_out, lse, delta, d_qkv, B, S, Hq, Hkv, softmax_scale, status, st);
+    return attn_bwd_impl<128>(qkv, out, d_out, lse, delta, scratch, d_qkv, B, S, Hq, Hkv, softmax_scale, num_sms, status, st);
+  return attn_bwd_impl<64>(qkv, out, d_out, lse, delta, scratch, d_qkv, B, S, Hq, Hkv, softmax_scale, num_sms, status, st);
 }
 
 }  // namespace piper

@@ -17,9 +17,13 @@ int attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int H
 int attn_tiles_per_cta(int B, int S, int Hq, int num_sms);
 
 // d_qkv has the layout of qkv and is fully overwritten.  delta is scratch of
-// B*Hq*S floats provided by the caller.
-int attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,
-             void* d_qkv, int B, int S, int Hq, int Hkv, int hd, float softmax_scale, int* status,
-             cudaStream_t st);
+// B*Hq*S floats provided by the caller, scratch attn_bwd_scratch() more or null (dK/dV CTAs are not split then).
+int attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta, float* scratch,
+             void* d_qkv, int B, int S, int Hq, int Hkv, int hd, float softmax_scale, int num_sms,
+             int* status, cudaStream_t st);
+
+// CTAs that share the query heads of a key block in attn_bwd, and the floats of scratch that they exchange sums in.
+int attn_bwd_parts(int B, int S, int Hq, int Hkv, int num_sms);
+long long attn_bwd_scratch(int B, int S, int Hq, int Hkv, int hd, int num_sms);
 
 }  // namespace piper

@@ -311,17 +311,33 @@ int64_t attn_tiles_per_cta(int64_t B, int64_t S, int64_t Hq, int64_t sms) {
   return piper::attn_tiles_per_cta(static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(sms));
 }
 
+// Floats that attn_bwd takes as `delta`, scratch included.
+int64_t attn_bwd_floats(int64_t B, int64_t S, int64_t Hq, int64_t Hkv, int64_t hd) {
+  return B * Hq * S + piper::attn_bwd_scratch(static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hq),
+                                              static_cast<int>(Hkv), static_cast<int>(hd), num_sms());
+}
+
 void attn_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, const Tensor& lse, Tensor delta,
               Tensor dqkv, int64_t B, int64_t S, int64_t Hq, int64_t Hkv, int64_t hd, double scale,
               Tensor status) {
   check_bf16(qkv, "qkv");
   check_bf16(dout, "dout");
   TORCH_CHECK(dout.is_contiguous() && dqkv.is_contiguous(), "attention expects contiguous tensors");
-  check_rc(piper::attn_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(),
-                           delta.data_ptr<float>(), dqkv.data_ptr(), static_cast<int>(B), static_cast<int>(S),
-                           static_cast<int>(Hq), static_cast<int>(Hkv), static_cast<int>(hd),
-                           static_cast<float>(scale), status.data_ptr<int>(), cur_stream()),
+  // delta holds B * Hq * S floats, and scratch behind them where the caller asked attn_bwd_floats for its size
+  const int64_t n = B * Hq * S;
+  TORCH_CHECK(delta.is_contiguous() && delta.numel() >= n, "delta must hold B * Hq * S floats");
+  float* d = delta.data_ptr<float>();
+  check_rc(piper::attn_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(), d,
+                           delta.numel() > n && delta.numel() >= attn_bwd_floats(B, S, Hq, Hkv, hd) ? d + n : nullptr,
+                           dqkv.data_ptr(), static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hq),
+                           static_cast<int>(Hkv), static_cast<int>(hd), static_cast<float>(scale), num_sms(),
+                           status.data_ptr<int>(), cur_stream()),
            "attn_bwd", 2);
+}
+
+int64_t attn_bwd_parts(int64_t B, int64_t S, int64_t Hq, int64_t Hkv, int64_t sms) {
+  return piper::attn_bwd_parts(static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(Hkv),
+                               static_cast<int>(sms));
 }
 
 }  // namespace
@@ -356,6 +372,8 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_tiles_per_cta", &attn_tiles_per_cta);
+  m.def("attn_bwd_parts", &attn_bwd_parts);
+  m.def("attn_bwd_floats", &attn_bwd_floats);
   register_moe_ops(m);
   register_fused_ops(m);
   register_native_ops(m);

@@ -665,7 +665,7 @@ def _attention_backward(ctx, dout, _dlse):
         if lse.data_ptr() % 16:            # the kernels copy pieces of it in bulk
             lse = lse.clone()
         dqkv = torch.empty_like(qc)
-        delta = torch.empty((B, Hq, S), dtype=torch.float32, device=qkv.device)
+        delta = torch.empty(native.lib().attn_bwd_floats(B, S, Hq, Hkv, hd), dtype=torch.float32, device=qkv.device)
         native.lib().attn_bwd(qc, out, dout.contiguous(), lse, delta, dqkv, B, S, Hq, Hkv, hd, scale,
                               native.status_tensor(qkv.device))
         return dqkv.view(qkv.shape), None, None, None, None, None, None

@@ -324,6 +324,36 @@ def test_attention_paired_tiles(B, S, Hq, Hkv, hd, growth, tiles):
         assert _close(qkv.grad[:, lo:hi], q2.grad[:, lo:hi], 3e-2), (lo, hi)
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,hd,parts", [(1, 640, 8, 2, 64, 4), (1, 1024, 8, 4, 128, 2), (1, 512, 16, 2, 128, 4),
+                                                 (1, 1024, 16, 2, 64, 8), (2, 1280, 8, 1, 128, 8), (1, 384, 12, 2, 128, 2)])
+def test_attention_backward_splits_a_group(B, S, Hq, Hkv, hd, parts):
+    """dK and dV of a key block by several CTAs: against an fp32 reference and, up to the order of the fp32 sums and one
+    bf16 rounding, against the launch without scratch, where one CTA adds all heads; the same bits every time."""
+    from piper_b200.ops import native
+    from piper_b200.ops.core import _attention_ref, attention_fwd
+
+    lib, st = native.lib(), native.status_tensor()
+    assert lib.attn_bwd_parts(B, S, Hq, Hkv, 148) == parts
+    torch.manual_seed(22)
+    scale = 1.0 / math.sqrt(hd)
+    qkv = torch.randn(B * S, (Hq + 2 * Hkv) * hd, device="cuda").to(torch.bfloat16)
+    g = torch.randn(B * S, Hq * hd, device="cuda").to(torch.bfloat16)
+    out, lse = attention_fwd(qkv, B, S, Hq, Hkv, hd, scale)
+    grads = []
+    for floats in (lib.attn_bwd_floats(B, S, Hq, Hkv, hd), lib.attn_bwd_floats(B, S, Hq, Hkv, hd), B * Hq * S):
+        delta = torch.full((floats,), float("nan"), device="cuda")
+        grads.append(torch.empty_like(qkv))
+        lib.attn_bwd(qkv, out, g, lse, delta, grads[-1], B, S, Hq, Hkv, hd, scale, st)
+    assert torch.equal(grads[0], grads[1])
+    assert _close(grads[0], grads[2], 2 ** -8) and torch.equal(grads[0][:, : Hq * hd], grads[2][:, : Hq * hd])
+    q2 = qkv.float().requires_grad_(True)
+    ref, _ = _attention_ref(q2, B, S, Hq, Hkv, hd, scale)
+    ref.backward(g.float())
+    nq, nk = Hq * hd, Hkv * hd
+    for lo, hi in ((0, nq), (nq, nq + nk), (nq + nk, nq + 2 * nk)):
+        assert _close(grads[0][:, lo:hi], q2.grad[:, lo:hi], 3e-2), (lo, hi)
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 def test_attention_largest_probability_is_exact(hd):
     """One key of the second block beats every earlier one by 2^0.1 to 2^7.9 and alone has a value, so a row is v / l.

@@ -92,6 +92,19 @@ def test_gemm_shape_rule(M, N, K, b_mn, f32, sms, shape):
     assert tuple(native.lib().gemm_shape(M, N, K, b_mn, f32, sms)) == shape
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,sms,parts", [
+    (1, 4096, 32, 32, 148, 1), (1, 4096, 32, 8, 148, 1), (1, 4096, 32, 4, 148, 2), (1, 5120, 16, 2, 148, 2),
+    (1, 512, 32, 4, 148, 4), (1, 2048, 16, 2, 148, 8), (8, 1024, 16, 2, 148, 1), (8, 128, 16, 4, 148, 1),
+    (1, 1024, 12, 2, 148, 2), (1, 1024, 9, 3, 148, 1), (1, 5120, 16, 2, 16, 1), (0, 128, 2, 1, 148, 1),
+])
+def test_attention_backward_parts_rule(B, S, Hq, Hkv, sms, parts):
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    assert native.lib().attn_bwd_parts(B, S, Hq, Hkv, sms) == parts
+
+
 @pytest.mark.parametrize("B,S,Hq,sms,tiles", [
     (1, 128, 148, 148, 1), (1, 128, 149, 148, 2),         # an SM for every tile, and one too few (one block each)
     (1, 512, 44, 148, 1), (1, 512, 45, 148, 2),           # 440 of 444 block times in which the longest tile is done
