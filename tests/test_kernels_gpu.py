@@ -221,6 +221,26 @@ def test_linear_gradients_around_the_fork_threshold(sizes, forked, monkeypatch):
     assert _close(results[0], want + held, 1e-4) and all(torch.equal(r, results[0]) for r in results)
 
 
+@pytest.mark.parametrize("T,D", [(1, 2048), (591, 4096), (593, 2048), (593, 8192), (1777, 2048)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_rows_per_cta(T, D, residual):
+    """One CTA per row up to 592 rows, several rows per CTA behind: every row against fp32, rounded to bf16 once (2^-8), the
+    residual sum exactly."""
+    from piper_b200.ops import core
+
+    torch.manual_seed(23)
+    x, r = (torch.randn(T, D, device="cuda").to(torch.bfloat16) for _ in range(2))
+    w = torch.randn(D, device="cuda").to(torch.bfloat16)
+    y, h, rstd = core.add_rmsnorm_fwd(x, r, w, 1e-6) if residual else (core.rmsnorm_fwd(x, w, 1e-6)[0], x,
+                                                                       core.rmsnorm_fwd(x, w, 1e-6)[1])
+    want_h = (x.float() + r.float()).to(torch.bfloat16) if residual else x
+    assert torch.equal(h, want_h)
+    want_r = torch.rsqrt(want_h.double().pow(2).mean(-1) + 1e-6)
+    assert torch.allclose(rstd.double(), want_r, rtol=1e-5)
+    want = want_h.double() * want_r.unsqueeze(-1) * w.double()
+    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
+
+
 @pytest.mark.parametrize("T,D", [(300, 256), (300, 2048), (1000, 4096), (300, 8192), (7, 4096)])
 def test_rmsnorm_and_residual(T, D):
     from piper_b200 import ops
