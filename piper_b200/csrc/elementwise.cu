@@ -382,8 +382,7 @@ reduce_partials_kernel(const float* __restrict__ partial, int nblocks, int D,
 // that both members of each of its eight rope pairs are its own: elements [16l, 16l+16) in the interleaved
 // form, [8l, 8l+8) and [hd/2 + 8l, hd/2 + 8l + 8) in the half-split form.  In both forms the lane's pairs use
 // cos/sin entries [8l, 8l+8).
-// A lane group walks this many consecutive heads of one token, so the token's cos/sin entries are loaded once.
-constexpr int ROPE_HEADS_PER_GROUP = 8;
+// A lane group walks several consecutive heads of one token, so the token's cos/sin entries are loaded once.
 
 template <int HD>
 struct RopeGroup {
@@ -438,17 +437,17 @@ qk_rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__
                const float* __restrict__ cosp, const float* __restrict__ sinp,
                const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
                float* __restrict__ rstd_out, long long T, int S, int Hq, int Hkv,
-               int interleaved, float eps, float sin_sign) {
+               int interleaved, float eps, float sin_sign, int heads_per_group) {
   const RopeGroup<HD> g(interleaved);
   constexpr int LANES = RopeGroup<HD>::LANES;
   const int heads = Hq + 2 * Hkv;
-  const int chunks = (heads + ROPE_HEADS_PER_GROUP - 1) / ROPE_HEADS_PER_GROUP;
+  const int chunks = (heads + heads_per_group - 1) / heads_per_group;
   const unsigned total = static_cast<unsigned>(T) * chunks;   // the launcher keeps this below 2^31
   const unsigned stride = gridDim.x * (blockDim.x / LANES);
   for (unsigned gi = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; gi < total; gi += stride) {
     const long long t = gi / static_cast<unsigned>(chunks);
-    const int h0 = static_cast<int>(gi - static_cast<unsigned>(t) * chunks) * ROPE_HEADS_PER_GROUP;
-    const int h1 = min(heads, h0 + ROPE_HEADS_PER_GROUP);
+    const int h0 = static_cast<int>(gi - static_cast<unsigned>(t) * chunks) * heads_per_group;
+    const int h1 = min(heads, h0 + heads_per_group);
     float c[8], s[8];
     const int cs = static_cast<int>(static_cast<unsigned>(t) % static_cast<unsigned>(S)) * (HD / 2) + 8 * g.lane;
     load8f(cosp + cs, c, 1.f);
@@ -503,7 +502,7 @@ qk_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
                    const float* __restrict__ sinp, const __nv_bfloat16* __restrict__ qw,
                    const __nv_bfloat16* __restrict__ kw, float* __restrict__ dqw,
                    float* __restrict__ dkw, long long T, int S, int Hq, int Hkv,
-                   int interleaved, float eps) {
+                   int interleaved, float eps, int heads_per_group) {
   __shared__ float sdw[2][HD];
   const bool want_dw = NORM && (dqw != nullptr || dkw != nullptr);
   if (want_dw) {
@@ -513,7 +512,7 @@ qk_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
   const RopeGroup<HD> g(interleaved);
   constexpr int LANES = RopeGroup<HD>::LANES;
   const int heads = Hq + 2 * Hkv;
-  const int chunks = (heads + ROPE_HEADS_PER_GROUP - 1) / ROPE_HEADS_PER_GROUP;
+  const int chunks = (heads + heads_per_group - 1) / heads_per_group;
   const unsigned total = static_cast<unsigned>(T) * chunks;   // the launcher keeps this below 2^31
   const unsigned stride = gridDim.x * (blockDim.x / LANES);
   float aq[NORM ? 16 : 1], ak[NORM ? 16 : 1];
@@ -521,8 +520,8 @@ qk_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
   for (int j = 0; j < (NORM ? 16 : 1); ++j) aq[j] = ak[j] = 0.f;
   for (unsigned gi = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; gi < total; gi += stride) {
     const long long t = gi / static_cast<unsigned>(chunks);
-    const int h0 = static_cast<int>(gi - static_cast<unsigned>(t) * chunks) * ROPE_HEADS_PER_GROUP;
-    const int h1 = min(heads, h0 + ROPE_HEADS_PER_GROUP);
+    const int h0 = static_cast<int>(gi - static_cast<unsigned>(t) * chunks) * heads_per_group;
+    const int h1 = min(heads, h0 + heads_per_group);
     float c[8], s[8];
     const int cs = static_cast<int>(static_cast<unsigned>(t) % static_cast<unsigned>(S)) * (HD / 2) + 8 * g.lane;
     load8f(cosp + cs, c, 1.f);
@@ -946,10 +945,25 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
   return PIPER_LAUNCH_OK();
 }
 
+// Heads that a lane group walks: more of them share one load of cos/sin, fewer make more groups to run at a time.  `blocks`
+// are the CTAs that one head per group makes.  In us, 8 heads per group and by this rule: 512 tokens of 4 + 2 x 4 heads x 64
+// forward 6.0 and 2.6, backward 5.8 and 2.3; 2048 x (32 + 2 x 8) x 64 12.4 and 9.8, 12.2 and 9.1; 8192 x (32 + 2 x 8) x 64 backward
+// 32.1 and 28.2; 4096 x (32 + 2 x 8) x 128 backward 31.6 and 30.1, forward 32.8 with 8, 33.7 with 4.  With norms a group has
+// more work per head: 4096 x (32 + 2 x 4) x 128 forward 24.9 with 8, 22.6 with 4, backward 60.3 with 8, 61.3 with 4 and 69
+// with 2 (there its weight-gradient sums end in more shuffles and atomics); 1000 x (16 + 2 x 2) x 64 backward 13.3 and 9.4.
+static int rope_heads_per_group(long long T, int heads, int hd, bool norm, bool backward) {
+  const long long blocks = T * heads * (hd / 16) / 256;
+  if (backward && norm) return blocks / 8 < 2 * 148 ? 4 : 8;
+  if (blocks <= 4 * 148) return 1;
+  if (backward || blocks <= 16 * 148) return 2;
+  return norm ? 4 : 8;
+}
+
 int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp, const void* qw,
                 const void* kw, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps,
                 cudaStream_t st) {
-  const long long groups = T * ((Hq + 2 * Hkv + ROPE_HEADS_PER_GROUP - 1) / ROPE_HEADS_PER_GROUP);
+  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, false);
+  const long long groups = T * ((Hq + 2 * Hkv + hpg - 1) / hpg);
   if (groups == 0) return 0;
   if (hd != 128 && hd != 64) return -1;
   if (groups >= (1ll << 31) || static_cast<long long>(S) * (hd / 2) >= (1ll << 31)) return -1;
@@ -962,10 +976,10 @@ int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp,
   auto k = static_cast<const __nv_bfloat16*>(kw);
   if (hd == 128)
     qk_rope_kernel<128><<<blocks, threads, 0, st>>>(a, o, cosp, sinp, q, k, nullptr, T, S, Hq, Hkv,
-                                                    interleaved, eps, 1.f);
+                                                    interleaved, eps, 1.f, hpg);
   else if (hd == 64)
     qk_rope_kernel<64><<<blocks, threads, 0, st>>>(a, o, cosp, sinp, q, k, nullptr, T, S, Hq, Hkv,
-                                                   interleaved, eps, 1.f);
+                                                   interleaved, eps, 1.f, hpg);
   else
     return -1;
   return PIPER_LAUNCH_OK();
@@ -974,7 +988,8 @@ int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp,
 int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, const float* sinp,
                 const void* qw, const void* kw, float* dqw, float* dkw, long long T, int S, int Hq,
                 int Hkv, int hd, int interleaved, float eps, cudaStream_t st) {
-  const long long groups = T * ((Hq + 2 * Hkv + ROPE_HEADS_PER_GROUP - 1) / ROPE_HEADS_PER_GROUP);
+  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, true);
+  const long long groups = T * ((Hq + 2 * Hkv + hpg - 1) / hpg);
   if (groups == 0) return 0;
   if (hd != 128 && hd != 64) return -1;
   if (groups >= (1ll << 31) || static_cast<long long>(S) * (hd / 2) >= (1ll << 31)) return -1;
@@ -989,7 +1004,7 @@ int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, 
   const bool norm = q != nullptr || k != nullptr;
   auto kern = hd == 128 ? (norm ? qk_rope_bwd_kernel<128, true> : qk_rope_bwd_kernel<128, false>)
                         : (norm ? qk_rope_bwd_kernel<64, true> : qk_rope_bwd_kernel<64, false>);
-  kern<<<blocks, threads, 0, st>>>(g, a, o, cosp, sinp, q, k, dqw, dkw, T, S, Hq, Hkv, interleaved, eps);
+  kern<<<blocks, threads, 0, st>>>(g, a, o, cosp, sinp, q, k, dqw, dkw, T, S, Hq, Hkv, interleaved, eps, hpg);
   return PIPER_LAUNCH_OK();
 }
 

@@ -241,6 +241,28 @@ def test_rmsnorm_rows_per_cta(T, D, residual):
     assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("T,Hq,Hkv,hd,norm", [(128, 2, 2, 64, False), (1024, 17, 2, 128, False), (4096, 30, 5, 128, False),
+                                              (256, 5, 1, 64, True), (1024, 16, 4, 128, True), (4096, 33, 4, 128, True)])
+def test_qk_rope_heads_per_group(T, Hq, Hkv, hd, norm):
+    """One, two, four and eight heads per lane group in both directions, with head counts that leave a shorter last group,
+    against the fp32 reference; bf16 rounding of results, fp32 sums for the weights."""
+    from piper_b200.ops import core
+
+    torch.manual_seed(24)
+    cos, sin = core.rope_tables(hd, T, 1e4, device="cuda")
+    x = torch.randn(T, (Hq + 2 * Hkv) * hd, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    ws = [torch.randn(hd, device="cuda").to(torch.bfloat16).requires_grad_(True) for _ in range(2)] if norm else [None, None]
+    out = core.qk_rope(x, cos, sin, *ws, T, Hq, Hkv, hd, False, 1e-6)
+    g = torch.randn_like(out)
+    out.backward(g)
+    leaves = [t.detach().float().requires_grad_(True) for t in (x, *ws) if t is not None]
+    ref = core._qk_rope_ref(leaves[0], cos, sin, *(leaves[1:] if norm else (None, None)), T, Hq, Hkv, hd, False, 1e-6)
+    ref.backward(g.float())
+    assert _close(out, ref, 2 ** -8) and _close(x.grad, leaves[0].grad, 2 ** -8)
+    for w, l in zip(ws, leaves[1:]):
+        assert _close(w.grad, l.grad, 2 ** -8)
+
+
 @pytest.mark.parametrize("T,D", [(300, 256), (300, 2048), (1000, 4096), (300, 8192), (7, 4096)])
 def test_rmsnorm_and_residual(T, D):
     from piper_b200 import ops
