@@ -41,7 +41,9 @@ constexpr int MAX_STAGES = 6;
 constexpr int NUM_THREADS = 384;     // TMA, MMA, TMEM-allocation and table warp, then eight epilogue warps
 constexpr int MAX_GROUPS = 1024;
 constexpr int EPI_WARPS = 8;
-constexpr int RING = 16;             // tiles handed out ahead: at most the stages + 2 accumulators + 1
+// Tiles handed out ahead.  Nothing tells the producer that a slot has been read: every tile has at least one k-block, so
+// it waits for a stage before the next one, and is at most the stages + 2 accumulators + 1 ahead of the slowest warp.
+constexpr int RING = 16;
 
 template <int MODE, int CTAS>
 struct Cfg {
@@ -51,9 +53,9 @@ struct Cfg {
   static constexpr int STAGES = CTAS == 2 ? (MODE == kGroupedWgrad ? 5 : 6) : (MODE == kGroupedWgrad ? 3 : 4);
   static constexpr int C_OFF = STAGES * STAGE_BYTES;
   static constexpr int BAR_OFF = C_OFF + EPI_WARPS * C_BYTES;
-  static constexpr int TABLE_OFF = BAR_OFF + 768;       // tile_prefix[MAX_GROUPS + 1], start[], len[]
+  static constexpr int TABLE_OFF = BAR_OFF + 768;       // table[MAX_GROUPS + 1], start[], len[]
   static constexpr int SMEM_BYTES = TABLE_OFF + (3 * MAX_GROUPS + 4) * 4 + 1024;
-  static_assert(STAGES <= MAX_STAGES && SMEM_BYTES <= 232448, "shared memory");
+  static_assert(STAGES <= MAX_STAGES && STAGES + 3 < RING && SMEM_BYTES <= 232448, "shared memory");
 };
 
 // What a tile is, as its producer hands it on.
@@ -82,6 +84,7 @@ struct GroupedParams {
   int experts;           // local experts
   int N, K;              // weight shape per expert [N, K]
   int accumulate;
+  void* out;
   int* status;
   int* sched;            // next tile, finished CTAs
 };
@@ -101,8 +104,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   Barriers* bars = reinterpret_cast<Barriers*>(smem + L::BAR_OFF);
-  int* tile_prefix = reinterpret_cast<int*>(smem + L::TABLE_OFF);
-  int* g_start = tile_prefix + MAX_GROUPS + 1;
+  // Token tiles before each segment and, behind them, of all; for a weight gradient the experts with rows from the front,
+  // those without from the back ([experts - 1] first), and the number with rows in [num_groups].
+  int* table = reinterpret_cast<int*>(smem + L::TABLE_OFF);
+  int* g_start = table + MAX_GROUPS + 1;
   int* g_len = g_start + MAX_GROUPS;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
@@ -146,13 +151,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (lane >= o) inc += v;
       }
       if (in) {
-        tile_prefix[q] = acc + inc - n;
+        if (MODE != kGroupedWgrad) table[q] = acc + inc - n;
         g_start[grp] = start;
         g_len[grp] = len;
       }
       acc += __shfl_sync(0xffffffffu, inc, 31);
     }
-    if (lane == 0) tile_prefix[p.num_groups] = acc;
+    if (MODE == kGroupedWgrad) {
+      __syncwarp();
+      acc = 0;
+      for (int e0 = 0; e0 < p.experts; e0 += 32) {
+        const int e = e0 + lane;
+        bool rows = false;
+        if (e < p.experts)
+          for (int src = 0; src < sources; ++src) rows = rows || g_len[src * p.experts + e] > 0;
+        const uint32_t mask = __ballot_sync(0xffffffffu, rows);
+        const int before = acc + __popc(mask & ((1u << lane) - 1));
+        if (e < p.experts) table[rows ? before : p.experts - 1 - (e - before)] = e;
+        acc += __popc(mask);
+      }
+    }
+    if (lane == 0) table[p.num_groups] = acc;
   }
   if (warp == 2) {
     tmem_alloc_n<CTAS>(&bars->tmem_base, 512);
@@ -175,7 +194,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer (both CTAs of a pair load their own halves)
     const int tiles_n = (p.K + BN - 1) / BN;           // weight gradient
-    const int num_tiles = tiles_m * (MODE == kGroupedWgrad ? p.experts * tiles_n : tile_prefix[p.num_groups]);
+    const int num_tiles = tiles_m * table[p.num_groups] * (MODE == kGroupedWgrad ? tiles_n : 1);
     const int contract_blocks = ((MODE == kGroupedFwd ? p.K : p.N) + BK - 1) / BK;
     uint32_t n = 0, fills = 0, ph = 0;
     int s = 0;
@@ -193,8 +212,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             // column tiles fastest: the CTAs that run at the same time write whole rows of dW
             const int u = i / tiles_n;
             t.n0 = (i - u * tiles_n) * BN;
-            t.expert = u / tiles_m;
-            t.m0 = (u - t.expert * tiles_m) * BM * CTAS;
+            const int j = u / tiles_m;
+            t.m0 = (u - j * tiles_m) * BM * CTAS;
+            t.expert = table[j];
             for (int src = 0; src < sources; ++src) t.count += g_len[src * p.experts + t.expert] / BK;
           } else {
             const int u = i / tiles_m;
@@ -202,14 +222,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             // Weight tiles of one token tile are consecutive, and token tiles are walked expert by expert (all sources
             // of an expert together): the CTAs that run at the same time share their tokens and a few experts'
             // weights through L2, so both stream from DRAM once.
-            int lo = 0, hi = p.num_groups;             // largest q with tile_prefix[q] <= u
+            int lo = 0, hi = p.num_groups;             // largest q with table[q] <= u
             while (hi - lo > 1) {
               const int mid = (lo + hi) >> 1;
-              if (tile_prefix[mid] <= u) lo = mid; else hi = mid;
+              if (table[mid] <= u) lo = mid; else hi = mid;
             }
-            t.expert = lo / sources;                   // tile_prefix is ordered (expert, source)
+            t.expert = lo / sources;                   // the table is ordered (expert, source)
             const int grp = (lo - t.expert * sources) * p.experts + t.expert;
-            const int r0 = (u - tile_prefix[lo]) * BN;
+            const int r0 = (u - table[lo]) * BN;
             t.n0 = g_start[grp] + r0;
             t.count = min(BN, g_len[grp] - r0);
           }
@@ -286,18 +306,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       constexpr int a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
       constexpr int b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
       const int contract_blocks = ((MODE == kGroupedFwd ? p.K : p.N) + BK - 1) / BK;
-      uint32_t tiles_done = 0, ph = 0;
+      uint32_t ph = 0;
       int s = 0;
       bool ok = true;
       for (uint32_t n = 0; ok; ++n) {
         Tile t;
         if (!(ok = tile_at(n, t)) || t.expert < 0) break;
         const int blocks = MODE == kGroupedWgrad ? t.count : contract_blocks;
-        if (blocks == 0) continue;
         const uint32_t idesc = umma_idesc_bf16(BM * CTAS, MODE == kGroupedWgrad ? BN : t.count, A_MN, B_MN);
-        const uint32_t acc = tiles_done & 1, acc_ph = (tiles_done >> 1) & 1;
-        ++tiles_done;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[acc], acc_ph ^ 1, p.status));
+        const uint32_t acc = n & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status));
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
         for (int kb = 0; kb < blocks && ok; ++kb) {
@@ -321,20 +339,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int q = warp & 3;                     // TMEM lanes [32q, 32q + 32)
     const int half = (warp - 4) >> 2;           // odd or even column chunks
     uint8_t* const blk = smem + L::C_OFF + (warp - 4) * L::C_BYTES;
-    uint32_t tiles_done = 0;
     for (uint32_t n = 0;; ++n) {
       Tile t;
       if (!tile_at(n, t) || t.expert < 0) break;
       const int row0 = t.m0 + rank * BM + q * 32;
-      // expert without rows: nothing to add; a weight gradient that does not accumulate is zero
-      const bool empty = MODE == kGroupedWgrad && t.count == 0;
-      if (empty && p.accumulate) continue;
-      const uint32_t acc = tiles_done & 1;
-      if (!empty) {
-        const uint32_t acc_ph = (tiles_done >> 1) & 1;
-        ++tiles_done;
-        if (!__all_sync(0xffffffffu, mbar_wait(&bars->acc_full[acc], acc_ph, p.status))) break;
-      }
+      const uint32_t acc = n & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->acc_full[acc], (n >> 1) & 1, p.status))) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       if (MODE == kGroupedWgrad) {
@@ -349,13 +359,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
           for (int h = 0; h < COLS / 32; ++h) {
             uint32_t r[32];
-            if (!empty) {
-              tmem_ld_32x32(taddr + c * COLS + h * 32, r);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0;
-            }
+            tmem_ld_32x32(taddr + c * COLS + h * 32, r);
+            tmem_ld_wait();
             if (OUT_BF16) {
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
@@ -402,7 +407,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
         }
       }
-      if (empty) continue;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -411,6 +415,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
     }
     if (lane == 0) bulk_wait_group<0>();         // staged blocks leave before the CTA does
+  } else if (MODE == kGroupedWgrad && !p.accumulate) {
+    // -------------------------------- experts without rows: their gradients are zero, written beside the other tiles
+    const long long vecs = static_cast<long long>(p.N) * p.K * (OUT_BF16 ? 2 : 4) / 16;      // K is a multiple of 8
+    for (int j = table[p.num_groups]; j < p.experts; ++j) {
+      uint4* dst = static_cast<uint4*>(p.out) + table[j] * vecs;
+      for (long long i = (blockIdx.x * 2 + warp - 2) * 32 + lane; i < vecs; i += gridDim.x * 64)
+        dst[i] = make_uint4(0, 0, 0, 0);
+    }
   }
 
   tc_fence_before();
@@ -520,6 +532,7 @@ int grouped_gemm_launch(const GroupedGemmArgs& g, int num_sms, cudaStream_t st) 
   p.N = g.N;
   p.K = g.K;
   p.accumulate = g.accumulate;
+  p.out = g.out;
   p.status = g.status;
   p.sched = gemm_sched_slot();
   CUtensorMap ta, tb, tc;

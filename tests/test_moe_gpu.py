@@ -1,4 +1,9 @@
 """MoE kernels on the GPU against the PyTorch fp32 reference bodies of the same ops."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -176,6 +181,57 @@ def test_grouped_products_by_pairs_and_single_ctas(E, N, K, sources):
             for got, want in ((y[s:s + n], x[s:s + n].double() @ w[gi % E].double().t()),
                               (dx[s:s + n], dy[s:s + n].double() @ w[gi % E].double())):
                 assert ((got.double() - want).abs().max() / want.abs().max()) < 2 ** -8
+
+
+def _weight_gradient_with_few_live_experts(E, N, K, sources, live):
+    """dW of E experts of which a few have rows: bf16 and fp32 stored over a filled buffer, fp32 accumulated.  fp32 sums of
+    up to 640 bf16 products (1e-5 of the largest); experts without rows are zero, or what the buffer held."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(8)
+    has_rows = {"first": lambda e: e < 3, "last": lambda e: e >= E - 3, "alternating": lambda e: e % 2 == 1,
+                "all": lambda e: True, "none": lambda e: False}[live]
+    lens = [[128 * (1 + (e + s) % 3) if has_rows(e) and (s == 0 or e % 4 != 1) else 0 for e in range(E)]
+            for s in range(sources)]
+    g_len = torch.tensor(lens, dtype=torch.int32).reshape(-1).cuda()
+    g_start = (torch.cumsum(g_len, 0) - g_len).to(torch.int32)
+    R = int(g_len.sum()) + 128                                # rows behind the last segment belong to nobody
+    x = torch.randn(R, K, device="cuda").to(torch.bfloat16)
+    dy = torch.randn(R, N, device="cuda").to(torch.bfloat16)
+    lib, st = native.lib(), native.status_tensor()
+    b16 = torch.full((E, N, K), 7.0, device="cuda", dtype=torch.bfloat16)
+    f32, added = torch.full((E, N, K), 7.0, device="cuda"), torch.full((E, N, K), 3.0, device="cuda")
+    for out, accumulate in ((b16, False), (f32, False), (added, True)):
+        lib.grouped_gemm(2, x, dy, None, out, g_start, g_len, E, N, K, accumulate, st)
+    native.check_status()
+    spans = list(zip(g_start.tolist(), g_len.tolist()))
+    for e in range(E):
+        want = sum((dy[s:s + n].double().t() @ x[s:s + n].double() for s, n in spans[e::E] if n),
+                   torch.zeros(N, K, dtype=torch.float64, device="cuda"))
+        bound = 1e-5 * max(1.0, float(want.abs().max()))
+        assert (f32[e].double() - want).abs().max() <= (bound if has_rows(e) else 0), e
+        assert torch.equal(b16[e], f32[e].to(torch.bfloat16)), e
+        assert (added[e].double() - 3 - want).abs().max() <= (bound if has_rows(e) else 0), e
+
+
+# 128 experts of 5 x 5 pair tiles: some forty tiles per pair, most of them of experts without rows; the smaller ones take
+# single CTAs.
+_FEW_LIVE = [(128, 1032, 1096, 1, "first"), (128, 1032, 1096, 1, "last"), (128, 1032, 1096, 2, "alternating"),
+             (128, 1032, 1096, 1, "none"), (40, 520, 328, 2, "all"), (8, 520, 72, 1, "first"), (12, 136, 264, 2, "last")]
+
+
+@pytest.mark.parametrize("E,N,K,sources,live", _FEW_LIVE)
+def test_grouped_weight_gradient_with_few_live_experts(E, N, K, sources, live):
+    _weight_gradient_with_few_live_experts(E, N, K, sources, live)
+
+
+def test_grouped_weight_gradient_with_few_live_experts_in_static_order():
+    """In a process of its own: the order of the tiles is read from the environment once."""
+    root = Path(__file__).resolve().parent.parent
+    code = ("from tests.test_moe_gpu import _FEW_LIVE, _weight_gradient_with_few_live_experts as check\n"
+            "for case in _FEW_LIVE: check(*case)")
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=root,
+                   env={**os.environ, "PIPER_GEMM_STATIC_TILES": "1"})
 
 
 def test_qwen3_moe_model_trains_on_one_gpu():
