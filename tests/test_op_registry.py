@@ -290,6 +290,23 @@ def test_native_formulas_under_a_recomputing_checkpoint():
     native.check_status()
 
 
+@pytest.mark.gpu
+def test_native_bodies_refuse_the_shapes_that_the_python_ones_refuse():
+    """The bodies unpack their arguments' shapes, and so does the fake body: [tokens, experts], [tokens, features], [experts, N,
+    K], [tokens, k], at least one dimension for the activation."""
+    def b16(*shape):
+        return torch.zeros(shape, device="cuda", dtype=torch.bfloat16)
+
+    i1, i2 = torch.zeros(4, device="cuda", dtype=torch.int32), torch.zeros(4, 2, device="cuda", dtype=torch.int32)
+    calls = [lambda: moe.moe_route(b16(4, 3, 8), 2, True), lambda: moe.moe_route(b16(8), 2, True), lambda: core.swiglu(b16()),
+             lambda: moe.moe_dispatch(b16(4, 3, 8), i2, i1), lambda: moe.moe_dispatch(b16(4, 8), i1, i1),
+             lambda: moe.grouped_linear(b16(128, 8), b16(8, 8), i1, i1),
+             lambda: moe.moe_combine(b16(128, 8), i1, torch.zeros(4, device="cuda"), i1, i1, i1)]
+    for call in calls:
+        with pytest.raises((RuntimeError, ValueError, IndexError)):
+            call()
+
+
 _CUDA_CHANGES = """
 import importlib, torch
 from piper_b200 import ops
