@@ -48,6 +48,12 @@ void check_rc(int rc, const char* what, int kernels = 1) {
 
 int64_t kernel_launch_count() { return g_kernel_launches.load(std::memory_order_relaxed); }
 
+// Rows of `inner` elements.  An empty row is refused: the division would end the process.
+int64_t rows_of(const Tensor& t, int64_t inner, const char* what) {
+  TORCH_CHECK(inner > 0, what, ": rows are empty");
+  return t.numel() / inner;
+}
+
 const void* opt_ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 float* opt_f32(const OptTensor& t) {
   if (!t.has_value()) return nullptr;
@@ -130,7 +136,7 @@ void rmsnorm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, Tensor 
   check_bf16(w, "w");
   TORCH_CHECK(x.is_contiguous() && y.is_contiguous(), "rmsnorm expects contiguous tensors");
   const int64_t D = x.size(-1);
-  const int64_t T = x.numel() / D;
+  const int64_t T = rows_of(x, D, "rmsnorm");
   TORCH_CHECK(res.has_value() == h_out.has_value(), "res and h_out go together");
   check_rc(piper::rmsnorm_fwd(x.data_ptr(), opt_ptr(res), w.data_ptr(), y.data_ptr(),
                               h_out.has_value() ? h_out->data_ptr() : nullptr, rstd.data_ptr<float>(), T,
@@ -146,7 +152,7 @@ void rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tenso
   check_bf16(dy, "dy");
   check_bf16(x, "x");
   const int64_t D = x.size(-1);
-  const int64_t T = x.numel() / D;
+  const int64_t T = rows_of(x, D, "rmsnorm");
   TORCH_CHECK(dw_partial.numel() >= piper::rmsnorm_bwd_num_partials(T) * D, "dw_partial too small");
   check_rc(piper::rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), opt_ptr(dres),
                               dx.data_ptr(), dw_partial.data_ptr<float>(), opt_f32(dw_f32),
@@ -162,7 +168,7 @@ void qk_rope_fwd(const Tensor& qkv, Tensor out, const Tensor& cos, const Tensor&
   TORCH_CHECK(qkv.is_contiguous() && out.is_contiguous(), "qk_rope expects contiguous tensors");
   TORCH_CHECK(cos.scalar_type() == at::kFloat && sin.scalar_type() == at::kFloat, "cos/sin must be fp32");
   TORCH_CHECK(cos.size(0) >= S && cos.size(-1) == hd / 2, "cos/sin must be [>=S, hd/2]");
-  const int64_t T = qkv.numel() / ((Hq + 2 * Hkv) * hd);
+  const int64_t T = rows_of(qkv, (Hq + 2 * Hkv) * hd, "qk_rope");
   check_rc(piper::qk_rope_fwd(qkv.data_ptr(), out.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(),
                               opt_ptr(qw), opt_ptr(kw), T, static_cast<int>(S), static_cast<int>(Hq),
                               static_cast<int>(Hkv), static_cast<int>(hd), interleaved ? 1 : 0,
@@ -174,7 +180,7 @@ void qk_rope_bwd(const Tensor& dout, const Tensor& qkv, Tensor din, const Tensor
                  const OptTensor& qw, const OptTensor& kw, const OptTensor& dqw, const OptTensor& dkw,
                  int64_t S, int64_t Hq, int64_t Hkv, int64_t hd, bool interleaved, double eps) {
   check_bf16(dout, "dout");
-  const int64_t T = dout.numel() / ((Hq + 2 * Hkv) * hd);
+  const int64_t T = rows_of(dout, (Hq + 2 * Hkv) * hd, "qk_rope");
   check_rc(piper::qk_rope_bwd(dout.data_ptr(), qkv.data_ptr(), din.data_ptr(), cos.data_ptr<float>(),
                               sin.data_ptr<float>(), opt_ptr(qw), opt_ptr(kw), opt_f32(dqw), opt_f32(dkw), T,
                               static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(Hkv),
@@ -187,7 +193,8 @@ void swiglu_fwd(const Tensor& h13, Tensor act) {
   check_bf16(h13, "h13");
   TORCH_CHECK(h13.is_contiguous() && act.is_contiguous(), "swiglu expects contiguous tensors");
   const int64_t F = act.size(-1);
-  check_rc(piper::swiglu_fwd(h13.data_ptr(), act.data_ptr(), act.numel() / F, static_cast<int>(F), cur_stream()),
+  check_rc(piper::swiglu_fwd(h13.data_ptr(), act.data_ptr(), rows_of(act, F, "swiglu"), static_cast<int>(F),
+                             cur_stream()),
            "swiglu_fwd");
 }
 
@@ -196,7 +203,7 @@ void swiglu_bwd(const Tensor& h13, const Tensor& dact, Tensor dh13) {
   check_bf16(dact, "dact");
   TORCH_CHECK(dact.is_contiguous() && dh13.is_contiguous(), "swiglu expects contiguous tensors");
   const int64_t F = dact.size(-1);
-  check_rc(piper::swiglu_bwd(h13.data_ptr(), dact.data_ptr(), dh13.data_ptr(), dact.numel() / F,
+  check_rc(piper::swiglu_bwd(h13.data_ptr(), dact.data_ptr(), dh13.data_ptr(), rows_of(dact, F, "swiglu"),
                              static_cast<int>(F), cur_stream()),
            "swiglu_bwd");
 }

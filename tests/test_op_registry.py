@@ -307,6 +307,20 @@ def test_native_bodies_refuse_the_shapes_that_the_python_ones_refuse():
             call()
 
 
+@pytest.mark.gpu
+def test_native_bodies_refuse_empty_rows():
+    """A last dimension of zero (or half of one) raises, as it did in Python, and does not divide by zero."""
+    def b16(*shape):
+        return torch.zeros(shape, device="cuda", dtype=torch.bfloat16)
+
+    cos = torch.zeros(4, 0, device="cuda")
+    for call in (lambda: core.rmsnorm_fwd(b16(4, 0), b16(0), 1e-5), lambda: core.add_rmsnorm_fwd(b16(4, 0), b16(4, 0), b16(0), 1e-5),
+                 lambda: core.swiglu(b16(4, 0)), lambda: core.swiglu(b16(4, 1)),
+                 lambda: core.qk_rope(b16(4, 0), cos, cos, None, None, 4, 2, 1, 0, False, 1e-5)):
+        with pytest.raises((RuntimeError, ZeroDivisionError)):
+            call()
+
+
 _CUDA_CHANGES = """
 import importlib, torch
 from piper_b200 import ops
