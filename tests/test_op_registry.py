@@ -321,6 +321,34 @@ def test_native_bodies_refuse_empty_rows():
             call()
 
 
+@pytest.mark.gpu
+def test_per_token_cross_entropy_gradient_keeps_its_graph():
+    """With a gradient per token the formula is tensor arithmetic: under create_graph its result can be differentiated by the
+    upstream gradient, by the C++ formula as by the Python one."""
+    from piper_b200.ops import native
+
+    torch.manual_seed(10)
+    logits = torch.randn(6, 64, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    labels = torch.tensor([3, -100, 0, 63, 7, 7], device="cuda")
+    up, v = torch.randn(6, device="cuda", requires_grad=True), torch.randn(6, 64, device="cuda")
+    results = []
+    for installed in (True, False):
+        if not installed:
+            native.lib().native_op_remove("cross_entropy_fwd")
+        try:
+            loss, _ = core.cross_entropy_fwd(logits, labels, -100)
+            (g,) = torch.autograd.grad(loss, logits, up, create_graph=True)
+            assert g.requires_grad
+            results.append([g, *torch.autograd.grad((g.float() * v).sum(), up)])
+        finally:
+            native.lib().native_op_install("cross_entropy_fwd")
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    p = torch.softmax(logits.detach().double(), -1) - torch.nn.functional.one_hot(labels.clamp(min=0), 64)
+    want = (p * v).sum(-1) * (labels != -100)
+    bound = 2 ** -8 * (p * v).abs().sum(-1)                  # every summand is rounded to bf16 (2^-9), in fp32 sums
+    assert ((results[0][1] - want).abs() <= bound).all()
+
+
 _CUDA_CHANGES = """
 import importlib, torch
 from piper_b200 import ops
