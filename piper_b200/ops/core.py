@@ -50,27 +50,30 @@ class GradSinks:
         self._sinks: dict[int, Tensor] = {}
 
     def _native(self):
-        return torch.ops.piper_c if native.loaded() and globals().get("grad_sinks") is self else None
+        return native.lib() if native.loaded() and globals().get("grad_sinks") is self else None
 
     def register(self, param: Tensor, sink: Tensor) -> None:
         assert sink.dtype == torch.float32 and sink.numel() == param.numel()
-        address = param.data_ptr()
-        self._sinks[address] = sink.view(param.shape)
-        if (lib := self._native()) is not None:
-            lib.sink_set.default(address, self._sinks[address])
+        address, sink = param.data_ptr(), sink.view(param.shape)
+        with native.lock:
+            self._sinks[address] = sink
+            if (lib := self._native()) is not None:
+                lib.sink_set.default(address, sink)
 
     def unregister(self, param: Tensor) -> None:
         address = param.data_ptr()
-        if self._sinks.pop(address, None) is not None and (lib := self._native()) is not None:
-            lib.sink_unset.default(address)
+        with native.lock:
+            if self._sinks.pop(address, None) is not None and (lib := self._native()) is not None:
+                lib.sink_unset.default(address)
 
     def get(self, param: Tensor) -> Optional[Tensor]:
         return self._sinks.get(param.data_ptr())
 
     def clear(self) -> None:
-        self._sinks.clear()
-        if (lib := self._native()) is not None:
-            lib.sink_clear()
+        with native.lock:
+            self._sinks.clear()
+            if (lib := self._native()) is not None:
+                lib.sink_clear.default()
 
 
 grad_sinks = GradSinks()
@@ -340,14 +343,15 @@ host_op("linear_backward_host", _linear_backward_host)
 
 def _hand_over(lib) -> None:
     lib.set_fork_macs(_FORK_MIN_MACS)
-    lib.sink_clear()
+    lib.sink_clear.default()
     for address, sink in grad_sinks._sinks.items():
-        lib.sink_set(address, sink)
+        lib.sink_set.default(address, sink)
 
 
-native.on_load["core"] = _hand_over
-if native.loaded():
-    _hand_over(native.lib())
+with native.lock:
+    native.hand_over["core"] = _hand_over
+    if native.loaded():
+        _hand_over(native.lib())
 
 # --------------------------------------------------------------------------
 # RMSNorm (optionally fused with the residual add)

@@ -17,12 +17,17 @@ import torch
 
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libpiper_b200.so"
 _loaded = False
-_load_lock = threading.RLock()
+# Held while the library is loaded, and by whoever changes state that the library keeps a copy of, so that a change is either
+# part of what is handed over or told to the loaded library.
+lock = threading.RLock()
 # What the op bodies and formulas in the library look at besides the gradient buckets: each flag sends the calls that it
 # concerns to the Python body or formula.
 DEFER_WGRAD, FORK_PENDING, GATHER_GEMMS, EXPERT_RUNTIME = range(4)
 _flags = [False] * 4
-on_load: dict = {}         # module -> function that hands its state to the library once that is loaded
+# Module -> function that runs when the library is loaded: all of the first kind, which hand state over, then all of the
+# second, which make the ops run in the library.
+hand_over: dict = {}
+install: dict = {}
 _status: dict[int, torch.Tensor] = {}
 _status_detail: dict[int, torch.Tensor] = {}
 _cdll = None
@@ -64,7 +69,7 @@ def lib():
 
 def _load() -> None:
     global _loaded
-    with _load_lock:
+    with lock:
         if _loaded:
             return
         if not _LIB_PATH.exists():
@@ -73,18 +78,19 @@ def _load() -> None:
                 "(CUDA tensors are never routed to a PyTorch fallback)"
             )
         torch.ops.load_library(str(_LIB_PATH))
-        _loaded = True
         for i, on in enumerate(_flags):
             torch.ops.piper_c.set_op_flag(i, on)
-        for hand_over in list(on_load.values()):
-            hand_over(torch.ops.piper_c)
+        for hook in [*hand_over.values(), *install.values()]:
+            hook(torch.ops.piper_c)
+        _loaded = True          # last: nobody else takes the library for loaded before it has the state
 
 
 def set_flag(flag: int, on: bool) -> None:
     if _flags[flag] != on:
-        _flags[flag] = on
-        if _loaded:
-            torch.ops.piper_c.set_op_flag.default(flag, on)
+        with lock:
+            _flags[flag] = on
+            if _loaded:
+                torch.ops.piper_c.set_op_flag.default(flag, on)
 
 
 def cdll() -> ctypes.CDLL:

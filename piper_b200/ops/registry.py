@@ -51,7 +51,7 @@ def _install_native(lib) -> None:
             lib.native_op_install(op.name)
 
 
-native.on_load["registry"] = _install_native
+native.install["registry"] = _install_native
 
 
 class Op:
@@ -72,14 +72,16 @@ class Op:
         for method in ("register_autocast", "register_autograd", "register_effect", "register_fake", "register_kernel",
                        "register_torch_dispatch", "register_vmap", "set_kernel_enabled"):
             setattr(self.overload, method, getattr(self, method))
-        _ops[name] = self
-        if native.loaded():
-            native.lib().native_op_install(name)
+        with native.lock:
+            _ops[name] = self
+            if native.loaded():
+                native.lib().native_op_install(name)
 
     def _drop_native(self) -> None:
-        self._use_native = False
-        if native.loaded():
-            native.lib().native_op_remove(self.name)
+        with native.lock:
+            self._use_native = False
+            if native.loaded():
+                native.lib().native_op_remove(self.name)
 
     def register_fake(self, fn: Callable) -> Callable:
         torch.library.register_fake(self.qualname, fn, lib=self._lib, allow_override=True)

@@ -164,6 +164,60 @@ def test_op_modules_reload_and_ops_take_further_registrations():
     subprocess.run([sys.executable, "-c", _MODULE_CHANGES], check=True, timeout=300, cwd=root)
 
 
+def test_the_library_has_the_state_before_it_counts_as_loaded(monkeypatch, tmp_path):
+    """A stand-in library that records its calls: flags and buckets are handed over before an op is installed, nobody sees
+    the library as loaded before that, and a bucket that another thread registers meanwhile is not lost."""
+    import threading
+    import types
+
+    from piper_b200.ops import native
+
+    calls, handing, registered = [], threading.Event(), threading.Event()
+
+    class Call:
+        def __init__(self, name):
+            self.name = name
+
+        def __call__(self, *args):
+            calls.append((self.name, native.loaded(), args))
+            if self.name == "sink_clear":
+                handing.set()
+                registered.wait(0.2)              # the other thread waits for the lock, so this runs out
+
+        default = property(lambda self: self)
+
+    fake = types.SimpleNamespace(**{n: Call(n) for n in (
+        "set_op_flag", "set_fork_macs", "sink_clear", "sink_set", "sink_unset", "native_op_install", "native_op_remove")})
+    (tmp_path / "lib.so").touch()
+    monkeypatch.setattr(native, "_LIB_PATH", tmp_path / "lib.so")
+    monkeypatch.setattr(native, "_loaded", False)
+    monkeypatch.setattr(native, "torch", types.SimpleNamespace(ops=types.SimpleNamespace(
+        piper_c=fake, load_library=lambda path: None)))
+    early, late = torch.randn(4), torch.randn(5)
+    core.grad_sinks.register(early, torch.zeros(4))
+
+    def register():
+        handing.wait(10)
+        core.grad_sinks.register(late, torch.zeros(5))
+        registered.set()
+
+    thread = threading.Thread(target=register)
+    thread.start()
+    try:
+        assert native.lib() is fake and native.loaded()
+        thread.join(10)
+        assert registered.is_set()
+        loading = [c for c in calls if not c[1]]
+        kinds = [name for name, _, _ in loading]
+        assert kinds == sorted(kinds, key=["set_op_flag", "set_fork_macs", "sink_clear", "sink_set", "native_op_install"].index)
+        assert {a[0] for n, _, a in loading if n == "native_op_install"} >= {"linear", "moe_dispatch"}
+        sinks = [a[0] for n, _, a in calls if n == "sink_set"]
+        assert early.data_ptr() in sinks and late.data_ptr() in sinks
+    finally:
+        core.grad_sinks.unregister(early)
+        core.grad_sinks.unregister(late)
+
+
 def _cuda_calls():
     """Calls on CUDA tensors, with the arguments that take gradients."""
     def rn(*shape):
