@@ -403,6 +403,42 @@ def test_per_token_cross_entropy_gradient_keeps_its_graph():
     assert ((results[0][1] - want).abs() <= bound).all()
 
 
+@pytest.mark.gpu
+def test_profilers_and_dispatch_modes_see_native_formulas_as_python_ones():
+    """The kernels that a pass launches are ops of their own, which a profiler lists; a dispatch mode sees the op itself and what a
+    backward pass allocates.  (The C++ formulas run below autograd, so there it sees their kernels as well.)"""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from piper_b200.ops import native
+
+    def listed(fn, args):
+        seen = []
+
+        class Mode(TorchDispatchMode):
+            def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+                seen.append(str(func))
+                return func(*args, **(kwargs or {}))
+
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+            _one_pass(fn, args, "plain")
+        with Mode():
+            _one_pass(fn, args, "plain")
+        asks = ("rmsnorm_bwd_num_partials", "attn_bwd_floats")       # sizes: no kernels
+        return (sorted(e.name for e in prof.events() if e.name.startswith("piper_c::") and not e.name.endswith(asks)),
+                [n for n in seen if n.startswith("piper.")], any(n.startswith("aten.empty") for n in seen))
+
+    torch.manual_seed(11)
+    for name, (fn, args) in _cuda_calls().items():
+        op = name.split()[0]
+        got = listed(fn, args)
+        native.lib().native_op_remove(op)
+        try:
+            want = listed(fn, args)
+        finally:
+            native.lib().native_op_install(op)
+        assert got == want and got[0], (name, got, want)
+
+
 _CUDA_CHANGES = """
 import importlib, torch
 from piper_b200 import ops
