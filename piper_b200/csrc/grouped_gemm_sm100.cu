@@ -74,6 +74,7 @@ struct Barriers {
   uint64_t tile_full[RING];
   Tile tile[RING];
   uint32_t tmem_base;
+  int first;         // the first tile of this CTA (or pair)
 };
 static_assert(sizeof(Barriers) <= 768, "barriers");
 
@@ -174,8 +175,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (lane == 0) table[p.num_groups] = acc;
   }
   if (warp == 2) {
+    // tiles come from a counter, as in the dense kernel; the first one is drawn beside the table
+    int first = static_cast<int>(blockIdx.x) / CTAS;
+    if (rank == 0 && lane == 0 && p.sched != nullptr) first = atomicAdd(&p.sched[0], 1);
+    __syncwarp();
     tmem_alloc_n<CTAS>(&bars->tmem_base, 512);
     tmem_relinquish_n<CTAS>();
+    if (lane == 0) bars->first = first;
   }
   tc_fence_before();
   if (CTAS == 2) cluster_sync();
@@ -201,11 +207,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     bool ok = true;
     for (;; ++n) {
       if (rank == 0 && elect_one()) {
-        // the first tile is the number of the CTA (or pair), the next ones come from a counter
         const int units = static_cast<int>(gridDim.x) / CTAS;
-        const int i = n == 0 || p.sched == nullptr || num_tiles <= units
-                          ? static_cast<int>(blockIdx.x) / CTAS + static_cast<int>(n) * units
-                          : units + atomicAdd(&p.sched[0], 1);
+        const int i = n > 0 && p.sched != nullptr && num_tiles > units ? atomicAdd(&p.sched[0], 1)
+                                                                       : bars->first + static_cast<int>(n) * units;
         Tile t = {0, 0, -1, 0};
         if (i < num_tiles) {
           if (MODE == kGroupedWgrad) {
