@@ -140,7 +140,7 @@ void rmsnorm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, Tensor 
   TORCH_CHECK(res.has_value() == h_out.has_value(), "res and h_out go together");
   check_rc(piper::rmsnorm_fwd(x.data_ptr(), opt_ptr(res), w.data_ptr(), y.data_ptr(),
                               h_out.has_value() ? h_out->data_ptr() : nullptr, rstd.data_ptr<float>(), T,
-                              static_cast<int>(D), static_cast<float>(eps), cur_stream()),
+                              static_cast<int>(D), static_cast<float>(eps), num_sms(), cur_stream()),
            "rmsnorm_fwd");
 }
 

@@ -196,12 +196,17 @@ __device__ __forceinline__ float block_sum_once(float v, float (*scratch)[NORM_T
   return t;
 }
 
-// Forward: bound by memory.  Four CTAs per SM walk the rows and fetch the next one before the current one is reduced: with a
-// CTA per row every row paid for its first loads, for the norm weights behind the barrier and for a last wave.  Residual and
-// norm, 4096 x 4096: 27.7 and 23.5 us (134 MB, 5.7 TB/s), 8192 x 8192 115 and 87 us, 8192 x 2048 28.2 and 24.2 us; 1000 x 4096 7.7 us
-// both ways; three CTAs per SM 23.6 / 105 / 26.2, five 29.0 / 97 / 23.5.
+// Forward: bound by memory.  Four CTAs per SM (two of rows of 8192 elements, which take 115 registers a thread) walk the
+// rows and fetch the next one before the current one is reduced: with a CTA per row every row paid for its first loads, for
+// the norm weights behind the barrier and for a last wave.  Residual and norm, 4096 x 4096: 27.7 and 23.5 us (134 MB, 5.7
+// TB/s), 8192 x 8192 115 and 87 us, 8192 x 2048 28.2 and 24.0 us; 1000 x 4096 7.7 us both ways.  The grid is what is resident
+// at once, and the launch bound keeps it so; four CTAs per SM of 8192-wide rows, in two waves, and two: 592 rows 10.6 and 9.5 us,
+// 1777 22.9 and 22.3, 8192 86.7 and 87.6, without residual 1000 rows 10.8 and 9.9.
 template <int VPT>
-__global__ void __launch_bounds__(NORM_THREADS)
+constexpr int NORM_FWD_CTAS = VPT == 4 ? 2 : 4;   // per SM
+
+template <int VPT>
+__global__ void __launch_bounds__(NORM_THREADS, NORM_FWD_CTAS<VPT>)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                        __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd, long long T, float eps) {
@@ -879,8 +884,16 @@ inline int grid_for(long long work, int threads, int max_blocks = 148 * 16) {
 
 #define PIPER_LAUNCH_OK() (cudaGetLastError() == cudaSuccess ? 0 : -3)
 
+template <int VPT>
+static int rmsnorm_fwd_rows(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
+                            __nv_bfloat16* h_out, float* rstd, long long T, float eps, int num_sms, cudaStream_t st) {
+  const int ctas = NORM_FWD_CTAS<VPT> * num_sms;
+  rmsnorm_fwd_reg_kernel<VPT><<<static_cast<unsigned>(T < ctas ? T : ctas), NORM_THREADS, 0, st>>>(x, res, w, y, h_out, rstd, T, eps);
+  return PIPER_LAUNCH_OK();
+}
+
 int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd,
-                long long T, int D, float eps, cudaStream_t st) {
+                long long T, int D, float eps, int num_sms, cudaStream_t st) {
   if (D % 8 != 0) return -1;
   if (T == 0) return 0;
   const auto* xp = static_cast<const __nv_bfloat16*>(x);
@@ -888,11 +901,10 @@ int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_
   const auto* wp = static_cast<const __nv_bfloat16*>(w);
   auto* yp = static_cast<__nv_bfloat16*>(y);
   auto* hp = static_cast<__nv_bfloat16*>(h_out);
-  const unsigned grid = static_cast<unsigned>(T < 148 * 4 ? T : 148 * 4);
   switch (D) {
-    case 2048: rmsnorm_fwd_reg_kernel<1><<<grid, NORM_THREADS, 0, st>>>(xp, rp, wp, yp, hp, rstd, T, eps); return PIPER_LAUNCH_OK();
-    case 4096: rmsnorm_fwd_reg_kernel<2><<<grid, NORM_THREADS, 0, st>>>(xp, rp, wp, yp, hp, rstd, T, eps); return PIPER_LAUNCH_OK();
-    case 8192: rmsnorm_fwd_reg_kernel<4><<<grid, NORM_THREADS, 0, st>>>(xp, rp, wp, yp, hp, rstd, T, eps); return PIPER_LAUNCH_OK();
+    case 2048: return rmsnorm_fwd_rows<1>(xp, rp, wp, yp, hp, rstd, T, eps, num_sms, st);
+    case 4096: return rmsnorm_fwd_rows<2>(xp, rp, wp, yp, hp, rstd, T, eps, num_sms, st);
+    case 8192: return rmsnorm_fwd_rows<4>(xp, rp, wp, yp, hp, rstd, T, eps, num_sms, st);
     default: break;
   }
   rmsnorm_fwd_kernel<<<static_cast<unsigned>(T), NORM_THREADS, 0, st>>>(

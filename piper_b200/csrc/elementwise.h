@@ -10,7 +10,7 @@ namespace piper {
 // y = rmsnorm(x (+ res)) * w; when res != nullptr the sum is also written to
 // h_out (the new residual stream).  rstd[T] is saved for backward.
 int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd,
-                long long T, int D, float eps, cudaStream_t st);
+                long long T, int D, float eps, int num_sms, cudaStream_t st);
 
 // Number of row-strips (and rows of dw_partial) rmsnorm_bwd uses for T rows.
 int rmsnorm_bwd_num_partials(long long T);

@@ -221,10 +221,10 @@ def test_linear_gradients_around_the_fork_threshold(sizes, forked, monkeypatch):
     assert _close(results[0], want + held, 1e-4) and all(torch.equal(r, results[0]) for r in results)
 
 
-@pytest.mark.parametrize("T,D", [(1, 2048), (591, 4096), (593, 2048), (593, 8192), (1777, 2048)])
+@pytest.mark.parametrize("T,D", [(1, 2048), (591, 4096), (593, 2048), (593, 8192), (1777, 2048), (297, 8192)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_rmsnorm_rows_per_cta(T, D, residual):
-    """One CTA per row up to 592 rows, several rows per CTA behind: every row against fp32, rounded to bf16 once (2^-8), the
+    """One CTA per row up to 592 rows (296 of 8192 elements), several rows per CTA behind: every row against fp32, rounded to bf16 once (2^-8), the
     residual sum exactly."""
     from piper_b200.ops import core
 
