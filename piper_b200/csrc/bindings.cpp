@@ -172,7 +172,7 @@ void qk_rope_fwd(const Tensor& qkv, Tensor out, const Tensor& cos, const Tensor&
   check_rc(piper::qk_rope_fwd(qkv.data_ptr(), out.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(),
                               opt_ptr(qw), opt_ptr(kw), T, static_cast<int>(S), static_cast<int>(Hq),
                               static_cast<int>(Hkv), static_cast<int>(hd), interleaved ? 1 : 0,
-                              static_cast<float>(eps), cur_stream()),
+                              static_cast<float>(eps), num_sms(), cur_stream()),
            "qk_rope_fwd");
 }
 
@@ -185,7 +185,7 @@ void qk_rope_bwd(const Tensor& dout, const Tensor& qkv, Tensor din, const Tensor
                               sin.data_ptr<float>(), opt_ptr(qw), opt_ptr(kw), opt_f32(dqw), opt_f32(dkw), T,
                               static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(Hkv),
                               static_cast<int>(hd), interleaved ? 1 : 0, static_cast<float>(eps),
-                              cur_stream()),
+                              num_sms(), cur_stream()),
            "qk_rope_bwd");
 }
 

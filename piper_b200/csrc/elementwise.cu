@@ -963,18 +963,18 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
 // 32.1 and 28.2; 4096 x (32 + 2 x 8) x 128 backward 31.6 and 30.1, forward 32.8 with 8, 33.7 with 4.  With norms a group has
 // more work per head: 4096 x (32 + 2 x 4) x 128 forward 24.9 with 8, 22.6 with 4, backward 60.3 with 8, 61.3 with 4 and 69
 // with 2 (there its weight-gradient sums end in more shuffles and atomics); 1000 x (16 + 2 x 2) x 64 backward 13.3 and 9.4.
-static int rope_heads_per_group(long long T, int heads, int hd, bool norm, bool backward) {
+static int rope_heads_per_group(long long T, int heads, int hd, bool norm, bool backward, int num_sms) {
   const long long blocks = T * heads * (hd / 16) / 256;
-  if (backward && norm) return blocks / 8 < 2 * 148 ? 4 : 8;
-  if (blocks <= 4 * 148) return 1;
-  if (backward || blocks <= 16 * 148) return 2;
+  if (backward && norm) return blocks / 8 < 2 * num_sms ? 4 : 8;
+  if (blocks <= 4 * num_sms) return 1;
+  if (backward || blocks <= 16 * num_sms) return 2;
   return norm ? 4 : 8;
 }
 
 int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp, const void* qw,
                 const void* kw, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps,
-                cudaStream_t st) {
-  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, false);
+                int num_sms, cudaStream_t st) {
+  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, false, num_sms);
   const long long groups = T * ((Hq + 2 * Hkv + hpg - 1) / hpg);
   if (groups == 0) return 0;
   if (hd != 128 && hd != 64) return -1;
@@ -999,8 +999,8 @@ int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp,
 
 int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, const float* sinp,
                 const void* qw, const void* kw, float* dqw, float* dkw, long long T, int S, int Hq,
-                int Hkv, int hd, int interleaved, float eps, cudaStream_t st) {
-  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, true);
+                int Hkv, int hd, int interleaved, float eps, int num_sms, cudaStream_t st) {
+  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, true, num_sms);
   const long long groups = T * ((Hq + 2 * Hkv + hpg - 1) / hpg);
   if (groups == 0) return 0;
   if (hd != 128 && hd != 64) return -1;

@@ -26,10 +26,10 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
 // (qw/kw, may be null) and rotary embedding applied to the q and k heads.
 int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp, const void* qw,
                 const void* kw, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps,
-                cudaStream_t st);
+                int num_sms, cudaStream_t st);
 int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, const float* sinp,
                 const void* qw, const void* kw, float* dqw, float* dkw, long long T, int S, int Hq,
-                int Hkv, int hd, int interleaved, float eps, cudaStream_t st);
+                int Hkv, int hd, int interleaved, float eps, int num_sms, cudaStream_t st);
 
 int swiglu_fwd(const void* h13, void* act, long long T, int F, cudaStream_t st);
 int swiglu_bwd(const void* h13, const void* dact, void* dh13, long long T, int F, cudaStream_t st);
