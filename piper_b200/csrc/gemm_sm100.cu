@@ -13,9 +13,10 @@
 //   warps 4-11  epilogue: tcgen05.ld of the finished accumulator, conversion, staging in shared memory, TMA store (or
 //               TMA reduce-add), while the MMAs of the next tile run in the other accumulator.
 //
-// What bounds it: an SM fills shared memory from L2 at about 80 bytes per cycle.  A k-block of a 128 x w tile is
-// (128 + w) x 128 bytes for 2w cycles of MMA, 614 cycles of fill against 512 at w = 256; in a pair each SM loads half
-// of B's rows, (128 + w / 2) x 128 bytes, 410 cycles of fill, and reads half as much of B from shared memory.
+// What bounds it: an SM fills shared memory from L2 at about 65 bytes per cycle while it multiplies (see gemm_cost).  A
+// k-block of a 128 x w tile is (128 + w) x 128 bytes for 2w cycles of MMA, 756 cycles of fill against 512 at w = 256; in a
+// pair each SM loads half of B's rows, (128 + w / 2) x 128 bytes, 504 cycles of fill, and reads half as much of B from
+// shared memory.
 //
 // Each operand can be K-major (contraction index contiguous in memory) or
 // MN-major (row index contiguous), which covers forward (X W^T), input
@@ -343,8 +344,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
 // library does not link against libcuda directly.
-// cuTensorMapEncodeTiled through the runtime's driver entry point, so the
-// library does not link against libcuda directly.
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
@@ -365,7 +364,7 @@ EncodeFn get_encode_fn() {
 
 }  // namespace
 
-// Pool of tile-scheduler slots (next tile, finished CTAs), one slot per launch in rotation.  It is the only
+// Pool of tile-scheduler slots (next tile, finished CTAs), one slot per dense or grouped launch in rotation.  It is the only
 // device memory this library allocates by itself: 32 KiB, once per process.
 constexpr int kSchedSlots = 4096;
 
@@ -486,12 +485,15 @@ static int forced_tile() {
   return v;
 }
 
-// The height of a tile of full width: 256 rows by a CTA pair or 128 by one CTA.  Pairs load a third fewer operand bytes
-// per flop and draw less power (4096 x 28672 x 4096 in a long loop 733 us with one CTA per tile, 690 us in pairs), but
+// One CTA (128 rows) or a pair (256) per tile where gemm_cost does not tell them apart.  Pairs load a third fewer operand
+// bytes per flop and draw less power (4096 x 28672 x 4096 in a long loop 733 us with one CTA per tile, 690 us in pairs), but
 // a pair starts later and hands every tile over between its SMs (512 x 768 x 256 5.2 us and 6.0 us, 1024 x 4096 x 4096
-// 25.8 and 26.4 us).  So they are taken where there are rounds enough: by the number of rounds if all SMs had a 256 x 256 tile each, and
-// in a single such round for long contractions over well-filled SMs.  Wide fp32 outputs (weight gradients that add into
-// a bucket) of fewer than two rounds take the small tiles.
+// 25.8 and 26.4 us).  So near ties go to pairs where there are rounds enough: by the number of rounds if all SMs had a 256 x
+// 256 tile each, and in a single such round for long contractions over well-filled SMs; wide fp32 outputs (weight gradients
+// that add into a bucket) of fewer than two rounds go to single CTAs.  Of 1,410 random products (M 100-8192, N 256-16384, K
+// 64-14400, both directions) 255 are near ties, and on 70 of those where this rule and the lower cost differ it is the faster one 55
+// times and 1.0 % behind the better choice on average, the lower cost 4.9 % (7641 x 3376 x 200 26.9 us by one CTA, 23.4 in pairs;
+// 536 x 6272 x 3968 into fp32 38.4 and 41.8 us).
 int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms) {
   const long long n_tiles = (N + 255) / 256;
   const long long tiles256 = (M + 255) / 256 * n_tiles;

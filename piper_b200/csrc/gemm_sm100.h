@@ -38,7 +38,7 @@ struct GemmArgs {
 // CUresult of a failed tensor-map encode.
 int gemm_bf16_launch(const GemmArgs& args, int num_sms, cudaStream_t stream);
 
-// The tile height (128: one CTA, 256: a CTA pair) that suits an [M, N] output in tiles of full width.
+// The tile height (128: one CTA, 256: a CTA pair) that gemm_shape takes where the model of its costs is undecided.
 int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms);
 
 // The tile shape that gemm_bf16_launch chooses: CTAs per tile (1 or 2, 128 rows each) and columns.
