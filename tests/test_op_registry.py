@@ -164,6 +164,33 @@ def test_op_modules_reload_and_ops_take_further_registrations():
     subprocess.run([sys.executable, "-c", _MODULE_CHANGES], check=True, timeout=300, cwd=root)
 
 
+_EARLIER_KERNEL = """
+import torch
+from piper_b200.ops import core, native
+torch.library.register_kernel("piper::swiglu", "cuda", lambda h: h[..., : h.shape[-1] // 2] * 0 + 2)
+lib = native.lib()                 # loaded by the first CUDA call of a program
+assert not lib.native_op_install("swiglu") and lib.native_op_install("linear")
+table = torch._C._dispatch_dump_table("piper::swiglu").splitlines()
+assert [line for line in table if line.startswith("CUDA:")] and not [line for line in table if "bindings_ops" in line]
+lib.native_op_remove("linear")
+assert lib.native_op_install("linear")
+if torch.cuda.is_available():
+    h = torch.ones(2, 8, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    assert (core.swiglu(h) == 2).all()
+"""
+
+
+@pytest.mark.parametrize("where", ["cpu", pytest.param("gpu", marks=pytest.mark.gpu)])
+def test_kernels_registered_before_the_library_is_loaded_stay(where):
+    """A program's own CUDA kernel, registered with the dispatcher, is not hidden by the library's."""
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    root = Path(__file__).resolve().parent.parent
+    subprocess.run([sys.executable, "-c", _EARLIER_KERNEL], check=True, timeout=300, cwd=root)
+
+
 def test_the_library_has_the_state_before_it_counts_as_loaded(monkeypatch, tmp_path):
     """A stand-in library that records its calls: flags and buckets are handed over before an op is installed, nobody sees
     the library as loaded before that, and a bucket that another thread registers meanwhile is not lost."""
