@@ -430,6 +430,10 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 // for 32 cycles of arithmetic.  Both passes and the delta kernel at S = 4096, 32 q / 8 kv heads x 128: 653 us with
 // probabilities through shared memory in two launches, 391 us so (this kernel alone 379 us, and 427 us with dQ on
 // 64-row tiles as well).  With eight softmax warps instead of sixteen: 376 and 374 us, 3 x 1408, 32 / 8 x 64 142 and 138 us.
+// The scores come out of tensor memory as fragments, not as rows: lse and delta belong to the columns here, and with a row
+// per lane every lane reads all 32 pairs of its columns, 1,784 shared-memory wavefronts per 128 x 128 scores beside the 1,024
+// (head dimension 64) that the MMAs read their operands in.  A fragment has 4 rows x 8 columns per thread: a quarter of them.
+// This kernel at 3 x 1408, 32 / 8 x 64: 139 us by rows, 128 us so; 1 x 4096, 32 / 8 x 128, which is short of power: 382 and 375 us.
 constexpr int BWD_THREADS = 576;
 constexpr int BWD_TMA_WARP = 16, BWD_MMA_WARP = 17;
 
@@ -628,11 +632,14 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     // ------------------------------------------- P' / dS' tiles + epilogue
     const int wg = warp >> 3;                  // tiles wg, wg + 2, ...; tensor memory stage wg
     const int ch = (warp >> 2) & 1;            // columns [32 ch, 32 ch + 32) of every tile
-    const int row = (warp & 3) * 32 + lane;    // stationary row == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t ts = tmem_base + lane_sel + wg * 64 + ch * 32;
     const uint32_t td = ts + 128;
-    const int xpos = xb * 128 + row;   // position of this row inside the sequence
+    // Fragment layout (tmem_ld_16x256b_x4): this thread has columns 8c + c0 + {0, 1} of rows 16 h + 8 j + lane / 4 of its
+    // warp's 32 x 32 block, c < 4, h, j < 2.
+    constexpr uint32_t kUpper = 16u << 16;     // upper 16 lanes of the warp's window
+    const int c0 = 2 * (lane & 3);
+    const int xpos = xb * 128 + (warp & 3) * 32 + (lane >> 2);   // position of the thread's first row in the sequence
     const float2 sl2 = make_float2(scale_log2, scale_log2);
     constexpr float kNegLog2e = -1.4426950408889634f;
     const float2 neg_one = make_float2(-1.f, -1.f);
@@ -641,60 +648,69 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     for (int it = wg; it < n_iter; it += 2) {
       const uint32_t ph = (it >> 1) & 1;
       const int st = it % L::Y_STAGES;
-      const float4* vl = reinterpret_cast<const float4*>(smem + L::VEC_OFF + st * 2 * L::VEC_BYTES) + ch * 8;
-      const float4* vd = vl + L::VEC_BYTES / 16;
+      const float* vl = reinterpret_cast<const float*>(smem + L::VEC_OFF + st * 2 * L::VEC_BYTES) + ch * 32 + c0;
+      const float* vd = vl + L::VEC_BYTES / 4;
       if (!await_all(&bars->y_full[st], (it / L::Y_STAGES) & 1, status)) { ok = false; break; }
+      float2 nl[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float2 l2 = *reinterpret_cast<const float2*>(vl + 8 * c);
+        nl[c] = make_float2(l2.x * kNegLog2e, l2.y * kNegLog2e);
+      }
       if (!await_all(&bars->s_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
-      uint32_t sv[32], w[16];
-      tmem_ld_32x32(ts, sv);
+      uint32_t sv[2][16], w[8];
+      tmem_ld_16x256b_x4(ts, sv[0]);
+      tmem_ld_16x256b_x4(ts + kUpper, sv[1]);
       tmem_ld_wait();
       // Causal mask, applied once to the registers of the tiles that cross the diagonal (element (x row, y col) is
       // kept iff key <= query): a score of -inf turns into a probability and a score gradient of exactly zero.
       const int ypos0 = ti * 64 + ch * 32;
       if (ypos0 < xb * 128 + 127) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (xpos > ypos0 + i) sv[i] = 0xff800000u;
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (xpos + 16 * h + 8 * ((i >> 1) & 1) > ypos0 + 8 * (i >> 2) + c0 + (i & 1)) sv[h][i] = 0xff800000u;
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 l4 = vl[q];
-        const float2 n0 = make_float2(l4.x * kNegLog2e, l4.y * kNegLog2e);
-        const float2 n1 = make_float2(l4.z * kNegLog2e, l4.w * kNegLog2e);
-        uint32_t* v = &sv[4 * q];
-        float2 p0 = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, n0);
-        float2 p1 = fma2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl2, n1);
-        p0.x = fast_exp2(p0.x); p0.y = fast_exp2(p0.y);
-        p1.x = fast_exp2(p1.x); p1.y = fast_exp2(p1.y);
-        v[0] = __float_as_uint(p0.x); v[1] = __float_as_uint(p0.y);
-        v[2] = __float_as_uint(p1.x); v[3] = __float_as_uint(p1.y);
-        w[2 * q] = pack_bf16x2(p0.x, p0.y);
-        w[2 * q + 1] = pack_bf16x2(p1.x, p1.y);
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {          // word i: columns of c = i / 2, row half i % 2
+          uint32_t* v = &sv[h][2 * i];
+          float2 p = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2, nl[i >> 1]);
+          p.x = fast_exp2(p.x);
+          p.y = fast_exp2(p.y);
+          v[0] = __float_as_uint(p.x);
+          v[1] = __float_as_uint(p.y);
+          w[i] = pack_bf16x2(p.x, p.y);
+        }
+        tmem_st_16x128b_x4(ts + h * kUpper, w);   // over columns this warp has already read
       }
-      tmem_st_32x16(ts, w);                    // over columns this thread has already read
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&bars->p_full[wg], lane);
+      float2 dl[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) dl[c] = *reinterpret_cast<const float2*>(vd + 8 * c);
       if (!await_all(&bars->dp_full[wg], ph, status)) { ok = false; break; }
       tc_fence_after();
-      uint32_t dv[32];
-      tmem_ld_32x32(td, dv);
+      uint32_t dv[2][16];
+      tmem_ld_16x256b_x4(td, dv[0]);
+      tmem_ld_16x256b_x4(td + kUpper, dv[1]);
       tmem_ld_wait();
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 d4 = vd[q];
-        float2 d0 = make_float2(d4.x, d4.y), d1 = make_float2(d4.z, d4.w);
-        const uint32_t* v = &dv[4 * q];
-        const uint32_t* p = &sv[4 * q];
-        d0 = fma2(d0, neg_one, make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])));
-        d1 = fma2(d1, neg_one, make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])));
-        d0 = mul2(d0, make_float2(__uint_as_float(p[0]), __uint_as_float(p[1])));
-        d1 = mul2(d1, make_float2(__uint_as_float(p[2]), __uint_as_float(p[3])));
-        w[2 * q] = pack_bf16x2(d0.x, d0.y);
-        w[2 * q + 1] = pack_bf16x2(d1.x, d1.y);
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t* v = &dv[h][2 * i];
+          const uint32_t* p = &sv[h][2 * i];
+          float2 d = fma2(dl[i >> 1], neg_one, make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])));
+          d = mul2(d, make_float2(__uint_as_float(p[0]), __uint_as_float(p[1])));
+          w[i] = pack_bf16x2(d.x, d.y);
+        }
+        tmem_st_16x128b_x4(td + h * kUpper, w);
       }
-      tmem_st_32x16(td, w);
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&bars->ds_full[wg], lane);
