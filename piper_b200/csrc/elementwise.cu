@@ -629,6 +629,17 @@ struct VecWalk {
   }
 };
 
+// sigmoid(g) as 1 / (1 + e) or e / (1 + e) with e = exp(-|g|): the divisor lies in (1, 2], where one approximate
+// reciprocal (1 ulp) has no range to check, and a large negative g keeps its small value instead of dividing by infinity.
+// An IEEE division per element made both kernels issue-bound.  With it and so, in us: 4096 x 14336 forward 72.9 and 58.8 (352 MB,
+// 6.0 TB/s), backward 109.4 and 101.3; 49,024 x 768 forward 52.4 and 37.0, backward 67.9 and 62.5.  Same error against 64 bits.
+__device__ __forceinline__ float sigmoid(float g) {
+  const float e = __expf(-fabsf(g));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return (g < 0.f ? e : 1.f) * r;
+}
+
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restrict__ act, long long T, int F,
                   int stride_rows, int stride_cols) {
@@ -639,7 +650,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restri
     unpack8(base[w.c], g);
     unpack8(base[vecs + w.c], u);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
+    for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid(g[j]) * u[j];
     reinterpret_cast<bf16x8*>(act + w.row * F)[w.c] = pack8(o);
   }
 }
@@ -656,7 +667,7 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ h13, const __nv_bfloat16* __
     unpack8(reinterpret_cast<const bf16x8*>(dact + w.row * F)[w.c], d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float sg = 1.f / (1.f + __expf(-g[j]));
+      const float sg = sigmoid(g[j]);
       const float silu = g[j] * sg;
       du[j] = d[j] * silu;
       dg[j] = d[j] * u[j] * sg * (1.f + g[j] * (1.f - sg));

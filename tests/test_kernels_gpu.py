@@ -471,6 +471,29 @@ def test_swiglu_grid_stride_walk(T, F):
     assert _close(a, ar, 1e-2) and _close(h.grad, hr.grad, 1e-2)
 
 
+def test_swiglu_large_gates():
+    """Gates of every magnitude: exp(-|g|) underflows on one side, and the small values on the other side stay."""
+    from piper_b200 import ops
+
+    g = torch.cat([torch.linspace(-120, 120, 4088, device="cuda"),
+                   torch.tensor([0.0, -0.0, 1e4, -1e4, 1e38, -1e38, float("inf"), float("nan")], device="cuda")])
+    u = torch.where(torch.arange(4096, device="cuda") % 2 == 0, 1.5, -0.75)
+    h = torch.cat([g, u])[None].bfloat16().requires_grad_(True)
+    a = ops.swiglu(h)
+    a.backward(torch.ones_like(a))
+    h64 = h.detach().double().requires_grad_(True)
+    a64 = torch.nn.functional.silu(h64[:, :4096]) * h64[:, 4096:]
+    a64.backward(torch.ones_like(a64))
+    # one rounding to bf16; exp of an argument of magnitude 88 is good to 2^-17; below 2^-126 results may be flushed.
+    # The gate's gradient is u s (1 + g (1 - s)), whose two terms cancel to their fp32 rounding near g = -1.28.
+    fin = slice(0, 4094)
+    assert torch.allclose(a.double()[:, fin], a64[:, fin], rtol=2 ** -8, atol=2 ** -126)
+    assert torch.allclose(h.grad.double()[:, fin], h64.grad[:, fin], rtol=2 ** -8, atol=1e-6)
+    assert torch.allclose(h.grad.double()[:, 4096:][:, fin], h64.grad[:, 4096:][:, fin], rtol=2 ** -8, atol=2 ** -126)
+    assert a[0, 4094] == float("inf") or a[0, 4094] == float("-inf")
+    assert a[0, 4095].isnan() and h.grad[0, 4095].isnan() and h.grad[0, 8191].isnan()
+
+
 def test_swiglu_embedding_ce_adam():
     from piper_b200 import ops
     from piper_b200.ops import native
