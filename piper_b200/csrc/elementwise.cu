@@ -383,35 +383,59 @@ reduce_partials_kernel(const float* __restrict__ partial, int nblocks, int D,
 // rope pairs: interleaved (x[2i], x[2i+1]) or half-split (x[i], x[i+hd/2]).
 // cos/sin are fp32 [S, hd/2]; position of token t is t % S.
 //
-// A group of hd/16 lanes handles one (token, head) vector.  Every lane owns two 16-byte vectors chosen so
-// that both members of each of its eight rope pairs are its own: elements [16l, 16l+16) in the interleaved
-// form, [8l, 8l+8) and [hd/2 + 8l, hd/2 + 8l + 8) in the half-split form.  In both forms the lane's pairs use
-// cos/sin entries [8l, 8l+8).
-// A lane group walks several consecutive heads of one token, so the token's cos/sin entries are loaded once.
-
+// A group of hd/16 lanes handles one (token, head) vector.  Lane l owns the two 16-byte vectors [8l, 8l + 8) and
+// [hd/2 + 8l, hd/2 + 8l + 8), so a group reads and writes contiguous memory with every instruction, and both members of
+// each of its eight rope pairs are its own: pairs 8l .. 8l + 7 in the half-split form, 4l .. 4l + 3 and hd/4 + 4l ..
+// hd/4 + 4l + 3 in the interleaved one.
+//
+// A warp takes (token, run of heads) tasks: its groups walk neighbouring heads of one token, whose cos/sin entries are
+// loaded once, and fetch the next head before they work on the current one.  The tasks are ordered by kind (query, key,
+// value heads), and the grid is what is resident at once: a warp has one kind at a time, hence one set of norm weights
+// and one set of weight-gradient sums in registers.
+// Bound by memory; 32 neighbouring bytes per lane (interleaved) or 640 to 2,368 CTAs of one pass each, without fetching ahead,
+// stayed far from it.  In us, forward and backward, so then and now: 4096 x (32 + 2 x 8) x 128 32.8 -> 19.4 (5.2 TB/s) and 30.1 ->
+// 19.6; 4096 x (32 + 2 x 4) x 128 with norms 23.7 -> 19.7 and 62.1 -> 32.7 (3.9 TB/s); 16384 x (32 + 2 x 4) x 128 with norms 84.8 ->
+// 64.0 and 185.7 -> 103.5; 8192 x (32 + 2 x 8) x 64 32.8 -> 29.2 and 28.1 -> 29.2; 512 x (4 + 2 x 4) x 64 2.6 -> 2.5 and 2.3 -> 2.5.
 template <int HD>
 struct RopeGroup {
   static constexpr int LANES = HD / 16;
-  int lane, off0, off1;
+  static constexpr int GROUPS = 32 / LANES;      // of a warp
+  int lane, group, off0, off1;
   unsigned mask;
-  __device__ __forceinline__ RopeGroup(int interleaved) {
+  __device__ __forceinline__ RopeGroup() {
     const int wl = threadIdx.x & 31;
     lane = wl & (LANES - 1);
-    mask = ((LANES == 32 ? 0u : (1u << LANES)) - 1u) << (wl & ~(LANES - 1));
-    off0 = interleaved ? 16 * lane : 8 * lane;
-    off1 = interleaved ? 16 * lane + 8 : HD / 2 + 8 * lane;
+    group = wl / LANES;
+    mask = ((1u << LANES) - 1u) << (wl & ~(LANES - 1));
+    off0 = 8 * lane;
+    off1 = HD / 2 + 8 * lane;
+  }
+  __device__ __forceinline__ void sum2(float& u, float& v) const {
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+      u += __shfl_xor_sync(mask, u, o);
+      v += __shfl_xor_sync(mask, v, o);
+    }
   }
   __device__ __forceinline__ float sum(float v) const {
 #pragma unroll
     for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
     return v;
   }
+  // The cos or sin entries of the lane's pairs, out of the row of one position.
+  template <bool INTER>
+  __device__ __forceinline__ void load_angles(const float* row, float sign, float (&f)[8]) const {
+    const float4 lo = *reinterpret_cast<const float4*>(row + (INTER ? 4 * lane : 8 * lane));
+    const float4 hi = *reinterpret_cast<const float4*>(row + (INTER ? HD / 4 + 4 * lane : 8 * lane + 4));
+    f[0] = lo.x * sign; f[1] = lo.y * sign; f[2] = lo.z * sign; f[3] = lo.w * sign;
+    f[4] = hi.x * sign; f[5] = hi.y * sign; f[6] = hi.z * sign; f[7] = hi.w * sign;
+  }
 };
 
 // (a, b) -> (a*c - b*s, a*s + b*c) on the lane's eight pairs.
-__device__ __forceinline__ void rope_rotate(float (&v0)[8], float (&v1)[8], const float (&c)[8], const float (&s)[8],
-                                            int interleaved) {
-  if (interleaved) {
+template <bool INTER>
+__device__ __forceinline__ void rope_rotate(float (&v0)[8], float (&v1)[8], const float (&c)[8], const float (&s)[8]) {
+  if (INTER) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const float a0 = v0[2 * p], b0 = v0[2 * p + 1], a1 = v1[2 * p], b1 = v1[2 * p + 1];
@@ -430,177 +454,173 @@ __device__ __forceinline__ void rope_rotate(float (&v0)[8], float (&v1)[8], cons
   }
 }
 
-__device__ __forceinline__ void load8f(const float* p, float (&f)[8], float scale) {
-  const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 4);
-  f[0] = lo.x * scale; f[1] = lo.y * scale; f[2] = lo.z * scale; f[3] = lo.w * scale;
-  f[4] = hi.x * scale; f[5] = hi.y * scale; f[6] = hi.z * scale; f[7] = hi.w * scale;
-}
+struct RopeArgs {
+  const __nv_bfloat16* x;        // forward: qkv; backward: the gradient of the output
+  const __nv_bfloat16* pre;      // backward with norms: qkv before them
+  __nv_bfloat16* out;
+  const float *cosp, *sinp;
+  const __nv_bfloat16 *qw, *kw;  // norm weights of the query and key heads, or null
+  float *dqw, *dkw;              // their gradients (accumulated), or null
+  long long T;
+  int S, Hq, Hkv;
+  float eps;
+  int run;                       // heads of a task
+};
 
-template <int HD>
-__global__ void __launch_bounds__(256)
-qk_rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
-               const float* __restrict__ cosp, const float* __restrict__ sinp,
-               const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
-               float* __restrict__ rstd_out, long long T, int S, int Hq, int Hkv,
-               int interleaved, float eps, float sin_sign, int heads_per_group) {
-  const RopeGroup<HD> g(interleaved);
-  constexpr int LANES = RopeGroup<HD>::LANES;
-  const int heads = Hq + 2 * Hkv;
-  const int chunks = (heads + heads_per_group - 1) / heads_per_group;
-  const unsigned total = static_cast<unsigned>(T) * chunks;   // the launcher keeps this below 2^31
-  const unsigned stride = gridDim.x * (blockDim.x / LANES);
-  for (unsigned gi = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; gi < total; gi += stride) {
-    const long long t = gi / static_cast<unsigned>(chunks);
-    const int h0 = static_cast<int>(gi - static_cast<unsigned>(t) * chunks) * heads_per_group;
-    const int h1 = min(heads, h0 + heads_per_group);
+enum RopeMode { kRopeCopy, kRopePlain, kRopeNorm };
+
+// The tasks of one kind: heads [first_head, first_head + n) of every token.  `task` is the warp's first one and becomes its
+// first one of the kind behind.  dw: sums of the weight gradient over the tasks, elements off0 .. and off1 ..
+template <int HD, RopeMode MODE, bool BWD, bool INTER>
+__device__ __forceinline__ void rope_tasks(const RopeArgs& a, const RopeGroup<HD>& g, int first_head, int n,
+                                           const __nv_bfloat16* w, unsigned& task, unsigned warps, float (&dw)[16]) {
+  constexpr bool PRE = BWD && MODE == kRopeNorm;
+  const int runs = (n + a.run - 1) / a.run;
+  const unsigned tasks = static_cast<unsigned>(a.T) * runs;     // the launcher keeps this below 2^31
+  const int heads = a.Hq + 2 * a.Hkv;
+  bf16x8 pw0, pw1;
+  if (MODE == kRopeNorm) {
+    pw0 = *reinterpret_cast<const bf16x8*>(w + g.off0);
+    pw1 = *reinterpret_cast<const bf16x8*>(w + g.off1);
+  }
+  for (; task < tasks; task += warps) {
+    const unsigned t = task / static_cast<unsigned>(runs);
+    const int r = static_cast<int>(task - t * runs);
+    int h = r * a.run + g.group;
+    const int h1 = min(n, (r + 1) * a.run);
+    if (h >= h1) continue;
+    long long at = (static_cast<long long>(t) * heads + first_head + h) * HD;
+    bf16x8 n0 = *reinterpret_cast<const bf16x8*>(a.x + at + g.off0), n1 = *reinterpret_cast<const bf16x8*>(a.x + at + g.off1);
+    bf16x8 m0, m1;
+    if (PRE) {
+      m0 = *reinterpret_cast<const bf16x8*>(a.pre + at + g.off0);
+      m1 = *reinterpret_cast<const bf16x8*>(a.pre + at + g.off1);
+    }
     float c[8], s[8];
-    const int cs = static_cast<int>(static_cast<unsigned>(t) % static_cast<unsigned>(S)) * (HD / 2) + 8 * g.lane;
-    load8f(cosp + cs, c, 1.f);
-    load8f(sinp + cs, s, sin_sign);
-#pragma unroll 4
-    for (int h = h0; h < h1; ++h) {
-      const __nv_bfloat16* src = in + (t * heads + h) * HD;
-      __nv_bfloat16* dst = out + (t * heads + h) * HD;
-      const bf16x8 p0 = *reinterpret_cast<const bf16x8*>(src + g.off0);
-      const bf16x8 p1 = *reinterpret_cast<const bf16x8*>(src + g.off1);
-      if (h >= Hq + Hkv) {   // value head: plain copy
+    if (MODE != kRopeCopy) {
+      const int pos = static_cast<int>(t % static_cast<unsigned>(a.S)) * (HD / 2);
+      g.template load_angles<INTER>(a.cosp + pos, 1.f, c);
+      g.template load_angles<INTER>(a.sinp + pos, BWD ? -1.f : 1.f, s);
+    }
+#pragma unroll 1
+    for (; h < h1; h += g.GROUPS) {
+      const bf16x8 p0 = n0, p1 = n1, q0 = m0, q1 = m1;
+      __nv_bfloat16* dst = a.out + at;
+      at += g.GROUPS * HD;
+      if (h + g.GROUPS < h1) {
+        n0 = *reinterpret_cast<const bf16x8*>(a.x + at + g.off0);
+        n1 = *reinterpret_cast<const bf16x8*>(a.x + at + g.off1);
+        if (PRE) {
+          m0 = *reinterpret_cast<const bf16x8*>(a.pre + at + g.off0);
+          m1 = *reinterpret_cast<const bf16x8*>(a.pre + at + g.off1);
+        }
+      }
+      if (MODE == kRopeCopy) {
         *reinterpret_cast<bf16x8*>(dst + g.off0) = p0;
         *reinterpret_cast<bf16x8*>(dst + g.off1) = p1;
         continue;
       }
-      float v0[8], v1[8];
+      float v0[8], v1[8], w0[8], w1[8];
       unpack8(p0, v0);
       unpack8(p1, v1);
-      const __nv_bfloat16* nw = (h < Hq) ? qw : kw;
-      if (nw != nullptr) {
-        float ss = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ss += v0[j] * v0[j] + v1[j] * v1[j];
-        ss = g.sum(ss);
-        const float r = rsqrtf(ss / HD + eps);
-        if (rstd_out != nullptr && g.lane == 0) rstd_out[t * (Hq + Hkv) + h] = r;
-        float w0[8], w1[8];
-        unpack8(*reinterpret_cast<const bf16x8*>(nw + g.off0), w0);
-        unpack8(*reinterpret_cast<const bf16x8*>(nw + g.off1), w1);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          v0[j] = v0[j] * r * w0[j];
-          v1[j] = v1[j] * r * w1[j];
-        }
+      if (MODE == kRopeNorm) {
+        unpack8(pw0, w0);
+        unpack8(pw1, w1);
       }
-      rope_rotate(v0, v1, c, s, interleaved);
+      if (BWD) {
+        rope_rotate<INTER>(v0, v1, c, s);
+        if (MODE == kRopeNorm) {
+          float x0[8], x1[8];
+          unpack8(q0, x0);
+          unpack8(q1, x1);
+          float ss = 0.f, dot = 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            ss += x0[j] * x0[j] + x1[j] * x1[j];
+            dot += v0[j] * w0[j] * x0[j] + v1[j] * w1[j] * x1[j];
+          }
+          g.sum2(ss, dot);
+          const float rs = rsqrtf(ss / HD + a.eps);
+          dot = dot * rs / HD;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xh0 = x0[j] * rs, xh1 = x1[j] * rs;
+            dw[j] += v0[j] * xh0;
+            dw[8 + j] += v1[j] * xh1;
+            v0[j] = rs * (v0[j] * w0[j] - xh0 * dot);
+            v1[j] = rs * (v1[j] * w1[j] - xh1 * dot);
+          }
+        }
+      } else {
+        if (MODE == kRopeNorm) {
+          float ss = 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ss += v0[j] * v0[j] + v1[j] * v1[j];
+          const float rs = rsqrtf(g.sum(ss) / HD + a.eps);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            v0[j] = v0[j] * rs * w0[j];
+            v1[j] = v1[j] * rs * w1[j];
+          }
+        }
+        rope_rotate<INTER>(v0, v1, c, s);
+      }
       *reinterpret_cast<bf16x8*>(dst + g.off0) = pack8(v0);
       *reinterpret_cast<bf16x8*>(dst + g.off1) = pack8(v1);
     }
   }
+  task -= tasks;
 }
 
-// Backward of QK-norm + RoPE: un-rotate the incoming gradient (RoPE is an orthogonal map, so its transpose is the
-// rotation by -theta), then apply the RMSNorm backward per head (NORM).  A lane's weight-gradient contributions stay in
-// registers over all heads it visits; they are summed over the warp, then the CTA, and added to fp32 dqw/dkw with one
-// atomic per element and CTA.  (Sixteen shared-memory atomics per lane and head made this kernel 7x slower than its
-// memory traffic: 147 us for 4096 tokens of 32 + 2 x 4 heads x 128.)
-template <int HD, bool NORM>
-__global__ void __launch_bounds__(256)
-qk_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ in /*pre-norm qkv*/,
-                   __nv_bfloat16* __restrict__ din, const float* __restrict__ cosp,
-                   const float* __restrict__ sinp, const __nv_bfloat16* __restrict__ qw,
-                   const __nv_bfloat16* __restrict__ kw, float* __restrict__ dqw,
-                   float* __restrict__ dkw, long long T, int S, int Hq, int Hkv,
-                   int interleaved, float eps, int heads_per_group) {
+// NORM: there are norm weights, of the query heads, the key heads or both.  Backward: un-rotate the gradient (RoPE is an
+// orthogonal map, so its transpose is the rotation by -theta), then the RMSNorm backward per head; the weight-gradient
+// sums of a warp are added over its lane groups, then over the CTA, and go to fp32 dw with one atomic per element and CTA.
+// (Sixteen shared-memory atomics per lane and head took 147 us for 4096 tokens of 32 + 2 x 4 heads x 128.)
+template <bool NORM, bool BWD>
+constexpr int ROPE_CTAS = !NORM ? 4 : BWD ? 2 : 3;     // per SM
+
+// The heads of one kind with the norm they have, and their weight gradient into sdw.
+template <int HD, bool NORM, bool BWD, bool INTER>
+__device__ __forceinline__ void rope_kind(const RopeArgs& a, const RopeGroup<HD>& g, int first_head, int n,
+                                          const __nv_bfloat16* w, bool want_dw, float* sdw, unsigned& task, unsigned warps) {
+  float dw[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) dw[j] = 0.f;
+  if (!NORM || w == nullptr) {
+    rope_tasks<HD, kRopePlain, BWD, INTER>(a, g, first_head, n, nullptr, task, warps, dw);
+    return;
+  }
+  rope_tasks<HD, kRopeNorm, BWD, INTER>(a, g, first_head, n, w, task, warps, dw);
+  if (!want_dw) return;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+#pragma unroll
+    for (int o = g.LANES; o < 32; o <<= 1) dw[j] += __shfl_xor_sync(0xffffffffu, dw[j], o);
+    if (g.group == 0) atomicAdd(sdw + (j < 8 ? g.off0 : g.off1) + (j & 7), dw[j]);
+  }
+}
+
+template <int HD, bool NORM, bool BWD, bool INTER>
+__global__ void __launch_bounds__(256, ROPE_CTAS<NORM, BWD>)
+qk_rope_kernel(const __grid_constant__ RopeArgs a) {
   __shared__ float sdw[2][HD];
-  const bool want_dw = NORM && (dqw != nullptr || dkw != nullptr);
+  const bool want_dw = NORM && BWD && (a.dqw != nullptr || a.dkw != nullptr);
   if (want_dw) {
     for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) (&sdw[0][0])[i] = 0.f;
     __syncthreads();
   }
-  const RopeGroup<HD> g(interleaved);
-  constexpr int LANES = RopeGroup<HD>::LANES;
-  const int heads = Hq + 2 * Hkv;
-  const int chunks = (heads + heads_per_group - 1) / heads_per_group;
-  const unsigned total = static_cast<unsigned>(T) * chunks;   // the launcher keeps this below 2^31
-  const unsigned stride = gridDim.x * (blockDim.x / LANES);
-  float aq[NORM ? 16 : 1], ak[NORM ? 16 : 1];
-#pragma unroll
-  for (int j = 0; j < (NORM ? 16 : 1); ++j) aq[j] = ak[j] = 0.f;
-  for (unsigned gi = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; gi < total; gi += stride) {
-    const long long t = gi / static_cast<unsigned>(chunks);
-    const int h0 = static_cast<int>(gi - static_cast<unsigned>(t) * chunks) * heads_per_group;
-    const int h1 = min(heads, h0 + heads_per_group);
-    float c[8], s[8];
-    const int cs = static_cast<int>(static_cast<unsigned>(t) % static_cast<unsigned>(S)) * (HD / 2) + 8 * g.lane;
-    load8f(cosp + cs, c, 1.f);
-    load8f(sinp + cs, s, -1.f);
-#pragma unroll (NORM ? 2 : 4)
-    for (int h = h0; h < h1; ++h) {
-      const __nv_bfloat16* gp = dout + (t * heads + h) * HD;
-      __nv_bfloat16* dst = din + (t * heads + h) * HD;
-      const bf16x8 p0 = *reinterpret_cast<const bf16x8*>(gp + g.off0);
-      const bf16x8 p1 = *reinterpret_cast<const bf16x8*>(gp + g.off1);
-      if (h >= Hq + Hkv) {
-        *reinterpret_cast<bf16x8*>(dst + g.off0) = p0;
-        *reinterpret_cast<bf16x8*>(dst + g.off1) = p1;
-        continue;
-      }
-      float d0[8], d1[8];
-      unpack8(p0, d0);
-      unpack8(p1, d1);
-      rope_rotate(d0, d1, c, s, interleaved);
-      const __nv_bfloat16* nw = (h < Hq) ? qw : kw;
-      if (NORM && nw != nullptr) {
-        const __nv_bfloat16* src = in + (t * heads + h) * HD;
-        float x0[8], x1[8], w0[8], w1[8];
-        unpack8(*reinterpret_cast<const bf16x8*>(src + g.off0), x0);
-        unpack8(*reinterpret_cast<const bf16x8*>(src + g.off1), x1);
-        unpack8(*reinterpret_cast<const bf16x8*>(nw + g.off0), w0);
-        unpack8(*reinterpret_cast<const bf16x8*>(nw + g.off1), w1);
-        float ss = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ss += x0[j] * x0[j] + x1[j] * x1[j];
-        ss = g.sum(ss);
-        const float r = rsqrtf(ss / HD + eps);
-        float dot = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) dot += (d0[j] * w0[j] * x0[j] + d1[j] * w1[j] * x1[j]) * r;
-        dot = g.sum(dot) / HD;
-        const bool is_q = h < Hq;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh0 = x0[j] * r, xh1 = x1[j] * r;
-          const float u0 = d0[j] * xh0, u1 = d1[j] * xh1;
-          if (is_q) {
-            aq[j] += u0;
-            aq[8 + j] += u1;
-          } else {
-            ak[j] += u0;
-            ak[8 + j] += u1;
-          }
-          d0[j] = r * (d0[j] * w0[j] - xh0 * dot);
-          d1[j] = r * (d1[j] * w1[j] - xh1 * dot);
-        }
-      }
-      *reinterpret_cast<bf16x8*>(dst + g.off0) = pack8(d0);
-      *reinterpret_cast<bf16x8*>(dst + g.off1) = pack8(d1);
-    }
-  }
+  const RopeGroup<HD> g;
+  unsigned task = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const unsigned warps = gridDim.x * 8;
+  rope_kind<HD, NORM, BWD, INTER>(a, g, 0, a.Hq, a.qw, want_dw, sdw[0], task, warps);
+  rope_kind<HD, NORM, BWD, INTER>(a, g, a.Hq, a.Hkv, a.kw, want_dw, sdw[1], task, warps);
+  float none[16];
+  rope_tasks<HD, kRopeCopy, BWD, INTER>(a, g, a.Hq + a.Hkv, a.Hkv, nullptr, task, warps, none);
   if (want_dw) {
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < (NORM ? 16 : 1); ++j) {
-#pragma unroll
-      for (int o = LANES; o < 32; o <<= 1) {       // over the warp's lane groups: same elements
-        aq[j] += __shfl_xor_sync(0xffffffffu, aq[j], o);
-        ak[j] += __shfl_xor_sync(0xffffffffu, ak[j], o);
-      }
-      if ((threadIdx.x & 31) < LANES) {
-        const int e = (j < 8 ? g.off0 : g.off1) + (j & 7);
-        atomicAdd(&sdw[0][e], aq[j]);
-        atomicAdd(&sdw[1][e], ak[j]);
-      }
-    }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) {
-      float* dwp = i < HD ? dqw : dkw;
+      float* dwp = i < HD ? a.dqw : a.dkw;
       const float v = (&sdw[0][0])[i];
       if (dwp != nullptr && v != 0.f) atomicAdd(dwp + (i < HD ? i : i - HD), v);
     }
@@ -981,67 +1001,54 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
   return PIPER_LAUNCH_OK();
 }
 
-// Heads that a lane group walks: more of them share one load of cos/sin, fewer make more groups to run at a time.  `blocks`
-// are the CTAs that one head per group makes.  In us, 8 heads per group and by this rule: 512 tokens of 4 + 2 x 4 heads x 64
-// forward 6.0 and 2.6, backward 5.8 and 2.3; 2048 x (32 + 2 x 8) x 64 12.4 and 9.8, 12.2 and 9.1; 8192 x (32 + 2 x 8) x 64 backward
-// 32.1 and 28.2; 4096 x (32 + 2 x 8) x 128 backward 31.6 and 30.1, forward 32.8 with 8, 33.7 with 4.  With norms a group has
-// more work per head: 4096 x (32 + 2 x 4) x 128 forward 24.9 with 8, 22.6 with 4, backward 60.3 with 8, 61.3 with 4 and 69
-// with 2 (there its weight-gradient sums end in more shuffles and atomics); 1000 x (16 + 2 x 2) x 64 backward 13.3 and 9.4.
-static int rope_heads_per_group(long long T, int heads, int hd, bool norm, bool backward, int num_sms) {
-  const long long blocks = T * heads * (hd / 16) / 256;
-  if (backward && norm) return blocks / 8 < 2 * num_sms ? 4 : 8;
-  if (blocks <= 4 * num_sms) return 1;
-  if (backward || blocks <= 16 * num_sms) return 2;
-  return norm ? 4 : 8;
+// Heads of a task: more of them share one load of cos/sin and fetch ahead, fewer make more tasks to run at a time.
+// Four per lane group at 128 (two at 64, whose runs would span half a token) where that leaves two tasks per resident warp.
+// In us for 1, 2, 4 and 8 heads per lane group: 4096 x (32 + 2 x 4) x 128 with norms forward 21.6 19.6 19.7 21.8, backward 36.5 32.9
+// 32.7 32.8; 16384 tokens 75.7 66.5 64.2 63.7, 123.3 108.8 103.8 101.1; 8192 x (32 + 2 x 8) x 128 38.0 35.8 35.4 36.1; 8192 x (32 +
+// 2 x 8) x 64 30.2 29.2 30.2 30.2; 128 x (32 + 2 x 8) x 128 2.6 2.7 3.4 4.6.
+template <int HD, bool NORM, bool BWD>
+static int qk_rope_launch(RopeArgs a, bool interleaved, int num_sms, cudaStream_t st) {
+  const int resident = ROPE_CTAS<NORM, BWD> * num_sms;
+  auto tasks = [&](int run) { return a.T * ((a.Hq + run - 1) / run + 2ll * ((a.Hkv + run - 1) / run)); };
+  constexpr int groups = RopeGroup<HD>::GROUPS;
+  a.run = (HD == 128 ? 4 : 2) * groups;
+  while (a.run > groups && tasks(a.run) < 2ll * 8 * resident) a.run /= 2;
+  if (tasks(a.run) >= (1ll << 31)) return -1;
+  const long long blocks = (tasks(a.run) + 7) / 8;
+  auto kern = interleaved ? qk_rope_kernel<HD, NORM, BWD, true> : qk_rope_kernel<HD, NORM, BWD, false>;
+  kern<<<static_cast<unsigned>(blocks < resident ? blocks : resident), 256, 0, st>>>(a);
+  return PIPER_LAUNCH_OK();
+}
+
+template <bool BWD>
+static int qk_rope(const RopeArgs& a, int hd, bool interleaved, int num_sms, cudaStream_t st) {
+  if (a.T == 0 || a.Hq + 2 * a.Hkv == 0) return 0;
+  if (hd != 128 && hd != 64) return -1;
+  if (static_cast<long long>(a.S) * (hd / 2) >= (1ll << 31)) return -1;
+  if (!aligned16(a.x, a.pre, a.out, a.cosp, a.sinp, a.qw, a.kw)) return -4;
+  if (a.qw != nullptr || a.kw != nullptr)
+    return hd == 128 ? qk_rope_launch<128, true, BWD>(a, interleaved, num_sms, st)
+                     : qk_rope_launch<64, true, BWD>(a, interleaved, num_sms, st);
+  return hd == 128 ? qk_rope_launch<128, false, BWD>(a, interleaved, num_sms, st)
+                   : qk_rope_launch<64, false, BWD>(a, interleaved, num_sms, st);
 }
 
 int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp, const void* qw,
                 const void* kw, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps,
                 int num_sms, cudaStream_t st) {
-  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, false, num_sms);
-  const long long groups = T * ((Hq + 2 * Hkv + hpg - 1) / hpg);
-  if (groups == 0) return 0;
-  if (hd != 128 && hd != 64) return -1;
-  if (groups >= (1ll << 31) || static_cast<long long>(S) * (hd / 2) >= (1ll << 31)) return -1;
-  if (!aligned16(in, out, cosp, sinp, qw, kw)) return -4;
-  const int threads = 256;
-  const int blocks = grid_for(groups * (hd / 16), threads);
-  auto a = static_cast<const __nv_bfloat16*>(in);
-  auto o = static_cast<__nv_bfloat16*>(out);
-  auto q = static_cast<const __nv_bfloat16*>(qw);
-  auto k = static_cast<const __nv_bfloat16*>(kw);
-  if (hd == 128)
-    qk_rope_kernel<128><<<blocks, threads, 0, st>>>(a, o, cosp, sinp, q, k, nullptr, T, S, Hq, Hkv,
-                                                    interleaved, eps, 1.f, hpg);
-  else if (hd == 64)
-    qk_rope_kernel<64><<<blocks, threads, 0, st>>>(a, o, cosp, sinp, q, k, nullptr, T, S, Hq, Hkv,
-                                                   interleaved, eps, 1.f, hpg);
-  else
-    return -1;
-  return PIPER_LAUNCH_OK();
+  const RopeArgs a{static_cast<const __nv_bfloat16*>(in), nullptr, static_cast<__nv_bfloat16*>(out), cosp, sinp,
+                   static_cast<const __nv_bfloat16*>(qw), static_cast<const __nv_bfloat16*>(kw), nullptr, nullptr,
+                   T, S, Hq, Hkv, eps, 0};
+  return qk_rope<false>(a, hd, interleaved != 0, num_sms, st);
 }
 
 int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, const float* sinp,
                 const void* qw, const void* kw, float* dqw, float* dkw, long long T, int S, int Hq,
                 int Hkv, int hd, int interleaved, float eps, int num_sms, cudaStream_t st) {
-  const int hpg = rope_heads_per_group(T, Hq + 2 * Hkv, hd, qw != nullptr || kw != nullptr, true, num_sms);
-  const long long groups = T * ((Hq + 2 * Hkv + hpg - 1) / hpg);
-  if (groups == 0) return 0;
-  if (hd != 128 && hd != 64) return -1;
-  if (groups >= (1ll << 31) || static_cast<long long>(S) * (hd / 2) >= (1ll << 31)) return -1;
-  if (!aligned16(dout, in, din, cosp, sinp, qw, kw)) return -4;
-  const int threads = 256;
-  const int blocks = grid_for(groups * (hd / 16), threads);
-  auto g = static_cast<const __nv_bfloat16*>(dout);
-  auto a = static_cast<const __nv_bfloat16*>(in);
-  auto o = static_cast<__nv_bfloat16*>(din);
-  auto q = static_cast<const __nv_bfloat16*>(qw);
-  auto k = static_cast<const __nv_bfloat16*>(kw);
-  const bool norm = q != nullptr || k != nullptr;
-  auto kern = hd == 128 ? (norm ? qk_rope_bwd_kernel<128, true> : qk_rope_bwd_kernel<128, false>)
-                        : (norm ? qk_rope_bwd_kernel<64, true> : qk_rope_bwd_kernel<64, false>);
-  kern<<<blocks, threads, 0, st>>>(g, a, o, cosp, sinp, q, k, dqw, dkw, T, S, Hq, Hkv, interleaved, eps, hpg);
-  return PIPER_LAUNCH_OK();
+  const RopeArgs a{static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(in),
+                   static_cast<__nv_bfloat16*>(din), cosp, sinp, static_cast<const __nv_bfloat16*>(qw),
+                   static_cast<const __nv_bfloat16*>(kw), dqw, dkw, T, S, Hq, Hkv, eps, 0};
+  return qk_rope<true>(a, hd, interleaved != 0, num_sms, st);
 }
 
 int swiglu_fwd(const void* h13, void* act, long long T, int F, cudaStream_t st) {

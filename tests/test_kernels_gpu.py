@@ -263,6 +263,32 @@ def test_qk_rope_heads_per_group(T, Hq, Hkv, hd, norm):
         assert _close(w.grad, l.grad, 2 ** -8)
 
 
+@pytest.mark.parametrize("T,Hq,Hkv,hd,norms,inter", [(1, 1, 1, 64, "qk", True), (1, 1, 1, 128, "", False), (3, 7, 1, 64, "k", False),
+                                                     (515, 9, 3, 64, "q", True), (2500, 21, 5, 128, "q", True),
+                                                     (2500, 21, 5, 128, "k", False), (6001, 9, 3, 64, "qk", True),
+                                                     (6001, 9, 3, 64, "", True)])
+def test_qk_rope_tasks(T, Hq, Hkv, hd, norms, inter):
+    """Fewer tasks than warps and several per warp, head counts that leave lane groups of a warp without a head, norms of
+    one kind of heads only, positions that repeat; against the fp32 reference, bf16 rounding of results."""
+    from piper_b200.ops import core
+
+    torch.manual_seed(25)
+    S = max(1, T // 2)
+    cos, sin = core.rope_tables(hd, S, 1e4, device="cuda")
+    x = torch.randn(T, (Hq + 2 * Hkv) * hd, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    ws = [torch.randn(hd, device="cuda").to(torch.bfloat16).requires_grad_(True) if c in norms else None for c in "qk"]
+    out = core.qk_rope(x, cos, sin, *ws, S, Hq, Hkv, hd, inter, 1e-6)
+    g = torch.randn_like(out)
+    out.backward(g)
+    xr, *wr = [None if t is None else t.detach().float().requires_grad_(True) for t in (x, *ws)]
+    ref = core._qk_rope_ref(xr, cos, sin, *wr, S, Hq, Hkv, hd, inter, 1e-6)
+    ref.backward(g.float())
+    assert _close(out, ref, 2 ** -8) and _close(x.grad, xr.grad, 2 ** -8)
+    assert torch.equal(out[:, (Hq + Hkv) * hd:], x[:, (Hq + Hkv) * hd:]) and torch.equal(x.grad[:, (Hq + Hkv) * hd:], g[:, (Hq + Hkv) * hd:])
+    for w, l in zip(ws, wr):
+        assert w is None or _close(w.grad, l.grad, 2 ** -8)
+
+
 @pytest.mark.parametrize("T,D", [(300, 256), (300, 2048), (1000, 4096), (300, 8192), (7, 4096)])
 def test_rmsnorm_and_residual(T, D):
     from piper_b200 import ops
