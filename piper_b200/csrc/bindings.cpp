@@ -176,17 +176,29 @@ void qk_rope_fwd(const Tensor& qkv, Tensor out, const Tensor& cos, const Tensor&
            "qk_rope_fwd");
 }
 
+// dqw / dkw: fp32 (added to) or bf16 (written); `partial` is [strips, 2 hd] floats where one of them is given.
 void qk_rope_bwd(const Tensor& dout, const Tensor& qkv, Tensor din, const Tensor& cos, const Tensor& sin,
-                 const OptTensor& qw, const OptTensor& kw, const OptTensor& dqw, const OptTensor& dkw,
-                 int64_t S, int64_t Hq, int64_t Hkv, int64_t hd, bool interleaved, double eps) {
+                 const OptTensor& qw, const OptTensor& kw, const OptTensor& partial, const OptTensor& dqw,
+                 const OptTensor& dkw, int64_t S, int64_t Hq, int64_t Hkv, int64_t hd, bool interleaved, double eps) {
   check_bf16(dout, "dout");
   const int64_t T = rows_of(dout, (Hq + 2 * Hkv) * hd, "qk_rope");
+  const int64_t strips = partial.has_value() && hd > 0 ? std::min<int64_t>(partial->numel() / (2 * hd), 1 << 16) : 0;
+  TORCH_CHECK(!partial.has_value() || (partial->is_contiguous() && strips > 0), "partial is too small");
+  TORCH_CHECK((!dqw.has_value() && !dkw.has_value()) || partial.has_value(), "weight gradients need partial");
+  auto f32 = [&](const OptTensor& t) { return t.has_value() && t->scalar_type() == at::kFloat ? t->data_ptr<float>() : nullptr; };
+  auto b16 = [&](const OptTensor& t) -> void* {
+    if (!t.has_value() || t->scalar_type() == at::kFloat) return nullptr;
+    check_bf16(*t, "weight gradient");
+    return t->data_ptr();
+  };
+  for (const OptTensor* t : {&dqw, &dkw})
+    TORCH_CHECK(!t->has_value() || ((*t)->numel() == hd && (*t)->is_contiguous()), "weight gradients have hd elements");
   check_rc(piper::qk_rope_bwd(dout.data_ptr(), qkv.data_ptr(), din.data_ptr(), cos.data_ptr<float>(),
-                              sin.data_ptr<float>(), opt_ptr(qw), opt_ptr(kw), opt_f32(dqw), opt_f32(dkw), T,
-                              static_cast<int>(S), static_cast<int>(Hq), static_cast<int>(Hkv),
-                              static_cast<int>(hd), interleaved ? 1 : 0, static_cast<float>(eps),
-                              num_sms(), cur_stream()),
-           "qk_rope_bwd");
+                              sin.data_ptr<float>(), opt_ptr(qw), opt_ptr(kw), opt_f32(partial), static_cast<int>(strips), f32(dqw), b16(dqw),
+                              f32(dkw), b16(dkw), T, static_cast<int>(S), static_cast<int>(Hq),
+                              static_cast<int>(Hkv), static_cast<int>(hd), interleaved ? 1 : 0,
+                              static_cast<float>(eps), num_sms(), cur_stream()),
+           "qk_rope_bwd", dqw.has_value() || dkw.has_value() ? 2 : 1);
 }
 
 void swiglu_fwd(const Tensor& h13, Tensor act) {

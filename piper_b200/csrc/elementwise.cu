@@ -349,15 +349,18 @@ rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
   }
 }
 
-// dw[c] (+)= sum_b partial[b][c]; fp32 output (the flat gradient bucket) or
-// bf16 when dw_bf16 is given.  A block owns 32 columns; its 32 thread rows each
-// sum a contiguous slice of the partials and the slices are added in a fixed
-// order, so the result does not depend on timing.
+// dw[c] (+)= sum_b partial[b][c]; fp32 output (the flat gradient bucket) or bf16 where that is given.  The columns from
+// `split` on go to a second weight.  A block owns 32 columns; its 32 thread rows each sum a contiguous slice of the partials
+// and the slices are added in a fixed order, so the result does not depend on timing.
+struct WeightGrad {
+  float* f32;
+  __nv_bfloat16* bf16;
+  int accumulate;
+};
+
 constexpr int RED_SLICES = 32;
 __global__ void __launch_bounds__(32 * RED_SLICES)
-reduce_partials_kernel(const float* __restrict__ partial, int nblocks, int D,
-                       float* __restrict__ dw_f32, __nv_bfloat16* __restrict__ dw_bf16,
-                       int accumulate) {
+reduce_partials_kernel(const float* __restrict__ partial, int nblocks, int D, WeightGrad first, WeightGrad second, int split) {
   __shared__ float part[RED_SLICES][32];
   const int c = blockIdx.x * 32 + threadIdx.x;
   const int per = (nblocks + RED_SLICES - 1) / RED_SLICES;
@@ -374,8 +377,10 @@ reduce_partials_kernel(const float* __restrict__ partial, int nblocks, int D,
   s = 0.f;
 #pragma unroll
   for (int i = 0; i < RED_SLICES; ++i) s += part[i][threadIdx.x];
-  if (dw_f32) dw_f32[c] = accumulate ? dw_f32[c] + s : s;
-  if (dw_bf16) dw_bf16[c] = __float2bfloat16(accumulate ? __bfloat162float(dw_bf16[c]) + s : s);
+  const WeightGrad o = c < split ? first : second;
+  const int i = c < split ? c : c - split;
+  if (o.f32) o.f32[i] = o.accumulate ? o.f32[i] + s : s;
+  if (o.bf16) o.bf16[i] = __float2bfloat16(o.accumulate ? __bfloat162float(o.bf16[i]) + s : s);
 }
 
 // --------------------------------------------------------- QK-norm + RoPE
@@ -460,7 +465,7 @@ struct RopeArgs {
   __nv_bfloat16* out;
   const float *cosp, *sinp;
   const __nv_bfloat16 *qw, *kw;  // norm weights of the query and key heads, or null
-  float *dqw, *dkw;              // their gradients (accumulated), or null
+  float* partial;                // sums of their gradients, [CTA][query, key][hd], or null
   long long T;
   int S, Hq, Hkv;
   float eps;
@@ -574,12 +579,13 @@ __device__ __forceinline__ void rope_tasks(const RopeArgs& a, const RopeGroup<HD
 
 // NORM: there are norm weights, of the query heads, the key heads or both.  Backward: un-rotate the gradient (RoPE is an
 // orthogonal map, so its transpose is the rotation by -theta), then the RMSNorm backward per head; the weight-gradient
-// sums of a warp are added over its lane groups, then over the CTA, and go to fp32 dw with one atomic per element and CTA.
-// (Sixteen shared-memory atomics per lane and head took 147 us for 4096 tokens of 32 + 2 x 4 heads x 128.)
+// sums of a warp are added over its lane groups, those of a CTA over its warps, and reduce_partials_kernel adds the CTAs', all in
+// a fixed order.  (Sixteen shared-memory atomics per lane and head took 147 us for 4096 tokens of 32 + 2 x 4 heads x 128.  One
+// atomic per element and CTA into cleared fp32 sums, which are then rounded, takes four launches more for two weights.)
 template <bool NORM, bool BWD>
 constexpr int ROPE_CTAS = !NORM ? 4 : BWD ? 2 : 3;     // per SM
 
-// The heads of one kind with the norm they have, and their weight gradient into sdw.
+// The heads of one kind with the norm they have, and the warp's sums of its weight gradient into sdw.
 template <int HD, bool NORM, bool BWD, bool INTER>
 __device__ __forceinline__ void rope_kind(const RopeArgs& a, const RopeGroup<HD>& g, int first_head, int n,
                                           const __nv_bfloat16* w, bool want_dw, float* sdw, unsigned& task, unsigned warps) {
@@ -597,32 +603,31 @@ __device__ __forceinline__ void rope_kind(const RopeArgs& a, const RopeGroup<HD>
   for (int j = 0; j < 16; ++j) {
 #pragma unroll
     for (int o = g.LANES; o < 32; o <<= 1) dw[j] += __shfl_xor_sync(0xffffffffu, dw[j], o);
-    if (g.group == 0) atomicAdd(sdw + (j < 8 ? g.off0 : g.off1) + (j & 7), dw[j]);
+    if (g.group == 0) sdw[(j < 8 ? g.off0 : g.off1) + (j & 7)] = dw[j];
   }
 }
 
 template <int HD, bool NORM, bool BWD, bool INTER>
 __global__ void __launch_bounds__(256, ROPE_CTAS<NORM, BWD>)
 qk_rope_kernel(const __grid_constant__ RopeArgs a) {
-  __shared__ float sdw[2][HD];
-  const bool want_dw = NORM && BWD && (a.dqw != nullptr || a.dkw != nullptr);
-  if (want_dw) {
-    for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) (&sdw[0][0])[i] = 0.f;
-    __syncthreads();
-  }
+  __shared__ float sdw[NORM && BWD ? 8 : 1][2 * HD];
+  const bool want_dw = NORM && BWD && a.partial != nullptr;
   const RopeGroup<HD> g;
+  const int w = NORM && BWD ? threadIdx.x >> 5 : 0;
   unsigned task = blockIdx.x * 8 + (threadIdx.x >> 5);
   const unsigned warps = gridDim.x * 8;
-  rope_kind<HD, NORM, BWD, INTER>(a, g, 0, a.Hq, a.qw, want_dw, sdw[0], task, warps);
-  rope_kind<HD, NORM, BWD, INTER>(a, g, a.Hq, a.Hkv, a.kw, want_dw, sdw[1], task, warps);
+  rope_kind<HD, NORM, BWD, INTER>(a, g, 0, a.Hq, a.qw, want_dw, sdw[w], task, warps);
+  rope_kind<HD, NORM, BWD, INTER>(a, g, a.Hq, a.Hkv, a.kw, want_dw, sdw[w] + HD, task, warps);
   float none[16];
   rope_tasks<HD, kRopeCopy, BWD, INTER>(a, g, a.Hq + a.Hkv, a.Hkv, nullptr, task, warps, none);
   if (want_dw) {
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) {
-      float* dwp = i < HD ? a.dqw : a.dkw;
-      const float v = (&sdw[0][0])[i];
-      if (dwp != nullptr && v != 0.f) atomicAdd(dwp + (i < HD ? i : i - HD), v);
+      if ((i < HD ? a.qw : a.kw) == nullptr) continue;
+      float v = 0.f;
+#pragma unroll
+      for (int k = 0; k < (NORM && BWD ? 8 : 1); ++k) v += sdw[k][i];
+      a.partial[static_cast<long long>(blockIdx.x) * 2 * HD + i] = v;
     }
   }
 }
@@ -973,6 +978,7 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
   if (T == 0) return 0;
   const int nb = rmsnorm_bwd_num_partials(T);
   const dim3 red_grid((D + 31) / 32), red_block(32, RED_SLICES);
+  const WeightGrad out{dw_f32, static_cast<__nv_bfloat16*>(dw_bf16), accumulate};
   if (D == 2048 || D == 4096 || D == 8192) {
     const auto* dyp = static_cast<const __nv_bfloat16*>(dy);
     const auto* xp = static_cast<const __nv_bfloat16*>(x);
@@ -983,8 +989,7 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
     if (D == 2048) rmsnorm_bwd_reg_kernel<1><<<nb, NORM_THREADS, 0, st>>>(dyp, xp, wp, rstd, ep, dxp, dw_partial, Ti);
     else if (D == 4096) rmsnorm_bwd_reg_kernel<2><<<nb, NORM_THREADS, 0, st>>>(dyp, xp, wp, rstd, ep, dxp, dw_partial, Ti);
     else rmsnorm_bwd_reg_kernel<4><<<nb, NORM_THREADS, 0, st>>>(dyp, xp, wp, rstd, ep, dxp, dw_partial, Ti);
-    reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, dw_f32,
-                                                           static_cast<__nv_bfloat16*>(dw_bf16), accumulate);
+    reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, out, out, D);
     return PIPER_LAUNCH_OK();
   }
   static bool configured = false;
@@ -996,59 +1001,78 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
       static_cast<const __nv_bfloat16*>(w), rstd, static_cast<const __nv_bfloat16*>(dres),
       static_cast<__nv_bfloat16*>(dx), dw_partial, static_cast<int>(T), D);
-  reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, dw_f32,
-                                                         static_cast<__nv_bfloat16*>(dw_bf16), accumulate);
+  reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, out, out, D);
   return PIPER_LAUNCH_OK();
 }
 
+// `grid` is the most CTAs that may run, or 0, and becomes those that do.
 // Heads of a task: more of them share one load of cos/sin and fetch ahead, fewer make more tasks to run at a time.
 // Four per lane group at 128 (two at 64, whose runs would span half a token) where that leaves two tasks per resident warp.
 // In us for 1, 2, 4 and 8 heads per lane group: 4096 x (32 + 2 x 4) x 128 with norms forward 21.6 19.6 19.7 21.8, backward 36.5 32.9
 // 32.7 32.8; 16384 tokens 75.7 66.5 64.2 63.7, 123.3 108.8 103.8 101.1; 8192 x (32 + 2 x 8) x 128 38.0 35.8 35.4 36.1; 8192 x (32 +
 // 2 x 8) x 64 30.2 29.2 30.2 30.2; 128 x (32 + 2 x 8) x 128 2.6 2.7 3.4 4.6.
 template <int HD, bool NORM, bool BWD>
-static int qk_rope_launch(RopeArgs a, bool interleaved, int num_sms, cudaStream_t st) {
-  const int resident = ROPE_CTAS<NORM, BWD> * num_sms;
+static int qk_rope_launch(RopeArgs a, bool interleaved, int num_sms, int& grid, cudaStream_t st) {
+  int resident = ROPE_CTAS<NORM, BWD> * num_sms;
+  if (grid > 0 && grid < resident) resident = grid;
   auto tasks = [&](int run) { return a.T * ((a.Hq + run - 1) / run + 2ll * ((a.Hkv + run - 1) / run)); };
   constexpr int groups = RopeGroup<HD>::GROUPS;
   a.run = (HD == 128 ? 4 : 2) * groups;
   while (a.run > groups && tasks(a.run) < 2ll * 8 * resident) a.run /= 2;
   if (tasks(a.run) >= (1ll << 31)) return -1;
   const long long blocks = (tasks(a.run) + 7) / 8;
+  grid = static_cast<int>(blocks < resident ? blocks : resident);
   auto kern = interleaved ? qk_rope_kernel<HD, NORM, BWD, true> : qk_rope_kernel<HD, NORM, BWD, false>;
-  kern<<<static_cast<unsigned>(blocks < resident ? blocks : resident), 256, 0, st>>>(a);
+  kern<<<grid, 256, 0, st>>>(a);
   return PIPER_LAUNCH_OK();
 }
 
 template <bool BWD>
-static int qk_rope(const RopeArgs& a, int hd, bool interleaved, int num_sms, cudaStream_t st) {
-  if (a.T == 0 || a.Hq + 2 * a.Hkv == 0) return 0;
+static int qk_rope(const RopeArgs& a, int hd, bool interleaved, int num_sms, int& grid, cudaStream_t st) {
+  if (a.T == 0 || a.Hq + 2 * a.Hkv == 0) {
+    grid = 0;
+    return 0;
+  }
   if (hd != 128 && hd != 64) return -1;
   if (static_cast<long long>(a.S) * (hd / 2) >= (1ll << 31)) return -1;
   if (!aligned16(a.x, a.pre, a.out, a.cosp, a.sinp, a.qw, a.kw)) return -4;
   if (a.qw != nullptr || a.kw != nullptr)
-    return hd == 128 ? qk_rope_launch<128, true, BWD>(a, interleaved, num_sms, st)
-                     : qk_rope_launch<64, true, BWD>(a, interleaved, num_sms, st);
-  return hd == 128 ? qk_rope_launch<128, false, BWD>(a, interleaved, num_sms, st)
-                   : qk_rope_launch<64, false, BWD>(a, interleaved, num_sms, st);
+    return hd == 128 ? qk_rope_launch<128, true, BWD>(a, interleaved, num_sms, grid, st)
+                     : qk_rope_launch<64, true, BWD>(a, interleaved, num_sms, grid, st);
+  return hd == 128 ? qk_rope_launch<128, false, BWD>(a, interleaved, num_sms, grid, st)
+                   : qk_rope_launch<64, false, BWD>(a, interleaved, num_sms, grid, st);
 }
 
 int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp, const void* qw,
                 const void* kw, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps,
                 int num_sms, cudaStream_t st) {
   const RopeArgs a{static_cast<const __nv_bfloat16*>(in), nullptr, static_cast<__nv_bfloat16*>(out), cosp, sinp,
-                   static_cast<const __nv_bfloat16*>(qw), static_cast<const __nv_bfloat16*>(kw), nullptr, nullptr,
+                   static_cast<const __nv_bfloat16*>(qw), static_cast<const __nv_bfloat16*>(kw), nullptr,
                    T, S, Hq, Hkv, eps, 0};
-  return qk_rope<false>(a, hd, interleaved != 0, num_sms, st);
+  int grid = 0;
+  return qk_rope<false>(a, hd, interleaved != 0, num_sms, grid, st);
 }
 
 int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, const float* sinp,
-                const void* qw, const void* kw, float* dqw, float* dkw, long long T, int S, int Hq,
-                int Hkv, int hd, int interleaved, float eps, int num_sms, cudaStream_t st) {
+                const void* qw, const void* kw, float* partial, int strips, float* dqw_f32, void* dqw_bf16, float* dkw_f32,
+                void* dkw_bf16, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps, int num_sms,
+                cudaStream_t st) {
+  // buckets add up, bf16 gradients are written (zeros where there are no tokens)
+  const WeightGrad q{dqw_f32, static_cast<__nv_bfloat16*>(dqw_bf16), dqw_f32 != nullptr};
+  const WeightGrad k{dkw_f32, static_cast<__nv_bfloat16*>(dkw_bf16), dkw_f32 != nullptr};
+  const bool want_q = q.f32 || q.bf16, want_k = k.f32 || k.bf16;
   const RopeArgs a{static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(in),
                    static_cast<__nv_bfloat16*>(din), cosp, sinp, static_cast<const __nv_bfloat16*>(qw),
-                   static_cast<const __nv_bfloat16*>(kw), dqw, dkw, T, S, Hq, Hkv, eps, 0};
-  return qk_rope<true>(a, hd, interleaved != 0, num_sms, st);
+                   static_cast<const __nv_bfloat16*>(kw), want_q || want_k ? partial : nullptr, T, S, Hq, Hkv, eps, 0};
+  if ((want_q && !qw) || (want_k && !kw) || ((want_q || want_k) && (!partial || strips < 1))) return -1;
+  int grid = want_q || want_k ? strips : 0;
+  const int rc = qk_rope<true>(a, hd, interleaved != 0, num_sms, grid, st);
+  if (rc != 0 || !(want_q || want_k)) return rc;
+  const WeightGrad none{nullptr, nullptr, 0};
+  const bool same = want_q && want_k && (q.f32 ? q.f32 == k.f32 : q.bf16 == k.bf16);   // one weight for both: in turn
+  reduce_partials_kernel<<<2 * hd / 32, dim3(32, RED_SLICES), 0, st>>>(partial, grid, 2 * hd, q, same ? none : k, hd);
+  if (same) reduce_partials_kernel<<<2 * hd / 32, dim3(32, RED_SLICES), 0, st>>>(partial, grid, 2 * hd, none, k, hd);
+  return PIPER_LAUNCH_OK();
 }
 
 int swiglu_fwd(const void* h13, void* act, long long T, int F, cudaStream_t st) {

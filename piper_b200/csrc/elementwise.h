@@ -27,9 +27,12 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
 int qk_rope_fwd(const void* in, void* out, const float* cosp, const float* sinp, const void* qw,
                 const void* kw, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps,
                 int num_sms, cudaStream_t st);
+// Gradients of the norm weights (each fp32, added to, or bf16, written; or null) go through `partial`, scratch of
+// `strips` x 2 hd floats; at most so many CTAs run then.
 int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, const float* sinp,
-                const void* qw, const void* kw, float* dqw, float* dkw, long long T, int S, int Hq,
-                int Hkv, int hd, int interleaved, float eps, int num_sms, cudaStream_t st);
+                const void* qw, const void* kw, float* partial, int strips, float* dqw_f32, void* dqw_bf16, float* dkw_f32,
+                void* dkw_bf16, long long T, int S, int Hq, int Hkv, int hd, int interleaved, float eps, int num_sms,
+                cudaStream_t st);
 
 int swiglu_fwd(const void* h13, void* act, long long T, int F, cudaStream_t st);
 int swiglu_bwd(const void* h13, const void* dact, void* dh13, long long T, int F, cudaStream_t st);

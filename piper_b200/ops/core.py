@@ -579,9 +579,18 @@ def _qk_rope_backward(ctx, dout):
         din = torch.empty_like(dc)
         sq = grad_sinks.get(qw) if qw is not None else None
         sk = grad_sinks.get(kw) if kw is not None else None
-        bq = sq.view(-1) if sq is not None else (torch.zeros(hd, dtype=torch.float32, device=dout.device) if qw is not None else None)
-        bk = sk.view(-1) if sk is not None else (torch.zeros(hd, dtype=torch.float32, device=dout.device) if kw is not None else None)
-        native.lib().qk_rope_bwd(dc, qkv if qkv is not None else dc, din, cos, sin, qw, kw, bq, bk, S, Hq, Hkv,
+        def target(w, sink):
+            # a bf16 weight's gradient is written by the kernels, another one is summed in fp32 and converted
+            if w is None or sink is not None:
+                return None if w is None else sink.view(-1)
+            return torch.empty(hd, dtype=w.dtype, device=w.device) if w.dtype == torch.bfloat16 else torch.zeros(hd, dtype=torch.float32, device=w.device)
+
+        bq, bk = target(qw, sq), target(kw, sk)
+        partial = None
+        if qkv is not None:
+            strips = native.lib().rmsnorm_bwd_num_partials(dc.numel() // max(1, dc.shape[-1]))
+            partial = torch.empty((strips, 2 * hd), dtype=torch.float32, device=dout.device)
+        native.lib().qk_rope_bwd(dc, qkv if qkv is not None else dc, din, cos, sin, qw, kw, partial, bq, bk, S, Hq, Hkv,
                                  hd, interleaved, eps)
         if qw is not None and sq is None:
             dqw = bq.to(qw.dtype)
