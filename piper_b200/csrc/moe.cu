@@ -127,10 +127,12 @@ __global__ void route_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const
   }
 }
 
-// One warp: a scan over each source's segments (one thread walking 128 groups took 5 us of dependent loads).
+// One warp: a scan over each source's segments (one thread walking 128 groups took 5 us of dependent loads).  It also clears
+// the permutation's cursors and copies the counts where a dispatch wants them: launches of their own took longer than this.
 __global__ void group_table_kernel(const int* __restrict__ counts, int num_groups, int experts,
                                    const int* __restrict__ row_base, int* __restrict__ g_start,
-                                   int* __restrict__ g_len, int* __restrict__ total) {
+                                   int* __restrict__ g_len, int* __restrict__ total, int* __restrict__ cursor,
+                                   int* __restrict__ copy) {
   const int lane = threadIdx.x;
   int run = 0, last = 0;
   for (int s0 = 0; s0 < num_groups; s0 += experts) {
@@ -140,7 +142,8 @@ __global__ void group_table_kernel(const int* __restrict__ counts, int num_group
     for (int e0 = 0; e0 < n; e0 += 32) {
       const int g = s0 + e0 + lane;
       const bool in = e0 + lane < n;
-      const int len = in ? (counts[g] + 127) / 128 * 128 : 0;
+      const int n_g = in ? counts[g] : 0;
+      const int len = (n_g + 127) / 128 * 128;
       int inc = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -150,12 +153,14 @@ __global__ void group_table_kernel(const int* __restrict__ counts, int num_group
       if (in) {
         g_start[g] = run + inc - len;
         g_len[g] = len;
+        if (cursor != nullptr) cursor[g] = 0;
+        if (copy != nullptr) copy[g] = n_g;
       }
       run += __shfl_sync(0xffffffffu, inc, 31);
       if (run > last) last = run;
     }
   }
-  if (lane == 0) total[0] = last;
+  if (lane == 0 && total != nullptr) total[0] = last;
 }
 
 constexpr int ROW_THREADS = 128;      // four tokens per CTA: enough CTAs for the small token counts
@@ -384,9 +389,9 @@ int moe_route_bwd(const void* logits, const int* idx, const float* weights, cons
 }
 
 int moe_group_table(const int* counts, int num_groups, int experts, const int* row_base, int* g_start, int* g_len,
-                    int* total, cudaStream_t st) {
+                    int* total, int* cursor, int* copy, cudaStream_t st) {
   if (num_groups <= 0 || experts <= 0) return -1;
-  group_table_kernel<<<1, 32, 0, st>>>(counts, num_groups, experts, row_base, g_start, g_len, total);
+  group_table_kernel<<<1, 32, 0, st>>>(counts, num_groups, experts, row_base, g_start, g_len, total, cursor, copy);
   return PIPER_LAUNCH_OK();
 }
 

@@ -22,8 +22,9 @@ int moe_route_bwd(const void* logits_bf16, const int* idx, const float* weights,
 // g_len[g] = counts[g] rounded up to 128, g_start = exclusive prefix sum of
 // g_len starting at row_base[source] when row_base != nullptr (region layout)
 // or running over all groups otherwise.  total[0] = one past the last row.
+// total may be null; cursor (zeroed) and copy (of counts) are for a dispatch, null otherwise.
 int moe_group_table(const int* counts, int num_groups, int experts, const int* row_base, int* g_start,
-                    int* g_len, int* total, cudaStream_t st);
+                    int* g_len, int* total, int* cursor, int* copy, cudaStream_t st);
 
 // Every kernel below that indexes a row buffer through pos or a group table checks the index against rows_cap
 // (rows of that buffer): a bad index is skipped and recorded in the status word.

@@ -149,13 +149,13 @@ def moe_dispatch(x: Tensor, idx: Tensor, counts: Tensor) -> tuple[Tensor, Tensor
             return _EP_RUNTIME.dispatch(x, idx, counts)
         g_start = torch.empty_like(counts)
         g_len = torch.empty_like(counts)
-        total = torch.empty(1, dtype=torch.int32, device=x.device)
-        native.lib().moe_group_table(counts, E, None, g_start, g_len, total)
+        cursor = torch.empty_like(counts)
+        copy = torch.empty_like(counts)
+        native.lib().moe_dispatch_table(counts, g_start, g_len, cursor, copy)
         rows = torch.empty((cap, D), dtype=x.dtype, device=x.device)
         pos = torch.empty(T * k, dtype=torch.int32, device=x.device)
-        cursor = torch.zeros(E, dtype=torch.int32, device=x.device)
         native.lib().moe_permute(x.contiguous(), idx, g_start, g_len, counts, cursor, pos, rows)
-        return rows, pos, g_start, g_len, counts.clone()
+        return rows, pos, g_start, g_len, copy
     g_len = (counts + (PAD - 1)) // PAD * PAD
     g_start = (torch.cumsum(g_len, 0) - g_len).to(torch.int32)
     flat_e = idx.reshape(-1).long()
