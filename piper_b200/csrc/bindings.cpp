@@ -267,6 +267,15 @@ void ce_fwd(const Tensor& logits, const Tensor& labels, Tensor loss, Tensor lse,
            "ce_fwd");
 }
 
+void ce_mean(const Tensor& loss, const Tensor& labels, Tensor mean, Tensor count, int64_t ignore_index) {
+  TORCH_CHECK(loss.is_cuda() && loss.scalar_type() == at::kFloat && loss.is_contiguous(), "loss must be contiguous fp32");
+  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == loss.numel(),
+              "labels must be contiguous int64, one per loss");
+  check_rc(piper::ce_mean(loss.data_ptr<float>(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()),
+                          mean.data_ptr<float>(), count.data_ptr<float>(), loss.numel(), ignore_index, cur_stream()),
+           "ce_mean");
+}
+
 void ce_bwd(const Tensor& logits, const Tensor& labels, const Tensor& lse, const Tensor& gscale, double row_scale,
             Tensor out, int64_t ignore_index) {
   check_bf16(logits, "logits");
@@ -383,6 +392,7 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("embedding_bwd", &embedding_bwd);
   m.def("embedding_bwd_bf16", &embedding_bwd_bf16);
   m.def("ce_fwd", &ce_fwd);
+  m.def("ce_mean", &ce_mean);
   m.def("ce_bwd", &ce_bwd);
   m.def("adam_flat", &adam_flat);
   m.def("cast_f32_to_bf16", &cast_f32_to_bf16);

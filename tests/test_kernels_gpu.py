@@ -521,6 +521,41 @@ def test_swiglu_large_gates():
     assert a[0, 4095].isnan() and h.grad[0, 4095].isnan() and h.grad[0, 8191].isnan()
 
 
+@pytest.mark.parametrize("T,ignored", [(0, 0.0), (1, 0.0), (33, 0.3), (1023, 1.0), (1024, 0.0), (5000, 0.3), (65536, 0.1), (65537, 0.1)])
+def test_cross_entropy_mean(T, ignored):
+    """One CTA's sum over any number of rows, and the sum by tensor ops above its limit: value, gradient, and the gradient of
+    the gradient by the upstream one, from the C++ formula and the Python one."""
+    from piper_b200.ops import core, native
+
+    torch.manual_seed(31)
+    logits = torch.randn(T, 16, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    labels = torch.randint(0, 16, (T,), device="cuda")
+    labels[torch.rand(T, device="cuda") < ignored] = -100
+    if ignored == 1.0:
+        labels.fill_(-100)
+    n = max(1, int((labels != -100).sum()))
+    up = torch.tensor(0.7, device="cuda", requires_grad=True)
+    results = []
+    for installed in (True, False):
+        if not installed:
+            native.lib().native_op_remove("cross_entropy_mean")
+        try:
+            rows, _ = core.cross_entropy_fwd(logits, labels, -100)
+            mean = core.cross_entropy(logits, labels)
+            per_row = rows.detach().requires_grad_(True)
+            by_op, count = core.cross_entropy_mean(per_row, labels, -100)
+            assert not count.requires_grad and int(count) == n
+            (g,) = torch.autograd.grad(by_op, per_row, up, create_graph=True)
+            results.append([mean.detach(), g.detach(), *torch.autograd.grad(g.sum(), up)])
+        finally:
+            native.lib().native_op_install("cross_entropy_mean")
+        want = rows.detach().double().sum() / n
+        # one rounding of a sum in 64 bits; above the limit fp32 partial sums of positive terms
+        assert abs(mean.double() - want) <= (2 ** -23 if T <= core.CE_MEAN_ROWS else 1e-6) * abs(want)
+        assert torch.equal(g.detach(), torch.full((T,), 0.7, device="cuda") / n)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 def test_swiglu_embedding_ce_adam():
     from piper_b200 import ops
     from piper_b200.ops import native
