@@ -64,8 +64,10 @@ float* opt_f32(const OptTensor& t) {
 // C[M,N] = A * B^T.  a: [M,K] (a_mn=false) or [K,M] (a_mn=true); b: [N,K]
 // (b_mn=false) or [K,N] (b_mn=true).  c bf16 -> store; c fp32 -> store or
 // accumulate.
-void gemm_shaped(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
-                 int64_t tile, int64_t width) {
+// shape: ctas 0 leaves the choice to the launcher, -1 to gemm_split_shape.  A split contraction is the one case that takes
+// memory: scratch, from the caching allocator.
+void gemm_run(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
+              piper::GemmShape shape) {
   check_bf16(a, "a");
   check_bf16(b, "b");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm expects 2-D tensors");
@@ -104,10 +106,37 @@ void gemm_shaped(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_m
   }
   g.accumulate = accumulate ? 1 : 0;
   g.status = status.data_ptr<int>();
+  if (shape.ctas < 0) {
+    shape = {0, 0, 1};
+    if (piper::gemm_forced_tile() == 0 && M > 0 && N > 0 && K > 0)
+      shape = piper::gemm_split_shape(g.M, g.N, g.K, b_mn, g.epilogue != piper::kEpiStoreBf16, num_sms());
+  }
+  Tensor scratch;
+  if (shape.splits > 1) {
+    try {
+      scratch = at::empty({piper::gemm_split_floats(g.M, g.N, shape.splits)}, c.options().dtype(at::kFloat));
+      g.scratch = scratch.data_ptr<float>();
+    } catch (const c10::OutOfMemoryError&) {
+      shape = {0, 0, 1};                         // in one part then
+    }
+  }
+  g.shape = shape;
+  check_rc(piper::gemm_bf16_launch(g, num_sms(), cur_stream()), "gemm", shape.splits > 1 ? 2 : 1);
+}
+
+void gemm_shaped(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
+                 int64_t tile, int64_t width) {
   TORCH_CHECK(tile == 0 || tile == 128 || tile == 256, "gemm tile must be 0 (auto), 128 or 256");
-  g.tile = static_cast<int>(tile);
-  g.width = static_cast<int>(width);
-  check_rc(piper::gemm_bf16_launch(g, num_sms(), cur_stream()), "gemm");
+  gemm_run(a, b, c, a_mn, b_mn, accumulate, status,
+           {static_cast<int>(tile) / 128, width != 0 ? static_cast<int>(width) : 256, 1});
+}
+
+// In `splits` parts, each with k-blocks of 64, by tiles of 128 x width or pairs of 256 x width.
+void gemm_split(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, Tensor status, int64_t tile, int64_t width,
+                int64_t splits) {
+  TORCH_CHECK(c.scalar_type() == at::kBFloat16 && splits >= 1 && (tile == 128 || tile == 256), "a split product is bf16");
+  gemm_run(a, b, c, a_mn, b_mn, false, status,
+           {static_cast<int>(tile) / 128, static_cast<int>(width), static_cast<int>(splits)});
 }
 
 void gemm_tiled(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status,
@@ -116,7 +145,14 @@ void gemm_tiled(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn
 }
 
 void gemm(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, bool accumulate, Tensor status) {
-  gemm_shaped(a, b, c, a_mn, b_mn, accumulate, status, 0, 0);
+  gemm_run(a, b, c, a_mn, b_mn, accumulate, status, {-1, 0, 1});
+}
+
+// (CTAs per tile, columns, parts of the contraction) of a product by gemm().
+std::tuple<int64_t, int64_t, int64_t> gemm_split_shape(int64_t M, int64_t N, int64_t K, bool b_mn, bool f32_out, int64_t sms) {
+  const piper::GemmShape s = piper::gemm_split_shape(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), b_mn,
+                                                     f32_out, static_cast<int>(sms));
+  return {s.ctas, s.width, s.splits};
 }
 
 int64_t gemm_tile_rows(int64_t M, int64_t N, int64_t K, bool f32_out, int64_t sms) {
@@ -379,6 +415,8 @@ TORCH_LIBRARY(piper_c, m) {
   m.def("gemm", &gemm);
   m.def("gemm_tiled", &gemm_tiled);
   m.def("gemm_shaped", &gemm_shaped);
+  m.def("gemm_split", &gemm_split);
+  m.def("gemm_split_shape", &gemm_split_shape);
   m.def("gemm_tile_rows", &gemm_tile_rows);
   m.def("gemm_shape", &gemm_shape);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);

@@ -23,7 +23,8 @@
 // gradient (dY W) and weight gradient (dY^T X) of a linear layer without any
 // transposed copy.  The epilogue either stores bf16 or adds into an fp32
 // buffer (gradient accumulation into the flat fp32 bucket).  Every output element is the sum of the same products in
-// the same order whatever the tile shape, so results do not depend on it.
+// the same order whatever the tile shape, so results do not depend on it, except where a gradient's contraction is split
+// (gemm_split_shape).
 //
 // All mbarrier waits are bounded; on expiry the kernel records a status code,
 // drains its TMA copies, frees TMEM and returns.
@@ -72,6 +73,9 @@ struct Params {
   int accumulate;
   int c_bufs;         // staging buffers per epilogue warp; the second ones take the room of operand stages
   int band;           // tiles of the faster dimension that are walked together
+  int splits;         // parts of the contraction, each a tile of its own
+  int k_per;          // k-blocks of a part
+  int split_rows;     // rows between the parts' outputs
   int* status;
   int* sched;
 };
@@ -93,7 +97,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const int stages = p.stages;
   const int tiles_m = (p.M + BM * CTAS - 1) / (BM * CTAS);
   const int tiles_n = (p.N + width - 1) / width;
-  const int num_tiles = tiles_m * tiles_n;
+  const int out_tiles = tiles_m * tiles_n;
+  const int num_tiles = out_tiles * p.splits;
   const int k_blocks = (p.K + BK - 1) / BK;
   const bool n_fast = tiles_n < tiles_m;
 
@@ -133,7 +138,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   // Tiles that run at the same time share operands: the dimension with fewer tiles is walked fastest, so that a wave
   // covers all of it and the operand of the other dimension streams through L2 once; in bands, where the operand of the
   // faster dimension would not stay in L2 from one wave to the next.
-  auto coords = [&](int tile, int& tm, int& tn) {
+  // The parts of a split contraction follow one another.
+  auto coords = [&](int tile, int& tm, int& tn, int& part) {
+    part = p.splits > 1 ? tile / out_tiles : 0;
+    tile -= part * out_tiles;
     const int fast = n_fast ? tiles_n : tiles_m, slow = n_fast ? tiles_m : tiles_n;
     const int b = tile / (p.band * slow), f0 = b * p.band;
     const int bw = min(p.band, fast - f0), r = tile - f0 * slow;
@@ -169,11 +177,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       __syncwarp();
       int tile;
       if (!(ok = tile_at(n, tile)) || tile < 0) break;
-      int tm, tn;
-      coords(tile, tm, tn);
+      int tm, tn, part;
+      coords(tile, tm, tn, part);
+      const int kb1 = min(k_blocks, (part + 1) * p.k_per);
       const int m0 = tm * (BM * CTAS) + static_cast<int>(rank) * BM;
       const int n0 = tn * width + static_cast<int>(rank) * b_rows;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = part * p.k_per; kb < kb1; ++kb) {
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->empty[s], ph ^ 1, p.status)))) break;
         if (elect_one()) {
           uint8_t* sa = smem + s * stage_bytes;
@@ -229,7 +238,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[acc], ((n >> 1) & 1) ^ 1, p.status)))) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * 256;
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        const int part = p.splits > 1 ? tile / out_tiles : 0;
+        const int kb0 = part * p.k_per, kb1 = min(k_blocks, kb0 + p.k_per);
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], ph, p.status)))) break;
           tc_fence_after();
           if (elect_one()) {
@@ -237,9 +248,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             const uint64_t db = db0 + (static_cast<uint32_t>(s * stage_bytes) >> 4);
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; ++k)
-              umma_bf16_ss_n<CTAS>(tmem_d, da + k * a_step, db + k * b_step, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              umma_bf16_ss_n<CTAS>(tmem_d, da + k * a_step, db + k * b_step, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
             umma_commit_n<CTAS>(&bars->empty[s]);
-            if (kb == k_blocks - 1) umma_commit_n<CTAS>(&bars->acc_full[acc]);
+            if (kb == kb1 - 1) umma_commit_n<CTAS>(&bars->acc_full[acc]);
           }
           __syncwarp();
           if (++s == stages) { s = 0; ph ^= 1; }
@@ -257,8 +268,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (!tile_at(n, tile) || tile < 0) break;
       const uint32_t acc = n & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(&bars->acc_full[acc], (n >> 1) & 1, p.status))) break;
-      int tm, tn;
-      coords(tile, tm, tn);
+      int tm, tn, part;
+      coords(tile, tm, tn, part);
       const int row0 = tm * (BM * CTAS) + static_cast<int>(rank) * BM + q * 32;
       const int n0 = tn * width;
       tc_fence_after();
@@ -311,7 +322,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             const int col0 = n0 + (c + 2 * j) * 32;
             if (j > 0 && (c + 2 * j >= width / 32 || col0 >= p.N)) continue;
             if (EPI == kEpiAccumF32 && p.accumulate) tma_reduce_add_2d_bulk(&tmap_c, stage + j * BLOCK, col0, row0);
-            else tma_store_2d_bulk(&tmap_c, stage + j * BLOCK, col0, row0);
+            else tma_store_2d_bulk(&tmap_c, stage + j * BLOCK, col0, row0 + part * p.split_rows);
           }
           bulk_commit_group();
         }
@@ -339,6 +350,36 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       p.sched[1] = 0;
       __threadfence();
     }
+  }
+}
+
+// C[m, n] = sum of the parts of a split contraction, in their order, rounded to bf16 once.  parts [splits][rows][ld]; a thread
+// has eight neighbouring columns, which the scratch holds for every row (ld is a multiple of eight).
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ c, int M, int N, int rows, int ld, long long ldc,
+                 int splits) {
+  const int vecs = ld / 8;
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= static_cast<long long>(M) * vecs) return;
+  const int m = static_cast<int>(i / vecs), n = static_cast<int>(i - static_cast<long long>(m) * vecs) * 8;
+  const float4* src = reinterpret_cast<const float4*>(parts + static_cast<long long>(m) * ld + n);
+  const long long step = static_cast<long long>(rows) * ld / 4;
+  float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float4 a = __ldcs(src + s * step), b = __ldcs(src + s * step + 1);
+    lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
+    hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+  }
+  const uint4 o = make_uint4(pack_bf16x2(lo.x, lo.y), pack_bf16x2(lo.z, lo.w), pack_bf16x2(hi.x, hi.y), pack_bf16x2(hi.z, hi.w));
+  __nv_bfloat16* dst = c + m * ldc + n;
+  if (n + 8 <= N) {
+    *reinterpret_cast<uint4*>(dst) = o;
+  } else {
+    const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (n + j < N) dst[j] = reinterpret_cast<const __nv_bfloat16*>(w)[j];
   }
 }
 
@@ -441,7 +482,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -2;
     configured = true;
   }
-  const int tiles = ((p.M + BM * CTAS - 1) / (BM * CTAS)) * ((p.N + p.width - 1) / p.width);
+  const int tiles = ((p.M + BM * CTAS - 1) / (BM * CTAS)) * ((p.N + p.width - 1) / p.width) * p.splits;
   const int units = num_sms / CTAS;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(CTAS * (tiles < units ? tiles : units)));
@@ -475,7 +516,7 @@ static int launch_layout(const GemmArgs& g, const CUtensorMap& ta, const CUtenso
 }
 
 // 0: choose by shape, 128 / 256: forced by PIPER_GEMM_TILE
-static int forced_tile() {
+int gemm_forced_tile() {
   static int v = -1;
   if (v < 0) {
     const char* env = getenv("PIPER_GEMM_TILE");
@@ -513,9 +554,10 @@ int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms) {
 // contraction), where 256 columns throughout are 17 % behind in pairs and 25 % by single CTAs.  Narrower tiles even out the last round: 4096 x 5120 x
 // 2048 in 23 x 16 tiles of 224 columns 56.3 us, in 20 x 16 of 256 columns 58.8 us; 1000 x 3072 x 8192 in 64 tiles of 192 columns
 // 37.6 us, in 48 of 256 columns 44.6 us; and a small problem covers more SMs: 512 x 768 x 256 5.2 and 7.2 us.
-static double gemm_cost(int M, int N, int K, bool b_mn, bool f32_out, int ctas, int width, int num_sms) {
-  const double k_blocks = (K + BK - 1) / BK;
-  const long long tiles = static_cast<long long>((M + BM * ctas - 1) / (BM * ctas)) * ((N + width - 1) / width);
+static double gemm_cost(int M, int N, int K, bool b_mn, bool f32_out, int ctas, int width, int num_sms, int splits = 1) {
+  const double k_blocks = ((K + BK - 1) / BK + splits - 1) / splits;
+  const long long tiles =
+      static_cast<long long>((M + BM * ctas - 1) / (BM * ctas)) * ((N + width - 1) / width) * splits;
   const long long units = num_sms / ctas;
   const double rounds = static_cast<double>((tiles + units - 1) / units);
   const int b_rows = b_mn ? (width / ctas + 63) / 64 * 64 : width / ctas;
@@ -525,7 +567,7 @@ static double gemm_cost(int M, int N, int K, bool b_mn, bool f32_out, int ctas, 
 }
 
 GemmShape gemm_shape(int M, int N, int K, bool b_mn, bool f32_out, int num_sms) {
-  GemmShape best[2] = {{1, 256}, {2, 256}};
+  GemmShape best[2] = {{1, 256, 1}, {2, 256, 1}};
   double cost[2];
   for (int i = 0; i < 2; ++i) {
     for (int width = 256; width >= 32; width -= 32) {
@@ -542,13 +584,55 @@ GemmShape gemm_shape(int M, int N, int K, bool b_mn, bool f32_out, int num_sms) 
   return best[pair ? 1 : 0];
 }
 
-int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
-  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 0;
-  const int tile = g.tile != 0 ? g.tile : forced_tile();
-  GemmShape shape = {tile / 128, g.width != 0 ? g.width : 256};
-  if (tile == 0) shape = gemm_shape(g.M, g.N, g.K, g.b_mn_major != 0, g.epilogue != kEpiStoreBf16, num_sms);
+constexpr long long kMaxSplitFloats = 16ll << 20;       // 64 MiB of scratch
+
+long long gemm_split_floats(int M, int N, int splits) {
+  return splits > 1 ? static_cast<long long>(splits) * ((M + 31) / 32 * 32) * ((N + 7) / 8 * 8) : 0;
+}
+
+// Parts of the contraction (and the shape of their tiles) where few output tiles leave most SMs without one: an input
+// gradient of few tokens, whose contraction is the layer's output width.  Every part is a tile that leaves fp32 sums in
+// scratch, and split_sum_kernel adds them in order.  Against one part by gemm_cost, a split launch takes its tiles as that has
+// them, or the time that the operands take out of memory (3,400 bytes per cycle), and 10,000 cycles and 3 per 1,000 sums
+// more for the sums' way through scratch; it has to save 8 %.  Fitted to 51 shapes (M 100-1500, N 256-4096, K 2048-128256) in 1 to 32
+// parts: the choice is 1 % behind the fastest on average, 15 % at most, and never behind one part.  us in one part and split:
+// 128 x 2048 x 128256 410 and 93 (floor 85), 500 x 2048 x 128256 563 and 211, 100 x 4096 x 28672 138 and 57, 512 x 2048 x 16384 75 and
+// 45, 128 x 1024 x 8192 30 and 15, 1500 x 256 x 32000 133 and 41; not split 1000 x 4096 x 28672 164 and 179, 512 x 4096 x 6144 25 and 31.
+// Products with both operands K-major are never split, although 100 x 4096 x 14336 would take 37 us instead of 64: they are the
+// forward pass, and what a model computes should not depend on how many SMs a device has.
+GemmShape gemm_split_shape(int M, int N, int K, bool b_mn, bool f32_out, int num_sms) {
+  const GemmShape whole = gemm_shape(M, N, K, b_mn, f32_out, num_sms);
+  const int k_blocks = (K + BK - 1) / BK;
+  if (!b_mn || f32_out || k_blocks < 8) return whole;
+  const double memory = 2.0 * K * (static_cast<double>(M) + N) / 3400;
+  const double unsplit = std::max(gemm_cost(M, N, K, b_mn, f32_out, whole.ctas, whole.width, num_sms), memory);
+  // no split is faster than the arithmetic of all SMs, or than memory
+  const double least = std::max(static_cast<double>(M) * N * K / (4096.0 * num_sms), memory);
+  if (least + 14000 > 0.92 * unsplit) return whole;
+  GemmShape best = whole;
+  double cost = 0.92 * unsplit;
+  for (const int splits : {2, 3, 4, 6, 8, 12, 16, 24, 32}) {
+    if (splits > k_blocks / 4 || gemm_split_floats(M, N, splits) > kMaxSplitFloats) break;
+    const double sums = 10000 + 0.003 * splits * M * N;
+    for (int ctas = 1; ctas <= 2 && ctas <= num_sms; ++ctas)
+      for (int width = 256; width >= 32; width -= 32) {
+        const double c = std::max(gemm_cost(M, N, K, b_mn, true, ctas, width, num_sms, splits), memory) + sums;
+        if (c < cost) {
+          cost = c;
+          best = {ctas, width, splits};
+        }
+      }
+  }
+  // as many parts as have k-blocks
+  const int per = (k_blocks + best.splits - 1) / best.splits;
+  best.splits = (k_blocks + per - 1) / per;
+  return best;
+}
+
+static int gemm_launch_shape(const GemmArgs& g, GemmShape shape, int num_sms, cudaStream_t stream) {
   if (shape.ctas < 1 || shape.ctas > 2 || shape.width < 32 || shape.width > 256 || shape.width % 32 != 0) return -1;
   if (num_sms < 2) shape.ctas = 1;
+  const int k_blocks = (g.K + BK - 1) / BK;
   const uint32_t b_rows = shape.width / shape.ctas;
   CUtensorMap ta, tb, tc;
   int rc;
@@ -559,8 +643,12 @@ int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
   rc = g.b_mn_major ? make_tmap_2d_bf16(&tb, g.b, g.N, g.K, g.ldb * 2, 64, BK)
                     : make_tmap_2d_bf16(&tb, g.b, g.K, g.N, g.ldb * 2, BK, b_rows);
   if (rc != 0) return rc;
-  rc = g.epilogue == kEpiAccumF32 ? make_tmap_c_f32(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 4)
-                                  : make_tmap_c_bf16(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 2);
+  const int rows = (g.M + 31) / 32 * 32, ld = (g.N + 7) / 8 * 8;      // of a part in scratch: the output boxes have 32 rows
+  if (shape.splits > 1)
+    rc = make_tmap_c_f32(&tc, g.scratch, g.N, static_cast<uint64_t>(shape.splits) * rows, static_cast<uint64_t>(ld) * 4);
+  else
+    rc = g.epilogue == kEpiAccumF32 ? make_tmap_c_f32(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 4)
+                                    : make_tmap_c_bf16(&tc, g.c, g.N, g.M, static_cast<uint64_t>(g.ldc) * 2);
   if (rc != 0) return rc;
   const int stage = A_STAGE_BYTES + (g.b_mn_major ? (b_rows + 63) / 64 * MN_BOX_BYTES : b_rows * BK * 2);
   Params p;
@@ -573,18 +661,43 @@ int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
   p.K = g.K;
   p.width = shape.width;
   p.stages = fit < MAX_STAGES ? fit : MAX_STAGES;
-  p.accumulate = g.accumulate;
+  p.accumulate = shape.splits > 1 ? 0 : g.accumulate;
+  p.splits = shape.splits;
+  p.k_per = (k_blocks + shape.splits - 1) / shape.splits;
+  p.split_rows = rows;
   const int tiles_m = (g.M + BM * shape.ctas - 1) / (BM * shape.ctas), tiles_n = (g.N + shape.width - 1) / shape.width;
   // An operand that stays in L2 (126 MB) is best read whole by every wave (4096 x 28672 x 4096: 701 us, in bands of 8
   // 717 us); one that does not is read from DRAM again by each, and bands of 8 tiles make the wave square (4096 x 4096 x
   // 28672: 799 and 761 us, x 14336: 389 and 381 us).
   const bool n_fast = tiles_n < tiles_m;
-  const long long fast_bytes = 2ll * (n_fast ? g.N : g.M) * g.K;
+  const long long fast_bytes = 2ll * (n_fast ? g.N : g.M) * g.K / shape.splits;
   p.band = fast_bytes > (96ll << 20) ? 8 : (n_fast ? tiles_n : tiles_m);
   p.status = g.status;
   p.sched = gemm_sched_slot();
-  return shape.ctas == 2 ? launch_layout<2>(g, ta, tb, tc, p, num_sms, stream)
-                         : launch_layout<1>(g, ta, tb, tc, p, num_sms, stream);
+  GemmArgs l = g;
+  if (shape.splits > 1) l.epilogue = kEpiAccumF32;
+  rc = shape.ctas == 2 ? launch_layout<2>(l, ta, tb, tc, p, num_sms, stream)
+                       : launch_layout<1>(l, ta, tb, tc, p, num_sms, stream);
+  if (rc != 0 || shape.splits == 1) return rc;
+  const long long threads = static_cast<long long>(g.M) * (ld / 8);
+  split_sum_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
+      g.scratch, static_cast<__nv_bfloat16*>(g.c), g.M, g.N, rows, ld, g.ldc, shape.splits);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+int gemm_bf16_launch(const GemmArgs& g, int num_sms, cudaStream_t stream) {
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return 0;
+  GemmShape shape = g.shape;
+  if (shape.ctas == 0) {
+    const int tile = gemm_forced_tile();
+    shape = tile != 0 ? GemmShape{tile / 128, 256, 1}
+                      : gemm_shape(g.M, g.N, g.K, g.b_mn_major != 0, g.epilogue != kEpiStoreBf16, num_sms);
+  }
+  if (shape.splits > 1) {
+    const int k_blocks = (g.K + BK - 1) / BK, per = (k_blocks + shape.splits - 1) / shape.splits;
+    if (g.scratch == nullptr || g.epilogue != kEpiStoreBf16 || (k_blocks + per - 1) / per != shape.splits) return -1;
+  }
+  return gemm_launch_shape(g, shape, num_sms, stream);
 }
 
 }  // namespace piper

@@ -13,6 +13,12 @@ enum : int {
   kEpiAccumF32 = 1,    // C (fp32) = acc, or C += acc when accumulate != 0
 };
 
+// The shape of a launch: CTAs per tile (1 or 2, 128 rows each), columns (a multiple of 32 up to 256), and parts of the
+// contraction.
+struct GemmShape {
+  int ctas, width, splits;
+};
+
 // C[M,N] = A[M,K] * B[N,K]^T.
 //   a_mn_major == 0: A is stored row-major [M, K] with row stride lda (elements).
 //   a_mn_major == 1: A is stored row-major [K, M] with row stride lda.
@@ -30,8 +36,8 @@ struct GemmArgs {
   int epilogue;     // kEpi*
   int accumulate;   // only for kEpiAccumF32
   int* status;      // device int, 0 = ok (see ptx.cuh)
-  int tile = 0;     // 0: chosen by shape (or PIPER_GEMM_TILE); 128: one CTA per tile, 256: a CTA pair
-  int width = 0;    // with tile != 0: columns of a tile, a multiple of 32 up to 256 (0: 256)
+  GemmShape shape = {0, 0, 1};   // ctas 0: by PIPER_GEMM_TILE or gemm_shape
+  float* scratch = nullptr;      // gemm_split_floats() floats where shape.splits > 1 (kEpiStoreBf16 only)
 };
 
 // Returns 0 on success, a negative code for a launch/set-up failure, or the
@@ -41,11 +47,13 @@ int gemm_bf16_launch(const GemmArgs& args, int num_sms, cudaStream_t stream);
 // The tile height (128: one CTA, 256: a CTA pair) that gemm_shape takes where the model of its costs is undecided.
 int gemm_tile_rows(int M, int N, int K, bool f32_out, int num_sms);
 
-// The tile shape that gemm_bf16_launch chooses: CTAs per tile (1 or 2, 128 rows each) and columns.
-struct GemmShape {
-  int ctas, width;
-};
+// The shape that gemm_bf16_launch chooses: the contraction in one part.
 GemmShape gemm_shape(int M, int N, int K, bool b_mn_major, bool f32_out, int num_sms);
+
+// The shape to launch where there may be scratch, and the scratch of one in `splits` parts (each with k-blocks of 64).
+GemmShape gemm_split_shape(int M, int N, int K, bool b_mn_major, bool f32_out, int num_sms);
+int gemm_forced_tile();   // of PIPER_GEMM_TILE, 0: none
+long long gemm_split_floats(int M, int N, int splits);
 
 enum : int {
   kGroupedFwd = 0,     // Y[rows, N]  = X[rows, K] * W[e]^T

@@ -173,6 +173,45 @@ def test_gemm_shapes_give_the_same_bits(M, N, K, tile):
             assert all(torch.equal(o, f) for o, f in zip(outs, first)), (xm, ym, width)
 
 
+@pytest.mark.parametrize("M,N,K,tile,width,splits", [(1, 8, 1024, 128, 32, 16), (100, 264, 5000, 128, 64, 7),
+                                                     (129, 1000, 4096, 128, 256, 3), (300, 520, 6016, 256, 96, 5),
+                                                     (513, 2056, 2112, 256, 256, 33), (1500, 256, 32000, 0, 0, 0),
+                                                     (33, 72, 20000, 0, 0, 0)])
+def test_gemm_split_contraction(M, N, K, tile, width, splits):
+    """Parts of equal and of unequal length, a k-block each, ragged rows and columns, and the shapes that the rule splits by
+    itself: against fp64, the same bits every time, and no further from it than the product in one part."""
+    from piper_b200.ops import native
+
+    lib, st = native.lib(), native.status_tensor()
+    torch.manual_seed(33)
+    for a_mn in (False, True):
+        a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+        b = torch.randn(K, (N + 7) // 8 * 8, device="cuda").to(torch.bfloat16)[:, :N]
+        if a_mn:
+            at = torch.zeros(K, (M + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)
+            at[:, :M] = a.t()
+            x = at[:, :M]
+        else:
+            x = torch.zeros(M, (K + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :K]
+            x.copy_(a)
+        want = a.double() @ b.double()
+        outs = [torch.full((M + 1, (N + 7) // 8 * 8), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+        for out in outs[:2]:
+            if splits:
+                lib.gemm_split(x, b, out[:M, :N], a_mn, True, st, tile, width, splits)
+            else:
+                assert lib.gemm_split_shape(M, N, K, True, False, 148)[2] > 1
+                lib.gemm(x, b, out[:M, :N], a_mn, True, False, st)
+        lib.gemm_shaped(x, b, outs[2][:M, :N], a_mn, True, False, st, 0, 0)
+        assert torch.equal(outs[0], outs[1])
+        assert (outs[0][M:] == 7).all() and (outs[0][:, N:] == 7).all()      # nothing beside the product
+        err = [((o[:M, :N].double() - want).norm() / want.norm()).item() for o in outs]
+        # one rounding to bf16 (rms 2^-9 / sqrt(3) at most); the sums in fp32 add far less
+        assert err[0] < 2 ** -9 and err[0] <= err[2] * 1.01
+        assert _close(outs[0][:M, :N], want, 2 ** -8)
+    native.check_status()
+
+
 @pytest.mark.parametrize("sizes,forked", [((4095,), []), ((4096,), [4096]), ((4096, 4095), [4096, 4095]),
                                           ((4095, 4096), [4096])])
 def test_linear_gradients_around_the_fork_threshold(sizes, forked, monkeypatch):

@@ -92,6 +92,44 @@ def test_gemm_shape_rule(M, N, K, b_mn, f32, sms, shape):
     assert tuple(native.lib().gemm_shape(M, N, K, b_mn, f32, sms)) == shape
 
 
+@pytest.mark.parametrize("M,N,K,b_mn,f32,sms,splits", [
+    (128, 2048, 128256, True, False, 148, 8), (1, 8, 32000, True, False, 148, 32),      # few tiles over a long contraction
+    (128, 2048, 128256, False, False, 148, 1), (128, 2048, 128256, True, True, 148, 1),  # forward pass, fp32 buckets
+    (1000, 4096, 28672, True, False, 148, 1), (4096, 4096, 28672, True, False, 148, 1),  # tiles for every SM
+    (512, 768, 256, True, False, 148, 1), (128, 256, 448, True, False, 148, 1),          # short contractions
+    (128, 1024, 8192, True, False, 1, 1),                                                # one SM gains nothing
+])
+def test_gemm_split_rule(M, N, K, b_mn, f32, sms, splits):
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    lib = native.lib()
+    ctas, width, got = lib.gemm_split_shape(M, N, K, b_mn, f32, sms)
+    assert got == splits
+    if got == 1:
+        assert (ctas, width) == tuple(lib.gemm_shape(M, N, K, b_mn, f32, sms))
+
+
+def test_gemm_split_parts_have_blocks_and_scratch_is_bounded():
+    import random
+
+    from piper_b200.ops import native
+
+    if not native.lib_path().exists():
+        pytest.skip("the native library has not been built")
+    rng, split = random.Random(3), 0
+    for _ in range(2000):
+        M, N, K = (int(2 ** rng.uniform(0, top)) for top in (12, 14, 17))
+        _, _, parts = native.lib().gemm_split_shape(M, N, K, True, False, rng.choice([148, 148, 64, 1]))
+        blocks = -(-K // 64)
+        per = -(-blocks // parts)
+        assert (parts - 1) * per < blocks <= parts * per                # none is empty
+        assert parts == 1 or parts * (M + 31) * (N + 7) * 4 <= (64 << 20) + parts * 4 * 31 * (M + N + 64)
+        split += parts > 1
+    assert split > 100
+
+
 @pytest.mark.parametrize("B,S,Hq,Hkv,sms,parts", [
     (1, 4096, 32, 32, 148, 1), (1, 4096, 32, 8, 148, 1), (1, 4096, 32, 4, 148, 2), (1, 5120, 16, 2, 148, 2),
     (1, 512, 32, 4, 148, 4), (1, 2048, 16, 2, 148, 8), (8, 1024, 16, 2, 148, 1), (8, 128, 16, 4, 148, 1),
