@@ -10,6 +10,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace piper {
 namespace {
 
@@ -182,44 +184,47 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   for (int i = threadIdx.x; i < D; i += NORM_THREADS) out[i] = dw_acc[i];
 }
 
-// Register-resident variants for D == VPT * 8 * NORM_THREADS (2048, 4096, 8192): every thread owns VPT
-// 8-element vectors of the row, so the row is read from memory exactly once and the block reduction needs a
-// single barrier (the per-warp sums alternate between two scratch rows; a thread can only reach the write of
-// row k+2 after every thread has passed the barrier of row k+1, i.e. after all reads of row k).
-__device__ __forceinline__ float block_sum_once(float v, float (*scratch)[NORM_THREADS / 32], int parity) {
+// Register-resident variants: THREADS threads (a multiple of 32, at most 256) own a row of 8 * VPT * THREADS elements, VPT
+// 8-element vectors each, so the row is read from memory exactly once and its reduction needs a single barrier (the per-warp
+// sums alternate between two scratch rows; a thread can only reach the write of row k+2 after every thread has passed the
+// barrier of row k+1, i.e. after all reads of row k).  A row of one warp needs none.
+// Sum over the THREADS threads of a row; barrier 1 + group is theirs.
+template <int THREADS>
+__device__ __forceinline__ float row_sum(float v, float* scratch, int warp, int group) {
   v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) scratch[parity][threadIdx.x >> 5] = v;
-  __syncthreads();
+  if (THREADS == 32) return v;
+  if ((threadIdx.x & 31) == 0) scratch[warp] = v;
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(THREADS) : "memory");
   float t = 0.f;
 #pragma unroll
-  for (int i = 0; i < NORM_THREADS / 32; ++i) t += scratch[parity][i];
+  for (int i = 0; i < THREADS / 32; ++i) t += scratch[i];
   return t;
 }
 
-// Forward: bound by memory.  Four CTAs per SM (two of rows of 8192 elements, which take 115 registers a thread) walk the
-// rows and fetch the next one before the current one is reduced: with a CTA per row every row paid for its first loads, for
-// the norm weights behind the barrier and for a last wave.  Residual and norm, 4096 x 4096: 27.7 and 23.5 us (134 MB, 5.7
-// TB/s), 8192 x 8192 115 and 87 us, 8192 x 2048 28.2 and 24.0 us; 1000 x 4096 7.7 us both ways.  The grid is what is resident
-// at once, and the launch bound keeps it so; four CTAs per SM of 8192-wide rows, in two waves, and two: 592 rows 10.6 and 9.5 us,
-// 1777 22.9 and 22.3, 8192 86.7 and 87.6, without residual 1000 rows 10.8 and 9.9.
-template <int VPT>
-constexpr int NORM_FWD_CTAS = VPT == 4 ? 2 : 4;   // per SM
+// Forward: bound by memory.  As many CTAs as are resident walk the rows (1,024 threads per SM, 512 of the widest rows, which
+// take 115 registers a thread) and fetch the next one before the current one is reduced: with a CTA per row every row paid for
+// its first loads, for the norm weights behind the barrier and for a last wave.  Residual and norm, 4096 x 4096: 27.7 and 23.5
+// us (134 MB, 5.7 TB/s), 8192 x 8192 115 and 87 us, 8192 x 2048 28.2 and 24.0 us; 1000 x 4096 7.7 us both ways.  With more CTAs than
+// fit, four per SM of 8192-wide rows, and two: 592 rows 10.6 and 9.5 us, 1777 22.9 and 22.3, 8192 86.7 and 87.6.  8192 rows
+// of 256, 1024, 2560 and 3072 by a CTA each that reads them twice and so: 13.4 19.9 39.7 47.5 and 5.7 12.6 27.1 34.1 us.
+template <int VPT, int THREADS>
+constexpr int NORM_FWD_CTAS = (VPT == 4 ? 512 : 1024) / THREADS;   // per SM, which holds 32
 
-template <int VPT>
-__global__ void __launch_bounds__(NORM_THREADS, NORM_FWD_CTAS<VPT>)
+template <int VPT, int THREADS>
+__global__ void __launch_bounds__(THREADS, NORM_FWD_CTAS<VPT, THREADS>)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                        __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd, long long T, float eps) {
-  constexpr int D = VPT * 8 * NORM_THREADS;
-  __shared__ float scratch[2][NORM_THREADS / 32];
+  constexpr int D = VPT * 8 * THREADS;
+  __shared__ float scratch[2][THREADS / 32];
   bf16x8 wv[VPT], nx[VPT], nr[VPT];
 #pragma unroll
-  for (int v = 0; v < VPT; ++v) wv[v] = reinterpret_cast<const bf16x8*>(w)[threadIdx.x + v * NORM_THREADS];
+  for (int v = 0; v < VPT; ++v) wv[v] = reinterpret_cast<const bf16x8*>(w)[threadIdx.x + v * THREADS];
   auto fetch = [&](long long rw) {
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
-      nx[v] = reinterpret_cast<const bf16x8*>(x + rw * D)[threadIdx.x + v * NORM_THREADS];
-      if (res) nr[v] = reinterpret_cast<const bf16x8*>(res + rw * D)[threadIdx.x + v * NORM_THREADS];
+      nx[v] = reinterpret_cast<const bf16x8*>(x + rw * D)[threadIdx.x + v * THREADS];
+      if (res) nr[v] = reinterpret_cast<const bf16x8*>(res + rw * D)[threadIdx.x + v * THREADS];
     }
   };
   long long row = blockIdx.x;
@@ -237,14 +242,14 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[v][j] += g[j];
         const bf16x8 hp = pack8(f[v]);   // the residual stream is bf16: normalise what is stored
-        reinterpret_cast<bf16x8*>(h_out + row * D)[threadIdx.x + v * NORM_THREADS] = hp;
+        reinterpret_cast<bf16x8*>(h_out + row * D)[threadIdx.x + v * THREADS] = hp;
         unpack8(hp, f[v]);
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss += f[v][j] * f[v][j];
     }
     if (row + gridDim.x < T) fetch(row + gridDim.x);
-    ss = block_sum_once(ss, scratch, parity);
+    ss = row_sum<THREADS>(ss, scratch[parity], threadIdx.x >> 5, 0);
     const float r = rsqrtf(ss / D + eps);
     if (threadIdx.x == 0) rstd[row] = r;
 #pragma unroll
@@ -253,51 +258,63 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
       unpack8(wv[v], g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[v][j] = f[v][j] * r * g[j];
-      reinterpret_cast<bf16x8*>(y + row * D)[threadIdx.x + v * NORM_THREADS] = pack8(f[v]);
+      reinterpret_cast<bf16x8*>(y + row * D)[threadIdx.x + v * THREADS] = pack8(f[v]);
     }
   }
 }
 
-// Two CTAs per SM (one for 8192-wide rows): the row vectors stay packed (bf16) in registers and are unpacked where they are used, which
-// keeps the kernel under 128 registers with the next row's loads in flight.
-template <int VPT>
-__global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 2 : 1)
+// Two CTAs per SM (one of the widest rows): the row vectors stay packed (bf16) in registers and are unpacked where they are
+// used, which keeps two vectors of 256 threads under 128 registers with the next row's loads in flight; with fewer registers
+// they spill (4096 columns under 102: 50 -> 69 us for 8192 rows).  CTAs are as many as there are strips of weight-gradient sums,
+// so narrow rows are worked on several at a time, whose sums a CTA adds in their order at the end.  8192 rows of
+// 256, 1024, 2560 and 3072 by a CTA of 256 threads a row, sums in shared memory, and so: 46.8 53.8 107.2 111.8 and 5.3 13.8 39.4
+// 42.7 us (4.7 TB/s).
+template <int VPT, int THREADS>
+constexpr int NORM_BWD_ROWS = VPT == 1 && THREADS < 384 ? 384 / THREADS : 1;
+
+template <int VPT, int THREADS>
+__global__ void __launch_bounds__(THREADS * NORM_BWD_ROWS<VPT, THREADS>, VPT <= 2 ? 2 : 1)
 rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                        float* __restrict__ dw_partial, int T) {
-  constexpr int D = VPT * 8 * NORM_THREADS;
-  __shared__ float scratch[2][NORM_THREADS / 32];
+  constexpr int D = VPT * 8 * THREADS, ROWS = NORM_BWD_ROWS<VPT, THREADS>;
+  const int rows = ROWS == 1 ? 1 : blockDim.x / THREADS;
+  const int group = ROWS == 1 ? 0 : threadIdx.x / THREADS, tid = threadIdx.x - group * THREADS;
+  __shared__ float scratch[2][THREADS * ROWS / 32];
+  extern __shared__ float strips[];              // [rows][D] where there are several
+  const int first_warp = group * (THREADS / 32);
   bf16x8 gw[VPT];
   float dw[VPT][8];
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
-    gw[v] = reinterpret_cast<const bf16x8*>(w)[threadIdx.x + v * NORM_THREADS];
+    gw[v] = reinterpret_cast<const bf16x8*>(w)[tid + v * THREADS];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dw[v][j] = 0.f;
   }
   // The next row's vectors are fetched before the current row is reduced, so the loads overlap the barrier.
   bf16x8 na[VPT], nb[VPT], ne[VPT];
   float nr = 0.f;
-  long long row = blockIdx.x;
+  const long long step = static_cast<long long>(gridDim.x) * rows;
+  long long row = static_cast<long long>(group) * gridDim.x + blockIdx.x;
   auto fetch = [&](long long rw) {
     const bf16x8* dyr = reinterpret_cast<const bf16x8*>(dy + rw * D);
     const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + rw * D);
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
-      na[v] = dyr[threadIdx.x + v * NORM_THREADS];
-      nb[v] = xr[threadIdx.x + v * NORM_THREADS];
+      na[v] = dyr[tid + v * THREADS];
+      nb[v] = xr[tid + v * THREADS];
     }
     if (dres) {
       const bf16x8* er = reinterpret_cast<const bf16x8*>(dres + rw * D);
 #pragma unroll
-      for (int v = 0; v < VPT; ++v) ne[v] = er[threadIdx.x + v * NORM_THREADS];
+      for (int v = 0; v < VPT; ++v) ne[v] = er[tid + v * THREADS];
     }
     nr = rstd[rw];
   };
   if (row < T) fetch(row);
   int parity = 0;
-  for (; row < T; row += gridDim.x, parity ^= 1) {
+  for (; row < T; row += step, parity ^= 1) {
     bf16x8 ca[VPT], cb[VPT], ce[VPT];
     const float r = nr;
 #pragma unroll
@@ -306,7 +323,7 @@ rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
       cb[v] = nb[v];
       if (dres) ce[v] = ne[v];
     }
-    if (row + gridDim.x < T) fetch(row + gridDim.x);
+    if (row + step < T) fetch(row + step);
     float dot = 0.f;
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
@@ -317,7 +334,7 @@ rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
 #pragma unroll
       for (int j = 0; j < 8; ++j) dot += a[j] * g[j] * (b[j] * r);
     }
-    dot = block_sum_once(dot, scratch, parity) / D;
+    dot = row_sum<THREADS>(dot, scratch[parity] + first_warp, tid >> 5, group) / D;
     bf16x8* dxr = reinterpret_cast<bf16x8*>(dx + row * D);
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
@@ -337,13 +354,28 @@ rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] += e[j];
       }
-      dxr[threadIdx.x + v * NORM_THREADS] = pack8(o);
+      dxr[tid + v * THREADS] = pack8(o);
     }
   }
   float* out = dw_partial + static_cast<long long>(blockIdx.x) * D;
+  if (rows > 1) {
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) {
+      float4* o4 = reinterpret_cast<float4*>(strips + group * D + (tid + v * THREADS) * 8);
+      o4[0] = make_float4(dw[v][0], dw[v][1], dw[v][2], dw[v][3]);
+      o4[1] = make_float4(dw[v][4], dw[v][5], dw[v][6], dw[v][7]);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < D; c += blockDim.x) {
+      float s = 0.f;
+      for (int g = 0; g < rows; ++g) s += strips[g * D + c];
+      out[c] = s;
+    }
+    return;
+  }
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
-    float4* o4 = reinterpret_cast<float4*>(out + (threadIdx.x + v * NORM_THREADS) * 8);
+    float4* o4 = reinterpret_cast<float4*>(out + (tid + v * THREADS) * 8);
     o4[0] = make_float4(dw[v][0], dw[v][1], dw[v][2], dw[v][3]);
     o4[1] = make_float4(dw[v][4], dw[v][5], dw[v][6], dw[v][7]);
   }
@@ -970,12 +1002,39 @@ inline int grid_for(long long work, int threads, int max_blocks = 148 * 16) {
 
 #define PIPER_LAUNCH_OK() (cudaGetLastError() == cudaSuccess ? 0 : -3)
 
-template <int VPT>
-static int rmsnorm_fwd_rows(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
-                            __nv_bfloat16* h_out, float* rstd, long long T, float eps, int num_sms, cudaStream_t st) {
-  const int ctas = NORM_FWD_CTAS<VPT> * num_sms;
-  rmsnorm_fwd_reg_kernel<VPT><<<static_cast<unsigned>(T < ctas ? T : ctas), NORM_THREADS, 0, st>>>(x, res, w, y, h_out, rstd, T, eps);
-  return PIPER_LAUNCH_OK();
+// Vectors per thread of the register-resident kernels: as few as leave a row at most 256 threads.  0: the row does not divide.
+static int norm_vectors(int D) {
+  if (D % 256 == 0 && D <= 2048) return 1;
+  if (D % 512 == 0 && D <= 4096) return 2;
+  return D % 1024 == 0 && D <= 8192 ? 4 : 0;
+}
+
+// Calls fn with the vectors and threads of a row of D elements as constants; false where there are none.
+template <class F>
+static bool with_norm_shape(int D, F fn) {
+  const int vpt = norm_vectors(D);
+  auto at = [&](auto v) {
+    constexpr int V = decltype(v)::value;
+    switch (D / (256 * V)) {
+      case 8: fn(v, std::integral_constant<int, 256>()); return;
+      case 7: fn(v, std::integral_constant<int, 224>()); return;
+      case 6: fn(v, std::integral_constant<int, 192>()); return;
+      case 5: fn(v, std::integral_constant<int, 160>()); return;
+      default: break;
+    }
+    if constexpr (V == 1) {
+      switch (D / 256) {
+        case 4: fn(v, std::integral_constant<int, 128>()); return;
+        case 3: fn(v, std::integral_constant<int, 96>()); return;
+        case 2: fn(v, std::integral_constant<int, 64>()); return;
+        default: fn(v, std::integral_constant<int, 32>()); return;
+      }
+    }
+  };
+  if (vpt == 1) at(std::integral_constant<int, 1>());
+  else if (vpt == 2) at(std::integral_constant<int, 2>());
+  else if (vpt == 4) at(std::integral_constant<int, 4>());
+  return vpt != 0;
 }
 
 int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd,
@@ -987,12 +1046,12 @@ int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_
   const auto* wp = static_cast<const __nv_bfloat16*>(w);
   auto* yp = static_cast<__nv_bfloat16*>(y);
   auto* hp = static_cast<__nv_bfloat16*>(h_out);
-  switch (D) {
-    case 2048: return rmsnorm_fwd_rows<1>(xp, rp, wp, yp, hp, rstd, T, eps, num_sms, st);
-    case 4096: return rmsnorm_fwd_rows<2>(xp, rp, wp, yp, hp, rstd, T, eps, num_sms, st);
-    case 8192: return rmsnorm_fwd_rows<4>(xp, rp, wp, yp, hp, rstd, T, eps, num_sms, st);
-    default: break;
-  }
+  const bool done = with_norm_shape(D, [&](auto vpt, auto threads) {
+    constexpr int VPT = decltype(vpt)::value, THREADS = decltype(threads)::value;
+    const long long ctas = static_cast<long long>(NORM_FWD_CTAS<VPT, THREADS>) * num_sms;
+    rmsnorm_fwd_reg_kernel<VPT, THREADS><<<static_cast<unsigned>(T < ctas ? T : ctas), THREADS, 0, st>>>(xp, rp, wp, yp, hp, rstd, T, eps);
+  });
+  if (done) return PIPER_LAUNCH_OK();
   rmsnorm_fwd_kernel<<<static_cast<unsigned>(T), NORM_THREADS, 0, st>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res),
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
@@ -1016,16 +1075,16 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
   const int nb = rmsnorm_bwd_num_partials(T);
   const dim3 red_grid((D + 31) / 32), red_block(32, RED_SLICES);
   const WeightGrad out{dw_f32, static_cast<__nv_bfloat16*>(dw_bf16), accumulate};
-  if (D == 2048 || D == 4096 || D == 8192) {
-    const auto* dyp = static_cast<const __nv_bfloat16*>(dy);
-    const auto* xp = static_cast<const __nv_bfloat16*>(x);
-    const auto* wp = static_cast<const __nv_bfloat16*>(w);
-    const auto* ep = static_cast<const __nv_bfloat16*>(dres);
-    auto* dxp = static_cast<__nv_bfloat16*>(dx);
-    const int Ti = static_cast<int>(T);
-    if (D == 2048) rmsnorm_bwd_reg_kernel<1><<<nb, NORM_THREADS, 0, st>>>(dyp, xp, wp, rstd, ep, dxp, dw_partial, Ti);
-    else if (D == 4096) rmsnorm_bwd_reg_kernel<2><<<nb, NORM_THREADS, 0, st>>>(dyp, xp, wp, rstd, ep, dxp, dw_partial, Ti);
-    else rmsnorm_bwd_reg_kernel<4><<<nb, NORM_THREADS, 0, st>>>(dyp, xp, wp, rstd, ep, dxp, dw_partial, Ti);
+  const bool done = with_norm_shape(D, [&](auto vpt, auto threads) {
+    constexpr int VPT = decltype(vpt)::value, THREADS = decltype(threads)::value;
+    // several rows at a time where a CTA has several to do
+    const long long each = (T + nb - 1) / nb;
+    const int rows = static_cast<int>(each < NORM_BWD_ROWS<VPT, THREADS> ? each : NORM_BWD_ROWS<VPT, THREADS>);
+    rmsnorm_bwd_reg_kernel<VPT, THREADS><<<nb, rows * THREADS, rows > 1 ? rows * D * sizeof(float) : 0, st>>>(
+        static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), rstd,
+        static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), dw_partial, static_cast<int>(T));
+  });
+  if (done) {
     reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, out, out, D);
     return PIPER_LAUNCH_OK();
   }

@@ -352,6 +352,32 @@ def test_rmsnorm_and_residual(T, D):
     assert _close(y2, x0 * torch.rsqrt(x0.pow(2).mean(-1, keepdim=True) + 1e-6) * w.detach().float(), 1e-2)
 
 
+@pytest.mark.parametrize("T", [1, 5, 299, 1801])
+@pytest.mark.parametrize("D", [8, 256, 512, 768, 1024, 1280, 1536, 1792, 2048, 2304, 2560, 3072, 3584, 4608, 5120, 6144, 7168, 8200])
+def test_rmsnorm_widths(T, D):
+    """Every number of threads and vectors per row, widths beside them for the general kernels, fewer rows than CTAs and
+    several per CTA; against fp64 with the residual rounded as the op rounds it."""
+    from piper_b200 import ops
+
+    torch.manual_seed(35)
+    x, r, gy, gh = (torch.randn(T, D, device="cuda").to(torch.bfloat16) for _ in range(4))
+    w = torch.randn(D, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    x.requires_grad_(True)
+    y, h = ops.add_rmsnorm(x, r, w, 1e-6)
+    dx, dw = torch.autograd.grad([y, h], [x, w], [gy, gh])
+    assert torch.equal(h, (x.float() + r.float()).to(torch.bfloat16))
+    h64, w64 = h.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    y64 = h64 * torch.rsqrt(h64.pow(2).mean(-1, keepdim=True) + 1e-6) * w64
+    dx64, dw64 = torch.autograd.grad(y64, [h64, w64], gy.double())
+    dx64 = dx64 + gh.double()
+    # one rounding to bf16 each; sums in fp32
+    assert ((y.double() - y64).abs() <= 2 ** -8 * y64.abs() + 1e-6).all()
+    assert ((dx.double() - dx64).abs() <= 2 ** -8 * dx64.abs() + 1e-4).all()
+    assert ((dw.double() - dw64).abs() <= 2 ** -8 * dw64.abs() + 1e-5 * max(1, T) ** 0.5 * 4).all()
+    plain = ops.rmsnorm(h.detach(), w.detach(), 1e-6)
+    assert torch.equal(plain, y)
+
+
 @pytest.mark.parametrize("hd,inter,qknorm,seqs", [(128, True, False, 2), (128, False, True, 2), (64, False, False, 2),
                                                   (64, True, True, 2), (128, False, True, 640), (64, True, True, 1200)])
 def test_qk_rope(hd, inter, qknorm, seqs):
