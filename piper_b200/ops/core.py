@@ -66,6 +66,15 @@ class GradSinks:
             if self._sinks.pop(address, None) is not None and (lib := self._native()) is not None:
                 lib.sink_unset.default(address)
 
+    def forget(self, address: int, sink_address: int) -> None:
+        """Drop the entry of a parameter that is gone, unless its address has another buffer by now."""
+        with native.lock:
+            sink = self._sinks.get(address)
+            if sink is not None and sink.data_ptr() == sink_address:
+                del self._sinks[address]
+                if (lib := self._native()) is not None:
+                    lib.sink_unset.default(address)
+
     def get(self, param: Tensor) -> Optional[Tensor]:
         return self._sinks.get(param.data_ptr())
 

@@ -25,6 +25,7 @@ single-process model start from identical weights.
 from __future__ import annotations
 
 import os
+import weakref
 import zlib
 from dataclasses import dataclass, field
 from typing import Any, Callable, Optional
@@ -85,6 +86,11 @@ class AdamConfig:
     decoupled: bool = False     # True: AdamW (decay shrinks the weight); False: torch.optim.Adam's L2 term in the gradient
 
 
+def _forget_sinks(sinks: dict) -> None:
+    for address, sink_address in sinks.items():
+        ops_core.grad_sinks.forget(address, sink_address)
+
+
 class ParamStorage:
     """Flat buffers of one bucket plus its (possibly sharded) Adam state."""
 
@@ -123,6 +129,10 @@ class ParamStorage:
         self.row_table: Optional[list] = None
         self.persistent_grads = False      # the full gradient buffer is never freed (it lives in symmetric memory)
         self.fused_stepped = False
+        # what this bucket has registered as gradient sinks: the allocator may hand a dead bucket's addresses to another
+        # tensor, which must not find the old buffer there
+        self._sinks: dict[int, int] = {}
+        weakref.finalize(self, _forget_sinks, self._sinks).atexit = False
         if self.numel == 0:
             return
         full = torch.zeros(self.numel, dtype=dtype, device=device)
@@ -230,7 +240,9 @@ class ParamStorage:
         for s in self.slots:
             p = self.param_views.get(s.pos)
             if p is not None:
-                ops_core.grad_sinks.register(p, self.flat_grads[s.offset:s.offset + s.numel])
+                sink = self.flat_grads[s.offset:s.offset + s.numel]
+                ops_core.grad_sinks.register(p, sink)
+                self._sinks[p.data_ptr()] = sink.data_ptr()
 
     def _unregister_sinks(self) -> None:
         for p in self.param_views.values():

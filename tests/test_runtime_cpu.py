@@ -397,6 +397,33 @@ def test_row_sharding_partitions_every_parameter_and_rebuilds_it():
             assert torch.allclose(master, w.detach(), atol=1e-6), cls
 
 
+def test_gradient_sinks_go_with_their_bucket():
+    """The address of a dead bucket's parameter can be another tensor's: it has no sink, unless that tensor has got its own."""
+    import gc
+
+    from piper_b200.ops import core
+    from piper_b200.runtime.storage import AdamConfig, ParamSlot, ParamStorage
+
+    def bucket():
+        slots = [ParamSlot(i, f"w{i}", (8, 16), torch.float32, True) for i in range(2)]
+        return ParamStorage("bucket", slots, torch.device("cpu"), torch.float32, "local", 0, 1, None, AdamConfig())
+
+    before = dict(core.grad_sinks._sinks)
+    st = bucket()
+    first, second = st.param_views[0], st.param_views[1]
+    assert core.grad_sinks.get(first) is not None and core.grad_sinks.get(second) is not None
+    own = torch.zeros(8, 16)
+    core.grad_sinks.register(second, own)
+    del st
+    gc.collect()
+    try:
+        assert core.grad_sinks.get(first) is None
+        assert core.grad_sinks.get(second).data_ptr() == own.data_ptr()
+    finally:
+        core.grad_sinks.unregister(second)
+    assert core.grad_sinks._sinks.keys() == before.keys()
+
+
 def test_optimizer_mapping_rejects_what_the_kernels_cannot_do():
     import functools
 
