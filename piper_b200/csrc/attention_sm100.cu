@@ -149,6 +149,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
+  grid_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -174,6 +175,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                       static_cast<int>(tok0) + (it >> 1) * 128);
         if (++s == L::STAGES) { s = 0; ph ^= 1; }
       }
+      grid_launch();
       if (it < 2 * n_blocks) {
         // Unwinding after a failed wait: let the copies already issued land
         // before the CTA and its shared memory go away.
@@ -396,6 +398,7 @@ template <int HD>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   float* __restrict__ delta, int* __restrict__ arrived, int n_arrived, long long T, int S, int Hq) {
+  grid_begin(o, d_o);
   for (int i = blockIdx.x * 256 + threadIdx.x; i < n_arrived; i += gridDim.x * 256) arrived[i] = 0;
   constexpr int LANES = HD / 8;
   const int wl = threadIdx.x & 31;
@@ -512,6 +515,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
+  grid_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -551,6 +555,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
         bulk_load(v + L::VEC_BYTES, delta + idx, L::VEC_BYTES, &bars->y_full[st]);
         if (++ti == S / 64) { ti = 2 * xb; ++hh; }
       }
+      grid_launch();
       if (it < n_iter) {
         // Unwinding: wait (bounded) for the copies in flight.
         await(&bars->x_full, 0, nullptr);
@@ -856,6 +861,7 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
+  grid_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -885,6 +891,7 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
           tma_load_2d(smem + L::V_OFF + (vj & 1) * L::TILE + h * 16384, tmap_qkv_x, &bars->v_full[vj & 1],
                       (Hq + Hkv + g) * HD + 64 * h, tok0 + vj * 128);
       }
+      grid_launch();
       if (vj < n_blocks) {
         // Unwinding: wait (bounded) for the copies in flight.
         await(&bars->x_full, 0, nullptr);
@@ -1095,7 +1102,7 @@ static int attn_fwd_impl(const CUtensorMap& tm, const CUtensorMap& to, float* ls
   const int tiles_per_cta = attn_tiles_per_cta(B, S, Hq, num_sms);
   const long long ctas = (per_head + tiles_per_cta - 1) / tiles_per_cta * Hkv * B;
   if (ctas > 0x7fffffffll) return -1;
-  attn_fwd_kernel<HD><<<static_cast<unsigned>(ctas), FWD_THREADS, FwdSmem<HD>::TOTAL, st>>>(
+  launch_overlapped(attn_fwd_kernel<HD>, static_cast<unsigned>(ctas), FWD_THREADS, FwdSmem<HD>::TOTAL, st, 
       tm, to, lse, S, Hq, Hkv, B, tiles_per_cta, scale_log2, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -1165,11 +1172,11 @@ static int attn_bwd_impl(const void* qkv, const void* out, const void* d_out, co
   int* arrived = reinterpret_cast<int*>(scratch);
   float* partial = scratch == nullptr ? nullptr : scratch + (n_kv + 3) / 4 * 4;
   const long long delta_blocks = (T * Hq * (HD / 8) + 255) / 256;
-  attn_delta_kernel<HD><<<static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st>>>(
+  launch_overlapped(attn_delta_kernel<HD>, static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st, 
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, arrived,
       parts > 1 ? n_kv : 0, T, S, Hq);
   if (cudaGetLastError() != cudaSuccess) return -3;
-  attn_bwd_kernel<HD><<<static_cast<unsigned>(n_kv * parts + S / 128 * Hq * B), BWD_THREADS, smem, st>>>(
+  launch_overlapped(attn_bwd_kernel<HD>, static_cast<unsigned>(n_kv * parts + S / 128 * Hq * B), BWD_THREADS, smem, st, 
       tqx, tqy, tdx, tdy, tdq, lse, delta, B, S, Hq, Hkv, parts, partial, arrived, softmax_scale,
       softmax_scale * 1.4426950408889634f, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                    __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd, int D, float eps) {
+  grid_begin(x, res, w);
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
@@ -137,6 +138,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int T, int D) {
+  grid_begin(dy, x, w, rstd, dres);
   extern __shared__ float dw_acc[];   // D floats
   __shared__ float scratch[32];
   for (int i = threadIdx.x; i < D; i += NORM_THREADS) dw_acc[i] = 0.f;
@@ -215,6 +217,7 @@ __global__ void __launch_bounds__(THREADS, NORM_FWD_CTAS<VPT, THREADS>)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                        __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd, long long T, float eps) {
+  grid_begin(x, res, w);
   constexpr int D = VPT * 8 * THREADS;
   __shared__ float scratch[2][THREADS / 32];
   bf16x8 wv[VPT], nx[VPT], nr[VPT];
@@ -278,6 +281,7 @@ rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                        float* __restrict__ dw_partial, int T) {
+  grid_begin(dy, x, w, rstd, dres);
   constexpr int D = VPT * 8 * THREADS, ROWS = NORM_BWD_ROWS<VPT, THREADS>;
   const int rows = ROWS == 1 ? 1 : blockDim.x / THREADS;
   const int group = ROWS == 1 ? 0 : threadIdx.x / THREADS, tid = threadIdx.x - group * THREADS;
@@ -393,6 +397,7 @@ struct WeightGrad {
 constexpr int RED_SLICES = 32;
 __global__ void __launch_bounds__(32 * RED_SLICES)
 reduce_partials_kernel(const float* __restrict__ partial, int nblocks, int D, WeightGrad first, WeightGrad second, int split) {
+  grid_begin(partial);
   __shared__ float part[RED_SLICES][32];
   const int c = blockIdx.x * 32 + threadIdx.x;
   const int per = (nblocks + RED_SLICES - 1) / RED_SLICES;
@@ -642,6 +647,7 @@ __device__ __forceinline__ void rope_kind(const RopeArgs& a, const RopeGroup<HD>
 template <int HD, bool NORM, bool BWD, bool INTER>
 __global__ void __launch_bounds__(256, ROPE_CTAS<NORM, BWD>)
 qk_rope_kernel(const __grid_constant__ RopeArgs a) {
+  grid_begin();
   __shared__ float sdw[NORM && BWD ? 8 : 1][2 * HD];
   const bool want_dw = NORM && BWD && a.partial != nullptr;
   const RopeGroup<HD> g;
@@ -714,6 +720,7 @@ __device__ __forceinline__ float sigmoid(float g) {
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restrict__ act, long long T, int F,
                   int stride_rows, int stride_cols) {
+  grid_begin(h13);
   const int vecs = F / 8;
   for (VecWalk w(vecs); w.row < T; w.next(vecs, stride_rows, stride_cols)) {
     const bf16x8* base = reinterpret_cast<const bf16x8*>(h13 + w.row * 2 * F);
@@ -729,6 +736,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restri
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ h13, const __nv_bfloat16* __restrict__ dact,
                   __nv_bfloat16* __restrict__ dh13, long long T, int F, int stride_rows, int stride_cols) {
+  grid_begin(h13, dact);
   const int vecs = F / 8;
   for (VecWalk w(vecs); w.row < T; w.next(vecs, stride_rows, stride_cols)) {
     const bf16x8* base = reinterpret_cast<const bf16x8*>(h13 + w.row * 2 * F);
@@ -752,6 +760,7 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ h13, const __nv_bfloat16* __
 __global__ void embedding_fwd_kernel(const long long* __restrict__ tokens,
                                      const __nv_bfloat16* __restrict__ table, __nv_bfloat16* __restrict__ out,
                                      long long T, int D, int V, int* status) {
+  grid_begin(tokens, table);
   const long long row = blockIdx.x;
   long long tok = tokens[row];
   if (tok < 0 || tok >= V) {   // recorded, not trapped
@@ -826,6 +835,7 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
               float* __restrict__ loss, float* __restrict__ lse, int V, long long ld,
               long long ignore_index) {
+  grid_begin(logits, labels);
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   const __nv_bfloat16* lr = logits + row * ld;
@@ -869,6 +879,7 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restr
 __global__ void __launch_bounds__(1024)
 ce_mean_kernel(const float* __restrict__ loss, const long long* __restrict__ labels, float* __restrict__ mean,
                float* __restrict__ count, long long T, long long ignore_index) {
+  grid_begin(loss, labels);
   __shared__ double sums[32];
   __shared__ int counts[32];
   double s = 0.0;
@@ -906,6 +917,7 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
               const float* __restrict__ lse, const float* __restrict__ gscale, float row_scale,
               __nv_bfloat16* __restrict__ out, int V, long long ld, long long ignore_index) {
+  grid_begin(logits, labels, lse, gscale);
   const long long row = blockIdx.x;
   const __nv_bfloat16* lr = logits + row * ld;
   __nv_bfloat16* orow = out + row * ld;
@@ -974,6 +986,7 @@ __global__ void accum_bf16_into_f32_kernel(const __nv_bfloat16* __restrict__ g, 
 // out = a + b over n bf16 elements (n % 8 == 0): the residual add at a stage boundary.
 __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                                 __nv_bfloat16* __restrict__ out, long long nvec) {
+  grid_begin(a, b);
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float x[8], y[8];
@@ -1049,10 +1062,10 @@ int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_
   const bool done = with_norm_shape(D, [&](auto vpt, auto threads) {
     constexpr int VPT = decltype(vpt)::value, THREADS = decltype(threads)::value;
     const long long ctas = static_cast<long long>(NORM_FWD_CTAS<VPT, THREADS>) * num_sms;
-    rmsnorm_fwd_reg_kernel<VPT, THREADS><<<static_cast<unsigned>(T < ctas ? T : ctas), THREADS, 0, st>>>(xp, rp, wp, yp, hp, rstd, T, eps);
+    launch_overlapped(rmsnorm_fwd_reg_kernel<VPT, THREADS>, static_cast<unsigned>(T < ctas ? T : ctas), THREADS, 0, st, xp, rp, wp, yp, hp, rstd, T, eps);
   });
   if (done) return PIPER_LAUNCH_OK();
-  rmsnorm_fwd_kernel<<<static_cast<unsigned>(T), NORM_THREADS, 0, st>>>(
+  launch_overlapped(rmsnorm_fwd_kernel, static_cast<unsigned>(T), NORM_THREADS, 0, st, 
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res),
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
       static_cast<__nv_bfloat16*>(h_out), rstd, D, eps);
@@ -1080,12 +1093,12 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
     // several rows at a time where a CTA has several to do
     const long long each = (T + nb - 1) / nb;
     const int rows = static_cast<int>(each < NORM_BWD_ROWS<VPT, THREADS> ? each : NORM_BWD_ROWS<VPT, THREADS>);
-    rmsnorm_bwd_reg_kernel<VPT, THREADS><<<nb, rows * THREADS, rows > 1 ? rows * D * sizeof(float) : 0, st>>>(
+    launch_overlapped(rmsnorm_bwd_reg_kernel<VPT, THREADS>, nb, rows * THREADS, rows > 1 ? rows * D * sizeof(float) : 0, st, 
         static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), rstd,
         static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), dw_partial, static_cast<int>(T));
   });
   if (done) {
-    reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, out, out, D);
+    launch_overlapped(reduce_partials_kernel, red_grid, red_block, 0, st, dw_partial, nb, D, out, out, D);
     return PIPER_LAUNCH_OK();
   }
   static bool configured = false;
@@ -1093,11 +1106,11 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
     cudaFuncSetAttribute(rmsnorm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     configured = true;
   }
-  rmsnorm_bwd_kernel<<<nb, NORM_THREADS, D * sizeof(float), st>>>(
+  launch_overlapped(rmsnorm_bwd_kernel, nb, NORM_THREADS, D * sizeof(float), st, 
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
       static_cast<const __nv_bfloat16*>(w), rstd, static_cast<const __nv_bfloat16*>(dres),
       static_cast<__nv_bfloat16*>(dx), dw_partial, static_cast<int>(T), D);
-  reduce_partials_kernel<<<red_grid, red_block, 0, st>>>(dw_partial, nb, D, out, out, D);
+  launch_overlapped(reduce_partials_kernel, red_grid, red_block, 0, st, dw_partial, nb, D, out, out, D);
   return PIPER_LAUNCH_OK();
 }
 
@@ -1119,7 +1132,7 @@ static int qk_rope_launch(RopeArgs a, bool interleaved, int num_sms, int& grid, 
   const long long blocks = (tasks(a.run) + 7) / 8;
   grid = static_cast<int>(blocks < resident ? blocks : resident);
   auto kern = interleaved ? qk_rope_kernel<HD, NORM, BWD, true> : qk_rope_kernel<HD, NORM, BWD, false>;
-  kern<<<grid, 256, 0, st>>>(a);
+  launch_overlapped(kern, grid, 256, 0, st, a);
   return PIPER_LAUNCH_OK();
 }
 
@@ -1166,8 +1179,8 @@ int qk_rope_bwd(const void* dout, const void* in, void* din, const float* cosp, 
   if (rc != 0 || !(want_q || want_k)) return rc;
   const WeightGrad none{nullptr, nullptr, 0};
   const bool same = want_q && want_k && (q.f32 ? q.f32 == k.f32 : q.bf16 == k.bf16);   // one weight for both: in turn
-  reduce_partials_kernel<<<2 * hd / 32, dim3(32, RED_SLICES), 0, st>>>(partial, grid, 2 * hd, q, same ? none : k, hd);
-  if (same) reduce_partials_kernel<<<2 * hd / 32, dim3(32, RED_SLICES), 0, st>>>(partial, grid, 2 * hd, none, k, hd);
+  launch_overlapped(reduce_partials_kernel, 2 * hd / 32, dim3(32, RED_SLICES), 0, st, partial, grid, 2 * hd, q, same ? none : k, hd);
+  if (same) launch_overlapped(reduce_partials_kernel, 2 * hd / 32, dim3(32, RED_SLICES), 0, st, partial, grid, 2 * hd, none, k, hd);
   return PIPER_LAUNCH_OK();
 }
 
@@ -1177,7 +1190,7 @@ int swiglu_fwd(const void* h13, void* act, long long T, int F, cudaStream_t st) 
   const int vecs = F / 8;
   const int blocks = grid_for(T * vecs, 256);
   const long long stride = static_cast<long long>(blocks) * 256;
-  swiglu_fwd_kernel<<<blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(h13), static_cast<__nv_bfloat16*>(act), T,
+  launch_overlapped(swiglu_fwd_kernel, blocks, 256, 0, st, static_cast<const __nv_bfloat16*>(h13), static_cast<__nv_bfloat16*>(act), T,
                                             F, static_cast<int>(stride / vecs), static_cast<int>(stride % vecs));
   return PIPER_LAUNCH_OK();
 }
@@ -1188,7 +1201,7 @@ int swiglu_bwd(const void* h13, const void* dact, void* dh13, long long T, int F
   const int vecs = F / 8;
   const int blocks = grid_for(T * vecs, 256);
   const long long stride = static_cast<long long>(blocks) * 256;
-  swiglu_bwd_kernel<<<blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(h13),
+  launch_overlapped(swiglu_bwd_kernel, blocks, 256, 0, st, static_cast<const __nv_bfloat16*>(h13),
                                             static_cast<const __nv_bfloat16*>(dact), static_cast<__nv_bfloat16*>(dh13),
                                             T, F, static_cast<int>(stride / vecs), static_cast<int>(stride % vecs));
   return PIPER_LAUNCH_OK();
@@ -1198,7 +1211,7 @@ int embedding_fwd(const long long* tokens, const void* table, void* out, long lo
                   int* status, cudaStream_t st) {
   if (D % 8 != 0) return -1;
   if (T == 0) return 0;
-  embedding_fwd_kernel<<<static_cast<unsigned>(T), 128, 0, st>>>(
+  launch_overlapped(embedding_fwd_kernel, static_cast<unsigned>(T), 128, 0, st, 
       tokens, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), T, D, V, status);
   return PIPER_LAUNCH_OK();
 }
@@ -1233,7 +1246,7 @@ int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse,
            long long ld, long long ignore_index, cudaStream_t st) {
   if (ld % 8 != 0) return -1;
   if (T == 0) return 0;
-  ce_fwd_kernel<<<static_cast<unsigned>(T), CE_THREADS, 0, st>>>(
+  launch_overlapped(ce_fwd_kernel, static_cast<unsigned>(T), CE_THREADS, 0, st, 
       static_cast<const __nv_bfloat16*>(logits), labels, loss, lse, V, ld, ignore_index);
   return PIPER_LAUNCH_OK();
 }
@@ -1241,7 +1254,7 @@ int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse,
 int ce_mean(const float* loss, const long long* labels, float* mean, float* count, long long T, long long ignore_index,
             cudaStream_t st) {
   if (T < 0 || T >= (1ll << 24)) return -1;      // the count is exact in fp32
-  ce_mean_kernel<<<1, 1024, 0, st>>>(loss, labels, mean, count, T, ignore_index);
+  launch_overlapped(ce_mean_kernel, 1, 1024, 0, st, loss, labels, mean, count, T, ignore_index);
   return PIPER_LAUNCH_OK();
 }
 
@@ -1250,7 +1263,7 @@ int ce_bwd(const void* logits, const long long* labels, const float* lse, const 
            cudaStream_t st) {
   if (ld % 8 != 0) return -1;
   if (T == 0) return 0;
-  ce_bwd_kernel<<<static_cast<unsigned>(T), CE_THREADS, 0, st>>>(
+  launch_overlapped(ce_bwd_kernel, static_cast<unsigned>(T), CE_THREADS, 0, st, 
       static_cast<const __nv_bfloat16*>(logits), labels, lse, gscale, row_scale,
       static_cast<__nv_bfloat16*>(out), V, ld, ignore_index);
   return PIPER_LAUNCH_OK();
@@ -1277,7 +1290,7 @@ int cast_f32_to_bf16(const float* in, void* out, long long n, float scale, cudaS
 int add_bf16(const void* a, const void* b, void* out, long long n, cudaStream_t st) {
   if (n % 8 != 0) return -1;
   if (n == 0) return 0;
-  add_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(a),
+  launch_overlapped(add_bf16_kernel, grid_for(n / 8, 256), 256, 0, st, static_cast<const __nv_bfloat16*>(a),
                                                        static_cast<const __nv_bfloat16*>(b),
                                                        static_cast<__nv_bfloat16*>(out), n / 8);
   return PIPER_LAUNCH_OK();

@@ -130,6 +130,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const bool draws = p.sched != nullptr && num_tiles > units;
   if (warp == 3 && rank == 0 && lane == 0)
     bars->first = draws ? atomicAdd(&p.sched[0], 1) : static_cast<int>(blockIdx.x) / CTAS;
+  grid_wait();
   tc_fence_before();
   if (CTAS == 2) cluster_sync(); else __syncthreads();
   tc_fence_after();
@@ -208,6 +209,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       }
       if (!ok) break;
     }
+    grid_launch();                               // the last loads are on their way
     if (ok) {
       // every stage handed back before the CTA may leave: no commit is still on its way to these barriers
       for (int i = 0; i < stages && ok; ++i) {
@@ -358,6 +360,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 __global__ void __launch_bounds__(256)
 split_sum_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ c, int M, int N, int rows, int ld, long long ldc,
                  int splits) {
+  grid_begin(parts);
   const int vecs = ld / 8;
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= static_cast<long long>(M) * vecs) return;
@@ -489,13 +492,15 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CTAS;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  cfg.numAttrs = CTAS > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p) == cudaSuccess ? 0 : -3;
 }
 
@@ -680,7 +685,7 @@ static int gemm_launch_shape(const GemmArgs& g, GemmShape shape, int num_sms, cu
                        : launch_layout<1>(l, ta, tb, tc, p, num_sms, stream);
   if (rc != 0 || shape.splits == 1) return rc;
   const long long threads = static_cast<long long>(g.M) * (ld / 8);
-  split_sum_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
+  launch_overlapped(split_sum_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, 
       g.scratch, static_cast<__nv_bfloat16*>(g.c), g.M, g.N, rows, ld, g.ldc, shape.splits);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -134,6 +134,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tma_prefetch_desc(&tmap_c);
   }
   if (warp == 3) {
+    grid_wait();
     // Token tiles before each segment, in the order q = expert * sources + source (group = source * experts + expert):
     // a warp scan, since one thread walking the table pays a memory latency per group in front of every launch.
     int acc = 0;
@@ -183,6 +184,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tmem_relinquish_n<CTAS>();
     if (lane == 0) bars->first = first;
   }
+  grid_wait();
   tc_fence_before();
   if (CTAS == 2) cluster_sync();
   else __syncthreads();
@@ -289,6 +291,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
       if (!ok) break;
     }
+    grid_launch();                                     // the last loads are on their way
     if (ok) {
       // every stage handed back before the CTA may leave: no commit is still on its way to these barriers
       for (int i = 0; i < STAGES && ok; ++i) {
@@ -494,13 +497,15 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CTAS;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  cfg.numAttrs = CTAS > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p) == cudaSuccess ? 0 : -3;
 }
 

@@ -58,6 +58,7 @@ template <int SLOTS>
 __global__ void route_kernel(const __nv_bfloat16* __restrict__ logits, float* __restrict__ weights,
                              int* __restrict__ idx, int* __restrict__ counts, long long T, int E, int k,
                              int renorm) {
+  grid_begin(logits);
   const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -94,6 +95,7 @@ __global__ void route_kernel(const __nv_bfloat16* __restrict__ logits, float* __
 __global__ void route_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const int* __restrict__ idx,
                                  const float* __restrict__ weights, const float* __restrict__ dweights,
                                  __nv_bfloat16* __restrict__ dlogits, long long T, int E, int k, int renorm) {
+  grid_begin(logits, idx, weights, dweights);
   const long long t = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -133,6 +135,7 @@ __global__ void group_table_kernel(const int* __restrict__ counts, int num_group
                                    const int* __restrict__ row_base, int* __restrict__ g_start,
                                    int* __restrict__ g_len, int* __restrict__ total, int* __restrict__ cursor,
                                    int* __restrict__ copy) {
+  grid_begin(counts, row_base);
   const int lane = threadIdx.x;
   int run = 0, last = 0;
   for (int s0 = 0; s0 < num_groups; s0 += experts) {
@@ -191,6 +194,7 @@ permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx,
                const int* __restrict__ g_len, const int* __restrict__ counts, int* __restrict__ cursor,
                int* __restrict__ pos, __nv_bfloat16* __restrict__ rows, long long T, int D, int k, int E,
                long long rows_cap, unsigned token_ctas, int* status) {
+  grid_begin(x, idx, g_start, g_len, counts);
   const unsigned pad_ctas = E * PAD_CTAS;
   if (blockIdx.x < pad_ctas) {
     const int b = static_cast<int>(blockIdx.x);
@@ -256,6 +260,7 @@ __global__ void __launch_bounds__(ROW_THREADS)
 gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ pos,
                   const float* __restrict__ weights, __nv_bfloat16* __restrict__ out, long long T, int D, int k,
                   long long rows_cap, int tag, int* status) {
+  grid_begin(rows, pos, weights);
   const long long t = (static_cast<long long>(blockIdx.x) * ROW_THREADS + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -311,6 +316,7 @@ combine_bwd_kernel(const __nv_bfloat16* __restrict__ rows, const __nv_bfloat16* 
                    __nv_bfloat16* __restrict__ drows, float* __restrict__ dweights,
                    const int* __restrict__ g_start, const int* __restrict__ g_len, const int* __restrict__ counts,
                    long long T, int D, int k, long long rows_cap, unsigned token_ctas, int* status) {
+  grid_begin(rows, dout, pos, weights, g_start, g_len, counts);
   if (blockIdx.x >= token_ctas) {
     const int b = static_cast<int>(blockIdx.x - token_ctas);
     zero_padding(drows, g_start, g_len, counts, b / PAD_CTAS, b % PAD_CTAS, D, rows_cap, status);
@@ -373,7 +379,7 @@ int moe_route(const void* logits, float* weights, int* idx, int* counts, long lo
   if (E > 32 * MAX_PER_LANE || k > MAX_K || k > E || k < 1) return -1;
   if (T == 0) return 0;
   auto kern = E <= 32 ? route_kernel<1> : E <= 64 ? route_kernel<2> : E <= 128 ? route_kernel<4> : route_kernel<8>;
-  kern<<<warps_grid(T, ROW_THREADS), ROW_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), weights, idx,
+  launch_overlapped(kern, warps_grid(T, ROW_THREADS), ROW_THREADS, 0, st, static_cast<const __nv_bfloat16*>(logits), weights, idx,
                                                            counts, T, E, k, renorm);
   return PIPER_LAUNCH_OK();
 }
@@ -382,7 +388,7 @@ int moe_route_bwd(const void* logits, const int* idx, const float* weights, cons
                   long long T, int E, int k, int renorm, cudaStream_t st) {
   if (E > 32 * MAX_PER_LANE || k > MAX_K) return -1;
   if (T == 0) return 0;
-  route_bwd_kernel<<<warps_grid(T, 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), idx, weights,
+  launch_overlapped(route_bwd_kernel, warps_grid(T, 256), 256, 0, st, static_cast<const __nv_bfloat16*>(logits), idx, weights,
                                                        dweights, static_cast<__nv_bfloat16*>(dlogits), T, E, k,
                                                        renorm);
   return PIPER_LAUNCH_OK();
@@ -391,7 +397,7 @@ int moe_route_bwd(const void* logits, const int* idx, const float* weights, cons
 int moe_group_table(const int* counts, int num_groups, int experts, const int* row_base, int* g_start, int* g_len,
                     int* total, int* cursor, int* copy, cudaStream_t st) {
   if (num_groups <= 0 || experts <= 0) return -1;
-  group_table_kernel<<<1, 32, 0, st>>>(counts, num_groups, experts, row_base, g_start, g_len, total, cursor, copy);
+  launch_overlapped(group_table_kernel, 1, 32, 0, st, counts, num_groups, experts, row_base, g_start, g_len, total, cursor, copy);
   return PIPER_LAUNCH_OK();
 }
 
@@ -400,7 +406,7 @@ int moe_permute(const void* x, const int* idx, const int* g_start, const int* g_
                 cudaStream_t st) {
   if (D % 8 != 0) return -1;
   const unsigned token_ctas = warps_grid(T, ROW_THREADS);
-  permute_kernel<<<token_ctas + E * PAD_CTAS, ROW_THREADS, 0, st>>>(
+  launch_overlapped(permute_kernel, token_ctas + E * PAD_CTAS, ROW_THREADS, 0, st, 
       static_cast<const __nv_bfloat16*>(x), idx, g_start, g_len, counts, cursor, pos, static_cast<__nv_bfloat16*>(rows),
       T, D, k, E, rows_cap, token_ctas, status);
   return PIPER_LAUNCH_OK();
@@ -413,7 +419,7 @@ static int gather_sum(const void* rows, const int* pos, const float* weights, vo
   if (T == 0) return 0;
   auto kern = k == 1 ? gather_sum_kernel<1> : k == 2 ? gather_sum_kernel<2> : k <= 4 ? gather_sum_kernel<4>
                                                                                       : gather_sum_kernel<8>;
-  kern<<<warps_grid(T, ROW_THREADS), ROW_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(rows), pos, weights,
+  launch_overlapped(kern, warps_grid(T, ROW_THREADS), ROW_THREADS, 0, st, static_cast<const __nv_bfloat16*>(rows), pos, weights,
                                                            static_cast<__nv_bfloat16*>(out), T, D, k, rows_cap, tag,
                                                            status);
   return PIPER_LAUNCH_OK();
@@ -437,7 +443,7 @@ int moe_combine_bwd(const void* rows, const void* dout, const int* pos, const fl
   if (token_ctas + num_groups == 0) return 0;
   auto kern = k == 1 ? combine_bwd_kernel<1> : k == 2 ? combine_bwd_kernel<2> : k <= 4 ? combine_bwd_kernel<4>
                                                                                         : combine_bwd_kernel<8>;
-  kern<<<token_ctas + num_groups * PAD_CTAS, ROW_THREADS, 0, st>>>(
+  launch_overlapped(kern, token_ctas + num_groups * PAD_CTAS, ROW_THREADS, 0, st, 
       static_cast<const __nv_bfloat16*>(rows), static_cast<const __nv_bfloat16*>(dout), pos, weights,
       static_cast<__nv_bfloat16*>(drows), dweights, g_start, g_len, counts, T, D, k, rows_cap, token_ctas, status);
   return PIPER_LAUNCH_OK();

@@ -586,6 +586,64 @@ def test_swiglu_large_gates():
     assert a[0, 4095].isnan() and h.grad[0, 4095].isnan() and h.grad[0, 8191].isnan()
 
 
+@pytest.mark.parametrize("T,D,F", [(128, 256, 512), (384, 512, 1536), (2048, 1024, 2048)])
+def test_overlapped_launches_keep_their_order(T, D, F):
+    """A kernel may start while the one before it runs, but reads what that one leaves: every op behind one that has just
+    written its input, weights that the optimizer kernel and a tensor op have just changed, a buffer that the allocator
+    hands on at once, the same with the device idle between any two ops, and in a captured graph."""
+    from piper_b200 import ops
+    from piper_b200.ops import moe, native
+
+    torch.manual_seed(37)
+    rn = lambda *shape: torch.randn(*shape, device="cuda").to(torch.bfloat16)
+    x, r, w13, w2, wn = rn(T, D), rn(T, D), rn(2 * F, D) * D ** -0.5, rn(D, F) * F ** -0.5, rn(D)
+    wqkv, labels = rn(3 * D, D) * D ** -0.5, torch.randint(0, D, (T,), device="cuda")
+    we, logits = rn(8, D, D) * D ** -0.5, rn(T, 8)
+    cos, sin = ops.rope_tables(64, 128, 1e4, device="cuda")
+    up = rn(T, D)
+    state = [torch.randn(w2.numel(), device="cuda") for _ in range(4)]
+
+    def chain(idle):
+        step = torch.cuda.synchronize if idle else lambda: None
+        w = w2.clone()
+        master, m, v, g = (t.clone() for t in state)
+        v.abs_()
+        step(); native.lib().adam_flat(master, m, v, g, w.view(-1), 1e-3, 0.9, 0.95, 1e-8, 0.0, 1, 1.0, True)
+        leaves = [t.clone().requires_grad_(True) for t in (x, w13, w, wn, wqkv, we, logits)]
+        xl, a13, a2, an, aq, ae, lg = leaves
+        with torch.no_grad():
+            step(); an.mul_(1.5)
+        step(); y, h = ops.add_rmsnorm(xl, r, an, 1e-6)
+        step(); qkv = ops.linear(y, aq)
+        step(); qkv = ops.qk_rope(qkv, cos, sin, None, None, 128, D // 64, D // 64, 64, True, 1e-6)
+        step(); o = ops.attention(qkv, T // 128, 128, D // 64, D // 64, 64)
+        step(); f = ops.linear(o, a13)
+        step(); f = ops.linear(ops.swiglu(f), a2)
+        step(); y, h = ops.add_rmsnorm(f, h, an, 1e-6)
+        step(); wts, idx, counts = moe.moe_route(lg, 1, True)
+        step(); rows, pos, gs, gl, ec = moe.moe_dispatch(y, idx, counts)
+        step(); e = moe.grouped_linear(rows, ae, *moe.moe_group_table(ec, ae))
+        step(); out = moe.moe_combine(e, pos, wts, gs, gl, counts) + h
+        step(); loss = ops.cross_entropy(out, labels)
+        step(); grads = torch.autograd.grad(loss, leaves)
+        return [loss.detach(), *grads]
+
+    want = chain(True)
+    for _ in range(20):
+        # rows of one expert come in the order of their arrival, and so do the sums of its weight's gradient
+        for i, (a, b) in enumerate(zip(chain(False), want)):
+            assert torch.equal(a, b) if i != 6 else _close(a, b, 2 ** -8), i
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = chain(False)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for i, (a, b) in enumerate(zip(captured, want)):
+        assert torch.equal(a, b) if i != 6 else _close(a, b, 2 ** -8), i
+    native.check_status()
+
+
 @pytest.mark.parametrize("T,ignored", [(0, 0.0), (1, 0.0), (33, 0.3), (1023, 1.0), (1024, 0.0), (5000, 0.3), (65536, 0.1), (65537, 0.1)])
 def test_cross_entropy_mean(T, ignored):
     """One CTA's sum over any number of rows, and the sum by tensor ops above its limit: value, gradient, and the gradient of
