@@ -72,6 +72,10 @@ __device__ __forceinline__ void store_row_chunk_sw128(uint8_t* tile, int row, in
 // which a row maximum of the warp has grown.  (Letting the maximum go stale until it has grown by 2^8 saves 8-15 % of
 // the time, but the largest probability of a row is then rounded to bf16 where it is exactly 1 otherwise: error against
 // 64 bits 2.05e-3 -> 2.09e-3 at S = 4096.)
+// Where there are too few tiles for pairs, a CTA works on one, and its even and odd key blocks take the places of two tiles,
+// each with its own maxima, sums and output in tensor memory, merged at the end: a block alone is a serial chain of scores,
+// softmax and P V, 1.3 us long at head dimension 64.  us with one chain and with two: 1 x 2048, 4 heads x 64 24.0 and 16.7, 1 x 4096, 8
+// heads x 64 45.8 and 31.7, 1 x 8192, 4 heads x 128 107.5 and 63.4, 1 x 512, 32 heads x 128 10.4 and 8.9.
 // Tiles of one kv head are numbered query block major, so a pair is two heads of the group on the same rows where
 // the group is even, and neighbouring query blocks otherwise.
 // S = 4096, 32 q / 8 kv heads x 128: 237 us with one CTA per 128 query rows and probabilities through shared memory,
@@ -100,7 +104,9 @@ struct FwdBars {
   uint32_t tmem_base;
 };
 
-template <int HD>
+// ONE: one tile per CTA, else tiles_per_cta, two.  A constant for the one case only: the loops of two tiles lose 0.6 % both to
+// the other case's decisions and with their own number as a constant (1 x 8192, 32 / 4 heads x 128, 523.5 and 526.6 us).
+template <int HD, bool ONE>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_out,
                 float* __restrict__ lse, int S, int Hq, int Hkv, int B, int tiles_per_cta, float scale_log2,
@@ -121,12 +127,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   const int g = gb % Hkv;
   const int b = gb / Hkv;
   const int t0 = pair * tiles_per_cta;
-  const bool two = tiles_per_cta == 2 && t0 + 1 < tiles;
+  const bool two = !ONE && tiles_per_cta == 2 && t0 + 1 < tiles;
   const int qblk0 = t0 / group, head0 = g * group + t0 % group;
   const int qblk1 = (t0 + 1) / group, head1 = g * group + (t0 + 1) % group;
-  const int n0 = qblk0 + 1;
-  const int n1 = two ? qblk1 + 1 : 0;           // n1 >= n0 where there are two tiles
-  const int n_blocks = two ? n1 : n0;
+  // one tile: its even key blocks take the place of tile A, the odd ones that of tile B, and the two are merged at the end
+  const bool halves = ONE && qblk0 > 0;
+  const int n0 = halves ? (qblk0 + 2) / 2 : qblk0 + 1;
+  const int n1 = two ? qblk1 + 1 : halves ? (qblk0 + 1) / 2 : 0;     // n1 >= n0 where there are two tiles
+  const int n_blocks = two ? n1 : qblk0 + 1;
   const long long tok0 = static_cast<long long>(b) * S;
 
   if (threadIdx.x == 0) {
@@ -195,7 +203,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const uint64_t dv_base = umma_desc_sw128(smem_u32(smem + L::KV_OFF), 16384, 1024);
 
     auto issue_s = [&](int t, int st) {
-      const uint64_t dq = dq0 + (t * L::TILE >> 4);
+      const uint64_t dq = dq0 + (halves ? 0 : t * L::TILE >> 4);
       const uint64_t dk = dk_base + (st * L::TILE >> 4);
 #pragma unroll
       for (int ks = 0; ks < HD / 16; ++ks) {
@@ -224,9 +232,42 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
       __syncwarp();
     }
+    if (halves) {
+      // block b belongs to half b % 2; its K is entry 2b of the ring, its V entry 2b + 1
+      auto entry = [&](int e) { return await_all(&bars->kv_full[e % L::STAGES], (e / L::STAGES) & 1, status); };
+      auto scores = [&](int b) -> bool {
+        if (!entry(2 * b)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          issue_s(b & 1, 2 * b % L::STAGES);
+          umma_commit(&bars->kv_empty[2 * b % L::STAGES]);
+        }
+        __syncwarp();
+        return true;
+      };
+      ok = ok && scores(1);
+      for (int b = 0; b < n_blocks && ok; ++b) {
+        const int t = b & 1, v_st = (2 * b + 1) % L::STAGES;
+        const uint32_t p_ph = (b >> 1) & 1;
+        ok = entry(2 * b + 1) && await_all(&bars->p_full[t][0], p_ph, status);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) issue_pv(t, v_st, 0, b < 2);
+        __syncwarp();
+        if (!(ok = await_all(&bars->p_full[t][1], p_ph, status))) break;
+        tc_fence_after();
+        if (elect_one()) {
+          issue_pv(t, v_st, 1, false);
+          if (b + 2 >= n_blocks) umma_commit(&bars->o_done[t]);
+          umma_commit(&bars->kv_empty[v_st]);
+        }
+        __syncwarp();
+        if (b + 2 < n_blocks) ok = scores(b + 2);
+      }
+    }
     int st = 1;                    // ring slot of V of block j; K of block j + 1 follows it
     uint32_t ph = 0;
-    for (int j = 0; j < n_blocks && ok; ++j) {
+    for (int j = 0; j < n_blocks && ok && (!ONE || !halves); ++j) {
       const int v_st = st;
       const uint32_t v_ph = ph;
       if (++st == L::STAGES) { st = 0; ph ^= 1; }
@@ -268,12 +309,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
       if (!more) break;
     }
-  } else if (warp < 4 || two) {
+  } else if (warp < 4 || two || halves) {
     // --------------------------------------------------- softmax + output
     const int t = warp >> 2;
     const int n_t = t ? n1 : n0;
-    const int qblk = t ? qblk1 : qblk0;
-    const int head = t ? head1 : head0;
+    const int qblk = t && !halves ? qblk1 : qblk0;
+    const int head = t && !halves ? head1 : head0;
     const int row = (warp & 3) * 32 + lane;      // query row == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t ts = tmem_base + lane_sel + t * 128;
@@ -288,7 +329,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, sv[c]);
       tmem_ld_wait();
-      if (j == qblk) {
+      if ((halves ? 2 * j + t : j) == qblk) {
         // causal mask, applied once to the registers of the only tile that needs it: a score of -inf then
         // drops out of the maximum and turns into a probability of exactly zero below
 #pragma unroll
@@ -355,19 +396,44 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
       l_run += (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
     }
-    if (ok && await_all(&bars->o_done[t], 0, status)) {
+    float wa = 1.f, wb = 0.f;                    // weights of the two halves' sums; the first half's warps write the tile
+    if (halves) {
+      // maxima and sums of the second half, through the buffer of the second query tile
+      float2* other = reinterpret_cast<float2*>(smem + L::Q_OFF + L::TILE);
+      if (t == 1) other[row] = make_float2(m_run, l_run);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (t == 0) {
+        const float2 o = other[row];
+        const float m = fmaxf(m_run, o.x);
+        wa = fast_exp2((m_run - m) * scale_log2);
+        wb = fast_exp2((o.x - m) * scale_log2);
+        l_run = l_run * wa + o.y * wb;
+        m_run = m;
+        ok = ok && await_all(&bars->o_done[1], 0, status);
+      }
+    }
+    if ((!ONE || !(halves && t == 1)) && ok && await_all(&bars->o_done[t], 0, status)) {
       // the tile's Q operand has been read for the last time; its buffer takes the output, 32 rows per warp
       tc_fence_after();
       const float inv = 1.f / l_run;
+      const float2 fa = make_float2(wa * inv, wa * inv), fb = make_float2(wb * inv, wb * inv);
       uint8_t* obuf = smem + L::Q_OFF + t * L::TILE;
 #pragma unroll
       for (int c = 0; c < HD / 32; ++c) {
-        uint32_t r[32], w[16];
+        uint32_t r[32], r2[32], w[16];
         tmem_ld_32x32(to + c * 32, r);
+        if (halves) tmem_ld_32x32(to + 128 + c * 32, r2);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+        for (int i = 0; i < 16; ++i) {
+          if (!ONE) {
+            w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+            continue;
+          }
+          float2 v = mul2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), fa);
+          if (halves) v = fma2(make_float2(__uint_as_float(r2[2 * i]), __uint_as_float(r2[2 * i + 1])), fb, v);
+          w[i] = pack_bf16x2(v.x, v.y);
+        }
         store_row_chunk_sw128(obuf + (c >> 1) * 16384, row, (c & 1) * 4, w);
       }
       lse[(static_cast<long long>(b) * Hq + head) * S + qblk * 128 + row] =
@@ -1078,12 +1144,12 @@ int set_smem(K kern, int bytes) {
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
-// Two query tiles per CTA overlap the softmax of one with the MMAs of the other, but last 1.1 to 1.3 times as long as
-// the longer of the two alone.  As long as every tile has an SM of its own, or the SMs get through all key blocks of all
+// Two query tiles per CTA read every K and V block once for both; one tile in two halves is done in little more than half the
+// time of a tile in one chain.  As long as every tile has an SM of its own, or the SMs get through all key blocks of all
 // tiles (longest first) before a longest tile and a block have passed, one tile per CTA finishes earlier.  One against
-// two on 148 SMs, head dimension 64 / 128: 16 key blocks, 256 tiles 29.0 against 35.1 / 35.0 against 37.1 us, 320
-// tiles 37.3 / 35.1 and 44.7 / 37.2; 4 blocks, 152 tiles 11.0 / 12.6 and 12.6 / 14.7, 208 tiles 14.6 / 12.9 and 16.7 / 14.7;
-// with one block two tiles are never slower.
+// two on 148 SMs, head dimension 64 / 128: 16 key blocks, 384 tiles 31.4 against 29.7 / 37.3 against 35.0 us, 512 tiles 40.3 against
+// 32.7 / 49.0 against 39.3; 4 blocks, 256 tiles 11.8 against 10.7 / 14.1 against 12.7; 8 blocks, 256 tiles, the first size that has
+// two, 14.9 against 17.0 / 17.5 against 20.0; with one block two tiles are never slower.
 int attn_tiles_per_cta(int B, int S, int Hq, int num_sms) {
   const long long blocks = S / 128, tiles = static_cast<long long>(B) * Hq * blocks;
   return tiles <= num_sms || tiles * (blocks + 1) / 2 <= (blocks - 1) * num_sms ? 1 : 2;
@@ -1094,7 +1160,8 @@ static int attn_fwd_impl(const CUtensorMap& tm, const CUtensorMap& to, float* ls
                          float softmax_scale, int num_sms, int* status, cudaStream_t st) {
   static bool cfg = false;
   if (!cfg) {
-    if (set_smem(attn_fwd_kernel<HD>, FwdSmem<HD>::TOTAL)) return -2;
+    if (set_smem(attn_fwd_kernel<HD, true>, FwdSmem<HD>::TOTAL) || set_smem(attn_fwd_kernel<HD, false>, FwdSmem<HD>::TOTAL))
+      return -2;
     cfg = true;
   }
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
@@ -1102,8 +1169,9 @@ static int attn_fwd_impl(const CUtensorMap& tm, const CUtensorMap& to, float* ls
   const int tiles_per_cta = attn_tiles_per_cta(B, S, Hq, num_sms);
   const long long ctas = (per_head + tiles_per_cta - 1) / tiles_per_cta * Hkv * B;
   if (ctas > 0x7fffffffll) return -1;
-  launch_overlapped(attn_fwd_kernel<HD>, static_cast<unsigned>(ctas), FWD_THREADS, FwdSmem<HD>::TOTAL, st, 
-      tm, to, lse, S, Hq, Hkv, B, tiles_per_cta, scale_log2, status);
+  launch_overlapped(tiles_per_cta == 1 ? attn_fwd_kernel<HD, true> : attn_fwd_kernel<HD, false>, static_cast<unsigned>(ctas),
+                    FWD_THREADS, FwdSmem<HD>::TOTAL, st, tm, to, lse, S, Hq, Hkv, B, tiles_per_cta, scale_log2,
+                    status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

@@ -644,6 +644,35 @@ def test_overlapped_launches_keep_their_order(T, D, F):
     native.check_status()
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,hd", [(1, 128, 2, 1, 64), (2, 256, 2, 2, 128), (1, 384, 3, 1, 64), (1, 640, 2, 2, 128),
+                                           (1, 1408, 4, 1, 64), (1, 2048, 8, 2, 128), (1, 2048, 16, 4, 64)])
+def test_attention_halves_of_key_blocks(B, S, Hq, Hkv, hd):
+    """One query tile per CTA, with no, one and several key blocks in its second half, an odd number of blocks, and more tiles
+    than SMs: output, log-sum-exp and gradients against fp64.  Large scores in single key blocks make the halves' maxima
+    differ by more than exp2 can hold in 16 bits."""
+    from piper_b200.ops import core, native
+
+    assert native.lib().attn_tiles_per_cta(B, S, Hq, 148) == 1
+    torch.manual_seed(39)
+    qkv = torch.randn(B * S, (Hq + 2 * Hkv) * hd, device="cuda")
+    qkv.view(B, S, -1)[:, 128:256, Hq * hd:(Hq + Hkv) * hd] *= 12          # keys of the second block
+    qkv = qkv.to(torch.bfloat16).requires_grad_(True)
+    out, lse = core.attention_fwd(qkv, B, S, Hq, Hkv, hd, hd ** -0.5)
+    g = torch.randn_like(out)
+    (dqkv,) = torch.autograd.grad(out, qkv, g)
+    x = qkv.detach().double().requires_grad_(True)
+    q, k, v = (t.transpose(1, 2) for t in x.view(B, S, Hq + 2 * Hkv, hd).split([Hq, Hkv, Hkv], 2))
+    k, v = (t.repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+    scores = (q @ k.transpose(2, 3) * hd ** -0.5).masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = (torch.softmax(scores, -1) @ v).transpose(1, 2).reshape(B * S, Hq * hd)
+    (dref,) = torch.autograd.grad(ref, x, g.double())
+    # probabilities are rounded to bf16 (2^-9 of a weighted mean of v), results once more; scores are fp32 sums
+    assert _close(out, ref, 2 ** -7) and _close(dqkv, dref, 2 ** -6)
+    assert ((out.double() - ref).norm() / ref.norm()) < 4e-3
+    want = torch.logsumexp(scores, -1)
+    assert ((lse.double() - want).abs() <= 1e-5 * want.abs().clamp(min=1)).all()
+
+
 @pytest.mark.parametrize("T,ignored", [(0, 0.0), (1, 0.0), (33, 0.3), (1023, 1.0), (1024, 0.0), (5000, 0.3), (65536, 0.1), (65537, 0.1)])
 def test_cross_entropy_mean(T, ignored):
     """One CTA's sum over any number of rows, and the sum by tensor ops above its limit: value, gradient, and the gradient of
