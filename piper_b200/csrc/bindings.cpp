@@ -1,7 +1,7 @@
 // torch.ops.piper_c.*: thin tensor-level wrappers over the launchers in this
 // directory.  Each wrapper validates shapes/dtypes, takes the current CUDA
 // stream, and writes into caller-allocated outputs; none of them allocates
-// device memory.  Higher-level autograd-aware ops live in piper_b200/ops.
+// device memory but a product whose contraction is split (gemm_run).  Higher-level autograd-aware ops live in piper_b200/ops.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <torch/library.h>
