@@ -586,6 +586,52 @@ def test_swiglu_large_gates():
     assert a[0, 4095].isnan() and h.grad[0, 4095].isnan() and h.grad[0, 8191].isnan()
 
 
+_SWIGLU_BY_DIVISION = """
+extern "C" __global__ void swiglu_by_division(const float* g, const float* u, const float* d, float* a, float* dg, float* du,
+                                              long long n) {
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= n) return;
+  a[i] = g[i] / (1.f + __expf(-g[i])) * u[i];
+  const float s = 1.f / (1.f + __expf(-g[i]));
+  du[i] = d[i] * (g[i] * s);
+  dg[i] = d[i] * u[i] * s * (1.f + g[i] * (1.f - s));
+}
+"""
+
+
+@pytest.mark.parametrize("backward", [False])
+def test_swiglu_has_the_bits_of_a_division(backward):
+    """Every bf16 gate with every up value (forward) or every upstream gradient (backward): the kernels, which do not divide,
+    against one that does, with the same exponential.  A sigmoid one unit in the last place of fp32 off shows in about one of
+    2^15 products, so nothing less than all of them pins it."""
+    from piper_b200 import ops
+
+    divided = torch.cuda._compile_kernel(_SWIGLU_BY_DIVISION, "swiglu_by_division")
+    torch.manual_seed(43)
+    every = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(torch.bfloat16)
+    rows, F = 64, every.numel()
+    g = every.expand(rows, F)
+    gf = g.float().contiguous()
+    bad = torch.zeros(3, dtype=torch.int64, device="cuda")
+    for values in every.split(rows):
+        u, up = values[:, None], torch.randn(rows, 1, device="cuda").bfloat16()
+        if backward:
+            u, up = up, u
+        u, up = u.expand(rows, F).contiguous(), up.expand(rows, F).contiguous()
+        h = torch.cat([g, u], 1).requires_grad_(backward)
+        act = ops.swiglu(h)
+        got = [act.detach()]
+        if backward:
+            (dh,) = torch.autograd.grad(act, h, up)
+            got += [dh[:, :F].contiguous(), dh[:, F:].contiguous()]
+        want = [torch.empty(rows, F, device="cuda") for _ in range(3)]
+        divided(grid=(rows * F // 256, 1, 1), block=(256, 1, 1), args=[gf, u.float(), up.float(), *want, rows * F])
+        for i, (x, y) in enumerate(zip(got, want)):
+            y = y.bfloat16()
+            bad[i] += ((x.view(torch.int16) != y.view(torch.int16)) & ~(x.isnan() & y.isnan())).sum()
+    assert bad.tolist() == [0, 0, 0]
+
+
 @pytest.mark.parametrize("T,D,F", [(128, 256, 512), (384, 512, 1536), (2048, 1024, 2048)])
 def test_overlapped_launches_keep_their_order(T, D, F):
     """A kernel may start while the one before it runs, but reads what that one leaves: every op behind one that has just
