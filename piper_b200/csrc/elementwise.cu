@@ -692,31 +692,24 @@ struct VecWalk {
   }
 };
 
-// (1 + exp(-g)) / 4 and its approximate reciprocal (1 ulp).  The quarter keeps the reciprocal of every finite divisor a normal
-// number; an infinite one is held at a value whose reciprocal is flushed to zero.  The forward pass brings its quotient to the
-// rounding of the exact one by Markstein's step, q - r (d q - n) with fused multiply-adds (IBM J. Res. Dev. 34, 1990), in which a
-// zero keeps its sign; his theorem wants a correctly rounded r, so it is the 65,536 gates that show it, and a test divides by them
-// all.  The gradients, of several such factors and sums, take the reciprocal as it is.  IEEE divisions, with the range checks that this
-// needs none of, made both kernels issue-bound.  With them and so, in us: 4096 x 14336 forward 72.9 and 59.5 (352 MB, 5.9 TB/s),
-// backward 109.4 and 101.3 (106.9 with the step); 49,024 x 768 forward 52.4 and 37.3, backward 67.9 and 62.5.  Forward results
-// keep their bits, errors of the gradients against 64 bits stay the same.
-__device__ __forceinline__ void sigmoid_divisor(float g, float& d, float& r) {
-  d = fminf(fmaf(__expf(-g), 0.25f, 0.25f), 0x1.8p126f);
+// 4 n / (1 + exp(-g)): both passes divide by d = (1 + exp(-g)) / 4 with its approximate reciprocal r (1 ulp).  The quarter keeps
+// the reciprocal of every finite divisor a normal number; an infinite one is held at a value whose reciprocal is flushed to zero.
+// One step of Markstein's, q - r (d q - n) with fused multiply-adds (IBM J. Res. Dev. 34, 1990), brings the quotient to the
+// rounding of the exact one; in this form of it a zero keeps its sign.  His theorem wants a correctly rounded r, so it is the gates
+// that show it: there are 65,536, and a test divides by all of them.  IEEE divisions have range checks that this needs
+// none of.  With them and so, in us: 4096 x 14336 forward 74.0 and 62.8 (352 MB, 5.6 TB/s), backward 107.7 and 106.9; 49,024 x 768
+// forward 51.0 and 43.2, backward 73.2 and 68.6.  Without the step a sigmoid that is a unit of fp32 off now and then turns the
+// rounding of gradients, and of all that follows from them, and nothing is faster (backward 108.6 and 73.0).
+__device__ __forceinline__ float over_sigmoid_divisor(float n, float g) {
+  const float d = fminf(fmaf(__expf(-g), 0.25f, 0.25f), 0x1.8p126f);
+  float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-}
-
-__device__ __forceinline__ float silu(float g) {
-  float d, r;
-  sigmoid_divisor(g, d, r);
-  const float n = 0.25f * g, q = n * r;
+  const float q = n * r;
   return fabsf(n) < 1e37f ? fmaf(-fmaf(d, q, -n), r, q) : q;     // an infinite q has no remainder
 }
 
-__device__ __forceinline__ float sigmoid(float g) {
-  float d, r;
-  sigmoid_divisor(g, d, r);
-  return 0.25f * r;
-}
+__device__ __forceinline__ float silu(float g) { return over_sigmoid_divisor(0.25f * g, g); }
+__device__ __forceinline__ float sigmoid(float g) { return over_sigmoid_divisor(0.25f, g); }
 
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restrict__ act, long long T, int F,

@@ -599,7 +599,7 @@ extern "C" __global__ void swiglu_by_division(const float* g, const float* u, co
 """
 
 
-@pytest.mark.parametrize("backward", [False])
+@pytest.mark.parametrize("backward", [False, True])
 def test_swiglu_has_the_bits_of_a_division(backward):
     """Every bf16 gate with every up value (forward) or every upstream gradient (backward): the kernels, which do not divide,
     against one that does, with the same exponential.  A sigmoid one unit in the last place of fp32 off shows in about one of
