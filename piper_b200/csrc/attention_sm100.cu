@@ -581,7 +581,7 @@ __device__ __forceinline__ void attn_dkv_cta(const CUtensorMap* tmap_qkv_x, cons
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
-  grid_wait();
+  grid_wait(lse, delta);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -927,7 +927,7 @@ __device__ __forceinline__ void attn_dq_cta(const CUtensorMap* tmap_qkv_x, const
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
-  grid_wait();
+  grid_wait(lse, delta);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -65,17 +65,20 @@ __device__ __forceinline__ bool elect_one() {
 // tokens, 32 / 8 heads x 64, 189 and 182 us (three launches), the 30B-A3B attention layer on 2 x 2048 794 and 785, the 3B MLP on
 // 1000 433 and 426, two layers of the 1B model 4526 and 4474; where power is short it gives nothing.  Kernels that wait for peers are not launched this way, and a
 // plain launch behind one of these waits for all of it, as ever.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// Both, and the pointers that the kernel reads through: the compiler takes what a const __restrict__ parameter points to for
-// constant over the kernel and may load it early, but not through a pointer that comes out of the wait.
+// The wait takes the const __restrict__ parameters that the kernel reads through: the compiler takes what they point to for constant
+// over the kernel and may load it early, but not through a pointer that comes out of the wait.
 template <class... P>
-__device__ __forceinline__ void grid_begin(P&... pointers) {
-  grid_launch();
+__device__ __forceinline__ void grid_wait(P&... pointers) {
   uint64_t zero;
   asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
   ((pointers += zero), ...);
+}
+__device__ __forceinline__ void grid_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P>
+__device__ __forceinline__ void grid_begin(P&... pointers) {
+  grid_launch();
+  grid_wait(pointers...);
 }
 
 template <class... P, class... A>

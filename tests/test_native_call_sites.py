@@ -3,6 +3,7 @@ in the package, the tests and the benchmark names an op the library registers an
 that op's schema accepts.  The ops themselves only run on a GPU, so a binding that drifted from its call sites
 would otherwise first show on a GPU box."""
 import ast
+import re
 from pathlib import Path
 
 import pytest
@@ -50,6 +51,22 @@ def test_native_op_call_sites_match_the_registered_schemas():
                                 f"its schema takes {required}..{len(args)}")
     assert not problems, "\n".join(problems)
     assert checked > 100
+
+
+def test_read_only_pointers_come_out_of_the_wait():
+    """A kernel that may start before the one in front of it has ended reads nothing early: what the compiler may take for
+    constant over the kernel (const __restrict__) goes through the wait."""
+    waits, problems = 0, []
+    for path in sorted((ROOT / "piper_b200" / "csrc").glob("*.cu")):
+        text = path.read_text()
+        for m in re.finditer(r"\bgrid_(?:wait|begin)\(([^)]*)\);", text):
+            function = text[text.rfind("\n}\n", 0, m.start()):m.start()]
+            params = re.findall(r"const [\w ]+\* __restrict__ (\w+)", function)
+            missing = set(params) - {a.strip() for a in m.group(1).split(",")}
+            waits += 1
+            if missing:
+                problems.append(f"{path.name}:{text[:m.start()].count(chr(10)) + 1}: {sorted(missing)}")
+    assert waits > 20 and not problems, problems
 
 
 @pytest.mark.parametrize("M,N,K,f32,sms,rows", [
