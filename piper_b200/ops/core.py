@@ -904,7 +904,8 @@ cross_entropy_mean.register_autograd(_ce_mean_backward, setup_context=_ce_mean_s
 
 def cross_entropy(logits: Tensor, labels: Tensor, ignore_index: int = -100, reduction: str = "mean") -> Tensor:
     """Cross-entropy over [.., V] logits without materialising fp32 probabilities."""
-    lg = logits if logits.dim() == 2 else logits.reshape(-1, logits.shape[-1])
+    # rows without a class take the view, which refuses them
+    lg = logits if logits.dim() == 2 and logits.shape[1] > 0 else logits.reshape(-1, logits.shape[-1])
     lb = labels if labels.dim() == 1 else labels.reshape(-1)
     loss, _ = cross_entropy_fwd(lg, lb, ignore_index)
     if reduction == "none":

@@ -403,6 +403,16 @@ def test_native_bodies_refuse_empty_rows():
 
 
 @pytest.mark.gpu
+def test_linear_and_cross_entropy_refuse_empty_rows_of_a_wider_matrix():
+    """Columns [0, 0) of a matrix are contiguous and keep its row stride: what the kernels check lets them by."""
+    x, w = (torch.zeros(4, 8, device="cuda", dtype=torch.bfloat16)[:, :0] for _ in range(2))
+    for call in (lambda: core.linear(x, w), lambda: core.linear(x.clone(), w.clone()), lambda: core.linear(x[None], w),
+                 lambda: core.cross_entropy(x, torch.zeros(4, device="cuda", dtype=torch.long))):
+        with pytest.raises(RuntimeError):
+            call()
+
+
+@pytest.mark.gpu
 def test_per_token_cross_entropy_gradient_keeps_its_graph():
     """With a gradient per token the formula is tensor arithmetic: under create_graph its result can be differentiated by the
     upstream gradient, by the C++ formula as by the Python one."""

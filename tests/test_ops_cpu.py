@@ -1,6 +1,7 @@
 """CPU checks of the custom ops' reference bodies and autograd formulas against plain PyTorch."""
 import math
 
+import pytest
 import torch
 
 from piper_b200 import ops
@@ -87,6 +88,12 @@ def test_qk_rope_is_orthogonal_and_backward_matches_autograd():
         q2 = qkv.detach().clone().requires_grad_(True)
         (gref,) = torch.autograd.grad(_qk_rope_ref(q2, cos, sin, None, None, S, Hq, Hkv, hd, inter, 1e-6), q2, g)
         assert torch.allclose(gin, gref, atol=1e-5)
+
+
+def test_cross_entropy_refuses_rows_without_a_class():
+    for rows in (0, 3):
+        with pytest.raises(RuntimeError):
+            ops.cross_entropy(torch.zeros(rows, 0), torch.full((rows,), -100))
 
 
 def test_swiglu_embedding_cross_entropy():
