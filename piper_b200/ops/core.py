@@ -52,13 +52,15 @@ class GradSinks:
     def _native(self):
         return native.lib() if native.loaded() and globals().get("grad_sinks") is self else None
 
-    def register(self, param: Tensor, sink: Tensor) -> None:
+    def register(self, param: Tensor, sink: Tensor) -> Tensor:
+        """Returns the entry, by which forget() knows it."""
         assert sink.dtype == torch.float32 and sink.numel() == param.numel()
         address, sink = param.data_ptr(), sink.view(param.shape)
         with native.lock:
             self._sinks[address] = sink
             if (lib := self._native()) is not None:
                 lib.sink_set.default(address, sink)
+        return sink
 
     def unregister(self, param: Tensor) -> None:
         address = param.data_ptr()
@@ -66,11 +68,10 @@ class GradSinks:
             if self._sinks.pop(address, None) is not None and (lib := self._native()) is not None:
                 lib.sink_unset.default(address)
 
-    def forget(self, address: int, sink_address: int) -> None:
-        """Drop the entry of a parameter that is gone, unless its address has another buffer by now."""
+    def forget(self, address: int, entry: Tensor) -> None:
+        """Drop an entry of a parameter that is gone, unless its address has another one by now (maybe of the same memory)."""
         with native.lock:
-            sink = self._sinks.get(address)
-            if sink is not None and sink.data_ptr() == sink_address:
+            if self._sinks.get(address) is entry:
                 del self._sinks[address]
                 if (lib := self._native()) is not None:
                     lib.sink_unset.default(address)

@@ -87,8 +87,9 @@ class AdamConfig:
 
 
 def _forget_sinks(sinks: dict) -> None:
-    for address, sink_address in sinks.items():
-        ops_core.grad_sinks.forget(address, sink_address)
+    for address, entry in sinks.items():
+        ops_core.grad_sinks.forget(address, entry)
+    sinks.clear()
 
 
 class ParamStorage:
@@ -129,9 +130,9 @@ class ParamStorage:
         self.row_table: Optional[list] = None
         self.persistent_grads = False      # the full gradient buffer is never freed (it lives in symmetric memory)
         self.fused_stepped = False
-        # what this bucket has registered as gradient sinks: the allocator may hand a dead bucket's addresses to another
-        # tensor, which must not find the old buffer there
-        self._sinks: dict[int, int] = {}
+        # what this bucket has registered as gradient sinks and not taken back: the allocator may hand a dead bucket's
+        # addresses to another tensor, which must not find the old buffer there
+        self._sinks: dict[int, torch.Tensor] = {}
         weakref.finalize(self, _forget_sinks, self._sinks).atexit = False
         if self.numel == 0:
             return
@@ -240,13 +241,12 @@ class ParamStorage:
         for s in self.slots:
             p = self.param_views.get(s.pos)
             if p is not None:
-                sink = self.flat_grads[s.offset:s.offset + s.numel]
-                ops_core.grad_sinks.register(p, sink)
-                self._sinks[p.data_ptr()] = sink.data_ptr()
+                self._sinks[p.data_ptr()] = ops_core.grad_sinks.register(p, self.flat_grads[s.offset:s.offset + s.numel])
 
     def _unregister_sinks(self) -> None:
         for p in self.param_views.values():
             ops_core.grad_sinks.unregister(p)
+        _forget_sinks(self._sinks)
 
     # -------------------------------------------------- zero-3 life cycle
     def params_ready(self) -> bool:
@@ -321,8 +321,7 @@ class ParamStorage:
     def free_grads(self, consumer_stream=None) -> None:
         if self.numel == 0 or not self.params_sharded or self.flat_grads is None or self.persistent_grads:
             return
-        for p in self.param_views.values():
-            ops_core.grad_sinks.unregister(p)
+        self._unregister_sinks()
         if consumer_stream is not None and self.flat_grads.is_cuda:
             self.flat_grads.record_stream(consumer_stream)
         self.flat_grads = None

@@ -424,6 +424,36 @@ def test_gradient_sinks_go_with_their_bucket():
     assert core.grad_sinks._sinks.keys() == before.keys()
 
 
+@pytest.mark.parametrize("freed", ["grads", "params"])
+def test_a_late_bucket_does_not_take_the_sinks_of_the_memory_s_next_owner(freed):
+    """A bucket frees its buffers, another one gets the same blocks and registers them, and only then is the first collected."""
+    import gc
+
+    from piper_b200.ops import core
+    from piper_b200.runtime.storage import AdamConfig, ParamSlot, ParamStorage
+
+    before = dict(core.grad_sinks._sinks)
+    st = ParamStorage("bucket", [ParamSlot(0, "w", (8, 16), torch.float32, True)], torch.device("cpu"), torch.float32, "zero3",
+                      0, 1, None, AdamConfig())
+    st.all_gather_params()
+    st.alloc_grads()
+    param, grads = st.param_views[0].detach(), st.flat_grads          # the same addresses, held here
+    assert core.grad_sinks.get(param).data_ptr() == grads.data_ptr()
+    if freed == "grads":
+        st.free_grads()
+    else:
+        st._unregister_sinks()                                        # what freeing the parameters does, without their memory
+    assert core.grad_sinks.get(param) is None
+    core.grad_sinks.register(param, grads[:128])
+    del st
+    gc.collect()
+    try:
+        assert core.grad_sinks.get(param) is not None
+    finally:
+        core.grad_sinks.unregister(param)
+    assert core.grad_sinks._sinks.keys() == before.keys()
+
+
 def test_optimizer_mapping_rejects_what_the_kernels_cannot_do():
     import functools
 
