@@ -1150,6 +1150,9 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
 // two on 148 SMs, head dimension 64 / 128: 16 key blocks, 384 tiles 31.4 against 29.7 / 37.3 against 35.0 us, 512 tiles 40.3 against
 // 32.7 / 49.0 against 39.3; 4 blocks, 256 tiles 11.8 against 10.7 / 14.1 against 12.7; 8 blocks, 256 tiles, the first size that has
 // two, 14.9 against 17.0 / 17.5 against 20.0; with one block two tiles are never slower.
+// The number also decides the order in which a row's sums are added (by halves or in one chain, with probabilities rounded
+// against other maxima), so that outputs depend in their rounding on batch, heads and SMs: the same sequence alone and in a batch
+// that takes two tiles differs by what two roundings to bf16 of every probability and of the output allow.
 int attn_tiles_per_cta(int B, int S, int Hq, int num_sms) {
   const long long blocks = S / 128, tiles = static_cast<long long>(B) * Hq * blocks;
   return tiles <= num_sms || tiles * (blocks + 1) / 2 <= (blocks - 1) * num_sms ? 1 : 2;

@@ -603,8 +603,9 @@ long long gemm_split_floats(int M, int N, int splits) {
 // parts: the choice is 1 % behind the fastest on average, 15 % at most, and never behind one part.  us in one part and split:
 // 128 x 2048 x 128256 410 and 93 (floor 85), 500 x 2048 x 128256 563 and 211, 100 x 4096 x 28672 138 and 57, 512 x 2048 x 16384 75 and
 // 45, 128 x 1024 x 8192 30 and 15, 1500 x 256 x 32000 133 and 41; not split 1000 x 4096 x 28672 164 and 179, 512 x 4096 x 6144 25 and 31.
-// Products with both operands K-major are never split, although 100 x 4096 x 14336 would take 37 us instead of 64: they are the
-// forward pass, and what a model computes should not depend on how many SMs a device has.
+// Products with both operands K-major, the forward pass, are never split, although 100 x 4096 x 14336 would take 37 us instead of
+// 64: a token's row has the same bits in a batch of any size.  (That is kept for products; the attention between them adds a
+// row's sums in an order that depends on the batch, see attn_tiles_per_cta.)
 GemmShape gemm_split_shape(int M, int N, int K, bool b_mn, bool f32_out, int num_sms) {
   const GemmShape whole = gemm_shape(M, N, K, b_mn, f32_out, num_sms);
   const int k_blocks = (K + BK - 1) / BK;

@@ -719,6 +719,45 @@ def test_attention_halves_of_key_blocks(B, S, Hq, Hkv, hd):
     assert ((lse.double() - want).abs() <= 1e-5 * want.abs().clamp(min=1)).all()
 
 
+@pytest.mark.parametrize("S,Hq,Hkv,hd,B", [(2048, 16, 4, 128, 2), (2048, 16, 16, 64, 3), (1024, 28, 4, 128, 2), (512, 44, 11, 64, 2)])
+def test_attention_of_a_sequence_alone_and_in_a_batch(S, Hq, Hkv, hd, B):
+    """Alone its tiles have a CTA each, in the batch they share one, and a row's sums are added in another order: the outputs
+    differ by roundings to bf16 only.  In batches of one kind they have the same bits."""
+    from piper_b200.ops import core, native
+
+    tiles = lambda n: native.lib().attn_tiles_per_cta(n, S, Hq, 148)
+    assert (tiles(1), tiles(B), tiles(B + 1)) == (1, 2, 2)
+    torch.manual_seed(41)
+    x = torch.randn(B + 1, S, (Hq + 2 * Hkv) * hd, device="cuda").to(torch.bfloat16)
+    run = lambda t: core.attention_fwd(t.reshape(-1, t.shape[-1]), t.shape[0], S, Hq, Hkv, hd, hd ** -0.5)
+    alone, lse = run(x[:1])
+    both, lse2 = run(x[:B])
+    more, lse3 = run(x)
+    assert torch.equal(both, more[:B * S]) and torch.equal(lse2, lse3[:B])
+    q, k, v = (t.double().transpose(0, 1) for t in x[0].view(S, Hq + 2 * Hkv, hd).split([Hq, Hkv, Hkv], 1))
+    k, v = (t.repeat_interleave(Hq // Hkv, 0) for t in (k, v))
+    scores = (q @ k.transpose(1, 2) * hd ** -0.5).masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    # every probability is rounded to bf16 once on either side (2^-9 of it each), and so is the output
+    spread = (torch.softmax(scores, -1) @ v.abs()).transpose(0, 1).reshape(S, Hq * hd)
+    a, b = alone.double(), both[:S].double()
+    assert not torch.equal(alone, both[:S])
+    assert ((a - b).abs() <= 2 ** -8 * spread + 2 ** -9 * (a.abs() + b.abs()) + 1e-5).all()
+    assert ((lse[0].double() - lse2[0].double()).abs() <= 1e-5 * lse[0].double().abs().clamp(min=1)).all()
+
+
+@pytest.mark.parametrize("N,K", [(4096, 14336), (512, 256), (2048, 2048)])
+def test_forward_products_of_a_row_do_not_depend_on_the_others(N, K):
+    """Tiles and their shapes follow the number of rows; the sum of a row is the same products in the same order."""
+    from piper_b200 import ops
+
+    torch.manual_seed(42)
+    x = torch.randn(2500, K, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    y = ops.linear(x, w)
+    for rows in (1, 100, 129, 700, 2048):
+        assert torch.equal(ops.linear(x[:rows], w), y[:rows]), rows
+
+
 @pytest.mark.parametrize("T,ignored", [(0, 0.0), (1, 0.0), (33, 0.3), (1023, 1.0), (1024, 0.0), (5000, 0.3), (65536, 0.1), (65537, 0.1)])
 def test_cross_entropy_mean(T, ignored):
     """One CTA's sum over any number of rows, and the sum by tensor ops above its limit: value, gradient, and the gradient of
