@@ -59,12 +59,16 @@ __device__ __forceinline__ bool elect_one() {
 // ------------------------------------------------------ launches that overlap
 // A kernel launched by launch_overlapped() may start while the one before it in the stream still runs, and has to wait for it
 // (and so for everything before that) in front of its first access to global memory: grid_wait().  grid_launch() lets the
-// kernel behind start once every CTA of this grid has called it or left; called late in a long kernel, so that the next one's
-// CTAs do not sit on SMs that other streams could use, and first thing in a short one (grid_begin()).  What overlaps is the
-// launch itself, the set-up of the CTAs and the tail.  A pass, forward and backward, without and so: attention on 3 x 1408
+// kernel behind start once every CTA of this grid has called it or left.  Products and attention call it with their last
+// loads, so that the next one's CTAs do not sit on SMs that other streams could use; all other kernels call it first thing
+// (grid_begin()), however long they take, so that behind one of hundreds of microseconds (cross-entropy of a large vocabulary) a
+// waiting product has its SMs' shared memory for as long.  First thing and not at all, in us: passes with a second stream, the 8B
+// MLP 3676 and 3713, the 3B MLP on 1000 tokens 432 and 437; the head of 128256 x 2048 5452 and 5439, two layers of the 1B model
+// 4512 and 4460, an attention layer on 4 x 128 tokens 173 and 175: within what two runs of one side differ by.  What overlaps is
+// the launch itself, the set-up of the CTAs and the tail.  A pass, forward and backward, without and so: attention on 3 x 1408
 // tokens, 32 / 8 heads x 64, 189 and 182 us (three launches), the 30B-A3B attention layer on 2 x 2048 794 and 785, the 3B MLP on
-// 1000 433 and 426, two layers of the 1B model 4526 and 4474; where power is short it gives nothing.  Kernels that wait for peers are not launched this way, and a
-// plain launch behind one of these waits for all of it, as ever.
+// 1000 433 and 426, two layers of the 1B model 4526 and 4474; where power is short it gives nothing.  Kernels that wait for peers
+// are not launched this way, and a plain launch behind one of these waits for all of it, as ever.
 // The wait takes the const __restrict__ parameters that the kernel reads through: the compiler takes what they point to for constant
 // over the kernel and may load it early, but not through a pointer that comes out of the wait.
 template <class... P>

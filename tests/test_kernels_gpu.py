@@ -690,6 +690,92 @@ def test_overlapped_launches_keep_their_order(T, D, F):
     native.check_status()
 
 
+def test_overlapped_launches_behind_another_stream():
+    """A kernel launched to overlap the one before it in its stream also waits for what the stream waits for: products and passes
+    handed from one stream to another and back through buffers that hold the step before, with the device idle between any two,
+    without, and in a captured graph."""
+    from piper_b200.ops import native
+
+    lib, status = native.lib(), native.status_tensor()
+    torch.manual_seed(44)
+    T, D, F, steps = 2048, 2048, 4096, 8
+    rn = lambda *shape: torch.randn(*shape, device="cuda").to(torch.bfloat16)
+    x, w13, w2 = rn(steps, T, D), rn(2 * F, D) * D ** -0.5, rn(D, F) * F ** -0.5
+    h, act, y, g, z = rn(T, 2 * F), rn(T, F), rn(T, D), rn(T, D), rn(T, D)
+    side = torch.cuda.Stream()
+
+    def run(idle):
+        step = torch.cuda.synchronize if idle else lambda: None
+        cur, out = torch.cuda.current_stream(), torch.zeros_like(x)
+        for i in range(steps):
+            step(); lib.gemm(x[i], w13, h, False, False, False, status)
+            step(); lib.swiglu_fwd(h, act)
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                step(); lib.gemm(act, w2, y, False, False, False, status)
+                step(); lib.add_bf16(y, x[i], g)
+            step(); lib.add_bf16(x[i], x[i - 1], z)
+            cur.wait_stream(side)
+            step(); lib.add_bf16(g, z, out[i])
+        return out
+
+    want = run(True)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        assert torch.equal(run(False), want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run(False)
+    for _ in range(3):
+        captured.zero_()
+        graph.replay()
+        assert torch.equal(captured, want)
+    native.check_status()
+
+
+@pytest.mark.parametrize("sinks", [False, True])
+def test_overlapped_launches_of_forked_gradients(sinks, monkeypatch):
+    """Layers whose weight gradients run on a second stream, joined layer by layer or, for buckets, at the end of the scope: the
+    gradients of the same layers on one stream."""
+    from piper_b200 import ops
+    from piper_b200.ops import core, native
+
+    torch.manual_seed(45)
+    T, D, F = 2048, 2048, 4096
+    rn = lambda *shape: torch.randn(*shape, device="cuda").to(torch.bfloat16)
+    x, up = rn(T, D), rn(T, D)
+    ws = [rn(2 * F, D) * D ** -0.5, rn(D, F) * F ** -0.5, rn(2 * F, D) * D ** -0.5, rn(D, F) * F ** -0.5]
+    assert all(T * w.numel() >= core._FORK_MIN_MACS for w in ws)
+    for t in (x, *ws):
+        t.requires_grad_(True)
+    buckets = [torch.zeros(w.shape, device="cuda") for w in ws]
+
+    def run():
+        for b in buckets:
+            b.zero_()
+        with core.deferred_join():
+            f = x
+            for a, b in ((ws[0], ws[1]), (ws[2], ws[3])):
+                f = ops.linear(ops.swiglu(ops.linear(f, a)), b)
+            grads = torch.autograd.grad(f, [x, *ws], up, allow_unused=sinks)
+        return [grads[0], *([b.clone() for b in buckets] if sinks else grads[1:])]
+
+    if sinks:
+        for w, b in zip(ws, buckets):
+            ops.grad_sinks.register(w, b)
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(core, "_GEMM_FORK", 0)
+            want = run()
+        for _ in range(10):
+            assert all(torch.equal(a, b) for a, b in zip(run(), want))
+    finally:
+        for w in ws:
+            ops.grad_sinks.unregister(w)
+    native.check_status()
+
+
 @pytest.mark.parametrize("B,S,Hq,Hkv,hd", [(1, 128, 2, 1, 64), (2, 256, 2, 2, 128), (1, 384, 3, 1, 64), (1, 640, 2, 2, 128),
                                            (1, 1408, 4, 1, 64), (1, 2048, 8, 2, 128), (1, 2048, 16, 4, 64)])
 def test_attention_halves_of_key_blocks(B, S, Hq, Hkv, hd):
