@@ -123,14 +123,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   }
   // Tiles come from a counter, so that none waits for a CTA that finds no SM until others are done: beside a kernel that
   // holds 16 SMs, with the CTA's own number as the first tile and so, 4096 x 8192 x 1024 65.3 and 58.9 us, 4096 x 14336 x 4096 297 and
-  // 289 us; alone 54.6 and 54.4, 254 and 253 us.  The first draw runs beside the allocation.  In a launch of one round a CTA
+  // 289 us; alone 54.6 and 54.4, 254 and 253 us.  The first draw runs beside the allocation, but behind the wait, as every access
+  // to global memory does (in front of it no pass is faster by more than its runs differ).  In a launch of one round a CTA
   // that comes late has as much to do as one that draws twice; there every CTA takes its number (512 x 256 x 688 6.5 us, with
   // the counter 6.9).
   const int units = static_cast<int>(gridDim.x) / CTAS;
   const bool draws = p.sched != nullptr && num_tiles > units;
+  grid_wait();
   if (warp == 3 && rank == 0 && lane == 0)
     bars->first = draws ? atomicAdd(&p.sched[0], 1) : static_cast<int>(blockIdx.x) / CTAS;
-  grid_wait();
   tc_fence_before();
   if (CTAS == 2) cluster_sync(); else __syncthreads();
   tc_fence_after();
@@ -408,8 +409,9 @@ EncodeFn get_encode_fn() {
 
 }  // namespace
 
-// Pool of tile-scheduler slots (next tile, finished CTAs), one slot per dense or grouped launch in rotation.  It is the only
-// device memory this library allocates by itself: 32 KiB, once per process.
+// Pool of tile-scheduler slots (next tile, finished CTAs), one slot per dense or grouped launch in rotation; the launch 4,096
+// before, whose last CTA rearms the slot, has to have ended on its stream by then.  It is the only device memory this library
+// allocates by itself: 32 KiB, once per process.
 constexpr int kSchedSlots = 4096;
 
 int* gemm_sched_slot() {

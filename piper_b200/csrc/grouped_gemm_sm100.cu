@@ -177,11 +177,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   }
   if (warp == 2) {
     // tiles come from a counter, as in the dense kernel; the first one is drawn beside the table
-    int first = static_cast<int>(blockIdx.x) / CTAS;
-    if (rank == 0 && lane == 0 && p.sched != nullptr) first = atomicAdd(&p.sched[0], 1);
-    __syncwarp();
     tmem_alloc_n<CTAS>(&bars->tmem_base, 512);
     tmem_relinquish_n<CTAS>();
+    grid_wait();
+    int first = static_cast<int>(blockIdx.x) / CTAS;
+    if (rank == 0 && lane == 0 && p.sched != nullptr) first = atomicAdd(&p.sched[0], 1);
     if (lane == 0) bars->first = first;
   }
   grid_wait();

@@ -69,6 +69,13 @@ def test_read_only_pointers_come_out_of_the_wait():
     assert waits > 20 and not problems, problems
 
 
+def test_products_draw_their_first_tile_behind_the_wait():
+    for name in ("gemm_sm100.cu", "grouped_gemm_sm100.cu"):
+        text = (ROOT / "piper_b200" / "csrc" / name).read_text()
+        lines = text[:text.index("atomicAdd(&p.sched[0], 1)")].splitlines()[-3:]
+        assert any(line.strip() == "grid_wait();" for line in lines), name
+
+
 @pytest.mark.parametrize("M,N,K,f32,sms,rows", [
     (2048, 4096, 4096, False, 148, 256),      # 128 big tiles in one round, 256 small ones in two
     (2048, 4096, 2048, False, 148, 128),      # the same with too short a contraction
