@@ -54,6 +54,11 @@ int64_t rows_of(const Tensor& t, int64_t inner, const char* what) {
   return t.numel() / inner;
 }
 
+// Kernels read device memory and pinned host memory; a pointer to any other faults.
+void check_readable(const Tensor& t, const char* what) {
+  TORCH_CHECK(t.is_cuda() || t.numel() == 0 || t.is_pinned(), what, " must be in device or pinned memory");
+}
+
 const void* opt_ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 float* opt_f32(const OptTensor& t) {
   if (!t.has_value()) return nullptr;
@@ -297,6 +302,7 @@ void ce_fwd(const Tensor& logits, const Tensor& labels, Tensor loss, Tensor lse,
   check_bf16(logits, "logits");
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1, "logits must be [T, V] with unit inner stride");
   TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous(), "labels must be contiguous int64");
+  check_readable(labels, "labels");
   check_rc(piper::ce_fwd(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()),
                          loss.data_ptr<float>(), lse.data_ptr<float>(), logits.size(0),
                          static_cast<int>(logits.size(1)), logits.stride(0), ignore_index, cur_stream()),
@@ -307,6 +313,7 @@ void ce_mean(const Tensor& loss, const Tensor& labels, Tensor mean, Tensor count
   TORCH_CHECK(loss.is_cuda() && loss.scalar_type() == at::kFloat && loss.is_contiguous(), "loss must be contiguous fp32");
   TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == loss.numel(),
               "labels must be contiguous int64, one per loss");
+  check_readable(labels, "labels");
   check_rc(piper::ce_mean(loss.data_ptr<float>(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()),
                           mean.data_ptr<float>(), count.data_ptr<float>(), loss.numel(), ignore_index, cur_stream()),
            "ce_mean");

@@ -413,6 +413,18 @@ def test_linear_and_cross_entropy_refuse_empty_rows_of_a_wider_matrix():
 
 
 @pytest.mark.gpu
+def test_cross_entropy_refuses_labels_that_the_device_cannot_read():
+    """Labels in host memory raise before a kernel gets their address, in the loss and in its mean; pinned ones are read."""
+    logits = torch.randn(4, 16, device="cuda").to(torch.bfloat16)
+    labels = torch.tensor([1, -100, 15, 3])
+    loss, _ = core.cross_entropy_fwd(logits, labels.cuda(), -100)
+    for call in (lambda: core.cross_entropy(logits, labels), lambda: core.cross_entropy_mean(loss, labels, -100)):
+        with pytest.raises(RuntimeError):
+            call()
+    assert torch.equal(core.cross_entropy(logits, labels.pin_memory()), core.cross_entropy(logits, labels.cuda()))
+
+
+@pytest.mark.gpu
 def test_per_token_cross_entropy_gradient_keeps_its_graph():
     """With a gradient per token the formula is tensor arithmetic: under create_graph its result can be differentiated by the
     upstream gradient, by the C++ formula as by the Python one."""
