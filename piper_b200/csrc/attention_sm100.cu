@@ -1147,9 +1147,12 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
 // Two query tiles per CTA read every K and V block once for both; one tile in two halves is done in little more than half the
 // time of a tile in one chain.  As long as every tile has an SM of its own, or the SMs get through all key blocks of all
 // tiles (longest first) before a longest tile and a block have passed, one tile per CTA finishes earlier.  One against
-// two on 148 SMs, head dimension 64 / 128: 16 key blocks, 384 tiles 31.4 against 29.7 / 37.3 against 35.0 us, 512 tiles 40.3 against
-// 32.7 / 49.0 against 39.3; 4 blocks, 256 tiles 11.8 against 10.7 / 14.1 against 12.7; 8 blocks, 256 tiles, the first size that has
-// two, 14.9 against 17.0 / 17.5 against 20.0; with one block two tiles are never slower.
+// two on 148 SMs, head dimension 64 / 128, in us: 2 key blocks, 148 tiles 5.4 against 7.1 / 6.6 against 8.4, 180 tiles 9.2 against 7.3 /
+// 10.8 against 8.8; 4 blocks, 256 tiles 11.8 against 11.0 / 13.9 against 13.0; 16 blocks, 256 tiles 20.9 against 31.7 / 24.0 against 34.1,
+// 448 tiles 35.7 against 32.3 / 41.4 against 34.7; with one block two tiles are never slower.
+// That line is right for a tile in one chain; the halves move it, to some 270 tiles at 8 blocks, 350 at 16 and 450 at 32, and in
+// between it takes two where one is faster: 8 blocks, 256 tiles 14.7 against 17.7 / 17.3 against 19.7; 16 blocks, 304 tiles 26.0 against
+// 31.9 / 30.3 against 34.5; 32 blocks, 288 tiles, the worst, 35.4 against 59.8 / 40.5 against 62.7.
 // The number also decides the order in which a row's sums are added (by halves or in one chain, with probabilities rounded
 // against other maxima), so that outputs depend in their rounding on batch, heads and SMs: the same sequence alone and in a batch
 // that takes two tiles differs by what two roundings to bf16 of every probability and of the output allow.
@@ -1243,11 +1246,11 @@ static int attn_bwd_impl(const void* qkv, const void* out, const void* d_out, co
   int* arrived = reinterpret_cast<int*>(scratch);
   float* partial = scratch == nullptr ? nullptr : scratch + (n_kv + 3) / 4 * 4;
   const long long delta_blocks = (T * Hq * (HD / 8) + 255) / 256;
-  launch_overlapped(attn_delta_kernel<HD>, static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st, 
+  launch_overlapped(attn_delta_kernel<HD>, static_cast<unsigned>(delta_blocks < 148 * 16 ? delta_blocks : 148 * 16), 256, 0, st,
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, arrived,
       parts > 1 ? n_kv : 0, T, S, Hq);
   if (cudaGetLastError() != cudaSuccess) return -3;
-  launch_overlapped(attn_bwd_kernel<HD>, static_cast<unsigned>(n_kv * parts + S / 128 * Hq * B), BWD_THREADS, smem, st, 
+  launch_overlapped(attn_bwd_kernel<HD>, static_cast<unsigned>(n_kv * parts + S / 128 * Hq * B), BWD_THREADS, smem, st,
       tqx, tqy, tdx, tdy, tdq, lse, delta, B, S, Hq, Hkv, parts, partial, arrived, softmax_scale,
       softmax_scale * 1.4426950408889634f, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

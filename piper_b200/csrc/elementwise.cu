@@ -619,6 +619,8 @@ __device__ __forceinline__ void rope_tasks(const RopeArgs& a, const RopeGroup<HD
 // sums of a warp are added over its lane groups, those of a CTA over its warps, and reduce_partials_kernel adds the CTAs', all in
 // a fixed order.  (Sixteen shared-memory atomics per lane and head took 147 us for 4096 tokens of 32 + 2 x 4 heads x 128.  One
 // atomic per element and CTA into cleared fp32 sums, which are then rounded, takes four launches more for two weights.)
+// The backward pass with norms has 128 registers, two CTAs of which fill an SM, and is the one form that spills (40 bytes of stores,
+// 96 of loads): 16 sums, two vectors each of gradient and input, the next ones and the weights.  It is at 3.9 TB/s, the others at 5.2.
 template <bool NORM, bool BWD>
 constexpr int ROPE_CTAS = !NORM ? 4 : BWD ? 2 : 3;     // per SM
 
@@ -1059,7 +1061,7 @@ int rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_
     launch_overlapped(rmsnorm_fwd_reg_kernel<VPT, THREADS>, static_cast<unsigned>(T < ctas ? T : ctas), THREADS, 0, st, xp, rp, wp, yp, hp, rstd, T, eps);
   });
   if (done) return PIPER_LAUNCH_OK();
-  launch_overlapped(rmsnorm_fwd_kernel, static_cast<unsigned>(T), NORM_THREADS, 0, st, 
+  launch_overlapped(rmsnorm_fwd_kernel, static_cast<unsigned>(T), NORM_THREADS, 0, st,
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res),
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
       static_cast<__nv_bfloat16*>(h_out), rstd, D, eps);
@@ -1087,7 +1089,7 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
     // several rows at a time where a CTA has several to do
     const long long each = (T + nb - 1) / nb;
     const int rows = static_cast<int>(each < NORM_BWD_ROWS<VPT, THREADS> ? each : NORM_BWD_ROWS<VPT, THREADS>);
-    launch_overlapped(rmsnorm_bwd_reg_kernel<VPT, THREADS>, nb, rows * THREADS, rows > 1 ? rows * D * sizeof(float) : 0, st, 
+    launch_overlapped(rmsnorm_bwd_reg_kernel<VPT, THREADS>, nb, rows * THREADS, rows > 1 ? rows * D * sizeof(float) : 0, st,
         static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), rstd,
         static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), dw_partial, static_cast<int>(T));
   });
@@ -1100,7 +1102,7 @@ int rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd,
     cudaFuncSetAttribute(rmsnorm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     configured = true;
   }
-  launch_overlapped(rmsnorm_bwd_kernel, nb, NORM_THREADS, D * sizeof(float), st, 
+  launch_overlapped(rmsnorm_bwd_kernel, nb, NORM_THREADS, D * sizeof(float), st,
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
       static_cast<const __nv_bfloat16*>(w), rstd, static_cast<const __nv_bfloat16*>(dres),
       static_cast<__nv_bfloat16*>(dx), dw_partial, static_cast<int>(T), D);
@@ -1205,7 +1207,7 @@ int embedding_fwd(const long long* tokens, const void* table, void* out, long lo
                   int* status, cudaStream_t st) {
   if (D % 8 != 0) return -1;
   if (T == 0) return 0;
-  launch_overlapped(embedding_fwd_kernel, static_cast<unsigned>(T), 128, 0, st, 
+  launch_overlapped(embedding_fwd_kernel, static_cast<unsigned>(T), 128, 0, st,
       tokens, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), T, D, V, status);
   return PIPER_LAUNCH_OK();
 }
@@ -1240,7 +1242,7 @@ int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse,
            long long ld, long long ignore_index, cudaStream_t st) {
   if (ld % 8 != 0) return -1;
   if (T == 0) return 0;
-  launch_overlapped(ce_fwd_kernel, static_cast<unsigned>(T), CE_THREADS, 0, st, 
+  launch_overlapped(ce_fwd_kernel, static_cast<unsigned>(T), CE_THREADS, 0, st,
       static_cast<const __nv_bfloat16*>(logits), labels, loss, lse, V, ld, ignore_index);
   return PIPER_LAUNCH_OK();
 }
@@ -1257,7 +1259,7 @@ int ce_bwd(const void* logits, const long long* labels, const float* lse, const 
            cudaStream_t st) {
   if (ld % 8 != 0) return -1;
   if (T == 0) return 0;
-  launch_overlapped(ce_bwd_kernel, static_cast<unsigned>(T), CE_THREADS, 0, st, 
+  launch_overlapped(ce_bwd_kernel, static_cast<unsigned>(T), CE_THREADS, 0, st,
       static_cast<const __nv_bfloat16*>(logits), labels, lse, gscale, row_scale,
       static_cast<__nv_bfloat16*>(out), V, ld, ignore_index);
   return PIPER_LAUNCH_OK();

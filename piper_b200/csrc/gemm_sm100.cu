@@ -688,7 +688,7 @@ static int gemm_launch_shape(const GemmArgs& g, GemmShape shape, int num_sms, cu
                        : launch_layout<1>(l, ta, tb, tc, p, num_sms, stream);
   if (rc != 0 || shape.splits == 1) return rc;
   const long long threads = static_cast<long long>(g.M) * (ld / 8);
-  launch_overlapped(split_sum_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, 
+  launch_overlapped(split_sum_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream,
       g.scratch, static_cast<__nv_bfloat16*>(g.c), g.M, g.N, rows, ld, g.ldc, shape.splits);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -406,7 +406,7 @@ int moe_permute(const void* x, const int* idx, const int* g_start, const int* g_
                 cudaStream_t st) {
   if (D % 8 != 0) return -1;
   const unsigned token_ctas = warps_grid(T, ROW_THREADS);
-  launch_overlapped(permute_kernel, token_ctas + E * PAD_CTAS, ROW_THREADS, 0, st, 
+  launch_overlapped(permute_kernel, token_ctas + E * PAD_CTAS, ROW_THREADS, 0, st,
       static_cast<const __nv_bfloat16*>(x), idx, g_start, g_len, counts, cursor, pos, static_cast<__nv_bfloat16*>(rows),
       T, D, k, E, rows_cap, token_ctas, status);
   return PIPER_LAUNCH_OK();
@@ -443,7 +443,7 @@ int moe_combine_bwd(const void* rows, const void* dout, const int* pos, const fl
   if (token_ctas + num_groups == 0) return 0;
   auto kern = k == 1 ? combine_bwd_kernel<1> : k == 2 ? combine_bwd_kernel<2> : k <= 4 ? combine_bwd_kernel<4>
                                                                                         : combine_bwd_kernel<8>;
-  launch_overlapped(kern, token_ctas + num_groups * PAD_CTAS, ROW_THREADS, 0, st, 
+  launch_overlapped(kern, token_ctas + num_groups * PAD_CTAS, ROW_THREADS, 0, st,
       static_cast<const __nv_bfloat16*>(rows), static_cast<const __nv_bfloat16*>(dout), pos, weights,
       static_cast<__nv_bfloat16*>(drows), dweights, g_start, g_len, counts, T, D, k, rows_cap, token_ctas, status);
   return PIPER_LAUNCH_OK();
