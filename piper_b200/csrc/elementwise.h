@@ -51,10 +51,10 @@ int embedding_bwd_bf16(const long long* tokens, const void* dout, int* scratch, 
 // Per-row loss and log-sum-exp of bf16 logits [T, V] with row stride ld.
 int ce_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long T, int V,
            long long ld, long long ignore_index, cudaStream_t st);
-// out = (softmax - onehot) * gscale[0] * row_scale; out may alias logits.
 // mean[0] = sum(loss) / count[0], count[0] = rows whose label is not ignore_index, at least 1.
 int ce_mean(const float* loss, const long long* labels, float* mean, float* count, long long T, long long ignore_index,
             cudaStream_t st);
+// out = (softmax - onehot) * gscale[0] * row_scale; out may alias logits.
 int ce_bwd(const void* logits, const long long* labels, const float* lse, const float* gscale,
            float row_scale, void* out, long long T, int V, long long ld, long long ignore_index,
            cudaStream_t st);
