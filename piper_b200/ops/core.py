@@ -867,14 +867,15 @@ def _ce_backward(ctx, dloss, _dlse):
 cross_entropy_fwd.register_autograd(_ce_backward, setup_context=_ce_setup)
 
 
-# Rows up to which one CTA takes the mean: 65,536 take it 10.7 us, and the sum alone by tensor ops 13.3; 4,096 take 2.6 us.
+# Rows up to which one CTA takes the mean: 65,536 take it 10.7 us, and the sum alone by tensor ops 13.3; 4,096 take 2.6 us.  The
+# op's body decides, and not its caller, so that a program traced with any number of rows has no guard on it.
 CE_MEAN_ROWS = 1 << 16
 
 
 @custom_op("piper::cross_entropy_mean")
 def cross_entropy_mean(loss: Tensor, labels: Tensor, ignore_index: int) -> tuple[Tensor, Tensor]:
     """Mean of per-token losses [T] over the tokens whose label counts, and their number (at least one), both fp32."""
-    if _is_native(loss):
+    if _is_native(loss) and loss.numel() <= CE_MEAN_ROWS and labels.shape == loss.shape:
         mean = torch.empty((), dtype=torch.float32, device=loss.device)
         count = torch.empty((), dtype=torch.float32, device=loss.device)
         native.lib().ce_mean(loss.contiguous(), labels.contiguous(), mean, count, ignore_index)
@@ -913,7 +914,7 @@ def cross_entropy(logits: Tensor, labels: Tensor, ignore_index: int = -100, redu
         return loss
     if reduction == "sum":
         return loss.sum()
-    if _is_native(loss) and loss.shape[0] <= CE_MEAN_ROWS and lb.shape == loss.shape:
+    if _is_native(loss):
         return cross_entropy_mean(loss, lb, ignore_index)[0]
     n = (lb != ignore_index).sum().clamp(min=1)
     return loss.sum() / n

@@ -425,6 +425,29 @@ def test_cross_entropy_refuses_labels_that_the_device_cannot_read():
 
 
 @pytest.mark.gpu
+def test_a_traced_mean_loss_has_no_guard_on_its_rows():
+    """A program exported or compiled with any number of rows runs with one token and with more than one CTA adds up."""
+    class Loss(torch.nn.Module):
+        def forward(self, logits, labels):
+            return core.cross_entropy(logits, labels)
+
+    def args(rows):
+        return torch.randn(rows, 64, device="cuda").to(torch.bfloat16), torch.randint(0, 64, (rows,), device="cuda")
+
+    rows, graphs = torch.export.Dim("rows"), []
+    exported = torch.export.export(Loss(), args(40), dynamic_shapes=({0: rows}, {0: rows})).module()
+    compiled = torch.compile(Loss(), backend=lambda gm, _: graphs.append(gm) or gm.forward, dynamic=True, fullgraph=True)
+    for n in (40, 50, core.CE_MEAN_ROWS + 1):
+        a, b = args(n)
+        want = core.cross_entropy(a, b)
+        assert torch.equal(exported(a, b), want) and torch.equal(compiled(a, b), want)
+    assert len(graphs) == 1
+    # more labels than rows, all of which count, as they do in tensor operations
+    losses, more = core.cross_entropy_fwd(a[:3], b[:3], -100)[0], b[:7]
+    assert torch.equal(core.cross_entropy(a[:3], more), losses.sum() / 7)
+
+
+@pytest.mark.gpu
 def test_per_token_cross_entropy_gradient_keeps_its_graph():
     """With a gradient per token the formula is tensor arithmetic: under create_graph its result can be differentiated by the
     upstream gradient, by the C++ formula as by the Python one."""
