@@ -212,6 +212,46 @@ def test_gemm_split_contraction(M, N, K, tile, width, splits):
     native.check_status()
 
 
+def test_gemm_split_contraction_in_a_captured_graph_and_on_two_streams():
+    """The sums' scratch belongs to the stream that runs the product: products of two streams at once, and a graph's, replayed on
+    other inputs beside products that take scratch of their own."""
+    from piper_b200.ops import native
+
+    lib, status = native.lib(), native.status_tensor()
+    torch.manual_seed(34)
+    M, N, K = 100, 512, 20000
+    assert lib.gemm_split_shape(M, N, K, True, False, 148)[2] > 1
+    rn = lambda *shape: torch.randn(*shape, device="cuda").to(torch.bfloat16)
+    xs, b = [rn(M, K) for _ in range(6)], rn(K, N)
+
+    def product(x):
+        out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        lib.gemm(x, b, out, False, True, False, status)
+        return out
+
+    want = [product(x) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(5):
+        got = [[], []]
+        for x in xs:
+            for stream, outs in zip(streams, got):
+                with torch.cuda.stream(stream):
+                    outs.append(product(x))
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for outs in got for a, b in zip(outs, want))
+    x = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        first, second = product(x), product(x)
+    for i in (3, 1, 5):
+        x.copy_(xs[i])
+        graph.replay()
+        other = product(xs[i - 1])
+        assert torch.equal(first, want[i]) and torch.equal(second, want[i]) and torch.equal(other, want[i - 1])
+    native.check_status()
+
+
 @pytest.mark.parametrize("sizes,forked", [((4095,), []), ((4096,), [4096]), ((4096, 4095), [4096, 4095]),
                                           ((4095, 4096), [4096])])
 def test_linear_gradients_around_the_fork_threshold(sizes, forked, monkeypatch):
